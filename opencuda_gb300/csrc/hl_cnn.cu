@@ -14,15 +14,18 @@
  * + ci (tap = ky * 3 + kx), K-major, so that one GEMM row of the weight
  * operand is one output channel.
  *
- * Implicit GEMM, one CTA of 128 threads per 128-pixel output tile:
- *   D[128 x N] = A[128 x K] * B[N x K]^T,
- *   A[m][k] = input pixel of output pixel m at tap k / Cin, channel k % Cin
- *   (zero outside the image), gathered into shared memory in the no-swizzle
- *   K-major core-matrix layout (8 rows x 16 bytes per core matrix), B the
- *   weights in the same layout.  Thread 0 issues K / 16 tcgen05.mma
- *   (M = 128, N = 32 or 16, K = 16) into a 32-column TMEM accumulator and
- *   commits them to an mbarrier; each warp then reads its 32 TMEM lanes
- *   (tcgen05.ld 32x32b) and runs the epilogue (bias, ReLU, bf16 store).
+ * Implicit GEMM, CTAs of 128 threads, one M = 128 tile of 8 x 16 output
+ * pixels at a time: D[128 x N] = sum over the taps of A_tap[128 x 32] *
+ * B_tap[N x 32]^T.  The input tile and its halo are copied into shared memory
+ * once (cp.async, zero outside the image) as rows of four channel planes,
+ * [row][8-channel group][pixel][8 channels]: 8 neighbouring pixels of a plane
+ * are 128 contiguous bytes, one core matrix of the no-swizzle K-major layout,
+ * whichever pixel they start at.  So every tap's A operand is the same halo
+ * at another start address (LBO one plane, SBO one output row), and nothing
+ * is gathered per tap.  One thread issues the tcgen05.mma in tap order (M = 128,
+ * N = 32 or 16, K = 16) into TMEM and commits them to an mbarrier; the next
+ * tile's copies are issued behind them; each warp reads its 32 TMEM lanes
+ * (tcgen05.ld 32x32b), runs the epilogue and stores whole 512-byte rows.
  */
 #include "hl_internal.h"
 #include "hl_cnn.h"
@@ -92,17 +95,17 @@ __device__ __forceinline__ bool cnn_mbar_wait(unsigned long long *bar,
     return false;
 }
 
-__device__ __forceinline__ void tmem_alloc32(unsigned *dst_smem)
+__device__ __forceinline__ void tmem_alloc(unsigned *dst_smem, int cols)
 {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 32;"
-                 ::"r"(cnn_smem_u32(dst_smem))
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 ::"r"(cnn_smem_u32(dst_smem)), "r"(cols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 
-__device__ __forceinline__ void tmem_dealloc32(unsigned taddr)
+__device__ __forceinline__ void tmem_dealloc(unsigned taddr, int cols)
 {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 32;" ::"r"(taddr)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols)
                  : "memory");
 }
 
@@ -115,6 +118,16 @@ __device__ __forceinline__ void umma_f16(unsigned tmem_d, unsigned long long ade
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+
+/* one lane of a converged warp: the branch stays warp-uniform, so descriptors
+ * are built in uniform registers */
+__device__ __forceinline__ bool elect_one()
+{
+    unsigned p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(p));
+    return p != 0;
 }
 
 __device__ __forceinline__ void umma_commit(unsigned long long *bar)
@@ -151,242 +164,512 @@ __device__ __forceinline__ void tmem_ld32(unsigned taddr, float (&v)[32])
 
 /* ---- the convolution ----------------------------------------------------- */
 
-/* Shared memory of one CTA: A (128 rows x K) and B (N rows x K) in core
- * matrices.  Core matrix (row group g, K group q) of an operand with KG K
- * groups sits at ((g * KG) + q) * 128 bytes, so the two K groups of MMA step
- * s start at 2 s * 128 (LBO = 128) and consecutive row groups are KG * 128
- * apart (SBO). */
-template <int KG, int NROWS>
-struct ConvSmem {
-    alignas(128) unsigned char a[CNN_TILE_M / 8][KG][128];
-    alignas(128) unsigned char b[NROWS / 8][KG][128];
-    unsigned long long bar;
-    unsigned tmem;
-    int tile;
+/* output tile: 8 x 16 pixels, GEMM row m = pixel (m / 8, m % 8) */
+#define CONV_TX 8
+#define CONV_TY 16
+
+/* Kinds of the 32-channel convolution. */
+enum { CONV_S1 = 0,     /* stride 1 */
+       CONV_S2 = 1,     /* stride 2 */
+       CONV_T2 = 2 };   /* x-gradient of a stride-2 convolution:
+                           dx[p] = sum w * dy[(p + 1 - tap) / 2] */
+
+/* The halo of a tile in shared memory: ROWS x COLS input pixels, a plane row
+ * of P bytes per (row, 8-channel group).  CONV_S2 keeps even and odd columns
+ * in two halves (HALF bytes apart), so that the 8 pixels of an output row,
+ * two columns apart, are neighbours.  A half starts 64 bytes off the banks of
+ * the other and P is 32 or 16 bytes off a multiple of 128, so the copies of
+ * 8 lanes (2 pixels x 4 planes) hit all banks. */
+template <int MODE> struct ConvHalo;
+template <> struct ConvHalo<CONV_S1> {
+    static constexpr int COLS = 10, ROWS = 18, P = 160, HALF = 0, BYTES = 18 * 4 * 160, NST = 2;
+    static constexpr int TMEM_COLS = 32, CTAS = 4;
+};
+template <> struct ConvHalo<CONV_S2> {
+    static constexpr int COLS = 17, ROWS = 33, P = 144, HALF = 33 * 4 * 144,
+                         BYTES = 2 * 33 * 4 * 144, NST = 1;
+    static constexpr int TMEM_COLS = 32, CTAS = 3;
+};
+template <> struct ConvHalo<CONV_T2> {
+    static constexpr int COLS = 9, ROWS = 17, P = 144, HALF = 0, BYTES = 17 * 4 * 144, NST = 2;
+    static constexpr int TMEM_COLS = 128, CTAS = 4;
 };
 
-/* Gather modes of the A operand. */
-enum { GATHER_CONV = 0,        /* y[p] = sum w * x[p * stride - 1 + tap] */
-       GATHER_CONVT2 = 1 };    /* x-gradient of a stride-2 conv:
-                                  dx[p] = sum w * dy[(p + 1 - tap) / 2] */
+/* B operand: core matrix (row group g, K group q) at (g * KG + q) * 128 bytes,
+ * so LBO = 128 and SBO = KG * 128. */
+template <int KG, int NROWS, int ABYTES>
+struct ConvSmem {
+    alignas(128) unsigned char b[NROWS / 8][KG][128];
+    alignas(128) unsigned char a[ABYTES];
+    alignas(128) unsigned char out[CNN_THREADS / 32][32 * 64];   /* a warp's output pixels */
+    alignas(16) float bias[32];
+    unsigned long long bar;
+    unsigned tmem;
+};
 
-/* One CTA per 128 output pixels, persistent over tiles.  Template:
- * CIN (1 or 32), N (GEMM N: 32, or 16 for a one-channel output padded with
- * zero weights), MODE (gather).  x: [B][H][W][CIN] bf16; y: [B][Ho][Wo][COUT]
- * bf16 (or f32 when y_f32 is set, COUT = 1). */
-template <int CIN, int N, int MODE>
-__global__ void __launch_bounds__(CNN_THREADS)
-hl_conv3x3_kernel(hl_conv_args a)
+/* weights -> B operand: row n = output channel, K group q = 8 consecutive k;
+ * rows n >= cout and k >= kreal are zero */
+template <int KG, int N>
+__device__ __forceinline__ void conv_weights(unsigned char (*b)[KG][128], const hl_conv_args &a)
 {
-    constexpr int K = (CIN == 1) ? 16 : 9 * CIN;   /* padded to 16 for CIN = 1 */
-    constexpr int KG = K / 8;
-    extern __shared__ __align__(128) unsigned char conv_raw[];
-    ConvSmem<KG, N> &sm = *reinterpret_cast<ConvSmem<KG, N> *>(conv_raw);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int HWo = a.Ho * a.Wo;
-    const int ntiles = (a.B * HWo + CNN_TILE_M - 1) / CNN_TILE_M;
-
-    /* weights -> B operand (once per CTA): row n = output channel, K group q
-     * = 8 consecutive k; rows n >= cout are zero */
-    for (int e = tid; e < N * KG; e += CNN_THREADS) {
-        const int n = e / KG, q = e % KG;
-        __nv_bfloat16 v8[8];
+    const bool vec = a.kreal % 8 == 0 && (((uintptr_t)a.w) & 15u) == 0;
+    constexpr int NE = N * KG / CNN_THREADS + (N * KG % CNN_THREADS != 0);
+    uint4 v[NE];   /* every load in flight before the first store */
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int k = q * 8 + j;
-            const bool ok = n < a.cout && k < a.kreal;
-            v8[j] = ok ? a.w[(size_t)n * a.kreal + k] : __float2bfloat16(0.0f);
+    for (int i = 0; i < NE; i++) {
+        /* 8 lanes take 4 channels x 2 K groups: whole sectors read, stores at
+         * most two to a bank */
+        const int e = threadIdx.x + i * CNN_THREADS;
+        const int q = ((e >> 3) % (KG / 2)) * 2 + (e & 1);
+        const int n = ((e >> 1) & 3) + 4 * (e / (4 * KG));
+        v[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (e < N * KG && vec) {
+            if (n < a.cout && q * 8 < a.kreal)
+                v[i] = *reinterpret_cast<const uint4 *>(a.w + (size_t)n * a.kreal + q * 8);
+        } else if (e < N * KG) {
+            __nv_bfloat16 v8[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const int k = q * 8 + j;
+                const bool ok = n < a.cout && k < a.kreal;
+                v8[j] = ok ? a.w[(size_t)n * a.kreal + k] : __float2bfloat16(0.0f);
+            }
+            v[i] = *reinterpret_cast<const uint4 *>(v8);
         }
-        unsigned char *dst = &sm.b[n >> 3][q][(n & 7) * 16];
-        *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(v8);
     }
-    if (warp == 0)
-        tmem_alloc32(&sm.tmem);
-    if (tid == 0) {
-        cnn_mbar_init(&sm.bar, 1);
+#pragma unroll
+    for (int i = 0; i < NE; i++) {
+        const int e = threadIdx.x + i * CNN_THREADS;
+        const int q = ((e >> 3) % (KG / 2)) * 2 + (e & 1);
+        const int n = ((e >> 1) & 3) + 4 * (e / (4 * KG));
+        if (e < N * KG)
+            *reinterpret_cast<uint4 *>(&b[n >> 3][q][(n & 7) * 16]) = v[i];
+    }
+}
+
+/* A tile of the output (CONV_T2: of the input): its image and first pixel. */
+struct ConvTile {
+    int b, y0, x0;
+};
+/* The tiles blockIdx.x, blockIdx.x + gridDim.x, ...: divisions once, then the
+ * grid's own (x, y, image) step with carries. */
+struct ConvTiles {
+    int tx_n, ty_n, x, y, b, dx, dy, db;
+    __device__ __forceinline__ ConvTiles(int tx, int ty) : tx_n(tx), ty_n(ty)
+    {
+        const int r = blockIdx.x / tx, gr = gridDim.x / tx;
+        x = blockIdx.x - r * tx;
+        b = r / ty;
+        y = r - b * ty;
+        dx = gridDim.x - gr * tx;
+        db = gr / ty;
+        dy = gr - db * ty;
+    }
+    __device__ __forceinline__ ConvTile get() const
+    {
+        ConvTile t;
+        t.b = b;
+        t.y0 = y * CONV_TY;
+        t.x0 = x * CONV_TX;
+        return t;
+    }
+    __device__ __forceinline__ void next()
+    {
+        x += dx;
+        y += dy;
+        b += db;
+        if (x >= tx_n) {
+            x -= tx_n;
+            y++;
+        }
+        if (y >= ty_n) {
+            y -= ty_n;
+            b++;
+        }
+    }
+};
+
+/* Start of a convolution kernel: TMEM columns and the mbarrier.  It comes
+ * before hl_pdl_begin lets the next launch in, so a waiting successor never
+ * holds columns this kernel still needs. */
+__device__ __forceinline__ unsigned conv_begin(unsigned *tmem_s, unsigned long long *bar,
+                                               int cols)
+{
+    if (threadIdx.x < 32)
+        tmem_alloc(tmem_s, cols);
+    if (threadIdx.x == 0) {
+        cnn_mbar_init(bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
-    const unsigned tmem = sm.tmem;
-    unsigned phase = 0;
-    bool failed = false;
+    return *tmem_s;
+}
 
-    for (int tile = blockIdx.x; tile < ntiles && !failed; tile += gridDim.x) {
-        /* A operand: row m = output pixel tile * 128 + m */
-        if (CIN == 32) {
-            /* thread m gathers row m (one output pixel): its coordinates once,
-             * then one 16-byte cp.async per K group (tap q / 4, channels
-             * (q % 4) * 8 .. +7) with compile-time tap offsets; every copy of
-             * the tile in flight at once, zero-filled outside the image */
-            static_assert(CNN_THREADS == CNN_TILE_M, "one thread per tile row");
-            const int m = tid;
-            const int p = tile * CNN_TILE_M + m;
-            const bool row_ok = p < a.B * HWo;
-            int bimg = 0, oy = 0, ox = 0;
-            if (row_ok) {
-                bimg = p / HWo;
-                const int r = p - bimg * HWo;
-                oy = r / a.Wo;
-                ox = r - oy * a.Wo;
-            }
-            const __nv_bfloat16 *ximg = a.x + (size_t)bimg * a.H * a.W * 32;
-            const unsigned arow = cnn_smem_u32(&sm.a[m >> 3][0][(m & 7) * 16]);
+/* two floats -> packed bf16 (the first in the low half) */
+__device__ __forceinline__ unsigned pack_bf16(float lo, float hi)
+{
+    const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const unsigned *>(&p);
+}
+
+/* Epilogue of a warp's 32 pixels (its TMEM lanes; columns tcol ..): bias and
+ * ReLU in fp32, bf16 rounding, then through the warp's staging buffer so that
+ * 8 neighbouring output pixels leave as one 512-byte store.  Tile row r (8
+ * pixels) goes to output row oy0 + r * osy, columns ox0 + x * osx. */
+__device__ __forceinline__ void conv_epilogue(const hl_conv_args &a, unsigned tcol,
+                                              unsigned char *stage, const float *bias, int bimg,
+                                              int oy0, int ox0, int osy, int osx)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float v[32];
+    tmem_ld32(tcol + ((unsigned)(32 * warp) << 16), v);
+    if (a.y_f32) {
+        const int m = 32 * warp + lane;
+        const int oy = oy0 + (m >> 3) * osy, ox = ox0 + (m & 7) * osx;
+        if (oy < a.Ho && ox < a.Wo) {
+            float o = v[0] + bias[0];
+            if (a.relu)
+                o = fmaxf(o, 0.0f);
+            a.y_f32[((size_t)bimg * a.Ho + oy) * a.Wo + ox] = o;
+        }
+        return;
+    }
 #pragma unroll
-            for (int tap = 0; tap < 9; tap++) {
-                const int ky = tap / 3, kx = tap % 3;
-                int iy, ix;
-                bool ok;
-                if (MODE == GATHER_CONV) {
-                    iy = oy * a.stride - 1 + ky;
-                    ix = ox * a.stride - 1 + kx;
-                    ok = row_ok && iy >= 0 && ix >= 0 && iy < a.H && ix < a.W;
-                } else {
-                    const int ty = oy + 1 - ky, tx = ox + 1 - kx;
-                    iy = ty >> 1;
-                    ix = tx >> 1;
-                    ok = row_ok && ty >= 0 && tx >= 0 && !(ty & 1) && !(tx & 1) &&
-                         iy < a.H && ix < a.W;
-                }
-                const __nv_bfloat16 *src = ok ? ximg + ((size_t)iy * a.W + ix) * 32 : a.x;
+    for (int c = 0; c < 8; c++) {
+        const float4 bb = reinterpret_cast<const float4 *>(bias)[c];
+        v[4 * c] += bb.x;
+        v[4 * c + 1] += bb.y;
+        v[4 * c + 2] += bb.z;
+        v[4 * c + 3] += bb.w;
+    }
+    if (a.relu) {
 #pragma unroll
-                for (int c = 0; c < 4; c++)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
-                                 ::"r"(arow + (unsigned)((tap * 4 + c) * 128)),
-                                 "l"(src + c * 8), "r"(ok ? 16 : 0)
-                                 : "memory");
-            }
-            asm volatile("cp.async.wait_all;" ::: "memory");
-        } else {
-            for (int e = tid; e < CNN_TILE_M * KG; e += CNN_THREADS) {
-                const int m = e / KG, q = e % KG;
-                const int p = tile * CNN_TILE_M + m;
-                uint4 val = make_uint4(0u, 0u, 0u, 0u);
-                if (p < a.B * HWo) {
-                    const int bimg = p / HWo, r = p % HWo;
-                    const int oy = r / a.Wo, ox = r % a.Wo;
-                    /* CIN = 1: k = tap, 9 taps then zeros */
-                    __nv_bfloat16 v8[8];
+        for (int c = 0; c < 32; c++)
+            v[c] = fmaxf(v[c], 0.0f);
+    }
+    if (a.cout < 32) {
 #pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        const int tap = q * 8 + j;
-                        __nv_bfloat16 v = __float2bfloat16(0.0f);
-                        if (tap < 9) {
-                            const int ky = tap / 3, kx = tap % 3;
-                            const int iy = oy * a.stride - 1 + ky;
-                            const int ix = ox * a.stride - 1 + kx;
-                            if (iy >= 0 && ix >= 0 && iy < a.H && ix < a.W)
-                                v = a.x[((size_t)bimg * a.H + iy) * a.W + ix];
-                        }
-                        v8[j] = v;
-                    }
-                    val = *reinterpret_cast<const uint4 *>(v8);
-                }
-                *reinterpret_cast<uint4 *>(&sm.a[m >> 3][q][(m & 7) * 16]) = val;
+        for (int c = 0; c < 32; c++)
+            v[c] = c < a.cout ? v[c] : 0.0f;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+        /* chunk c of pixel p at 16-byte slot 4 p + (c ^ (p / 2) % 4) */
+        *reinterpret_cast<uint4 *>(stage + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) =
+            make_uint4(pack_bf16(v[8 * c], v[8 * c + 1]), pack_bf16(v[8 * c + 2], v[8 * c + 3]),
+                       pack_bf16(v[8 * c + 4], v[8 * c + 5]),
+                       pack_bf16(v[8 * c + 6], v[8 * c + 7]));
+    __syncwarp();
+    const int x = lane >> 2, q = lane & 3;
+    const int ox = ox0 + x * osx;
+#pragma unroll
+    for (int it = 0; it < 4; it++) {
+        const int p = it * 8 + x;
+        const uint4 o = *reinterpret_cast<const uint4 *>(stage + p * 64 +
+                                                         ((q ^ ((p >> 1) & 3)) << 4));
+        const int oy = oy0 + (4 * warp + it) * osy;
+        if (oy < a.Ho && ox < a.Wo)
+            *reinterpret_cast<uint4 *>(a.y + (((size_t)bimg * a.Ho + oy) * a.Wo + ox) * 32 +
+                                       q * 8) = o;
+    }
+    __syncwarp();
+}
+
+/* 32 input channels.  What bounds it: shared memory -- the tensor cores read
+ * each pixel once a tap (18 MMAs x 5 KB of operands, about 720 cycles a tile,
+ * and 460 of copies and staging); the MMAs themselves are busy 12%.  Several
+ * CTAs an SM overlap one tile's copies and epilogue with another's MMAs, and
+ * weights that are ready are read while the launch before still runs.  64
+ * images of 64 x 64, stride 1, ncu: 15.5 us a launch, against 55.0 us when
+ * every tap was gathered into an im2col tile; stride 2 (bound by the 67 MB it
+ * reads) 28.9 against 55.5, one-channel output 12.9 against 41.5. */
+template <int N, int MODE>
+__global__ void __launch_bounds__(CNN_THREADS)
+hl_conv32_kernel(hl_conv_args a)
+{
+    using H = ConvHalo<MODE>;
+    constexpr int KG = 36;
+    extern __shared__ __align__(128) unsigned char conv_raw[];
+    typedef ConvSmem<KG, N, H::NST * ((H::BYTES + 127) / 128 * 128)> Smem;
+    Smem &sm = *reinterpret_cast<Smem *>(conv_raw);
+    constexpr unsigned STAGE = (H::BYTES + 127) / 128 * 128;
+    const int tid = threadIdx.x;
+    const unsigned tmem = conv_begin(&sm.tmem, &sm.bar, H::TMEM_COLS);
+
+    /* weights written before the previous launch began are read while it
+     * still runs */
+    if (!a.w_ready)
+        hl_pdl_begin();
+    conv_weights<KG, N>(sm.b, a);
+    if (tid < 32)
+        sm.bias[tid] = (a.bias && tid < a.cout) ? a.bias[tid] : 0.0f;
+    if (a.w_ready)
+        hl_pdl_begin();
+    /* tiles cover the output (CONV_T2: the input, four outputs a position) */
+    const int EX = MODE == CONV_T2 ? a.W : a.Wo, EY = MODE == CONV_T2 ? a.H : a.Ho;
+    const int tx_n = (EX + CONV_TX - 1) / CONV_TX, ty_n = (EY + CONV_TY - 1) / CONV_TY;
+    const int ntiles = a.B * tx_n * ty_n;
+    const unsigned abase = cnn_smem_u32(sm.a), bbase = cnn_smem_u32(sm.b);
+
+    /* a thread copies plane q of every 32nd halo pixel */
+    auto load = [&](const ConvTile &t, unsigned st) {
+        constexpr int S = MODE == CONV_S2 ? 2 : 1;
+        const int iy0 = t.y0 * S - (MODE == CONV_T2 ? 0 : 1);
+        const int ix0 = t.x0 * S - (MODE == CONV_T2 ? 0 : 1);
+        const int q = tid & 3;
+        const __nv_bfloat16 *x = a.x + (size_t)t.b * a.H * a.W * 32 + q * 8;
+        int hy = (tid >> 2) / H::COLS, hx = (tid >> 2) % H::COLS;
+        for (int px = tid >> 2; px < H::ROWS * H::COLS; px += CNN_THREADS / 4) {
+            const int iy = iy0 + hy, ix = ix0 + hx;
+            const bool ok = (unsigned)iy < (unsigned)a.H && (unsigned)ix < (unsigned)a.W;
+            const __nv_bfloat16 *src = ok ? x + (size_t)(iy * a.W + ix) * 32 : a.x;
+            const unsigned dst =
+                abase + st + (unsigned)((hy * 4 + q) * H::P) +
+                (MODE == CONV_S2 ? (unsigned)((hx & 1) * H::HALF + (hx >> 1) * 16)
+                                 : (unsigned)(hx * 16));
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                         ::"r"(dst), "l"(src), "r"(ok ? 16 : 0)
+                         : "memory");
+            hx += 32 % H::COLS;
+            hy += 32 / H::COLS;
+            if (hx >= H::COLS) {
+                hx -= H::COLS;
+                hy++;
             }
         }
-        /* make the generic-proxy writes visible to the tensor cores */
+    };
+
+    unsigned phase = 0, st = 0;
+    bool failed = false;
+    ConvTiles walk(tx_n, ty_n);
+    ConvTile cur = walk.get();
+    if ((int)blockIdx.x < ntiles)
+        load(cur, 0);
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        /* the copies (and the weights) visible to the tensor cores */
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
+        if (__syncthreads_or(failed))
+            break;
+        if (tid < 32 && elect_one()) {
             tmem_fence_after();
-            const unsigned abase = cnn_smem_u32(&sm.a[0][0][0]);
-            const unsigned bbase = cnn_smem_u32(&sm.b[0][0][0]);
             constexpr unsigned idesc = mma_idesc(CNN_TILE_M, N);
+            constexpr unsigned sbo = (MODE == CONV_S2 ? 8 : 4) * H::P;
+            /* descriptors of tap 0; a tap's differ by a constant in the
+             * 16-byte address field */
+            const unsigned long long ad0 = smem_desc(abase + st, H::P, sbo);
+            const unsigned long long bd0 = smem_desc(bbase, 128, KG * 128);
+            /* CONV_T2: output parity class cls = 2 py + px; others one class */
 #pragma unroll
-            for (int s = 0; s < K / 16; s++) {
-                const unsigned long long ad = smem_desc(abase + s * 256, 128, KG * 128);
-                const unsigned long long bd = smem_desc(bbase + s * 256, 128, KG * 128);
-                umma_f16(tmem, ad, bd, idesc, s > 0);
+            for (int cls = 0; cls < (MODE == CONV_T2 ? 4 : 1); cls++) {
+                bool first = true;
+#pragma unroll
+                for (int tap = 0; tap < 9; tap++) {
+                    const int ky = tap / 3, kx = tap % 3;
+                    unsigned off;
+                    if (MODE == CONV_T2) {
+                        /* rows with (p + 1 - tap) odd take no tap; an even row
+                         * takes ky = 1 at j, an odd one ky = 0 at j + 1 and
+                         * ky = 2 at j */
+                        if (((cls >> 1) + 1 - ky) & 1 || ((cls & 1) + 1 - kx) & 1)
+                            continue;
+                        const int dy = ((cls >> 1) + 1 - ky) >> 1, dx = ((cls & 1) + 1 - kx) >> 1;
+                        off = (unsigned)(dy * 4 * H::P + dx * 16);
+                    } else if (MODE == CONV_S2) {
+                        off = (unsigned)(ky * 4 * H::P + (kx & 1) * H::HALF + (kx >> 1) * 16);
+                    } else {
+                        off = (unsigned)(ky * 4 * H::P + kx * 16);
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        umma_f16(tmem + (unsigned)(cls * 32),
+                                 ad0 + ((off + (unsigned)(2 * h * H::P)) >> 4),
+                                 bd0 + (unsigned)((tap * 2 + h) * 16), idesc, !first);
+                        first = false;
+                    }
+                }
             }
             umma_commit(&sm.bar);
         }
         __syncwarp();
+        const int next = tile + (int)gridDim.x;
+        walk.next();
+        const ConvTile nt = walk.get();
+        if (H::NST == 2 && next < ntiles)
+            load(nt, st ^ STAGE);
         const bool got = cnn_mbar_wait(&sm.bar, phase);
         phase ^= 1u;
         tmem_fence_after();
         if (!got) {
             failed = true;
-            if (lane == 0)
+            if ((tid & 31) == 0)
                 atomicOr(a.status, HL_ST_CNN_TIMEOUT);
-        } else {
-            /* epilogue: warp w holds rows 32 w .. 32 w + 31 (its TMEM lanes) */
-            float v[32];
-            tmem_ld32(tmem + ((unsigned)(32 * warp) << 16), v);
-            const int m = 32 * warp + lane;
-            const int p = tile * CNN_TILE_M + m;
-            if (p < a.B * HWo) {
-                if (a.y_f32) {
-                    float o = v[0] + (a.bias ? a.bias[0] : 0.0f);
-                    if (a.relu)
-                        o = fmaxf(o, 0.0f);
-                    a.y_f32[p] = o;
-                } else {
-                    __nv_bfloat16 o8[32];
-#pragma unroll
-                    for (int c = 0; c < 32; c++) {
-                        float o = v[c] + ((a.bias && c < a.cout) ? a.bias[c] : 0.0f);
-                        if (a.relu)
-                            o = fmaxf(o, 0.0f);
-                        if (c >= a.cout)
-                            o = 0.0f;
-                        o8[c] = __float2bfloat16(o);
-                    }
-                    uint4 *dst = reinterpret_cast<uint4 *>(a.y + (size_t)p * 32);
-#pragma unroll
-                    for (int c = 0; c < 4; c++)
-                        dst[c] = reinterpret_cast<const uint4 *>(o8)[c];
-                }
-            }
+            continue;
         }
-        /* TMEM reads and shared-memory reads done before the next tile */
+        if (H::NST == 1 && next < ntiles)
+            load(nt, 0);   /* the MMAs have read the halo */
+        else if (H::NST == 2)
+            st ^= STAGE;
+        if (MODE == CONV_T2) {
+#pragma unroll 1
+            for (int cls = 0; cls < 4; cls++)
+                conv_epilogue(a, tmem + (unsigned)(cls * 32), sm.out[tid >> 5], sm.bias, cur.b,
+                              2 * cur.y0 + (cls >> 1), 2 * cur.x0 + (cls & 1), 2, 2);
+        } else {
+            conv_epilogue(a, tmem, sm.out[tid >> 5], sm.bias, cur.b, cur.y0, cur.x0, 1, 1);
+        }
+        cur = nt;
+        /* TMEM reads done before the next tile's MMAs (ordered by the
+         * barrier at the loop's top) */
         tmem_fence_before();
-        __syncthreads();
-        tmem_fence_after();
     }
     if (failed) {
         /* a commit that never arrived: nothing more is issued; wait once
          * more (bounded) so no MMA still writes the TMEM being released */
-        cnn_mbar_wait(&sm.bar, phase);
+        cnn_mbar_wait(&sm.bar, phase ^ 1u);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    if (warp == 0)
-        tmem_dealloc32(tmem);
+    if (tid < 32)
+        tmem_dealloc(tmem, H::TMEM_COLS);
 }
 
-template <int CIN, int N, int MODE>
-static cudaError_t launch_conv(const hl_conv_args *a, int sms, cudaStream_t s)
+/* One input channel, stride 1 or 2: K = 16 (9 taps, then zeros), a thread
+ * gathers the 9 values of its output pixel into its row of A; the next tile's
+ * values are loaded behind the MMA.  Bound by its epilogue's instructions and
+ * the output's 64 bytes a pixel: 64 maps of 256 x 256, stride 2, 23.8 us
+ * (46.6 us before). */
+__global__ void __launch_bounds__(CNN_THREADS)
+hl_conv1_kernel(hl_conv_args a)
 {
-    constexpr int K = (CIN == 1) ? 16 : 9 * CIN;
-    const size_t smem = sizeof(ConvSmem<K / 8, N>) + 128;
-    cudaError_t e = cudaFuncSetAttribute(hl_conv3x3_kernel<CIN, N, MODE>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess)
-        return e;
-    const int ntiles = (a->B * a->Ho * a->Wo + CNN_TILE_M - 1) / CNN_TILE_M;
-    /* CTAs per SM: 32-channel inputs hold ~92 KB of operands (two fit);
-     * one-channel inputs ~5 KB (eight fit, 8 x 32 TMEM columns) */
-    const int grid = std::max(1, std::min(ntiles, sms * (CIN == 1 ? 8 : 2)));
-    hl_conv3x3_kernel<CIN, N, MODE><<<grid, CNN_THREADS, smem, s>>>(*a);
-    return cudaGetLastError();
+    constexpr int KG = 2, N = 32;
+    extern __shared__ __align__(128) unsigned char conv_raw[];
+    typedef ConvSmem<KG, N, CNN_TILE_M * 32> Smem;
+    Smem &sm = *reinterpret_cast<Smem *>(conv_raw);
+    const int tid = threadIdx.x;
+    const unsigned tmem = conv_begin(&sm.tmem, &sm.bar, 32);
+    hl_pdl_begin();
+    conv_weights<KG, N>(sm.b, a);
+    if (tid < 32)
+        sm.bias[tid] = (a.bias && tid < a.cout) ? a.bias[tid] : 0.0f;
+    const int tx_n = (a.Wo + CONV_TX - 1) / CONV_TX, ty_n = (a.Ho + CONV_TY - 1) / CONV_TY;
+    const int ntiles = a.B * tx_n * ty_n;
+    const unsigned abase = cnn_smem_u32(sm.a), bbase = cnn_smem_u32(sm.b);
+
+    unsigned short v[9];   /* the pixel's taps, as bf16 bits */
+    auto gather = [&](const ConvTile &t) {
+        const int iy0 = (t.y0 + (tid >> 3)) * a.stride - 1;
+        const int ix0 = (t.x0 + (tid & 7)) * a.stride - 1;
+        const unsigned short *x =
+            reinterpret_cast<const unsigned short *>(a.x) + (size_t)t.b * a.H * a.W;
+        bool okx[3];
+#pragma unroll
+        for (int kx = 0; kx < 3; kx++)
+            okx[kx] = (unsigned)(ix0 + kx) < (unsigned)a.W;
+#pragma unroll
+        for (int ky = 0; ky < 3; ky++) {
+            const bool oky = (unsigned)(iy0 + ky) < (unsigned)a.H;
+            const unsigned short *row = x + (ptrdiff_t)(iy0 + ky) * a.W + ix0;
+#pragma unroll
+            for (int kx = 0; kx < 3; kx++)
+                v[3 * ky + kx] = oky && okx[kx] ? row[kx] : (unsigned short)0;
+        }
+    };
+    unsigned phase = 0;
+    bool failed = false;
+    ConvTiles walk(tx_n, ty_n);
+    ConvTile cur = walk.get();
+    if ((int)blockIdx.x < ntiles)
+        gather(cur);
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        unsigned char *row = sm.a + (tid >> 3) * 256 + (tid & 7) * 16;
+        *reinterpret_cast<uint4 *>(row) =
+            make_uint4(v[0] | ((unsigned)v[1] << 16), v[2] | ((unsigned)v[3] << 16),
+                       v[4] | ((unsigned)v[5] << 16), v[6] | ((unsigned)v[7] << 16));
+        *reinterpret_cast<uint4 *>(row + 128) = make_uint4(v[8], 0u, 0u, 0u);
+        asm volatile("cp.async.wait_all;" ::: "memory");   /* the weights */
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (__syncthreads_or(failed))
+            break;
+        if (tid < 32 && elect_one()) {
+            tmem_fence_after();
+            umma_f16(tmem, smem_desc(abase, 128, 256), smem_desc(bbase, 128, 256),
+                     mma_idesc(CNN_TILE_M, N), 0);
+            umma_commit(&sm.bar);
+        }
+        __syncwarp();
+        const int next = tile + (int)gridDim.x;
+        walk.next();
+        const ConvTile nt = walk.get();
+        if (next < ntiles)
+            gather(nt);
+        const bool got = cnn_mbar_wait(&sm.bar, phase);
+        phase ^= 1u;
+        tmem_fence_after();
+        if (!got) {
+            failed = true;
+            if ((tid & 31) == 0)
+                atomicOr(a.status, HL_ST_CNN_TIMEOUT);
+            continue;
+        }
+        conv_epilogue(a, tmem, sm.out[tid >> 5], sm.bias, cur.b, cur.y0, cur.x0, 1, 1);
+        cur = nt;
+        tmem_fence_before();
+    }
+    if (failed)
+        cnn_mbar_wait(&sm.bar, phase ^ 1u);   /* as in hl_conv32_kernel */
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (tid < 32)
+        tmem_dealloc(tmem, 32);
 }
 
-cudaError_t hl_launch_conv3x3(const hl_conv_args *a, int mode, cudaStream_t s)
+template <typename K>
+static cudaError_t launch_conv(K kernel, size_t smem, long long ntiles, int ctas_per_sm,
+                               const hl_conv_args *a, cudaStream_t s)
 {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (a->cin == 1 && a->cout <= 32 && mode == GATHER_CONV)
-        return launch_conv<1, 32, GATHER_CONV>(a, sms, s);
-    if (a->cin == 32 && a->cout <= 16 && mode == GATHER_CONV)
-        return launch_conv<32, 16, GATHER_CONV>(a, sms, s);
-    if (a->cin == 32 && a->cout <= 32 && mode == GATHER_CONV)
-        return launch_conv<32, 32, GATHER_CONV>(a, sms, s);
-    if (a->cin == 32 && a->cout <= 32 && mode == GATHER_CONVT2)
-        return launch_conv<32, 32, GATHER_CONVT2>(a, sms, s);
-    return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem);
+    if (e != cudaSuccess)
+        return e;
+    if (ntiles > 0x7fffffffLL)
+        return cudaErrorInvalidValue;
+    const int grid = (int)std::max(1LL, std::min(ntiles, (long long)sms * ctas_per_sm));
+    return hl_launch_pdl(kernel, dim3(grid), dim3(CNN_THREADS), smem, s, false, *a);
+}
+
+template <int N, int MODE>
+static cudaError_t launch_conv32(const hl_conv_args *a, cudaStream_t s)
+{
+    typedef ConvHalo<MODE> H;
+    typedef ConvSmem<36, N, H::NST * ((H::BYTES + 127) / 128 * 128)> Smem;
+    const int ex = MODE == CONV_T2 ? a->W : a->Wo, ey = MODE == CONV_T2 ? a->H : a->Ho;
+    const long long nt = (long long)a->B * ((ex + CONV_TX - 1) / CONV_TX) *
+                         ((ey + CONV_TY - 1) / CONV_TY);
+    return launch_conv(hl_conv32_kernel<N, MODE>, sizeof(Smem), nt, H::CTAS, a, s);
+}
+
+cudaError_t hl_launch_conv3x3(const hl_conv_args *a, int mode, cudaStream_t s)
+{
+    if (a->cin == 1 && a->cout <= 32 && mode == 0) {
+        const long long nt = (long long)a->B * ((a->Wo + CONV_TX - 1) / CONV_TX) *
+                             ((a->Ho + CONV_TY - 1) / CONV_TY);
+        return launch_conv(hl_conv1_kernel, sizeof(ConvSmem<2, 32, CNN_TILE_M * 32>), nt, 8, a, s);
+    }
+    if (a->cin != 32 || a->cout > 32)
+        return cudaErrorInvalidValue;
+    if (mode == 1)
+        return launch_conv32<32, CONV_T2>(a, s);
+    if (mode != 0)
+        return cudaErrorInvalidValue;
+    if (a->stride == 2)
+        return a->cout <= 16 ? launch_conv32<16, CONV_S2>(a, s) : launch_conv32<32, CONV_S2>(a, s);
+    return a->cout <= 16 ? launch_conv32<16, CONV_S1>(a, s) : launch_conv32<32, CONV_S1>(a, s);
 }
 
 /* ---- occupancy pooling ---------------------------------------------------- */
@@ -594,63 +877,158 @@ __device__ __forceinline__ int head_bin(const hl_head_geom &g, int qy, int qx,
 
 /* logits[b][t][r] = alpha * sum_{cells with bin r at angle t} e[b][cell] + beta
  * One CTA per (image, group of HEAD_TG angles), the group's [HEAD_TG][R] sums
- * in shared memory.  A thread walks one line of evidence cells for one angle
- * -- a column when the angle's rho changes less along y (|sin| < |cos|), else
- * a row -- keeping a running sum while consecutive cells fall in one bin and
- * adding it to that bin when the bin changes: the cells of a line mostly
- * share bins, so this issues a few shared reductions per line instead of one
- * per cell.  The sums are 64-bit fixed point (2^-24 units), so they do not
- * depend on the order of the additions. */
+ * and the image's evidence map in shared memory (rows one word longer than the
+ * map, so a walk along x or y is free of bank conflicts).  A thread walks one
+ * line of evidence cells for one angle -- a column when the angle's rho
+ * changes less along y (|sin| < |cos|), else a row -- keeping a running sum
+ * while consecutive cells fall in one bin and adding it to that bin when the
+ * bin changes: the cells of a line mostly share bins, so this issues a few
+ * shared reductions per line instead of one per cell.  Bound by its
+ * instructions and shared reductions: 64 images 30.3 us, 95 us with 64-bit
+ * shared atomics and a double conversion per cell; prefix sums along the lines
+ * with one difference per bin measured 38 us.  The sums are 64-bit
+ * fixed point (2^-24 units), so they do not depend on the order of the
+ * additions; a sum is kept in two 32-bit words (a 64-bit shared reduction is a
+ * compare-and-swap loop): where every cell fits 32 bits, run = hi * 2^20 + lo
+ * (at most 64 runs reach a bin, one a line, so neither word overflows and
+ * neither reduction needs its result back), else low and high word with the
+ * carry. */
 #define HEAD_TG 6
+#define HEAD_EV 64          /* side of the evidence map */
 #define HEAD_FIX 16777216.0f
+#define HEAD_WORDS (HEAD_TG * HL_HEAD_R + 32)   /* the bins, a dump word per lane */
+__device__ __forceinline__ void head_add64(unsigned *lo, unsigned *hi, unsigned long long v)
+{
+    const unsigned l = (unsigned)v;
+    const unsigned old = atomicAdd(lo, l);
+    const unsigned h = (unsigned)(v >> 32) + (old + l < old ? 1u : 0u);
+    if (h)
+        atomicAdd(hi, h);
+}
+/* 64-bit conversions run on the FP64 pipe (16 cycles a warp even when
+ * predicated off), so they are kept out of line */
+static __device__ __noinline__ float head_sum64(long long fx)
+{
+    return (float)((double)fx * (1.0 / HEAD_FIX));
+}
+
+/* the bin of rho (head_bin) */
+__device__ __forceinline__ int head_cell(float fi, float fixed, float mc, const hl_head_geom &g)
+{
+    /* head_bin's roundings; fl(x c) + fl(y s) does not depend on the order */
+    const float rho = __fadd_rn(fixed, __fmul_rn(__fmul_rn(fi, g.cell), mc));
+    const int bin = (int)floorf(__fmul_rn(__fsub_rn(rho, g.rho_min), g.inv_rw));
+    return min(max(bin, 0), HL_HEAD_R - 1);
+}
+
+/* One thread's walk of a line of n cells: cell i adds s_e[i * step] to the
+ * bin of rho = fixed + m(i).  At every cell each lane issues the two
+ * reductions of its run, to the bin where it leaves one and to its dump word
+ * elsewhere: neighbouring lines change bins at different cells, so a branch
+ * would be taken at nearly every cell. */
+__device__ __forceinline__ void head_walk(const int *s_e, int step, int n, float fixed, float mc,
+                                          const hl_head_geom &g, unsigned lo, unsigned dump)
+{
+    long long run = 0;
+    int cur = 0;
+    float fi = 0.5f;
+    auto flush = [&](bool p) {
+        const unsigned addr = p ? lo + 4u * (unsigned)cur : dump;
+        asm volatile("red.shared.add.u32 [%0], %1;\n\tred.shared.add.u32 [%0 + %3], %2;"
+                     ::"r"(addr), "r"((unsigned)run & 0xfffffu), "r"((unsigned)(run >> 20)),
+                     "n"(HEAD_WORDS * 4)
+                     : "memory");
+    };
+#pragma unroll 4
+    for (int i = 0; i < n; i++, s_e += step, fi += 1.0f) {
+        const int bin = head_cell(fi, fixed, mc, g);
+        const int v = *s_e;
+        const bool p = bin != cur;
+        flush(p);
+        run = p ? (long long)v : run + v;
+        cur = bin;
+    }
+    flush(n > 0);
+}
+
+/* the same with the evidence read from global memory, where a cell's fixed
+ * point needs more than 32 bits */
+__device__ __noinline__ void head_walk_wide(const float *g_e, int gstep, int n, float fixed,
+                                            float mc, const hl_head_geom &g, unsigned *lo,
+                                            unsigned *hi)
+{
+    unsigned long long run = 0ull;
+    int cur = 0;
+    float fi = 0.5f;
+    for (int i = 0; i < n; i++, fi += 1.0f) {
+        const int bin = head_cell(fi, fixed, mc, g);
+        if (bin != cur) {
+            head_add64(lo + cur, hi + cur, run);
+            cur = bin;
+            run = 0ull;
+        }
+        run += (unsigned long long)__float2ll_rn(g_e[i * gstep] * HEAD_FIX);
+    }
+    head_add64(lo + cur, hi + cur, run);
+}
+
 __global__ void __launch_bounds__(384)
-hl_head_fwd_kernel(const float *e, int ev, const hl_head_geom *geo,
+hl_head_fwd_kernel(const float *e, const hl_head_geom *geo,
                    const float *ab, float *hsum, float *logits, HeadTrig tr)
 {
-    __shared__ unsigned long long sh[HEAD_TG * HL_HEAD_R];
+    __shared__ unsigned s_sum[2 * HEAD_WORDS];     /* low words, high words */
+    __shared__ int s_e[HEAD_EV * (HEAD_EV + 1)];   /* the evidence in fixed point */
     __shared__ float cs[HEAD_TG], sn[HEAD_TG];
     const int b = blockIdx.y, t0 = blockIdx.x * HEAD_TG;
     const int nt = min(HEAD_TG, HL_HEAD_T - t0);
-    for (int i = threadIdx.x; i < HEAD_TG * HL_HEAD_R; i += blockDim.x)
-        sh[i] = 0ull;
+    unsigned *const s_lo = s_sum, *const s_hi = s_sum + HEAD_WORDS;
+    for (int i = threadIdx.x; i < 2 * HEAD_WORDS; i += blockDim.x)
+        s_sum[i] = 0u;
     if (threadIdx.x < nt) {
         cs[threadIdx.x] = tr.c[t0 + threadIdx.x];
         sn[threadIdx.x] = tr.s[t0 + threadIdx.x];
     }
-    __syncthreads();
+    hl_pdl_begin();
     const hl_head_geom g = geo[b];
-    const float *eb = e + (size_t)b * ev * ev;
-    for (int job = threadIdx.x; job < nt * ev; job += blockDim.x) {
-        const int t = job / ev, line = job % ev;
+    const float *eb = e + (size_t)b * HEAD_EV * HEAD_EV;
+    bool big = false;   /* a value whose fixed point needs more than 32 bits */
+    for (int i = threadIdx.x; i < HEAD_EV * HEAD_EV; i += blockDim.x) {
+        const float x = eb[i] * HEAD_FIX;
+        big |= !(fabsf(x) < 2147483648.0f);
+        s_e[(i / HEAD_EV) * (HEAD_EV + 1) + i % HEAD_EV] = __float2int_rn(x);
+    }
+    const bool wide = __syncthreads_or(big);
+    for (int job = threadIdx.x; job < nt * HEAD_EV; job += blockDim.x) {
+        const int t = job / HEAD_EV, line = job % HEAD_EV;
         const float c = cs[t], sv = sn[t];
         const bool walk_y = fabsf(sv) < fabsf(c);
-        unsigned long long run = 0ull;
-        int cur = -1;
-        for (int i = 0; i < ev; i++) {
-            const int qy = walk_y ? i : line, qx = walk_y ? line : i;
-            if (qy >= g.qh || qx >= g.qw)
-                continue;
-            const float v = eb[qy * ev + qx];
-            if (v == 0.0f)
-                continue;
-            const int bin = head_bin(g, qy, qx, c, sv);
-            if (bin != cur) {
-                if (cur >= 0)
-                    atomicAdd(&sh[t * HL_HEAD_R + cur], run);
-                cur = bin;
-                run = 0ull;
-            }
-            run += (unsigned long long)__float2ll_rn(v * HEAD_FIX);
-        }
-        if (cur >= 0)
-            atomicAdd(&sh[t * HL_HEAD_R + cur], run);
+        /* the walk's fixed and moving coordinates */
+        const int n = line < (walk_y ? g.qw : g.qh) ? min(walk_y ? g.qh : g.qw, HEAD_EV) : 0;
+        const float fixed = __fmul_rn(__fmul_rn(__fadd_rn((float)line, 0.5f), g.cell),
+                                      walk_y ? c : sv);
+        const float mc = walk_y ? sv : c;
+        const int *p = s_e + (walk_y ? line : line * (HEAD_EV + 1));
+        const int step = walk_y ? HEAD_EV + 1 : 1;
+        if (!wide)
+            head_walk(p, step, n, fixed, mc, g, cnn_smem_u32(s_lo + t * HL_HEAD_R),
+                      cnn_smem_u32(s_lo + HEAD_TG * HL_HEAD_R + (threadIdx.x & 31)));
+        else
+            head_walk_wide(eb + (walk_y ? line : line * HEAD_EV), walk_y ? HEAD_EV : 1, n, fixed,
+                           mc, g, s_lo + t * HL_HEAD_R, s_hi + t * HL_HEAD_R);
     }
     __syncthreads();
     const float alpha = ab[0], beta = ab[1];
     for (int i = threadIdx.x; i < nt * HL_HEAD_R; i += blockDim.x) {
         const size_t o = (size_t)b * HL_HEAD_T * HL_HEAD_R + (size_t)t0 * HL_HEAD_R + i;
-        const float sum = (float)((double)(long long)sh[i] * (1.0 / HEAD_FIX));
-        hsum[o] = sum;
+        const long long fx =
+            wide ? (long long)(((unsigned long long)s_hi[i] << 32) | s_lo[i])
+                 : (((long long)(int)s_hi[i]) << 20) + (long long)s_lo[i];
+        /* the double only where the sum needs more than 32 bits: both give
+         * the float nearest the sum */
+        const float sum = fx == (int)fx ? __int2float_rn((int)fx) * (1.0f / HEAD_FIX)
+                                        : head_sum64(fx);
+        if (hsum)
+            hsum[o] = sum;
         logits[o] = alpha * sum + beta;
     }
 }
@@ -685,13 +1063,12 @@ hl_head_bwd_kernel(const float *dz, int ev, const hl_head_geom *geo,
     }
 }
 
-cudaError_t hl_launch_head_fwd(const float *e, int ev, const hl_head_geom *geo,
+cudaError_t hl_launch_head_fwd(const float *e, const hl_head_geom *geo,
                                int nimg, const float *ab, float *hsum,
                                float *logits, cudaStream_t s)
 {
-    hl_head_fwd_kernel<<<dim3((HL_HEAD_T + HEAD_TG - 1) / HEAD_TG, nimg), 384, 0, s>>>(
-        e, ev, geo, ab, hsum, logits, head_trig());
-    return cudaGetLastError();
+    return hl_launch_pdl(hl_head_fwd_kernel, dim3((HL_HEAD_T + HEAD_TG - 1) / HEAD_TG, nimg),
+                         dim3(384), 0, s, false, e, geo, ab, hsum, logits, head_trig());
 }
 
 cudaError_t hl_launch_head_bwd(const float *dz, int ev, const hl_head_geom *geo,

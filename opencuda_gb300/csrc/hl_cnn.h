@@ -22,6 +22,9 @@ typedef struct hl_conv_args {
     int cin, cout, kreal;
     int stride;
     int relu;
+    /* w and bias were written before the launch preceding this one on its
+     * stream began: they may be read while that one still runs */
+    int w_ready;
     int *status;
 } hl_conv_args;
 
@@ -71,7 +74,8 @@ typedef struct hl_head_geom {
     int qh, qw;      /* evidence cells covering the ROI */
     int pad;
 } hl_head_geom;
-cudaError_t hl_launch_head_fwd(const float *e, int ev, const hl_head_geom *geo,
+/* e: [nimg][64][64] evidence; hsum may be NULL (no training) */
+cudaError_t hl_launch_head_fwd(const float *e, const hl_head_geom *geo,
                                int nimg, const float *ab, float *hsum,
                                float *logits, cudaStream_t s);
 cudaError_t hl_launch_head_bwd(const float *dz, int ev, const hl_head_geom *geo,

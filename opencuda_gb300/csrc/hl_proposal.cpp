@@ -304,12 +304,15 @@ static int conv_layer(hl_net *n, int l, const __nv_bfloat16 *x, int B,
     a.kreal = 9 * L_CIN[l];
     a.stride = L_STRIDE[l];
     a.relu = L_RELU[l];
+    a.w_ready = l > 0;   /* the launch before is the previous layer's */
     a.status = n->status;
     CKN(hl_launch_conv3x3(&a, 0, s));
     return HL_NO_ERROR;
 }
 
-static int net_forward(hl_net *n, const __nv_bfloat16 *occ, int B, cudaStream_t s)
+/* logits into `logits` (device); the head's sums into n->hsum when training */
+static int net_forward(hl_net *n, const __nv_bfloat16 *occ, int B, float *logits, bool train,
+                       cudaStream_t s)
 {
     int rc;
     const __nv_bfloat16 *x = occ;
@@ -322,8 +325,8 @@ static int net_forward(hl_net *n, const __nv_bfloat16 *occ, int B, cudaStream_t 
             return rc;
         x = n->act[l];
     }
-    CKN(hl_launch_head_fwd(n->ev, NET_EV, n->geo, B, n->w + ab_off(), n->hsum,
-                           n->logits, s));
+    CKN(hl_launch_head_fwd(n->ev, n->geo, B, n->w + ab_off(), train ? n->hsum : nullptr,
+                           logits, s));
     return HL_NO_ERROR;
 }
 
@@ -347,13 +350,7 @@ extern "C" int hl_net_forward(hl_net *n, const void *occ_dev,
     int rc = net_reserve(n, B);
     if (rc != HL_NO_ERROR || (rc = upload_geo(n, geo_host, B, s)) != HL_NO_ERROR)
         return rc;
-    if ((rc = net_forward(n, static_cast<const __nv_bfloat16 *>(occ_dev), B, s)) !=
-        HL_NO_ERROR)
-        return rc;
-    CKN(cudaMemcpyAsync(logits_dev, n->logits,
-                        (size_t)B * HL_HEAD_T * HL_HEAD_R * sizeof(float),
-                        cudaMemcpyDeviceToDevice, s));
-    return HL_NO_ERROR;
+    return net_forward(n, static_cast<const __nv_bfloat16 *>(occ_dev), B, logits_dev, false, s);
 }
 
 /* dW and db of layer l from the f32 gradient dy (rows of dy_c values) */
@@ -424,7 +421,7 @@ extern "C" int hl_net_train_step(hl_net *n, const void *occ_dev,
     int rc = net_reserve(n, B);
     if (rc != HL_NO_ERROR || (rc = upload_geo(n, geo_host, B, s)) != HL_NO_ERROR)
         return rc;
-    if ((rc = net_forward(n, occ, B, s)) != HL_NO_ERROR)
+    if ((rc = net_forward(n, occ, B, n->logits, true, s)) != HL_NO_ERROR)
         return rc;
     const int np = n_params();
     CKN(cudaMemsetAsync(n->g, 0, np * sizeof(float), s));
@@ -550,7 +547,7 @@ int hl_net_run(hl_net *n, const __nv_bfloat16 *occ, const hl_head_geom *geo_dev,
         return rc;
     CKN(cudaMemcpyAsync(n->geo, geo_dev, (size_t)B * sizeof(hl_head_geom),
                         cudaMemcpyDeviceToDevice, s));
-    if ((rc = net_forward(n, occ, B, s)) != HL_NO_ERROR)
+    if ((rc = net_forward(n, occ, B, n->logits, false, s)) != HL_NO_ERROR)
         return rc;
     *logits = n->logits;
     return HL_NO_ERROR;
