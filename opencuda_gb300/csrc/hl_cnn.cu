@@ -253,6 +253,7 @@ struct ConvTile {
 };
 /* The tiles blockIdx.x, blockIdx.x + gridDim.x, ...: divisions once, then the
  * grid's own (x, y, image) step with carries. */
+template <int TX, int TY>
 struct ConvTiles {
     int tx_n, ty_n, x, y, b, dx, dy, db;
     __device__ __forceinline__ ConvTiles(int tx, int ty) : tx_n(tx), ty_n(ty)
@@ -269,8 +270,8 @@ struct ConvTiles {
     {
         ConvTile t;
         t.b = b;
-        t.y0 = y * CONV_TY;
-        t.x0 = x * CONV_TX;
+        t.y0 = y * TY;
+        t.x0 = x * TX;
         return t;
     }
     __device__ __forceinline__ void next()
@@ -314,13 +315,30 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi)
     return *reinterpret_cast<const unsigned *>(&p);
 }
 
+/* v with the halves zeroed where m's bf16 half is not above zero (the ReLU
+ * mask), the kept values added to s0 (low half) and s1 */
+__device__ __forceinline__ unsigned mask_bf16(unsigned v, unsigned m, float &s0, float &s1)
+{
+    if (!(__uint_as_float(m << 16) > 0.0f))
+        v &= 0xffff0000u;
+    if (!(__uint_as_float(m & 0xffff0000u) > 0.0f))
+        v &= 0x0000ffffu;
+    s0 += __uint_as_float(v << 16);
+    s1 += __uint_as_float(v & 0xffff0000u);
+    return v;
+}
+
 /* Epilogue of a warp's 32 pixels (its TMEM lanes; columns tcol ..): bias and
  * ReLU in fp32, bf16 rounding, then through the warp's staging buffer so that
  * 8 neighbouring output pixels leave as one 512-byte store.  Tile row r (8
- * pixels) goes to output row oy0 + r * osy, columns ox0 + x * osx. */
+ * pixels) goes to output row oy0 + r * osy, columns ox0 + x * osx.  GRAD: the
+ * values are an input gradient; they are masked by the layer's ReLU output
+ * a.mask on the way out and summed over the pixels (its bias gradient), lane
+ * l holding channels 8 (l % 4) .. in db. */
+template <bool GRAD>
 __device__ __forceinline__ void conv_epilogue(const hl_conv_args &a, unsigned tcol,
                                               unsigned char *stage, const float *bias, int bimg,
-                                              int oy0, int ox0, int osy, int osx)
+                                              int oy0, int ox0, int osy, int osx, float (&db)[8])
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float v[32];
@@ -367,14 +385,42 @@ __device__ __forceinline__ void conv_epilogue(const hl_conv_args &a, unsigned tc
 #pragma unroll
     for (int it = 0; it < 4; it++) {
         const int p = it * 8 + x;
-        const uint4 o = *reinterpret_cast<const uint4 *>(stage + p * 64 +
-                                                         ((q ^ ((p >> 1) & 3)) << 4));
+        uint4 o = *reinterpret_cast<const uint4 *>(stage + p * 64 + ((q ^ ((p >> 1) & 3)) << 4));
         const int oy = oy0 + (4 * warp + it) * osy;
-        if (oy < a.Ho && ox < a.Wo)
-            *reinterpret_cast<uint4 *>(a.y + (((size_t)bimg * a.Ho + oy) * a.Wo + ox) * 32 +
-                                       q * 8) = o;
+        if (oy < a.Ho && ox < a.Wo) {
+            const size_t at = (((size_t)bimg * a.Ho + oy) * a.Wo + ox) * 32 + q * 8;
+            if (GRAD) {
+                const uint4 m = *reinterpret_cast<const uint4 *>(a.mask + at);
+                o.x = mask_bf16(o.x, m.x, db[0], db[1]);
+                o.y = mask_bf16(o.y, m.y, db[2], db[3]);
+                o.z = mask_bf16(o.z, m.z, db[4], db[5]);
+                o.w = mask_bf16(o.w, m.w, db[6], db[7]);
+            }
+            *reinterpret_cast<uint4 *>(a.y + at) = o;
+        }
     }
     __syncwarp();
+}
+
+/* the CTA's bias-gradient sums (conv_epilogue's db) added to its copy of a.db:
+ * lanes, then warps (s: 4 x 32 floats), then one 32-channel reduction */
+__device__ __forceinline__ void conv_add_db(const hl_conv_args &a, float (&db)[8], float *s)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1)
+            db[j] += __shfl_xor_sync(FULL, db[j], o);
+    __syncthreads();
+    if (lane < 4)
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            s[warp * 32 + lane * 8 + j] = db[j];
+    __syncthreads();
+    if (warp == 0 && lane < a.cout)
+        atomicAdd(a.db + (size_t)(blockIdx.x % HL_GRAD_COPIES) * a.db_stride + lane,
+                  (s[lane] + s[32 + lane]) + (s[64 + lane] + s[96 + lane]));
 }
 
 /* 32 input channels.  What bounds it: shared memory -- the tensor cores read
@@ -385,10 +431,11 @@ __device__ __forceinline__ void conv_epilogue(const hl_conv_args &a, unsigned tc
  * images of 64 x 64, stride 1, ncu: 15.5 us a launch, against 55.0 us when
  * every tap was gathered into an im2col tile; stride 2 (bound by the 67 MB it
  * reads) 28.9 against 55.5, one-channel output 12.9 against 41.5. */
-template <int N, int MODE>
+template <int N, int MODE, bool GRAD>
 __global__ void __launch_bounds__(CNN_THREADS)
 hl_conv32_kernel(hl_conv_args a)
 {
+    float db[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     using H = ConvHalo<MODE>;
     constexpr int KG = 36;
     extern __shared__ __align__(128) unsigned char conv_raw[];
@@ -443,7 +490,7 @@ hl_conv32_kernel(hl_conv_args a)
 
     unsigned phase = 0, st = 0;
     bool failed = false;
-    ConvTiles walk(tx_n, ty_n);
+    ConvTiles<CONV_TX, CONV_TY> walk(tx_n, ty_n);
     ConvTile cur = walk.get();
     if ((int)blockIdx.x < ntiles)
         load(cur, 0);
@@ -515,10 +562,12 @@ hl_conv32_kernel(hl_conv_args a)
         if (MODE == CONV_T2) {
 #pragma unroll 1
             for (int cls = 0; cls < 4; cls++)
-                conv_epilogue(a, tmem + (unsigned)(cls * 32), sm.out[tid >> 5], sm.bias, cur.b,
-                              2 * cur.y0 + (cls >> 1), 2 * cur.x0 + (cls & 1), 2, 2);
+                conv_epilogue<GRAD>(a, tmem + (unsigned)(cls * 32), sm.out[tid >> 5], sm.bias,
+                                    cur.b, 2 * cur.y0 + (cls >> 1), 2 * cur.x0 + (cls & 1), 2, 2,
+                                    db);
         } else {
-            conv_epilogue(a, tmem, sm.out[tid >> 5], sm.bias, cur.b, cur.y0, cur.x0, 1, 1);
+            conv_epilogue<GRAD>(a, tmem, sm.out[tid >> 5], sm.bias, cur.b, cur.y0, cur.x0, 1, 1,
+                                db);
         }
         cur = nt;
         /* TMEM reads done before the next tile's MMAs (ordered by the
@@ -530,6 +579,8 @@ hl_conv32_kernel(hl_conv_args a)
          * more (bounded) so no MMA still writes the TMEM being released */
         cnn_mbar_wait(&sm.bar, phase ^ 1u);
     }
+    if (GRAD)
+        conv_add_db(a, db, reinterpret_cast<float *>(sm.out));
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     if (tid < 32)
@@ -541,9 +592,11 @@ hl_conv32_kernel(hl_conv_args a)
  * values are loaded behind the MMA.  Bound by its epilogue's instructions and
  * the output's 64 bytes a pixel: 64 maps of 256 x 256, stride 2, 23.8 us
  * (46.6 us before). */
+template <bool GRAD>
 __global__ void __launch_bounds__(CNN_THREADS)
 hl_conv1_kernel(hl_conv_args a)
 {
+    float db[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     constexpr int KG = 2, N = 32;
     extern __shared__ __align__(128) unsigned char conv_raw[];
     typedef ConvSmem<KG, N, CNN_TILE_M * 32> Smem;
@@ -579,7 +632,7 @@ hl_conv1_kernel(hl_conv_args a)
     };
     unsigned phase = 0;
     bool failed = false;
-    ConvTiles walk(tx_n, ty_n);
+    ConvTiles<CONV_TX, CONV_TY> walk(tx_n, ty_n);
     ConvTile cur = walk.get();
     if ((int)blockIdx.x < ntiles)
         gather(cur);
@@ -614,12 +667,14 @@ hl_conv1_kernel(hl_conv_args a)
                 atomicOr(a.status, HL_ST_CNN_TIMEOUT);
             continue;
         }
-        conv_epilogue(a, tmem, sm.out[tid >> 5], sm.bias, cur.b, cur.y0, cur.x0, 1, 1);
+        conv_epilogue<GRAD>(a, tmem, sm.out[tid >> 5], sm.bias, cur.b, cur.y0, cur.x0, 1, 1, db);
         cur = nt;
         tmem_fence_before();
     }
     if (failed)
         cnn_mbar_wait(&sm.bar, phase ^ 1u);   /* as in hl_conv32_kernel */
+    if (GRAD)
+        conv_add_db(a, db, reinterpret_cast<float *>(sm.out));
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     if (tid < 32)
@@ -643,7 +698,7 @@ static cudaError_t launch_conv(K kernel, size_t smem, long long ntiles, int ctas
     return hl_launch_pdl(kernel, dim3(grid), dim3(CNN_THREADS), smem, s, false, *a);
 }
 
-template <int N, int MODE>
+template <int N, int MODE, bool GRAD>
 static cudaError_t launch_conv32(const hl_conv_args *a, cudaStream_t s)
 {
     typedef ConvHalo<MODE> H;
@@ -651,25 +706,33 @@ static cudaError_t launch_conv32(const hl_conv_args *a, cudaStream_t s)
     const int ex = MODE == CONV_T2 ? a->W : a->Wo, ey = MODE == CONV_T2 ? a->H : a->Ho;
     const long long nt = (long long)a->B * ((ex + CONV_TX - 1) / CONV_TX) *
                          ((ey + CONV_TY - 1) / CONV_TY);
-    return launch_conv(hl_conv32_kernel<N, MODE>, sizeof(Smem), nt, H::CTAS, a, s);
+    return launch_conv(hl_conv32_kernel<N, MODE, GRAD>, sizeof(Smem), nt, H::CTAS, a, s);
 }
 
 cudaError_t hl_launch_conv3x3(const hl_conv_args *a, int mode, cudaStream_t s)
 {
+    const bool grad = a->mask != nullptr;   /* an input gradient of the network */
     if (a->cin == 1 && a->cout <= 32 && mode == 0) {
         const long long nt = (long long)a->B * ((a->Wo + CONV_TX - 1) / CONV_TX) *
                              ((a->Ho + CONV_TY - 1) / CONV_TY);
-        return launch_conv(hl_conv1_kernel, sizeof(ConvSmem<2, 32, CNN_TILE_M * 32>), nt, 8, a, s);
+        const size_t smem = sizeof(ConvSmem<2, 32, CNN_TILE_M * 32>);
+        return grad ? launch_conv(hl_conv1_kernel<true>, smem, nt, 8, a, s)
+                    : launch_conv(hl_conv1_kernel<false>, smem, nt, 8, a, s);
     }
     if (a->cin != 32 || a->cout > 32)
         return cudaErrorInvalidValue;
     if (mode == 1)
-        return launch_conv32<32, CONV_T2>(a, s);
+        return grad ? launch_conv32<32, CONV_T2, true>(a, s)
+                    : launch_conv32<32, CONV_T2, false>(a, s);
     if (mode != 0)
         return cudaErrorInvalidValue;
     if (a->stride == 2)
-        return a->cout <= 16 ? launch_conv32<16, CONV_S2>(a, s) : launch_conv32<32, CONV_S2>(a, s);
-    return a->cout <= 16 ? launch_conv32<16, CONV_S1>(a, s) : launch_conv32<32, CONV_S1>(a, s);
+        return a->cout <= 16 ? launch_conv32<16, CONV_S2, false>(a, s)
+                             : launch_conv32<32, CONV_S2, false>(a, s);
+    if (grad)
+        return launch_conv32<32, CONV_S1, true>(a, s);
+    return a->cout <= 16 ? launch_conv32<16, CONV_S1, false>(a, s)
+                         : launch_conv32<32, CONV_S1, false>(a, s);
 }
 
 /* ---- occupancy pooling ---------------------------------------------------- */
@@ -715,129 +778,364 @@ cudaError_t hl_launch_pool(const hl_pool_img *imgs, int nimg, int side,
     return cudaGetLastError();
 }
 
-/* ---- weight and bias gradients (CUDA cores, FP32) ------------------------ */
+/* ---- weight gradients ------------------------------------------------------ */
 
-/* dw[co][tap * cin + ci] += sum over pixels of dy[p][co] * x[in(p, tap)][ci].
- * Thread (tap, ci) keeps 32 accumulators (one per co); a CTA walks chunks of
- * DW_CHUNK output pixels grid-stride, with the chunk's dy rows in shared
- * memory, and adds its sums into dw once at the end.  dy: [P][32] f32 (the
- * output gradient after the ReLU mask), x: bf16 NHWC with cin channels
- * (32-channel rows for cin = 32, one value for cin = 1). */
-#define DW_CHUNK 64
-__global__ void __launch_bounds__(288)
-hl_conv_dw_kernel(hl_dw_args a)
+/* dw[co][tap][ci] += sum over output pixels p of dy[p][co] * x[in(p, tap)][ci]:
+ * a GEMM whose contraction runs over the pixels, K = 16 neighbouring pixels of
+ * a row an MMA, both operands MN-major (a core matrix is 8 pixels x 8 channels,
+ * the same 128 bytes as in the convolutions).
+ *   A (M = 128): the x halo as rows of four channel planes; row group
+ *     4 ky + q of a pixel row is plane q of the halo row ky further down, all
+ *     one plane row apart, so one descriptor holds three ky x 32 channels
+ *     (rows 0..95; rows 96..127 run into the row after and are not read
+ *     back).  kx is a start address, with its own accumulator.
+ *   B: dy, N = 32 channels -- or, for the one-channel FP32 gradient, N = 16
+ *     with dy split exactly into three bf16 pieces (columns 0..2), whose sums
+ *     are added at the end.
+ * dy of the 32-channel layers is bf16 already, so the products are exact.  The
+ * tensor cores truncate their FP32 sums, which over hundreds of additions
+ * outgrows the rounding of FP32 fused multiply-adds (measured against 64 bits:
+ * up to 2e-6 where those had 4e-7), so an accumulator takes DW_SEQ MMAs only
+ * and is then added, rounded to nearest, to a thread's register sums (1.3e-7
+ * to 4e-7, at or below the FP32 kernel's).  Bound by the copies into shared
+ * memory and the MMAs' reads of A.  32 maps: 64 x 64 x 32 layers 12.8 us a
+ * launch, the stride-2 layer 18, the input layer 19, the one-channel output 11,
+ * where FP32 multiply-adds took 222, 222, 400 and 210. */
+#define DW_SEQ 4       /* MMAs (rows of 16 pixels) an accumulator takes */
+#define DW_SETS (DW_TY / DW_SEQ)
+#define DW_TX 16
+#define DW_TY 8
+template <int STRIDE> struct DwHalo;
+template <> struct DwHalo<1> {
+    /* 10 rows of 18 pixels, one more row for the unused row groups */
+    static constexpr int COLS = 18, ROWS = 10, P = 288, HALF = 0, BYTES = 11 * 4 * 288;
+};
+template <> struct DwHalo<2> {
+    /* 17 rows of 33 pixels, even and odd columns apart (64 bytes off each
+     * other's banks) */
+    static constexpr int COLS = 33, ROWS = 17, P = 272, HALF = 18 * 4 * 272 + 64,
+                         BYTES = 2 * (18 * 4 * 272 + 64);
+};
+#define DW_DYP 288     /* plane row of the dy tile: 16 pixels and 32 bytes of padding */
+
+template <int XBYTES, int DYG>
+struct DwSmem {
+    alignas(128) unsigned char x[2][(XBYTES + 127) / 128 * 128];
+    alignas(128) unsigned char dy[2][DW_TY * DYG * DW_DYP];
+    unsigned long long bar;
+    unsigned tmem;
+};
+
+/* D f32, A and B bf16, both MN-major */
+__host__ __device__ constexpr unsigned mma_idesc_mn(int M, int N)
 {
-    __shared__ float s_dy[DW_CHUNK][32];
-    const int t = threadIdx.x;
-    const int tap = t / 32 < 9 ? t / 32 : 8, ci = t % 32;
-    const bool act = t < 9 * a.cin;   /* cin = 1: threads 0..8 (ci = t) */
-    const int my_tap = a.cin == 32 ? tap : t, my_ci = a.cin == 32 ? ci : 0;
-    const int ky = my_tap / 3, kx = my_tap % 3;
-    float acc[32];
+    return mma_idesc(M, N) | (1u << 15) | (1u << 16);
+}
+
+/* copies of a dy tile: 16 x 8 pixels, four planes a row, zero past the map */
+__device__ __forceinline__ void dw_load_dy(const hl_dw_args &a, const ConvTile &t, unsigned dst)
+{
+    const int q = threadIdx.x & 3;
+    for (int px = threadIdx.x >> 2; px < DW_TX * DW_TY; px += CNN_THREADS / 4) {
+        const int y = px / DW_TX, x = px % DW_TX;
+        const bool ok = t.y0 + y < a.Ho && t.x0 + x < a.Wo;
+        const __nv_bfloat16 *src =
+            ok ? a.dy + (((size_t)t.b * a.Ho + t.y0 + y) * a.Wo + t.x0 + x) * 32 + q * 8 : a.dy;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                     ::"r"(dst + (unsigned)((y * 4 + q) * DW_DYP + x * 16)), "l"(src),
+                     "r"(ok ? 16 : 0)
+                     : "memory");
+    }
+}
+
+template <int STRIDE, bool SPLIT>
+__global__ void __launch_bounds__(CNN_THREADS)
+hl_dw32_kernel(hl_dw_args a)
+{
+    using H = DwHalo<STRIDE>;
+    constexpr int DYG = SPLIT ? 2 : 4;
+    constexpr int N = SPLIT ? 16 : 32;
+    extern __shared__ __align__(128) unsigned char conv_raw[];
+    typedef DwSmem<H::BYTES, DYG> Smem;
+    Smem &sm = *reinterpret_cast<Smem *>(conv_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned tmem = conv_begin(&sm.tmem, &sm.bar, 256);
+    hl_pdl_begin();
+    const int tx_n = (a.Wo + DW_TX - 1) / DW_TX, ty_n = (a.Ho + DW_TY - 1) / DW_TY;
+    const int ntiles = a.B * tx_n * ty_n;
+    const unsigned xbase = cnn_smem_u32(sm.x[0]), dybase = cnn_smem_u32(sm.dy[0]);
+    constexpr unsigned XST = sizeof(sm.x[0]), DYST = sizeof(sm.dy[0]);
+
+    auto load = [&](const ConvTile &t, unsigned st) {
+        const int iy0 = t.y0 * STRIDE - 1, ix0 = t.x0 * STRIDE - 1;
+        const int q = tid & 3;
+        const __nv_bfloat16 *x = a.x + (size_t)t.b * a.H * a.W * 32 + q * 8;
+        int hy = (tid >> 2) / H::COLS, hx = (tid >> 2) % H::COLS;
+        for (int px = tid >> 2; px < H::ROWS * H::COLS; px += CNN_THREADS / 4) {
+            const int iy = iy0 + hy, ix = ix0 + hx;
+            const bool ok = (unsigned)iy < (unsigned)a.H && (unsigned)ix < (unsigned)a.W;
+            const __nv_bfloat16 *src = ok ? x + (size_t)(iy * a.W + ix) * 32 : a.x;
+            const unsigned dst =
+                xbase + st * XST + (unsigned)((hy * 4 + q) * H::P) +
+                (STRIDE == 2 ? (unsigned)((hx & 1) * H::HALF + (hx >> 1) * 16)
+                             : (unsigned)(hx * 16));
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                         ::"r"(dst), "l"(src), "r"(ok ? 16 : 0)
+                         : "memory");
+            hx += 32 % H::COLS;
+            hy += 32 / H::COLS;
+            if (hx >= H::COLS) {
+                hx -= H::COLS;
+                hy++;
+            }
+        }
+        if (!SPLIT) {
+            dw_load_dy(a, t, dybase + st * DYST);
+        } else {
+            /* one pixel a thread: f = hi + mid + lo exactly (24 bits in three
+             * pieces of 8); an infinity or NaN stays in hi alone */
+            const int y = tid / DW_TX, xx = tid % DW_TX;
+            const bool ok = t.y0 + y < a.Ho && t.x0 + xx < a.Wo;
+            const float f =
+                ok ? a.dy_f32[((size_t)t.b * a.Ho + t.y0 + y) * a.Wo + t.x0 + xx] : 0.0f;
+            const __nv_bfloat16 hi = __float2bfloat16(f);
+            float r = __fsub_rn(f, __bfloat162float(hi));
+            r = fabsf(f) < 3.0e38f ? r : 0.0f;
+            const __nv_bfloat16 mid = __float2bfloat16(r);
+            const __nv_bfloat16 lo = __float2bfloat16(__fsub_rn(r, __bfloat162float(mid)));
+            unsigned char *d = sm.dy[st] + (y * 2) * DW_DYP + xx * 16;
+            *reinterpret_cast<uint4 *>(d) = make_uint4(
+                (unsigned)__bfloat16_as_ushort(hi) | ((unsigned)__bfloat16_as_ushort(mid) << 16),
+                (unsigned)__bfloat16_as_ushort(lo), 0u, 0u);
+            *reinterpret_cast<uint4 *>(d + DW_DYP) = make_uint4(0u, 0u, 0u, 0u);
+        }
+    };
+
+    ConvTiles<DW_TX, DW_TY> walk(tx_n, ty_n);
+    float acc[3][SPLIT ? 1 : 32];   /* warp = ky, lane = ci: this thread's sums */
+#pragma unroll
+    for (int kx = 0; kx < 3; kx++)
+#pragma unroll
+        for (int c = 0; c < (SPLIT ? 1 : 32); c++)
+            acc[kx][c] = 0.0f;
+    bool failed = false;
+    unsigned it = 0;
+    if ((int)blockIdx.x < ntiles)
+        load(walk.get(), 0);
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
+        const unsigned st = it & 1u;
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (__syncthreads_or(failed))
+            break;
+        if (tid < 32 && elect_one()) {
+            tmem_fence_after();
+            const unsigned long long ad0 = smem_desc(xbase + st * XST, 128, H::P);
+            const unsigned long long bd0 = smem_desc(dybase + st * DYST, 128, DW_DYP);
+#pragma unroll
+            for (int y = 0; y < DW_TY; y++)
+#pragma unroll
+                for (int kx = 0; kx < 3; kx++) {
+                    const unsigned off =
+                        (unsigned)(y * STRIDE * 4 * H::P) +
+                        (STRIDE == 2 ? (unsigned)((kx & 1) * H::HALF + (kx >> 1) * 16)
+                                     : (unsigned)(kx * 16));
+                    umma_f16(tmem + (unsigned)((y / DW_SEQ * 3 + kx) * 32), ad0 + (off >> 4),
+                             bd0 + (unsigned)(y * DYG * DW_DYP >> 4),
+                             mma_idesc_mn(CNN_TILE_M, N), y % DW_SEQ > 0);
+                }
+            umma_commit(&sm.bar);
+        }
+        __syncwarp();
+        /* the other buffer's MMAs were waited for in the round before */
+        if (tile + (int)gridDim.x < ntiles) {
+            walk.next();
+            load(walk.get(), st ^ 1u);
+        }
+        if (!cnn_mbar_wait(&sm.bar, it & 1u)) {
+            failed = true;
+            if (lane == 0)
+                atomicOr(a.status, HL_ST_CNN_TIMEOUT);
+            continue;
+        }
+        tmem_fence_after();
+        if (warp < 3) {   /* rows 32 ky + ci of every accumulator */
+#pragma unroll
+            for (int set = 0; set < DW_SETS; set++)
+#pragma unroll
+                for (int kx = 0; kx < 3; kx++) {
+                    float v[32];
+                    tmem_ld32(tmem + ((unsigned)(32 * warp) << 16) +
+                                  (unsigned)((set * 3 + kx) * 32), v);
+                    if (SPLIT) {
+                        acc[kx][0] += v[0] + (v[1] + v[2]);
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < (SPLIT ? 1 : 32); c++)
+                            acc[kx][c] += v[c];
+                    }
+                }
+        }
+        tmem_fence_before();
+    }
+    if (failed)
+        cnn_mbar_wait(&sm.bar, it & 1u);   /* as in hl_conv32_kernel */
+    if (!__syncthreads_or(failed) && it > 0 && warp < 3) {
+#pragma unroll
+        for (int kx = 0; kx < 3; kx++) {
+            float *dst = a.dw + (size_t)(blockIdx.x % HL_GRAD_COPIES) * a.dw_stride +
+                         (warp * 3 + kx) * 32 + lane;
+#pragma unroll
+            for (int c = 0; c < (SPLIT ? 1 : 32); c++)
+                atomicAdd(dst + c * 288, acc[kx][c]);
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    tmem_fence_before();
+    __syncthreads();
+    if (tid < 32)
+        tmem_dealloc(tmem, 256);
+}
+
+/* One input channel (stride 1 or 2): A's rows are the 9 taps, two 8-tap
+ * groups a pixel gathered by its thread; the row groups past them run into the
+ * rows after (14 spare plane rows at the end) and are not read back. */
+#define DW1_X ((DW_TY * 2 + 14) * DW_DYP)
+__global__ void __launch_bounds__(CNN_THREADS)
+hl_dw1_kernel(hl_dw_args a)
+{
+    extern __shared__ __align__(128) unsigned char conv_raw[];
+    typedef DwSmem<DW1_X, 4> Smem;
+    Smem &sm = *reinterpret_cast<Smem *>(conv_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned tmem = conv_begin(&sm.tmem, &sm.bar, 64);
+    hl_pdl_begin();
+    const int tx_n = (a.Wo + DW_TX - 1) / DW_TX, ty_n = (a.Ho + DW_TY - 1) / DW_TY;
+    const int ntiles = a.B * tx_n * ty_n;
+    const unsigned xbase = cnn_smem_u32(sm.x[0]), dybase = cnn_smem_u32(sm.dy[0]);
+    constexpr unsigned XST = sizeof(sm.x[0]), DYST = sizeof(sm.dy[0]);
+    const int py = tid / DW_TX, px = tid % DW_TX;   /* the thread's pixel */
+
+    auto load = [&](const ConvTile &t, unsigned st) {
+        dw_load_dy(a, t, dybase + st * DYST);
+        const int iy0 = (t.y0 + py) * a.stride - 1, ix0 = (t.x0 + px) * a.stride - 1;
+        const unsigned short *x =
+            reinterpret_cast<const unsigned short *>(a.x) + (size_t)t.b * a.H * a.W;
+        unsigned short v[9];
+#pragma unroll
+        for (int ky = 0; ky < 3; ky++) {
+            const bool oky = (unsigned)(iy0 + ky) < (unsigned)a.H;
+            const unsigned short *row = x + (ptrdiff_t)(iy0 + ky) * a.W + ix0;
+#pragma unroll
+            for (int kx = 0; kx < 3; kx++)
+                v[3 * ky + kx] = oky && (unsigned)(ix0 + kx) < (unsigned)a.W ? row[kx]
+                                                                             : (unsigned short)0;
+        }
+        unsigned char *d = sm.x[st] + (py * 2) * DW_DYP + px * 16;
+        *reinterpret_cast<uint4 *>(d) =
+            make_uint4(v[0] | ((unsigned)v[1] << 16), v[2] | ((unsigned)v[3] << 16),
+                       v[4] | ((unsigned)v[5] << 16), v[6] | ((unsigned)v[7] << 16));
+        *reinterpret_cast<uint4 *>(d + DW_DYP) = make_uint4(v[8], 0u, 0u, 0u);
+    };
+
+    ConvTiles<DW_TX, DW_TY> walk(tx_n, ty_n);
+    float acc[32];   /* warp 0, lane = tap: this thread's sums */
 #pragma unroll
     for (int c = 0; c < 32; c++)
         acc[c] = 0.0f;
-    const int HWo = a.Ho * a.Wo;
-    const long long P = (long long)a.B * HWo;
-    for (long long p0 = (long long)blockIdx.x * DW_CHUNK; p0 < P;
-         p0 += (long long)gridDim.x * DW_CHUNK) {
-        for (int e = t; e < DW_CHUNK * 32; e += blockDim.x) {
-            const long long p = p0 + e / 32;
-            s_dy[e / 32][e % 32] =
-                (p < P && (e % 32) < a.dy_c) ? a.dy[p * a.dy_c + (e % 32)] : 0.0f;
+    bool failed = false;
+    unsigned it = 0;
+    if ((int)blockIdx.x < ntiles)
+        load(walk.get(), 0);
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
+        const unsigned st = it & 1u;
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (__syncthreads_or(failed))
+            break;
+        if (tid < 32 && elect_one()) {
+            tmem_fence_after();
+            const unsigned long long ad0 = smem_desc(xbase + st * XST, 128, DW_DYP);
+            const unsigned long long bd0 = smem_desc(dybase + st * DYST, 128, DW_DYP);
+#pragma unroll
+            for (int y = 0; y < DW_TY; y++)
+                umma_f16(tmem + (unsigned)(y / DW_SEQ * 32), ad0 + (unsigned)(y * 2 * DW_DYP >> 4),
+                         bd0 + (unsigned)(y * 4 * DW_DYP >> 4), mma_idesc_mn(CNN_TILE_M, 32),
+                         y % DW_SEQ > 0);
+            umma_commit(&sm.bar);
         }
-        __syncthreads();
-        if (act) {
-            for (int q = 0; q < DW_CHUNK; q++) {
-                const long long p = p0 + q;
-                if (p >= P)
-                    break;
-                const int b = (int)(p / HWo), r = (int)(p % HWo);
-                const int oy = r / a.Wo, ox = r % a.Wo;
-                const int iy = oy * a.stride - 1 + ky, ix = ox * a.stride - 1 + kx;
-                float xv = 0.0f;
-                if (iy >= 0 && ix >= 0 && iy < a.H && ix < a.W)
-                    xv = __bfloat162float(
-                        a.x[(((size_t)b * a.H + iy) * a.W + ix) * a.cin + my_ci]);
+        __syncwarp();
+        if (tile + (int)gridDim.x < ntiles) {
+            walk.next();
+            load(walk.get(), st ^ 1u);
+        }
+        if (!cnn_mbar_wait(&sm.bar, it & 1u)) {
+            failed = true;
+            if (lane == 0)
+                atomicOr(a.status, HL_ST_CNN_TIMEOUT);
+            continue;
+        }
+        tmem_fence_after();
+        if (warp == 0) {
+#pragma unroll
+            for (int set = 0; set < DW_SETS; set++) {
+                float v[32];
+                tmem_ld32(tmem + (unsigned)(set * 32), v);
 #pragma unroll
                 for (int c = 0; c < 32; c++)
-                    acc[c] = fmaf(s_dy[q][c], xv, acc[c]);
+                    acc[c] += v[c];
             }
         }
-        __syncthreads();
+        tmem_fence_before();
     }
-    if (act) {
-        const int kreal = 9 * a.cin;
-        const int k = my_tap * a.cin + my_ci;
-        for (int c = 0; c < a.cout; c++)
-            atomicAdd(&a.dw[(size_t)c * kreal + k], acc[c]);
+    if (failed)
+        cnn_mbar_wait(&sm.bar, it & 1u);   /* as in hl_conv32_kernel */
+    if (!__syncthreads_or(failed) && it > 0 && warp == 0 && lane < 9) {
+#pragma unroll
+        for (int co = 0; co < 32; co++)
+            atomicAdd(a.dw + (size_t)(blockIdx.x % HL_GRAD_COPIES) * a.dw_stride + co * 9 + lane,
+                      acc[co]);
     }
-}
-
-/* db[c] += sum over pixels of dy[p][c] (dy rows of dy_c values) */
-__global__ void hl_bias_grad_kernel(const float *dy, int dy_c, long long P, int cout,
-                                    float *db)
-{
-    __shared__ float s[32][33];
-    const int c = threadIdx.x & 31, row = threadIdx.x >> 5;   /* 256 threads */
-    float acc = 0.0f;
-    if (c < dy_c)
-        for (long long p = (long long)blockIdx.x * 8 + row; p < P;
-             p += (long long)gridDim.x * 8)
-            acc += dy[p * dy_c + c];
-    s[row][c] = acc;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    tmem_fence_before();
     __syncthreads();
-    if (threadIdx.x < 32) {
-        float t = 0.0f;
-        for (int r = 0; r < 8; r++)
-            t += s[r][threadIdx.x];
-        if (threadIdx.x < cout)
-            atomicAdd(&db[threadIdx.x], t);
-    }
+    if (tid < 32)
+        tmem_dealloc(tmem, 64);
 }
 
-cudaError_t hl_launch_conv_dw(const hl_dw_args *a, cudaStream_t s)
+template <typename K>
+static cudaError_t launch_dw(K kernel, size_t smem, int ctas_per_sm, const hl_dw_args *a,
+                             cudaStream_t s)
 {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long P = (long long)a->B * a->Ho * a->Wo;
-    const int chunks = (int)((P + DW_CHUNK - 1) / DW_CHUNK);
-    hl_conv_dw_kernel<<<std::max(1, std::min(chunks, sms * 4)), 288, 0, s>>>(*a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || !a->db)
+    const cudaError_t e =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess)
         return e;
-    const int blocks = (int)std::max(1LL, std::min((P + 7) / 8, (long long)sms * 4));
-    hl_bias_grad_kernel<<<blocks, 256, 0, s>>>(a->dy, a->dy_c, P, a->cout, a->db);
-    return cudaGetLastError();
+    const long long nt = (long long)a->B * ((a->Wo + DW_TX - 1) / DW_TX) *
+                         ((a->Ho + DW_TY - 1) / DW_TY);
+    if (nt > 0x7fffffffLL)
+        return cudaErrorInvalidValue;
+    const int grid = (int)std::max(1LL, std::min(nt, (long long)sms * ctas_per_sm));
+    return hl_launch_pdl(kernel, dim3(grid), dim3(CNN_THREADS), smem, s, false, *a);
 }
 
-/* dy (bf16 NHWC 32) * [y > 0] -> f32 [P][32] and a bf16 copy (the next
- * backward convolution's operand); y is the layer's ReLU output.  For a
- * one-channel gradient (dy32 == NULL): g [P] f32 -> bf16 [P]. */
-__global__ void hl_relu_mask_kernel(const __nv_bfloat16 *dx, const __nv_bfloat16 *y,
-                                    long long n, float *out_f32,
-                                    __nv_bfloat16 *out_bf16)
+cudaError_t hl_launch_conv_dw(const hl_dw_args *a, cudaStream_t s)
 {
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n;
-         e += (long long)gridDim.x * blockDim.x) {
-        float g = __bfloat162float(dx[e]);
-        if (y && !(__bfloat162float(y[e]) > 0.0f))
-            g = 0.0f;
-        if (out_f32)
-            out_f32[e] = g;
-        if (out_bf16)
-            out_bf16[e] = __float2bfloat16(g);
-    }
-}
-
-cudaError_t hl_launch_relu_mask(const __nv_bfloat16 *dx, const __nv_bfloat16 *y,
-                                long long n, float *out_f32,
-                                __nv_bfloat16 *out_bf16, cudaStream_t s)
-{
-    const int blocks = (int)std::max(1LL, std::min((n + 255) / 256, 8192LL));
-    hl_relu_mask_kernel<<<blocks, 256, 0, s>>>(dx, y, n, out_f32, out_bf16);
-    return cudaGetLastError();
+    if (a->cin == 1 && a->dy)
+        return launch_dw(hl_dw1_kernel, sizeof(DwSmem<DW1_X, 4>), 3, a, s);
+    if (a->cin != 32)
+        return cudaErrorInvalidValue;
+    if (!a->dy)
+        return a->stride == 1 ? launch_dw(hl_dw32_kernel<1, true>,
+                                          sizeof(DwSmem<DwHalo<1>::BYTES, 2>), 2, a, s)
+                              : cudaErrorInvalidValue;
+    return a->stride == 2 ? launch_dw(hl_dw32_kernel<2, false>,
+                                      sizeof(DwSmem<DwHalo<2>::BYTES, 4>), 2, a, s)
+                          : launch_dw(hl_dw32_kernel<1, false>,
+                                      sizeof(DwSmem<DwHalo<1>::BYTES, 4>), 2, a, s);
 }
 
 /* ---- coarse Hough head ------------------------------------------------------ */
@@ -1034,24 +1332,29 @@ hl_head_fwd_kernel(const float *e, const hl_head_geom *geo,
 }
 
 /* de[b][cell] = alpha * sum_t dz[b][t][bin(cell, t)] (the gather transpose of
- * the head); one CTA per (image, 512 cells), each thread one cell summing its
- * angles in order */
+ * the head), its bf16 copy (the next convolution's operand) and its sum (the
+ * last layer's bias gradient); one CTA per (image, 512 cells), each thread one
+ * cell summing its angles in order */
 __global__ void __launch_bounds__(512)
 hl_head_bwd_kernel(const float *dz, int ev, const hl_head_geom *geo,
-                   const float *ab, float *de, HeadTrig tr)
+                   const float *ab, float *de, __nv_bfloat16 *de_b, float *db, int db_stride,
+                   HeadTrig tr)
 {
+    __shared__ float s_tot[16];
     __shared__ float sd[HL_HEAD_T * HL_HEAD_R];
     __shared__ float cs[HL_HEAD_T], sn[HL_HEAD_T];
     const int b = blockIdx.y;
-    for (int i = threadIdx.x; i < HL_HEAD_T * HL_HEAD_R; i += blockDim.x)
-        sd[i] = dz[(size_t)b * HL_HEAD_T * HL_HEAD_R + i];
     if (threadIdx.x < HL_HEAD_T) {
         cs[threadIdx.x] = tr.c[threadIdx.x];
         sn[threadIdx.x] = tr.s[threadIdx.x];
     }
+    hl_pdl_begin();
+    for (int i = threadIdx.x; i < HL_HEAD_T * HL_HEAD_R; i += blockDim.x)
+        sd[i] = dz[(size_t)b * HL_HEAD_T * HL_HEAD_R + i];
     __syncthreads();
     const hl_head_geom g = geo[b];
     const float alpha = ab[0];
+    float tot = 0.0f;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < ev * ev;
          p += gridDim.x * blockDim.x) {
         const int qy = p / ev, qx = p % ev;
@@ -1059,7 +1362,21 @@ hl_head_bwd_kernel(const float *dz, int ev, const hl_head_geom *geo,
         if (qy < g.qh && qx < g.qw)
             for (int t = 0; t < HL_HEAD_T; t++)
                 acc += sd[t * HL_HEAD_R + head_bin(g, qy, qx, cs[t], sn[t])];
-        de[(size_t)b * ev * ev + p] = alpha * acc;
+        const float v = alpha * acc;
+        de[(size_t)b * ev * ev + p] = v;
+        de_b[(size_t)b * ev * ev + p] = __float2bfloat16(v);
+        tot += v;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        tot += __shfl_xor_sync(FULL, tot, o);
+    if ((threadIdx.x & 31) == 0)
+        s_tot[threadIdx.x >> 5] = tot;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 16; w++)
+            tot += s_tot[w];
+        atomicAdd(db + (size_t)((blockIdx.x + blockIdx.y) % HL_GRAD_COPIES) * db_stride, tot);
     }
 }
 
@@ -1072,11 +1389,12 @@ cudaError_t hl_launch_head_fwd(const float *e, const hl_head_geom *geo,
 }
 
 cudaError_t hl_launch_head_bwd(const float *dz, int ev, const hl_head_geom *geo,
-                               int nimg, const float *ab, float *de, cudaStream_t s)
+                               int nimg, const float *ab, float *de, __nv_bfloat16 *de_b,
+                               float *db, int db_stride, cudaStream_t s)
 {
-    hl_head_bwd_kernel<<<dim3((unsigned)((ev * ev + 511) / 512), nimg), 512, 0, s>>>(
-        dz, ev, geo, ab, de, head_trig());
-    return cudaGetLastError();
+    return hl_launch_pdl(hl_head_bwd_kernel, dim3((unsigned)((ev * ev + 511) / 512), nimg),
+                         dim3(512), 0, s, false, dz, ev, geo, ab, de, de_b, db, db_stride,
+                         head_trig());
 }
 
 /* ---- loss ------------------------------------------------------------------- */
@@ -1086,10 +1404,11 @@ cudaError_t hl_launch_head_bwd(const float *dz, int ev, const hl_head_geom *geo,
  * n; also d alpha = sum dz * hsum, d beta = sum dz and the summed loss. */
 __global__ void hl_bce_kernel(const float *z, const float *y, const float *hsum,
                               long long n, float wpos, float *dz, float *dab,
-                              float *loss)
+                              float *loss, int stride)
 {
     __shared__ float r[3][256];
     float la = 0.0f, ga = 0.0f, gb = 0.0f;
+    hl_pdl_begin();
     const float inv = 1.0f / (float)n;
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n;
          e += (long long)gridDim.x * blockDim.x) {
@@ -1116,89 +1435,78 @@ __global__ void hl_bce_kernel(const float *z, const float *y, const float *hsum,
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        atomicAdd(loss, r[0][0] * inv);
-        atomicAdd(&dab[0], r[1][0]);
-        atomicAdd(&dab[1], r[2][0]);
+        const size_t c = (size_t)(blockIdx.x % HL_GRAD_COPIES) * stride;
+        atomicAdd(loss + c, r[0][0] * inv);
+        atomicAdd(dab + c, r[1][0]);
+        atomicAdd(dab + c + 1, r[2][0]);
     }
 }
 
 cudaError_t hl_launch_bce(const float *z, const float *y, const float *hsum,
                           long long n, float wpos, float *dz, float *dab,
-                          float *loss, cudaStream_t s)
+                          float *loss, int stride, cudaStream_t s)
 {
-    hl_bce_kernel<<<256, 256, 0, s>>>(z, y, hsum, n, wpos, dz, dab, loss);
-    return cudaGetLastError();
+    return hl_launch_pdl(hl_bce_kernel, dim3(256), dim3(256), 0, s, false, z, y, hsum, n, wpos,
+                         dz, dab, loss, stride);
 }
 
 /* ---- Adam and weight layouts ---------------------------------------------- */
 
-__global__ void hl_adam_kernel(float *w, const float *g, float *m, float *v, int n,
-                               float lr, float b1, float b2, float eps, float c1,
-                               float c2, float clip)
+/* One thread per parameter: the sum of the gradient copies, the Adam update
+ * (lr > 0), then the bf16 copies of
+ * a layer's FP32 master weights [cout][9 * cin]: the forward operand (same
+ * layout) and, past the first layer, the backward one -- stride 1: flipped and
+ * transposed ([cin][8 - tap][cout], the input gradient as a convolution),
+ * stride 2: transposed ([cin][tap][cout], the input-gradient gather). */
+__global__ void hl_update_kernel(hl_update_args a)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += gridDim.x * blockDim.x) {
-        const float gi = fminf(fmaxf(g[i], -clip), clip);
-        const float mi = b1 * m[i] + (1.0f - b1) * gi;
-        const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        w[i] -= lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+    hl_pdl_begin();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.n)
+        return;
+    if (a.gsum) {   /* a step: the copies' gradient (and, last, the loss) */
+        float gs = 0.0f;
+#pragma unroll
+        for (int c = 0; c < HL_GRAD_COPIES; c++)
+            gs += a.gpart[(size_t)c * a.gstride + i];
+        a.g[i] = gs;
+        if (i == 0) {
+            float ls = 0.0f;
+#pragma unroll
+            for (int c = 0; c < HL_GRAD_COPIES; c++)
+                ls += a.gpart[(size_t)c * a.gstride + a.n];
+            a.g[a.n] = ls;
+        }
+    }
+    float w = a.w[i];
+    if (a.lr > 0.0f) {
+        const float b1 = 0.9f, b2 = 0.999f;
+        const float gi = fminf(fmaxf(a.g[i], -a.clip), a.clip);
+        const float mi = b1 * a.m[i] + (1.0f - b1) * gi;
+        const float vi = b2 * a.v[i] + (1.0f - b2) * gi * gi;
+        a.m[i] = mi;
+        a.v[i] = vi;
+        w -= a.lr * (mi * a.c1) / (sqrtf(vi * a.c2) + 1e-8f);
+        a.w[i] = w;
+    }
+    for (int l = 0; l < a.nlayers; l++) {
+        const hl_update_layer &L = a.layer[l];
+        const int r = i - L.off;
+        if (r < 0 || r >= L.cout * 9 * L.cin)
+            continue;
+        const __nv_bfloat16 v = __float2bfloat16(w);
+        L.wf[r] = v;
+        if (L.wb) {
+            const int co = r / (9 * L.cin), k = r % (9 * L.cin);
+            const int tap = k / L.cin, ci = k % L.cin;
+            L.wb[((size_t)ci * 9 + (L.flip ? 8 - tap : tap)) * L.cout + co] = v;
+        }
     }
 }
 
-cudaError_t hl_launch_adam(float *w, const float *g, float *m, float *v, int n,
-                           float lr, int step, float clip, cudaStream_t s)
+cudaError_t hl_launch_update(hl_update_args *a, int step, cudaStream_t s)
 {
-    const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = 1.0f / (1.0f - powf(b1, (float)step));
-    const float c2 = 1.0f / (1.0f - powf(b2, (float)step));
-    hl_adam_kernel<<<(n + 255) / 256, 256, 0, s>>>(w, g, m, v, n, lr, b1, b2, 1e-8f,
-                                                   c1, c2, clip);
-    return cudaGetLastError();
-}
-
-/* FP32 master weights [cout][9 * cin] -> the bf16 operand of one layer:
- * mode 0 forward (same layout), mode 1 flipped and transposed ([cin][tap][cout]
- * with tap -> 8 - tap: the stride-1 input gradient as a convolution), mode 2
- * transposed ([cin][tap][cout]: the stride-2 input-gradient gather). */
-__global__ void hl_weight_layout_kernel(const float *w, int cout, int cin, int mode,
-                                        __nv_bfloat16 *out)
-{
-    const int n = cout * 9 * cin;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += gridDim.x * blockDim.x) {
-        const int co = i / (9 * cin), r = i % (9 * cin);
-        const int tap = r / cin, ci = r % cin;
-        const float v = w[i];
-        if (mode == 0)
-            out[i] = __float2bfloat16(v);
-        else if (mode == 1)
-            out[((size_t)ci * 9 + (8 - tap)) * cout + co] = __float2bfloat16(v);
-        else
-            out[((size_t)ci * 9 + tap) * cout + co] = __float2bfloat16(v);
-    }
-}
-
-cudaError_t hl_launch_weight_layout(const float *w, int cout, int cin, int mode,
-                                    __nv_bfloat16 *out, cudaStream_t s)
-{
-    const int n = cout * 9 * cin;
-    hl_weight_layout_kernel<<<(n + 255) / 256, 256, 0, s>>>(w, cout, cin, mode, out);
-    return cudaGetLastError();
-}
-
-__global__ void hl_f32_to_bf16_kernel(const float *in, long long n, __nv_bfloat16 *out)
-{
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n;
-         e += (long long)gridDim.x * blockDim.x)
-        out[e] = __float2bfloat16(in[e]);
-}
-
-cudaError_t hl_launch_f32_to_bf16(const float *in, long long n, __nv_bfloat16 *out,
-                                  cudaStream_t s)
-{
-    const int blocks = (int)std::max(1LL, std::min((n + 255) / 256, 8192LL));
-    hl_f32_to_bf16_kernel<<<blocks, 256, 0, s>>>(in, n, out);
-    return cudaGetLastError();
+    a->c1 = 1.0f / (1.0f - powf(0.9f, (float)step));
+    a->c2 = 1.0f / (1.0f - powf(0.999f, (float)step));
+    return hl_launch_pdl(hl_update_kernel, dim3((a->n + 255) / 256), dim3(256), 0, s, false, *a);
 }

@@ -11,6 +11,11 @@
 
 #include <algorithm>
 
+/* The gradients are summed into this many copies of the flat parameters (a
+ * CTA adds to copy blockIdx % HL_GRAD_COPIES), which the update kernel adds up:
+ * hundreds of CTAs reducing into one address otherwise queue at its L2 line. */
+#define HL_GRAD_COPIES 8
+
 /* 3x3 convolution, padding 1: x [B][H][W][cin] -> y [B][Ho][Wo][cout] */
 typedef struct hl_conv_args {
     const __nv_bfloat16 *x;
@@ -26,6 +31,12 @@ typedef struct hl_conv_args {
      * stream began: they may be read while that one still runs */
     int w_ready;
     int *status;
+    /* an input gradient of the network (NULL: none): masked by the ReLU output
+     * mask (the layout of y), its sums over the pixels added to db [cout] of a
+     * gradient copy (db_stride floats apart) */
+    const __nv_bfloat16 *mask;
+    float *db;
+    int db_stride;
 } hl_conv_args;
 
 /* mode 0: convolution; mode 1: input gradient of a stride-2 convolution
@@ -33,24 +44,22 @@ typedef struct hl_conv_args {
  * size of the forward convolution) */
 cudaError_t hl_launch_conv3x3(const hl_conv_args *a, int mode, cudaStream_t s);
 
-/* Weight gradient of a 3x3 convolution (padding 1): dw [cout][9 * cin] +=,
- * db [cout] += (NULL: none).  x as in the forward pass, dy [P][dy_c] f32
- * (dy_c = 32, or 1 for a one-channel output). */
+/* Weight gradient of a 3x3 convolution (padding 1): dw [cout][9 * cin] of a
+ * gradient copy (dw_stride floats apart) +=.
+ * x as in the forward pass; dy bf16 [P][32] (cout = 32), or dy NULL and
+ * dy_f32 [P] (cout = 1, cin = 32, stride 1). */
 typedef struct hl_dw_args {
     const __nv_bfloat16 *x;
-    const float *dy;          /* [P][dy_c] */
-    int dy_c;
+    const __nv_bfloat16 *dy;
+    const float *dy_f32;
     float *dw;
-    float *db;
+    int dw_stride;
     int B, H, W, Ho, Wo;
-    int cin, cout;
+    int cin;
     int stride;
+    int *status;
 } hl_dw_args;
 cudaError_t hl_launch_conv_dw(const hl_dw_args *a, cudaStream_t s);
-
-cudaError_t hl_launch_relu_mask(const __nv_bfloat16 *dx, const __nv_bfloat16 *y,
-                                long long n, float *out_f32,
-                                __nv_bfloat16 *out_bf16, cudaStream_t s);
 
 /* Average pooling of 0/255 images into side x side occupancy maps. */
 typedef struct hl_pool_img {
@@ -79,16 +88,31 @@ cudaError_t hl_launch_head_fwd(const float *e, const hl_head_geom *geo,
                                int nimg, const float *ab, float *hsum,
                                float *logits, cudaStream_t s);
 cudaError_t hl_launch_head_bwd(const float *dz, int ev, const hl_head_geom *geo,
-                               int nimg, const float *ab, float *de, cudaStream_t s);
+                               int nimg, const float *ab, float *de, __nv_bfloat16 *de_b,
+                               float *db, int db_stride, cudaStream_t s);
 cudaError_t hl_launch_bce(const float *z, const float *y, const float *hsum,
                           long long n, float wpos, float *dz, float *dab,
-                          float *loss, cudaStream_t s);
-cudaError_t hl_launch_adam(float *w, const float *g, float *m, float *v, int n,
-                           float lr, int step, float clip, cudaStream_t s);
-cudaError_t hl_launch_f32_to_bf16(const float *in, long long n, __nv_bfloat16 *out,
-                                  cudaStream_t s);
-cudaError_t hl_launch_weight_layout(const float *w, int cout, int cin, int mode,
-                                    __nv_bfloat16 *out, cudaStream_t s);
+                          float *loss, int stride, cudaStream_t s);
+/* The optimiser step and the bf16 weight copies of every layer. */
+#define HL_NET_LAYERS 6
+typedef struct hl_update_layer {
+    int off, cout, cin;       /* its weights in the flat parameters */
+    int flip;                 /* wb: taps mirrored (stride 1) */
+    __nv_bfloat16 *wf, *wb;   /* wb NULL: no backward copy */
+} hl_update_layer;
+typedef struct hl_update_args {
+    float *w;
+    float *g;                 /* [n] and the loss: the copies' sums (gsum) */
+    float *m, *v;
+    const float *gpart;       /* HL_GRAD_COPIES x gstride: [n] and the loss each */
+    int gstride, gsum;
+    int n;
+    float lr, clip;           /* lr = 0: only the copies */
+    float c1, c2;             /* bias corrections (set by the launcher) */
+    int nlayers;
+    hl_update_layer layer[HL_NET_LAYERS];
+} hl_update_args;
+cudaError_t hl_launch_update(hl_update_args *a, int step, cudaStream_t s);
 
 struct hl_net;
 /* the network's forward pass on device-resident geometry (hl_proposal.cpp);

@@ -76,7 +76,7 @@ extern "C" int hl_cnn_conv3x3(const void *x, const void *w, const float *bias,
 /* ==================================================================== */
 
 /* Layers: (cin, cout, stride, relu); input 256 x 256 x 1, evidence 64 x 64. */
-#define NET_LAYERS 6
+#define NET_LAYERS HL_NET_LAYERS
 static const int L_CIN[NET_LAYERS] = {1, 32, 32, 32, 32, 32};
 static const int L_COUT[NET_LAYERS] = {32, 32, 32, 32, 32, 1};
 static const int L_STRIDE[NET_LAYERS] = {2, 2, 1, 1, 1, 1};
@@ -96,6 +96,8 @@ static int w_off(int l)
 static int b_off(int l) { return w_off(l) + L_COUT[l] * 9 * L_CIN[l]; }
 static int ab_off(void) { return w_off(NET_LAYERS); }
 static int n_params(void) { return ab_off() + 2; }
+/* floats of a gradient copy: the parameters and the loss, whole 128-byte lines */
+static int g_stride(void) { return (n_params() + 1 + 31) / 32 * 32; }
 
 /* side of layer l's input and output */
 static int l_in_side(int l) { return l == 0 ? NET_IN : (l == 1 ? NET_IN / 2 : NET_EV); }
@@ -104,6 +106,7 @@ static int l_out_side(int l) { return l == 0 ? NET_IN / 2 : NET_EV; }
 struct hl_net {
     int B;                             /* capacity (images) */
     float *w, *g, *m, *v;              /* FP32 master weights, grads, Adam */
+    float *gpart;                      /* gradient copies, each [np] and the loss */
     __nv_bfloat16 *wf[NET_LAYERS];     /* forward bf16 weights */
     __nv_bfloat16 *wb[NET_LAYERS];     /* backward layouts (l >= 1) */
     __nv_bfloat16 *act[NET_LAYERS];    /* outputs of layers 0..4 (bf16) */
@@ -111,27 +114,24 @@ struct hl_net {
     float *hsum, *logits, *dz;         /* [B][90][128] */
     float *de;                         /* [B][64][64] */
     __nv_bfloat16 *de_b;
-    __nv_bfloat16 *gx, *gx2;           /* input gradients (bf16, 32 ch) */
-    float *gm;                         /* masked gradient f32 [P][32] */
-    __nv_bfloat16 *gm_b;
-    float *loss;                       /* [1] */
-    int *status;
+    __nv_bfloat16 *gx, *gx2;           /* masked input gradients (bf16, 32 ch) */
+    float *loss;                       /* after the gradients */
+    int *status;                       /* after the loss: read back with it */
     hl_head_geom *geo;                 /* [B] */
     int step;
 };
 
 static void net_free_bufs(hl_net *n)
 {
-    void *p[] = {n->ev, n->hsum, n->logits, n->dz, n->de, n->de_b, n->gx, n->gx2,
-                 n->gm, n->gm_b, n->geo};
+    void *p[] = {n->ev, n->hsum, n->logits, n->dz, n->de, n->de_b, n->gx, n->gx2, n->geo};
     for (void *q : p)
         if (q)
             cudaFree(q);
     for (int l = 0; l < NET_LAYERS; l++)
         if (n->act[l])
             cudaFree(n->act[l]);
-    n->ev = n->hsum = n->logits = n->dz = n->de = n->gm = nullptr;
-    n->de_b = n->gx = n->gx2 = n->gm_b = nullptr;
+    n->ev = n->hsum = n->logits = n->dz = n->de = nullptr;
+    n->de_b = n->gx = n->gx2 = nullptr;
     n->geo = nullptr;
     for (int l = 0; l < NET_LAYERS; l++)
         n->act[l] = nullptr;
@@ -156,22 +156,37 @@ static int net_reserve(hl_net *n, int B)
     CKN(cudaMalloc(&n->de_b, s64 * sizeof(__nv_bfloat16)));
     CKN(cudaMalloc(&n->gx, s128 * 32 * sizeof(__nv_bfloat16)));
     CKN(cudaMalloc(&n->gx2, s128 * 32 * sizeof(__nv_bfloat16)));
-    CKN(cudaMalloc(&n->gm, s128 * 32 * sizeof(float)));
-    CKN(cudaMalloc(&n->gm_b, s128 * 32 * sizeof(__nv_bfloat16)));
     CKN(cudaMalloc(&n->geo, (size_t)B * sizeof(hl_head_geom)));
     n->B = B;
     return HL_NO_ERROR;
 }
 
-/* bf16 copies of the master weights in every layout the passes use */
-static int net_refresh(hl_net *n, cudaStream_t s)
+/* one optimiser step (lr > 0) and the bf16 copies of the master weights in
+ * every layout the passes use */
+static int net_update(hl_net *n, float lr, bool gsum, cudaStream_t s)
 {
+    hl_update_args a;
+    memset(&a, 0, sizeof(a));
+    a.w = n->w;
+    a.g = n->g;
+    a.m = n->m;
+    a.v = n->v;
+    a.gpart = n->gpart;
+    a.gstride = g_stride();
+    a.gsum = gsum ? 1 : 0;
+    a.n = n_params();
+    a.lr = lr;
+    a.clip = 1.0f;
+    a.nlayers = NET_LAYERS;
     for (int l = 0; l < NET_LAYERS; l++) {
-        CKN(hl_launch_weight_layout(n->w + w_off(l), L_COUT[l], L_CIN[l], 0, n->wf[l], s));
-        if (l >= 1)
-            CKN(hl_launch_weight_layout(n->w + w_off(l), L_COUT[l], L_CIN[l],
-                                        L_STRIDE[l] == 1 ? 1 : 2, n->wb[l], s));
+        a.layer[l].off = w_off(l);
+        a.layer[l].cout = L_COUT[l];
+        a.layer[l].cin = L_CIN[l];
+        a.layer[l].flip = L_STRIDE[l] == 1;
+        a.layer[l].wf = n->wf[l];
+        a.layer[l].wb = l >= 1 ? n->wb[l] : nullptr;
     }
+    CKN(hl_launch_update(&a, std::max(n->step, 1), s));
     return HL_NO_ERROR;
 }
 
@@ -199,12 +214,13 @@ extern "C" int hl_net_create(hl_net **out, unsigned long long seed)
     int rc = HL_NO_ERROR;
     auto fail = [&](int r) { hl_net_destroy(n); return r; };
     if (cudaMalloc(&n->w, np * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&n->g, np * sizeof(float)) != cudaSuccess ||
+        cudaMalloc(&n->g, (np + 2) * sizeof(float)) != cudaSuccess ||
+        cudaMalloc(&n->gpart, sizeof(float) * HL_GRAD_COPIES * g_stride()) != cudaSuccess ||
         cudaMalloc(&n->m, np * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&n->v, np * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&n->loss, sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&n->status, sizeof(int)) != cudaSuccess)
+        cudaMalloc(&n->v, np * sizeof(float)) != cudaSuccess)
         return fail(HL_OUT_OF_MEM);
+    n->loss = n->g + np;
+    n->status = reinterpret_cast<int *>(n->loss + 1);
     for (int l = 0; l < NET_LAYERS; l++) {
         const size_t k = (size_t)L_COUT[l] * 9 * L_CIN[l];
         if (cudaMalloc(&n->wf[l], k * sizeof(__nv_bfloat16)) != cudaSuccess ||
@@ -228,9 +244,9 @@ extern "C" int hl_net_create(hl_net **out, unsigned long long seed)
     if (cudaMemcpy(n->w, h.data(), np * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(n->m, 0, np * sizeof(float)) != cudaSuccess ||
         cudaMemset(n->v, 0, np * sizeof(float)) != cudaSuccess ||
-        cudaMemset(n->status, 0, sizeof(int)) != cudaSuccess)
+        cudaMemset(n->g, 0, (np + 2) * sizeof(float)) != cudaSuccess)
         return fail(HL_CUDA_ERROR);
-    if ((rc = net_refresh(n, 0)) != HL_NO_ERROR || cudaStreamSynchronize(0) != cudaSuccess)
+    if ((rc = net_update(n, 0.0f, false, 0)) != HL_NO_ERROR || cudaStreamSynchronize(0) != cudaSuccess)
         return fail(rc != HL_NO_ERROR ? rc : HL_CUDA_ERROR);
     *out = n;
     return HL_NO_ERROR;
@@ -241,7 +257,7 @@ extern "C" int hl_net_destroy(hl_net *n)
     if (!n)
         return HL_NULL_POINTER;
     net_free_bufs(n);
-    void *p[] = {n->w, n->g, n->m, n->v, n->loss, n->status};
+    void *p[] = {n->w, n->g, n->gpart, n->m, n->v};
     for (void *q : p)
         if (q)
             cudaFree(q);
@@ -279,7 +295,7 @@ extern "C" int hl_net_set_params(hl_net *n, const float *host)
     CKN(cudaMemset(n->m, 0, n_params() * sizeof(float)));
     CKN(cudaMemset(n->v, 0, n_params() * sizeof(float)));
     n->step = 0;
-    int rc = net_refresh(n, 0);
+    int rc = net_update(n, 0.0f, false, 0);
     if (rc != HL_NO_ERROR)
         return rc;
     CKN(cudaStreamSynchronize(0));
@@ -353,28 +369,30 @@ extern "C" int hl_net_forward(hl_net *n, const void *occ_dev,
     return net_forward(n, static_cast<const __nv_bfloat16 *>(occ_dev), B, logits_dev, false, s);
 }
 
-/* dW and db of layer l from the f32 gradient dy (rows of dy_c values) */
-static int layer_dw(hl_net *n, int l, const __nv_bfloat16 *x, const float *dy,
-                    int dy_c, int B, cudaStream_t s)
+/* dW of layer l from the masked gradient of its output: dy (bf16), or the
+ * one-channel FP32 gradient dy_f32 of the last layer */
+static int layer_dw(hl_net *n, int l, const __nv_bfloat16 *x, const __nv_bfloat16 *dy,
+                    const float *dy_f32, int B, cudaStream_t s)
 {
     hl_dw_args a;
     memset(&a, 0, sizeof(a));
     a.x = x;
     a.dy = dy;
-    a.dy_c = dy_c;
-    a.dw = n->g + w_off(l);
-    a.db = n->g + b_off(l);
+    a.dy_f32 = dy_f32;
+    a.dw = n->gpart + w_off(l);
+    a.dw_stride = g_stride();
     a.B = B;
     a.H = a.W = l_in_side(l);
     a.Ho = a.Wo = l_out_side(l);
     a.cin = L_CIN[l];
-    a.cout = L_COUT[l];
     a.stride = L_STRIDE[l];
+    a.status = n->status;
     CKN(hl_launch_conv_dw(&a, s));
     return HL_NO_ERROR;
 }
 
-/* input gradient of layer l (l >= 1) from the bf16 gradient g of its output */
+/* input gradient of layer l (l >= 1) from the bf16 gradient g of its output,
+ * masked by the ReLU of layer l - 1, whose bias gradient is its sum */
 static int layer_dx(hl_net *n, int l, const __nv_bfloat16 *g, int B,
                     __nv_bfloat16 *dx, cudaStream_t s)
 {
@@ -384,25 +402,19 @@ static int layer_dx(hl_net *n, int l, const __nv_bfloat16 *g, int B,
     a.w = n->wb[l];
     a.y = dx;
     a.B = B;
+    a.H = a.W = l_out_side(l);
+    a.Ho = a.Wo = l_in_side(l);
+    a.cin = L_COUT[l];
+    a.cout = L_CIN[l];
+    a.kreal = 9 * L_COUT[l];
+    a.stride = L_STRIDE[l];
+    a.w_ready = 1;   /* the weights are the forward pass's */
     a.status = n->status;
-    if (L_STRIDE[l] == 1) {
-        /* dx = conv(g, flipped transposed weights): cin = cout_fwd */
-        a.H = a.W = l_out_side(l);
-        a.Ho = a.Wo = l_in_side(l);
-        a.cin = L_COUT[l];
-        a.cout = L_CIN[l];
-        a.kreal = 9 * L_COUT[l];
-        a.stride = 1;
-        CKN(hl_launch_conv3x3(&a, 0, s));
-    } else {
-        a.H = a.W = l_out_side(l);
-        a.Ho = a.Wo = l_in_side(l);
-        a.cin = L_COUT[l];
-        a.cout = L_CIN[l];
-        a.kreal = 9 * L_COUT[l];
-        a.stride = 2;
-        CKN(hl_launch_conv3x3(&a, 1, s));
-    }
+    a.mask = n->act[l - 1];
+    a.db = n->gpart + b_off(l - 1);
+    a.db_stride = g_stride();
+    /* stride 1: a convolution with the flipped transposed weights */
+    CKN(hl_launch_conv3x3(&a, L_STRIDE[l] == 1 ? 0 : 1, s));
     return HL_NO_ERROR;
 }
 
@@ -424,62 +436,36 @@ extern "C" int hl_net_train_step(hl_net *n, const void *occ_dev,
     if ((rc = net_forward(n, occ, B, n->logits, true, s)) != HL_NO_ERROR)
         return rc;
     const int np = n_params();
-    CKN(cudaMemsetAsync(n->g, 0, np * sizeof(float), s));
-    CKN(cudaMemsetAsync(n->loss, 0, sizeof(float), s));
+    CKN(cudaMemsetAsync(n->gpart, 0, sizeof(float) * HL_GRAD_COPIES * g_stride(), s));
     const long long cells = (long long)B * HL_HEAD_T * HL_HEAD_R;
     CKN(hl_launch_bce(n->logits, target_dev, n->hsum, cells, pos_weight, n->dz,
-                      n->g + ab_off(), n->loss, s));
-    CKN(hl_launch_head_bwd(n->dz, NET_EV, n->geo, B, n->w + ab_off(), n->de, s));
-    const long long P64 = (long long)B * NET_EV * NET_EV;
-    const long long P128 = (long long)B * 128 * 128;
-    /* layer 5 (32 -> 1, no ReLU): dW from de, dx = conv(de, flipped W) */
-    if ((rc = layer_dw(n, 5, n->act[4], n->de, 1, B, s)) != HL_NO_ERROR)
-        return rc;
-    CKN(hl_launch_f32_to_bf16(n->de, P64, n->de_b, s));
-    {
-        hl_conv_args a;
-        memset(&a, 0, sizeof(a));
-        a.x = n->de_b;
-        a.w = n->wb[5];            /* [32][9]: cin 1 -> cout 32, flipped */
-        a.y = n->gx;
-        a.B = B;
-        a.H = a.W = NET_EV;
-        a.Ho = a.Wo = NET_EV;
-        a.cin = 1;
-        a.cout = 32;
-        a.kreal = 9;
-        a.stride = 1;
-        a.status = n->status;
-        CKN(hl_launch_conv3x3(&a, 0, s));
-    }
-    /* layers 4 .. 1 */
+                      n->gpart + ab_off(), n->gpart + np, g_stride(), s));
+    CKN(hl_launch_head_bwd(n->dz, NET_EV, n->geo, B, n->w + ab_off(), n->de, n->de_b,
+                           n->gpart + b_off(5), g_stride(), s));
+    /* layer 5 (32 -> 1, no ReLU): dW from the FP32 gradient, dx from its bf16
+     * copy; then layers 4 .. 1, and dW of layer 0 from the input map */
     __nv_bfloat16 *gin = n->gx, *gout = n->gx2;
-    for (int l = 4; l >= 0; l--) {
-        const long long P = (l == 0) ? P128 : P64;
-        CKN(hl_launch_relu_mask(gin, n->act[l], P * 32, n->gm, n->gm_b, s));
-        const __nv_bfloat16 *xin = (l == 0) ? occ : n->act[l - 1];
-        if ((rc = layer_dw(n, l, xin, n->gm, 32, B, s)) != HL_NO_ERROR)
+    if ((rc = layer_dw(n, 5, n->act[4], nullptr, n->de, B, s)) != HL_NO_ERROR ||
+        (rc = layer_dx(n, 5, n->de_b, B, gin, s)) != HL_NO_ERROR)
+        return rc;
+    for (int l = 4; l >= 1; l--) {
+        if ((rc = layer_dw(n, l, n->act[l - 1], gin, nullptr, B, s)) != HL_NO_ERROR ||
+            (rc = layer_dx(n, l, gin, B, gout, s)) != HL_NO_ERROR)
             return rc;
-        if (l >= 1) {
-            if ((rc = layer_dx(n, l, n->gm_b, B, gout, s)) != HL_NO_ERROR)
-                return rc;
-            std::swap(gin, gout);
-        }
+        std::swap(gin, gout);
     }
+    if ((rc = layer_dw(n, 0, occ, gin, nullptr, B, s)) != HL_NO_ERROR)
+        return rc;
     n->step++;
-    if (lr > 0.0f)
-        CKN(hl_launch_adam(n->w, n->g, n->m, n->v, np, lr, n->step, 1.0f, s));
-    if ((rc = net_refresh(n, s)) != HL_NO_ERROR)
+    if ((rc = net_update(n, lr, true, s)) != HL_NO_ERROR)
         return rc;
     if (loss_host) {
-        float l = 0.0f;
-        int st = 0;
-        CKN(cudaMemcpyAsync(&l, n->loss, sizeof(float), cudaMemcpyDeviceToHost, s));
-        CKN(cudaMemcpyAsync(&st, n->status, sizeof(int), cudaMemcpyDeviceToHost, s));
+        int ret[2] = {0, 0};   /* loss (bits), status */
+        CKN(cudaMemcpyAsync(ret, n->loss, sizeof(ret), cudaMemcpyDeviceToHost, s));
         CKN(cudaStreamSynchronize(s));
-        if (st != 0)
+        if (ret[1] != 0)
             return HL_CUDA_ERROR;
-        *loss_host = l;
+        memcpy(loss_host, &ret[0], sizeof(float));
     }
     return HL_NO_ERROR;
 }

@@ -74,3 +74,34 @@ def test_head_beyond_32_bits(lib, scale):  # noqa: F811
     zr, _, e, _, _ = CO.net_forward(occ, geos, p.astype(np.float64))
     assert (np.abs(e).max() > 128) == (scale > 1)
     assert np.abs(z - zr).max() <= 1e-2 * max(1.0, np.abs(zr).max())
+
+
+@pytest.mark.parametrize("B", [1, 3])
+def test_training_step_gradients_and_update(lib, B):  # noqa: F811
+    """Gradients of one to three maps against the oracle (5% of a layer's
+    norm: BF16 activations and gradients, 2^-9 each, through six layers), and
+    the first Adam step from them: w - lr g / (|g| + eps), both bias
+    corrections cancelling, to FP32 rounding."""
+    import torch
+    from opencuda_gb300.proposal import HoughNet
+    rng = np.random.default_rng(40 + B)
+    occ = CO.bf16_round((rng.random((B, 256, 256)) < 0.05).astype(np.float32) * 0.125)
+    geos = [(32.0, -2896.0, 128 / 5793.0, 64, 64), (16.0, -1448.0, 128 / 2897.0, 64, 50),
+            (4.0, -300.0, 128 / 601.0, 9, 64)][:B]
+    net = HoughNet(seed=21)
+    p = net.get_params()
+    tgt = (rng.random((B, 90, 128)) < 0.005).astype(np.float32)
+    loss = net.train_step(_dev_bf16(torch, occ), HoughNet.geos(geos), torch.from_numpy(tgt).cuda(),
+                          1e-3, 30.0)
+    g, q = net.get_grads(), net.get_params()
+    lref, gref = CO.net_loss_grads(occ, geos, p.astype(np.float64), tgt, 30.0)
+    assert abs(loss - lref) <= 1e-3 * abs(lref) + 1e-5
+    o = 0
+    for ci, co, _, _ in CO.LAYERS:
+        for n in (co * 9 * ci, co):
+            a, b = g[o:o + n], gref[o:o + n]
+            assert np.linalg.norm(a - b) <= 0.05 * max(np.linalg.norm(b), 1e-12), (o, n)
+            o += n
+    assert np.allclose(g[o:], gref[o:], rtol=1e-3, atol=1e-6)
+    gc = np.clip(g.astype(np.float64), -1, 1)
+    assert np.allclose(q, p - 1e-3 * gc / (np.abs(gc) + 1e-8), rtol=1e-5, atol=2e-6)
