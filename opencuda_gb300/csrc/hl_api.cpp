@@ -38,6 +38,7 @@ struct hl_handle {
     int device;
     int sms;
     float *d_cos, *d_sin;
+    float *h_cos, *h_sin;    /* host copies of the table */
 
     uint32_t *d_pts;
     size_t cap_pts;
@@ -53,8 +54,10 @@ struct hl_handle {
     unsigned char *d_result; /* hl_result_hdr + lines */
     size_t cap_result;
     unsigned char *h_result; /* pinned mirror */
-    /* counters: [0] ncand, [1] status, [2] points, [3] ticket, [4..7] bbox */
+    /* counters: [0] ncand, [1] status, [2] points, [3] ticket, [4] bbox ticket */
     int *d_counters;
+    int4 *d_bbox;            /* partial boxes of a coordinate list */
+    int *h_bbox;             /* its box (pinned; the kernel writes it) */
 
     unsigned ticket_base;
     unsigned epoch;
@@ -189,6 +192,14 @@ static int build_table(hl_handle *h)
     CK(cudaMalloc(&h->d_cos, sizeof(float) * h->Tp));
     CK(cudaMalloc(&h->d_sin, sizeof(float) * h->Tp));
     CK(hl_launch_trig(h->d_cos, h->d_sin, h->T, h->Tp, h->p.detheta, 0));
+    free(h->h_cos);
+    free(h->h_sin);
+    h->h_cos = (float *)malloc(sizeof(float) * h->Tp);
+    h->h_sin = (float *)malloc(sizeof(float) * h->Tp);
+    if (!h->h_cos || !h->h_sin)
+        return HL_OUT_OF_MEM;
+    CK(cudaMemcpyAsync(h->h_cos, h->d_cos, sizeof(float) * h->Tp, cudaMemcpyDeviceToHost, 0));
+    CK(cudaMemcpyAsync(h->h_sin, h->d_sin, sizeof(float) * h->Tp, cudaMemcpyDeviceToHost, 0));
     CK(cudaStreamSynchronize(0));
     return HL_NO_ERROR;
 }
@@ -250,7 +261,7 @@ extern "C" int hl_destroy(hl_handle *h)
                     h->d_tile_off, h->d_acc, h->d_keys, h->d_aux,
                     h->d_result, h->d_counters, h->order_dev,
                     h->d_merge, h->d_scratch, h->d_tmask,
-                    h->d_ckeys, h->d_ccnt, h->d_cres};
+                    h->d_ckeys, h->d_ccnt, h->d_cres, h->d_bbox};
     for (void *q : ptrs)
         if (q)
             cudaFree(q);
@@ -258,6 +269,10 @@ extern "C" int hl_destroy(hl_handle *h)
         cudaFreeHost(h->h_result);
     if (h->h_cres)
         cudaFreeHost(h->h_cres);
+    if (h->h_bbox)
+        cudaFreeHost(h->h_bbox);
+    free(h->h_cos);
+    free(h->h_sin);
     if (h->prof_ev) {
         for (int i = 0; i < HL_PROF_MAX * (HL_NSTAGE + 1); i++)
             cudaEventDestroy(h->prof_ev[i]);
@@ -1147,6 +1162,27 @@ extern "C" int hl_lines_from_accumulator(hl_handle *h, const int32_t *acc_dev,
     return fetch_result(h, linesmax, lines, s);
 }
 
+/* Rows of the widest rho range a theta slice reaches over the box [x0, x1] x
+ * [y0, y1] (in double, two rows of slack an end for the vote rule's floats and
+ * 2^-20 of the value). */
+static int points_span(const hl_handle *h, const int bb[4], int R)
+{
+    const double irho = (double)(float)(1.0 / h->p.derho);
+    double span = 0.0;
+    for (int k0 = 0; k0 < h->T; k0 += HL_SLICE) {
+        double lo = 1e300, hi = -1e300;
+        for (int k = k0; k < std::min(k0 + HL_SLICE, h->T); k++) {
+            const double c = h->h_cos[k] * irho, s = h->h_sin[k] * irho;
+            const double xa = bb[0] * c, xb = bb[2] * c, ya = bb[1] * s, yb = bb[3] * s;
+            lo = std::min(lo, std::min(xa, xb) + std::min(ya, yb));
+            hi = std::max(hi, std::max(xa, xb) + std::max(ya, yb));
+        }
+        const double slack = 3.0 + std::max(fabs(lo), fabs(hi)) / 1048576.0;
+        span = std::max(span, hi - lo + 2.0 * slack);
+    }
+    return (int)std::min(span, (double)R);
+}
+
 extern "C" int hl_plain_points(hl_handle *h, const int *xy_dev, int n,
                                int *linesmax, hl_line *lines, void *stream)
 {
@@ -1157,14 +1193,14 @@ extern "C" int hl_plain_points(hl_handle *h, const int *xy_dev, int n,
     if (n <= 0)
         return HL_INVALID_DATA;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    int init[4] = {0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000};
-    CK(cudaMemcpyAsync(h->d_counters + 4, init, sizeof(init),
-                       cudaMemcpyHostToDevice, s));
-    CK(hl_launch_bbox(xy_dev, n, h->d_counters + 4, s));
-    int bb[4];
-    CK(cudaMemcpyAsync(bb, h->d_counters + 4, sizeof(bb), cudaMemcpyDeviceToHost,
-                       s));
+    if (!h->d_bbox)
+        CK(cudaMalloc(&h->d_bbox, sizeof(int4) * HL_BBOX_CTAS));
+    if (!h->h_bbox)
+        CK(cudaMallocHost(&h->h_bbox, sizeof(int4)));
+    CK(hl_launch_bbox(xy_dev, n, h->d_bbox, reinterpret_cast<unsigned *>(h->d_counters + 4),
+                      h->h_bbox, s));
     CK(cudaStreamSynchronize(s));
+    const int bb[4] = {h->h_bbox[0], h->h_bbox[1], h->h_bbox[2], h->h_bbox[3]};
     /* the reference's accumulator height uses the box extent,
      * okano_3_0/HoughLine.cu:374-375,387 */
     int w = bb[2] - bb[0], hh = bb[3] - bb[1];
@@ -1180,11 +1216,25 @@ extern "C" int hl_plain_points(hl_handle *h, const int *xy_dev, int n,
     int rc = ensure_acc(h, g.numrho, *linesmax);
     if (rc != HL_NO_ERROR)
         return rc;
-    int rows, nwin, threads;
-    vote_shape(h, g.numrho, &rows, &nwin, &threads);
-    CK(hl_launch_vote_points(xy_dev, n, h->d_cos, h->d_sin, h->T, h->Tp,
-                             g.rho_min, g.numrho, rows, nwin,
-                             (float)(1.0 / h->p.derho), h->d_acc, threads, s));
+    hl_points_args pa;
+    memset(&pa, 0, sizeof(pa));
+    pa.xy = reinterpret_cast<const int2 *>(xy_dev);
+    pa.n = n;
+    pa.x0 = bb[0];
+    pa.y0 = bb[1];
+    pa.x1 = bb[2];
+    pa.y1 = bb[3];
+    pa.cosv = h->d_cos;
+    pa.sinv = h->d_sin;
+    pa.T = h->T;
+    pa.Tp = h->Tp;
+    pa.rho_min = g.rho_min;
+    pa.R = g.numrho;
+    pa.span = points_span(h, bb, g.numrho);
+    pa.exact = g.numrho >= (1 << 22);
+    pa.irho = (float)(1.0 / h->p.derho);
+    pa.acc = h->d_acc;
+    CK(hl_launch_vote_points(&pa, std::max(h->sms, 1), s));
     int launches = 2;
     h->prof_open = 0;
     if ((rc = run_c(h, g, *linesmax, nullptr, nullptr, s, &launches)) !=

@@ -384,12 +384,21 @@ cudaError_t hl_launch_merge(const hl_merge_args *a, int max_rows, cudaStream_t s
 cudaError_t hl_launch_vote(const hl_vote_args *a, int threads, int grid,
                            cudaStream_t s);
 size_t hl_vote_smem_bytes(int win_rows);
-size_t hl_vote_points_smem_bytes(int win_rows);
-cudaError_t hl_launch_vote_points(const int *xy, int n, const float *cosv,
-                                  const float *sinv, int T, int Tp,
-                                  int rho_min, int R, int win_rows, int nwin,
-                                  float irho, int32_t *acc, int threads,
-                                  cudaStream_t s);
+/* the vote over a coordinate list: clears acc, then votes */
+typedef struct hl_points_args {
+    const int2 *xy;
+    int n;
+    int x0, y0, x1, y1;       /* its bounding box */
+    const float *cosv, *sinv; /* [Tp] */
+    int T, Tp;
+    int rho_min, R;
+    int span;                 /* rows any slice's range over the box needs at most */
+    int win_rows;             /* set by the launcher */
+    int exact;                /* |rho| may reach 2^22: convert exactly */
+    float irho;
+    int32_t *acc;             /* [R][Tp] */
+} hl_points_args;
+cudaError_t hl_launch_vote_points(hl_points_args *a, int sms, cudaStream_t s);
 cudaError_t hl_launch_peaks(const hl_peak_args *a, cudaStream_t s);
 cudaError_t hl_launch_finalize(const hl_final_args *a, int nimg, cudaStream_t s);
 cudaError_t hl_launch_to_tight(const int32_t *acc, int R, int T, int Tp,
@@ -399,7 +408,12 @@ cudaError_t hl_launch_to_ref(const int32_t *acc, int R, int T, int Tp,
                              cudaStream_t s);
 cudaError_t hl_launch_from_tight(const int32_t *acc, int R, int T, int Tp,
                                  int32_t *out, cudaStream_t s);
-cudaError_t hl_launch_bbox(const int *xy, int n, int *bbox, cudaStream_t s);
+/* CTAs of the bounding-box kernel at most (their partial boxes in part) */
+#define HL_BBOX_CTAS 152
+/* bounding box {xmin, ymin, xmax, ymax} of a list; bbox may be mapped host
+ * memory, *ticket is zero before and after */
+cudaError_t hl_launch_bbox(const int *xy, int n, int4 *part, unsigned *ticket, int *bbox,
+                           cudaStream_t s);
 cudaError_t hl_launch_draw(uint8_t *out, long pitch, int w, int h,
                            const hl_line *lines, int nlines, int derho,
                            cudaStream_t s);

@@ -670,42 +670,63 @@ cudaError_t hl_launch_compact(const hl_compact_args *a, cudaStream_t s)
 
 /* Bounding box of an interleaved (x, y) list: bbox = {xmin, ymin, xmax, ymax}
  * (the reference's _findMinMaxCoordinates, okano_3_0/HoughLine.cu:287-334,
- * done on the device).  bbox must be preset to {INT_MAX, INT_MAX, INT_MIN,
- * INT_MIN}. */
-__global__ void hl_bbox_kernel(const int *xy, int n, int *bbox)
+ * done on the device).  Every CTA writes its own box; the last one to finish
+ * combines them and writes the result straight into mapped host memory, which
+ * the host reads after its one synchronisation. */
+#define BBOX_THREADS 512
+__device__ __forceinline__ int4 bbox_join(int4 a, int4 b)
 {
-    int xmin = 0x7fffffff, ymin = 0x7fffffff, xmax = (int)0x80000000,
-        ymax = (int)0x80000000;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += gridDim.x * blockDim.x) {
-        int2 p = reinterpret_cast<const int2 *>(xy)[i];
-        xmin = min(xmin, p.x);
-        xmax = max(xmax, p.x);
-        ymin = min(ymin, p.y);
-        ymax = max(ymax, p.y);
-    }
+    return make_int4(min(a.x, b.x), min(a.y, b.y), max(a.z, b.z), max(a.w, b.w));
+}
+__device__ __forceinline__ int4 bbox_block(int4 b, int4 *s)
+{
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        xmin = min(xmin, __shfl_xor_sync(FULL, xmin, o));
-        xmax = max(xmax, __shfl_xor_sync(FULL, xmax, o));
-        ymin = min(ymin, __shfl_xor_sync(FULL, ymin, o));
-        ymax = max(ymax, __shfl_xor_sync(FULL, ymax, o));
+    for (int o = 16; o > 0; o >>= 1)
+        b = bbox_join(b, make_int4(__shfl_xor_sync(FULL, b.x, o), __shfl_xor_sync(FULL, b.y, o),
+                                   __shfl_xor_sync(FULL, b.z, o), __shfl_xor_sync(FULL, b.w, o)));
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0)
+        s[threadIdx.x >> 5] = b;
+    __syncthreads();
+    for (int w = 0; w < BBOX_THREADS / 32; w++)
+        b = bbox_join(b, s[w]);
+    return b;
+}
+__global__ void __launch_bounds__(BBOX_THREADS)
+hl_bbox_kernel(const int *xy, int n, int4 *part, unsigned *ticket, int *bbox)
+{
+    __shared__ int4 s[BBOX_THREADS / 32];
+    __shared__ bool s_last;
+    const int4 none = make_int4(0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000);
+    int4 b = none;
+    for (int i = blockIdx.x * BBOX_THREADS + threadIdx.x; i < n; i += gridDim.x * BBOX_THREADS) {
+        const int2 p = reinterpret_cast<const int2 *>(xy)[i];
+        b = bbox_join(b, make_int4(p.x, p.y, p.x, p.y));
     }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(&bbox[0], xmin);
-        atomicMin(&bbox[1], ymin);
-        atomicMax(&bbox[2], xmax);
-        atomicMax(&bbox[3], ymax);
+    b = bbox_block(b, s);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = b;
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last)
+        return;
+    __threadfence();
+    b = threadIdx.x < gridDim.x ? __ldcg(part + threadIdx.x) : none;
+    b = bbox_block(b, s);
+    if (threadIdx.x == 0) {
+        *reinterpret_cast<int4 *>(bbox) = b;
+        *ticket = 0u;
+        __threadfence_system();
     }
 }
 
-cudaError_t hl_launch_bbox(const int *xy, int n, int *bbox, cudaStream_t s)
+cudaError_t hl_launch_bbox(const int *xy, int n, int4 *part, unsigned *ticket, int *bbox,
+                           cudaStream_t s)
 {
-    int blocks = (n + 255) / 256;
-    if (blocks > 1216)
-        blocks = 1216;
-    if (blocks < 1)
-        blocks = 1;
-    hl_bbox_kernel<<<blocks, 256, 0, s>>>(xy, n, bbox);
+    const int blocks =
+        std::max(1, std::min((n + 4 * BBOX_THREADS - 1) / (4 * BBOX_THREADS), HL_BBOX_CTAS));
+    hl_bbox_kernel<<<blocks, BBOX_THREADS, 0, s>>>(xy, n, part, ticket, bbox);
     return cudaGetLastError();
 }

@@ -57,6 +57,8 @@
 #include "hl_internal.h"
 #include "hl_device.cuh"
 
+#include <algorithm>
+
 #define FULL 0xffffffffu
 #define MBAR_WAIT_LIMIT (1 << 14)
 /* float2 entries of one ring slot (runs are gap-free: the compaction pads
@@ -798,84 +800,140 @@ cudaError_t hl_launch_vote(const hl_vote_args *a, int threads, int grid,
                 : launch_vote_t<false, false>(a, threads, grid, smem, s);
 }
 
-size_t hl_vote_points_smem_bytes(int win_rows)
+/* ---- voting over a coordinate list ------------------------------------------
+ * The guidingset path (okano_3_0/HoughLine.cu:133-165): interleaved int (x, y),
+ * any order, so no tile filter.  A CTA takes one theta slice (blockIdx.x), one
+ * rho window of it (blockIdx.y) and one part of the points (blockIdx.z): the
+ * parts spread a list over the chip however few slices there are.  A slice's
+ * windows start at the lowest row its bounding box can reach and there are as
+ * many as its range needs (one up to about 1200 x 1200), so most points vote
+ * once a theta.  Votes go to shared memory on the vote kernel's diagonal
+ * schedule, four rounds' points in flight; then the window's nonzero bins are
+ * added to the accumulator (cleared before), a row of 32 thetas a reduction.
+ * Bound by latency: clearing, voting and adding one window a CTA.  24 K points
+ * of 1024 x 1024, T = 180, ncu: 10.7 us (100 us with every point broadcast to
+ * every window of 66 CTAs); the whole call 147 -> 53 us. */
+#define PTS_THREADS 1024
+#define PTS_PART_MIN 1024      /* points a part at least holds */
+
+static int points_max_rows(void)
 {
-    return (size_t)win_rows * HL_SLICE * sizeof(int);
+    return (int)((227u * 1024u - 1024u) / (HL_SLICE * sizeof(int))) - 1;
 }
 
-/* Voting over an interleaved int (x, y) list (the guidingset path,
- * okano_3_0/HoughLine.cu:133-165).  No tile order here, so every window
- * reads every point; the per-vote row test keeps it exact. */
+template <bool UNIT, int CV>
+__device__ __forceinline__ void points_vote(const int2 *xy, int p0, int p1, const DiagTab &t,
+                                            f2x ir, int base, unsigned lim)
+{
+    const int warp = threadIdx.x >> 5, p = threadIdx.x & 7;
+    constexpr int STEP = PTS_THREADS / 32 * 8;
+    for (int g0 = p0 + warp * 8; g0 < p1; g0 += 4 * STEP) {
+        float2 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int i = g0 + u * STEP + p;
+            const int2 v = i < p1 ? xy[i] : make_int2(0, 0);
+            q[u] = i < p1 ? make_float2((float)v.x, (float)v.y) : make_float2(1e30f, 0.0f);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (g0 + u * STEP < p1)
+                diag_point<UNIT, CV>(q[u].x, q[u].y, t, ir, base, lim);
+    }
+}
+
 template <bool UNIT>
-__global__ void __launch_bounds__(1024, 1)
-hl_vote_points_kernel(const int2 *xy, int n, const float *cosv,
-                      const float *sinv, int T, int Tp, int rho_min, int R,
-                      int win_rows, float irho, int32_t *acc)
+__global__ void __launch_bounds__(PTS_THREADS, 1)
+hl_vote_points_kernel(hl_points_args a)
 {
     extern __shared__ __align__(16) int s_pacc[];
+    __shared__ float s_c[HL_SLICE], s_s[HL_SLICE];
+    __shared__ int s_lo, s_hi;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nwarps = blockDim.x >> 5;
-    const int k0 = blockIdx.x * HL_SLICE, k = k0 + lane;
-    const bool kvalid = k < T;
-    const float c = cosv[k], s = sinv[k];
-    const int w0 = blockIdx.y * win_rows;
-    const int rows = min(win_rows, R - w0);
-    const int row_base = rho_min + w0;
-    for (int i = tid; i < rows * HL_SLICE; i += blockDim.x)
-        s_pacc[i] = 0;
-    __syncthreads();
-    for (int b = warp * 32; b < n; b += nwarps * 32) {
-        const int i = b + lane;
-        int2 p = (i < n) ? xy[i] : make_int2(0, 0);
-        const float xf = (float)p.x, yf = (float)p.y;
-        const int nb = min(32, n - b);
-        for (int j = 0; j < nb; j++) {
-            const float x = __shfl_sync(FULL, xf, j);
-            const float y = __shfl_sync(FULL, yf, j);
-            const int row = rho_of<UNIT>(x, y, c, s, irho) - row_base;
-            if (kvalid && (unsigned)row < (unsigned)rows)
-                atomicAdd(&s_pacc[row * HL_SLICE + lane], 1);
+    const int k0 = blockIdx.x * HL_SLICE;
+    hl_pdl_begin();
+    if (tid < HL_SLICE) {
+        /* rho range of the slice over the bounding box: every rounded step
+         * of the vote rule is monotone in x and in y, so the corners' values
+         * bound it exactly */
+        const float c = a.cosv[k0 + lane], s = a.sinv[k0 + lane];
+        s_c[lane] = c;
+        s_s[lane] = s;
+        float lo = 3.0e38f, hi = -3.0e38f;
+        if (k0 + lane < a.T)
+            for (int i = 0; i < 4; i++) {
+                const float v = rho_f<UNIT>((float)((i & 1) ? a.x1 : a.x0),
+                                            (float)((i & 2) ? a.y1 : a.y0), c, s, a.irho);
+                lo = fminf(lo, v);
+                hi = fmaxf(hi, v);
+            }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(FULL, lo, o));
+            hi = fmaxf(hi, __shfl_xor_sync(FULL, hi, o));
+        }
+        if (lane == 0) {
+            s_lo = max(__float2int_rd(lo) - a.rho_min, 0);
+            s_hi = min(__float2int_ru(hi) - a.rho_min, a.R - 1);
         }
     }
     __syncthreads();
-    int4 *dst4 = reinterpret_cast<int4 *>(acc);
-    const int4 *src4 = reinterpret_cast<const int4 *>(s_pacc);
-    const int tp4 = Tp >> 2;
-    for (int i = tid; i < rows * (HL_SLICE / 4); i += blockDim.x) {
-        int r = i >> 3, q = i & 7;
-        dst4[(size_t)(w0 + r) * tp4 + (k0 >> 2) + q] = src4[i];
+    const int w0 = s_lo + blockIdx.y * a.win_rows;   /* first row of the window */
+    const int rows = min(a.win_rows, s_hi + 1 - w0);
+    if (rows <= 0)
+        return;
+    int4 *z = reinterpret_cast<int4 *>(s_pacc);
+    for (int i = tid; i < (rows + 1) * (HL_SLICE / 4); i += PTS_THREADS)
+        z[i] = make_int4(0, 0, 0, 0);
+    const int p0 = (int)((long long)a.n * blockIdx.z / gridDim.z);
+    const int p1 = (int)((long long)a.n * (blockIdx.z + 1) / gridDim.z);
+    DiagTab tab;
+    diag_table(tab, s_c, s_s, smem_u32(s_pacc), lane);
+    const f2x ir = f2_pack(a.irho, a.irho);
+    const int row_base = a.rho_min + w0;
+    __syncthreads();
+    if (a.exact)   /* coordinates beyond the magic constant's range */
+        points_vote<UNIT, CV_EXACT>(a.xy, p0, p1, tab, ir, row_base, (unsigned)rows);
+    else if (row_base >= 1)
+        points_vote<UNIT, CV_FLOOR>(a.xy, p0, p1, tab, ir, RHO_MAGIC_BITS + row_base,
+                                    (unsigned)rows);
+    else
+        points_vote<UNIT, CV_SIGN>(a.xy, p0, p1, tab, ir, RHO_MAGIC_BITS + row_base,
+                                   (unsigned)rows);
+    __syncthreads();
+    /* a warp a row, four rows in flight; the padding columns are left zero */
+    const bool kvalid = k0 + lane < a.T;
+    int *dst = a.acc + (size_t)w0 * a.Tp + k0 + lane;
+    for (int r0 = warp * 4; r0 < rows; r0 += PTS_THREADS / 32 * 4) {
+        int v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            v[u] = r0 + u < rows && kvalid ? s_pacc[(r0 + u) * HL_SLICE + lane] : 0;
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (v[u])
+                atomicAdd(dst + (size_t)(r0 + u) * a.Tp, v[u]);
     }
 }
 
-cudaError_t hl_launch_vote_points(const int *xy, int n, const float *cosv,
-                                  const float *sinv, int T, int Tp,
-                                  int rho_min, int R, int win_rows, int nwin,
-                                  float irho, int32_t *acc, int threads,
-                                  cudaStream_t s)
+cudaError_t hl_launch_vote_points(hl_points_args *a, int sms, cudaStream_t s)
 {
-    dim3 grid(Tp / HL_SLICE, nwin);
-    size_t smem = hl_vote_points_smem_bytes(win_rows);
-    cudaError_t e;
-    if (irho == 1.0f) {
-        e = cudaFuncSetAttribute(hl_vote_points_kernel<true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem);
-        if (e != cudaSuccess)
-            return e;
-        hl_vote_points_kernel<true><<<grid, threads, smem, s>>>(
-            reinterpret_cast<const int2 *>(xy), n, cosv, sinv, T, Tp, rho_min,
-            R, win_rows, irho, acc);
-    } else {
-        e = cudaFuncSetAttribute(hl_vote_points_kernel<false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem);
-        if (e != cudaSuccess)
-            return e;
-        hl_vote_points_kernel<false><<<grid, threads, smem, s>>>(
-            reinterpret_cast<const int2 *>(xy), n, cosv, sinv, T, Tp, rho_min,
-            R, win_rows, irho, acc);
-    }
-    return cudaGetLastError();
+    const int slices = a->Tp / HL_SLICE;
+    const int maxr = points_max_rows();
+    const int nwin = std::max(1, (a->span + maxr - 1) / maxr);
+    a->win_rows = std::max(1, std::min(maxr, (a->span + nwin - 1) / nwin));
+    /* parts: one CTA an SM, all at once */
+    const int parts = std::max(1, std::min(std::min((a->n + PTS_PART_MIN - 1) / PTS_PART_MIN,
+                                                    sms / std::max(1, slices * nwin)), 64));
+    const size_t smem = (size_t)(a->win_rows + 1) * HL_SLICE * sizeof(int);
+    cudaError_t e = cudaMemsetAsync(a->acc, 0, sizeof(int) * (size_t)a->R * a->Tp, s);
+    if (e != cudaSuccess)
+        return e;
+    const auto kernel = a->irho == 1.0f ? hl_vote_points_kernel<true> : hl_vote_points_kernel<false>;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess)
+        return e;
+    return hl_launch_pdl(kernel, dim3(slices, nwin, parts), dim3(PTS_THREADS), smem, s, false, *a);
 }
 
 /* Shared-memory atomic ceiling: every lane adds to its own bank, 8
