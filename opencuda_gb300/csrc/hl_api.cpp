@@ -1308,21 +1308,27 @@ extern "C" int hl_plain_draw(hl_handle *h, const hl_image_desc *in,
     if (rc != HL_NO_ERROR)
         return rc;
     const int launches = h->last_launches;
+    /* the drawing kernel reads the records in the device result block; with
+     * room for few lines it is queued behind the tail and takes the count
+     * from the block, so the call waits once */
+    const hl_line *dl = reinterpret_cast<const hl_line *>(h->d_result + sizeof(hl_result_hdr));
+    const int derho_i = (int)h->p.derho;   /* _houghoutKer takes an int derho */
+    const bool queued = derho_i != 0 && *linesmax > 0 && *linesmax <= 1024;
+    if (queued)
+        CK(hl_launch_draw(const_cast<uint8_t *>(rout.base), rout.pitch, w, hh, dl, *linesmax,
+                          reinterpret_cast<const hl_result_hdr *>(h->d_result), derho_i, s));
     rc = fetch_result(h, linesmax, lines, s);
     if (rc != HL_NO_ERROR)
         return rc;
     if (*linesmax > 0) {
-        /* the drawing kernel reads the records still held in the device
-         * result block */
-        const hl_line *dl = reinterpret_cast<const hl_line *>(h->d_result +
-                                                              sizeof(hl_result_hdr));
-        int derho_i = (int)h->p.derho;   /* _houghoutKer takes an int derho */
         if (derho_i == 0)
             return HL_INVALID_DATA;
-        CK(hl_launch_draw(const_cast<uint8_t *>(rout.base), rout.pitch, w, hh, dl,
-                          *linesmax, derho_i, s));
-        CK(cudaStreamSynchronize(s));
-        h->last_launches = launches + (*linesmax + 1023) / 1024;
+        if (!queued) {
+            CK(hl_launch_draw(const_cast<uint8_t *>(rout.base), rout.pitch, w, hh, dl,
+                              *linesmax, nullptr, derho_i, s));
+            CK(cudaStreamSynchronize(s));
+        }
+        h->last_launches = launches + (*linesmax + HL_DRAW_LINES - 1) / HL_DRAW_LINES;
     }
     return HL_NO_ERROR;
 }
@@ -1350,10 +1356,10 @@ extern "C" int hl_draw_lines(hl_handle *h, const hl_image_desc *out,
     CK(cudaMemcpyAsync(h->d_aux, lines, sizeof(hl_line) * (size_t)nlines,
                        cudaMemcpyHostToDevice, s));
     CK(hl_launch_draw(const_cast<uint8_t *>(r.base), r.pitch, r.w, r.h,
-                      reinterpret_cast<const hl_line *>(h->d_aux), nlines,
+                      reinterpret_cast<const hl_line *>(h->d_aux), nlines, nullptr,
                       derho_i, s));
     CK(cudaStreamSynchronize(s));
-    h->last_launches = (nlines + 1023) / 1024;
+    h->last_launches = (nlines + HL_DRAW_LINES - 1) / HL_DRAW_LINES;
     return HL_NO_ERROR;
 }
 

@@ -414,8 +414,12 @@ cudaError_t hl_launch_from_tight(const int32_t *acc, int R, int T, int Tp,
  * memory, *ticket is zero before and after */
 cudaError_t hl_launch_bbox(const int *xy, int n, int4 *part, unsigned *ticket, int *bbox,
                            cudaStream_t s);
+/* lines of one drawing launch */
+#define HL_DRAW_LINES 32768
+/* hdr NULL: nlines lines; else at most HL_DRAW_LINES, and only the hdr->count
+ * that were found (none after an error) */
 cudaError_t hl_launch_draw(uint8_t *out, long pitch, int w, int h,
-                           const hl_line *lines, int nlines, int derho,
+                           const hl_line *lines, int nlines, const hl_result_hdr *hdr, int derho,
                            cudaStream_t s);
 cudaError_t hl_launch_real_line(const uint8_t *img, long pitch, int w, int h,
                                 int x1, int y1, int x2, int y2, int delta,
