@@ -31,6 +31,9 @@
 #endif
 
 struct hl_batch_ws;   /* batched-path workspace (hl_batch*) */
+/* a handle's accumulator: anything; zero in the rows that the plan's votes never
+ * reach; all zero */
+enum { ACC_ANY = 0, ACC_UNREACHED, ACC_ZERO };
 
 struct hl_handle {
     hl_params p;
@@ -54,7 +57,8 @@ struct hl_handle {
     unsigned char *d_result; /* hl_result_hdr + lines */
     size_t cap_result;
     unsigned char *h_result; /* pinned mirror */
-    /* counters: [0] ncand, [1] status, [2] points, [3] ticket, [4] bbox ticket */
+    /* counters: [0] ncand, [1] status, [2] points, [3] ticket, [4] bbox
+     * ticket, [8] realLine, [9] vote work, [10] peak candidates */
     int *d_counters;
     int4 *d_bbox;            /* partial boxes of a coordinate list */
     int *h_bbox;             /* its box (pinned; the kernel writes it) */
@@ -64,17 +68,20 @@ struct hl_handle {
     int win_rows_override, threads_override;
     int last_launches;
 
-    /* vote work items: heaviest-first order (cached per geometry) and the
-     * persistent-CTA counter base */
-    int4 *order_dev;
-    size_t cap_order;
-    int order_w, order_h, order_rows, order_R, order_T, order_ctas;
-    int order_n, order_nmerge, order_nslots;
-    /* the split blocks (summed from their parts' scratch slots) */
-    hl_merge_region *d_merge;
-    size_t cap_merge;
-    int4 *d_scratch;
+    /* the vote plan of the last geometry (reused while it is the same) and
+     * the persistent-CTA counter base */
+    struct vote_plan *plan;
+    int plan_w, plan_h, plan_R, plan_T, plan_cap, plan_thr;
+    int acc_state;           /* what is known of d_acc (ACC_*) ... */
+    size_t acc_bytes;        /* ... as long as cap_acc is still this */
+    int cand_par;            /* the noted candidates' counter: [10 + cand_par] */
+    double plan_detheta, plan_derho;
+    unsigned char *d_plan;   /* items, merge blocks, slab list */
+    size_t cap_plan;
+    unsigned char *d_scratch;
     size_t cap_scratch;
+    unsigned long long *d_cand;   /* noted peak candidates */
+    size_t cap_cand;
     /* HoughCircle: candidate keys, [ncand, status] counters, results; the
      * workspace of circle batches */
     struct hl_cb_ws *cb;
@@ -82,12 +89,6 @@ struct hl_handle {
     int *d_ccnt;
     unsigned char *d_cres;
     unsigned char *h_cres;
-    /* admitted-tile masks of the cached geometry (see hl_tile_mask_kernel) */
-    unsigned *d_tmask;
-    size_t cap_tmask;
-    int masks_dirty;
-    double order_detheta;
-    double order_derho;
     unsigned work_base;
 
     /* batched path: workspace, CUDA-graph switch; whether the last
@@ -158,16 +159,6 @@ static int grow(void **ptr, size_t *cap, size_t need_bytes)
     }
     *cap = nb;
     return HL_NO_ERROR;
-}
-
-/* grow() that raises *moved when the buffer was (re)allocated */
-static int grow_tracked(void **ptr, size_t *cap, size_t need_bytes, int *moved)
-{
-    const void *old = *ptr;
-    int rc = grow(ptr, cap, need_bytes);
-    if (rc == HL_NO_ERROR && *ptr != old)
-        *moved = 1;
-    return rc;
 }
 
 static int check_params(const hl_params *p)
@@ -250,6 +241,7 @@ extern "C" int hl_create(hl_handle **out, const hl_params *params)
 
 static void batch_free(hl_handle *h);
 static void circle_batch_free(hl_handle *h);
+static void plan_free(struct vote_plan *p);
 
 extern "C" int hl_destroy(hl_handle *h)
 {
@@ -257,10 +249,10 @@ extern "C" int hl_destroy(hl_handle *h)
         return HL_NULL_POINTER;
     batch_free(h);
     circle_batch_free(h);
+    plan_free(h->plan);
     void *ptrs[] = {h->d_cos, h->d_sin, h->d_pts, h->d_tile_state,
                     h->d_tile_off, h->d_acc, h->d_keys, h->d_aux,
-                    h->d_result, h->d_counters, h->order_dev,
-                    h->d_merge, h->d_scratch, h->d_tmask,
+                    h->d_result, h->d_counters, h->d_plan, h->d_scratch, h->d_cand,
                     h->d_ckeys, h->d_ccnt, h->d_cres, h->d_bbox};
     for (void *q : ptrs)
         if (q)
@@ -393,236 +385,428 @@ extern "C" int hl_last_launch_count(const hl_handle *h)
     return h ? h->last_launches : 0;
 }
 
-/* Rho-window rows per work item: at most what one CTA holds next to its
- * staging ring (one CTA of 1024 threads per SM), and enough windows that
- * there are about two items per SM (the heaviest-first order then balances
- * the tail), but no window below 256 rows. */
-static void vote_shape(const hl_handle *h, int R, int *rows, int *nwin,
-                       int *threads)
-{
-    const int slices = h->Tp / HL_SLICE;
-    const int maxr = hl_vote_max_rows();
-    int nw;
-    if (h->win_rows_override > 0) {
-        nw = (R + std::min(h->win_rows_override, maxr) - 1) /
-             std::min(h->win_rows_override, maxr);
-    } else {
-        /* windows as tall as one CTA's shared memory allows (the fastest
-         * measured at 4096 x 4096, T = 720: fewer tile-filter passes and
-         * less vote waste than smaller windows; heavy blocks are split into
-         * parts anyway), unless that leaves fewer blocks than SMs: then
-         * about two blocks per SM, 256 rows at least */
-        int nmin = (R + maxr - 1) / maxr;
-        nw = nmin;
-        if (nw * slices < std::max(h->sms, 1)) {
-            int want = (2 * std::max(h->sms, 1) + slices - 1) / slices;
-            int nmax = std::max(1, R / 256);
-            nw = std::max(nmin, std::min(want, nmax));
-        }
-    }
-    int r = (R + nw - 1) / nw;
-    r = (r + 7) / 8 * 8;
-    nw = (R + r - 1) / r;
-    *rows = r;
-    *nwin = nw;
-    *threads = h->threads_override > 0 ? h->threads_override : 1024;
-}
+/* ---- the vote plan ---------------------------------------------------------
+ * Every image's theta slices are voted in regions, rectangles of compaction
+ * tiles whose rho range over the slice fits a window in shared memory
+ * (hl_vote_item).  A region's rows are its width times max|cos| plus its
+ * height times max|sin| over the slice, so slices near an axis take long
+ * regions across it.  The number of regions is at least what the rows need and
+ * what spreads the launch's work over the CTAs (weight cap); among the grids
+ * with enough of them the one that stores the fewest rows is taken.  Weights
+ * are in pixels; a row of a window costs about HL_ROW_PIXELS of them (its
+ * clearing, storing and merging against votes at the 2-3% of edge pixels that
+ * maps hold).  Items go heaviest first; those that a list schedule starts in
+ * the last 40% of the launch are halved, so the CTAs finish together. */
+/* Rows: 24 or 160 pixels change a 4096 x 4096 image, T = 720, by less than 0.3 us,
+ * 160 cost 64 cells of 256 x 256 10 us of 82. */
+#define HL_ROW_PIXELS 64.0
+/* Items per CTA the plan aims at.  More balance better, fewer store and merge
+ * less: 1, 2, 3, 5 a CTA take 151.5, 147.2, 150.2, 153.2 us at 4096 x 4096, T =
+ * 720, and 1036, 993, 1005, 1007 us in a proposal batch of 32 x 2048 x 2048. */
+#define HL_PLAN_SHARE 2.0
+/* No region below this for balance alone: a region's own start and its slab
+ * then cost more than its votes.  1913 x 1077, T = 360: 64 K, 128 K, 192 K pixels
+ * 45.6, 45.5, 43.1 us; 2048 x 2048, T = 360, lines drawn: 72.6, 73.6, 67.9 us. */
+#define HL_MIN_REGION (192.0 * 1024.0)
 
-/* Weight of every (slice, window) block of a w x hh ROI: the area of the
- * tiles that the vote kernel's tile filter (tile_hits) admits for it.  The
- * kernel votes every point of an admitted tile with all 32 lanes (a last,
- * partial slice too: its lanes past T vote into the padding), so with a
- * uniform point density this is its work, waste included.  Per slice
- * each tile's rho range over the slice (corners at both end angles, plus
- * x + y when the corner's direction lies inside the slice, three bins of
- * slack) gives the run of windows it reaches. */
-static void block_weights_tiles(const hl_handle *h, int w, int hh, int rho_min,
-                                int R, int rows, int nwin,
-                                std::vector<double> &wt)
+struct vote_plan {
+    std::vector<hl_vote_item> items;
+    std::vector<hl_merge_block> blocks;
+    std::vector<int2> slabs;
+    long long scratch_units;   /* 64 bytes each */
+    int part16, win_rows, exact;
+    /* the blocks' items add to the accumulator instead of going through slabs:
+     * where a tile needs several windows (rho steps below 0.1 pixels) or the
+     * slabs would take more than HL_MAX_SCRATCH (images of 32 K and more a
+     * side, or a handful of angles: a slab's column groups are as tall as their
+     * thetas lie apart).  Dense: the accumulator is cleared before and scanned
+     * after */
+    int add;
+};
+#define HL_MAX_SCRATCH (1LL << 30)
+static void plan_free(vote_plan *p) { delete p; }
+
+struct plan_img {
+    int w, h, R;
+};
+
+/* max|cos| and max|sin| of a slice's thetas times irho, with a little slack
+ * for the vote rule's floats */
+struct slice_ext {
+    double c, s;
+};
+
+static void slice_extents(const hl_handle *h, std::vector<slice_ext> &ext)
 {
-    const int slices = h->Tp / HL_SLICE;
-    const int tx_n = (w + HL_TILE_W - 1) / HL_TILE_W;
-    const int ty_n = (hh + HL_TILE_H - 1) / HL_TILE_H;
     const double irho = 1.0 / h->p.derho;
-    wt.assign((size_t)slices * nwin, 0.0);
-    for (int sl = 0; sl < slices; sl++) {
-        const int k0 = sl * HL_SLICE;
-        if (k0 >= h->T)
-            continue;
-        const int k1 = std::min(k0 + HL_SLICE, h->T) - 1;
-        const double c0 = cos(k0 * h->p.detheta), s0 = sin(k0 * h->p.detheta);
-        const double c1 = cos(k1 * h->p.detheta), s1 = sin(k1 * h->p.detheta);
-        for (int ty = 0; ty < ty_n; ty++) {
-            const double ya = (double)ty * HL_TILE_H;
-            const double yb = std::min(ya + HL_TILE_H - 1, hh - 1.0);
-            for (int tx = 0; tx < tx_n; tx++) {
-                const double xa = (double)tx * HL_TILE_W;
-                const double xb = std::min(xa + HL_TILE_W - 1, w - 1.0);
-                double mn = 1e300, mx = -1e300;
-                for (int i = 0; i < 4; i++) {
-                    const double x = (i & 1) ? xb : xa, y = (i & 2) ? yb : ya;
-                    const double f0 = x * c0 + y * s0, f1 = x * c1 + y * s1;
-                    mn = std::min(mn, std::min(f0, f1));
-                    double hi = std::max(f0, f1);
-                    if (c0 * y - s0 * x >= 0.0 && x * s1 - y * c1 >= 0.0)
-                        hi = std::max(hi, x + y);
-                    mx = std::max(mx, hi);
-                }
-                const double lo_r = mn * irho - 3.0 - rho_min;
-                const double hi_r = mx * irho + 3.0 - rho_min;
-                if (hi_r < 0.0 || lo_r > R - 1.0)
-                    continue;
-                int wlo = nwin > 1 ? (int)floor(std::max(lo_r, 0.0) / rows) : 0;
-                int whi = nwin > 1 ? (int)floor(std::min(hi_r, R - 1.0) / rows) : 0;
-                wlo = std::min(std::max(wlo, 0), nwin - 1);
-                whi = std::min(std::max(whi, wlo), nwin - 1);
-                const double area = (xb - xa + 1.0) * (yb - ya + 1.0);
-                for (int wn = wlo; wn <= whi; wn++)
-                    wt[(size_t)sl + (size_t)slices * wn] += area;
-            }
-        }
+    const int slices = h->Tp / HL_SLICE;
+    ext.assign((size_t)slices, {0.0, 0.0});
+    for (int k = 0; k < h->T; k++) {
+        slice_ext &e = ext[(size_t)(k / HL_SLICE)];
+        e.c = std::max(e.c, fabs((double)h->h_cos[k]) * irho * (1.0 + 1e-6));
+        e.s = std::max(e.s, fabs((double)h->h_sin[k]) * irho * (1.0 + 1e-6));
     }
 }
 
-/* Split plan of the vote blocks (weights wt in pixels of admitted tiles,
- * ctas persistent CTAs): a block heavier than cap = total / (capf * ctas) is
- * cut into ceil(wt / cap) parts (at most 16, none below HL_MIN_PART pixels:
- * a part's fixed cost -- its scratch slot, written and merged -- would
- * outweigh its votes).  Then one pass over a list schedule of the parts (each CTA
- * takes the next part, heaviest first, when it is free -- the vote kernel's
- * own order): a part that would start after 60% of the estimated makespan and
- * weighs more than cap / 4 is halved (part p of n becomes parts 2p and 2p + 1
- * of 2n, the same range of the block's batches), so the last parts to start
- * are small and the CTAs finish together.  Returns the parts heaviest first;
- * pieces[b] counts block b's parts. */
-struct vote_part { double wt; int blk, part, nparts; };
-#define HL_MIN_PART (256.0 * 1024.0)
-static std::vector<vote_part> plan_parts(const std::vector<double> &wt, int ctas,
-                                         double capf, std::vector<int> &pieces)
+/* rows a region of gw x gh pixels needs over a slice (its range, both ends,
+ * truncation and rounding) */
+static double region_rows(const slice_ext &e, double gw, double gh)
 {
-    double total = 0.0;
-    for (double v : wt)
-        total += v;
-    const double cap = total / (capf * std::max(ctas, 1));
-    std::vector<vote_part> parts;
-    parts.reserve(wt.size() * 2);
-    for (size_t b = 0; b < wt.size(); b++) {
-        int np = 1;
-        if (cap > 0.0 && wt[b] > cap)
-            np = std::min(16, (int)ceil(wt[b] / cap));
-        np = std::max(1, std::min(np, (int)(wt[b] / HL_MIN_PART)));
-        for (int q = 0; q < np; q++)
-            parts.push_back({wt[b] / np, (int)b, q, np});
+    return (gw - 1.0) * e.c + (gh - 1.0) * e.s + 4.0;
+}
+
+struct plan_region {
+    double wt;
+    hl_vote_item it;
+    int blk;
+};
+
+/* the grid of regions of one (image, slice): nx x ny; nwin windows each (more
+ * than one only where a single tile needs it) */
+static void best_grid(const slice_ext &e, int w, int hh, int cap, double n_min, int *bx, int *by,
+                      int *nwin)
+{
+    const int tx = (w + HL_TILE_W - 1) / HL_TILE_W, ty = (hh + HL_TILE_H - 1) / HL_TILE_H;
+    double best = 1e300;
+    *bx = tx;
+    *by = ty;
+    *nwin = 0;
+    for (int nx = 1; nx <= tx; nx++) {
+        const int gtx = (tx + nx - 1) / nx;
+        if (nx > 1 && gtx == (tx + nx - 2) / (nx - 1))
+            continue;   /* no narrower than with one column less */
+        const double gw = std::min(gtx * HL_TILE_W, w);
+        const double left = cap - 4.0 - (gw - 1.0) * e.c;
+        if (left < 0.0)
+            continue;
+        /* tile rows a region may have */
+        double tr = e.s > 0.0 ? floor((left / e.s + 1.0) / HL_TILE_H) : ty;
+        if (tr < ty && hh <= HL_TILE_H && (hh - 1.0) * e.s <= left)
+            tr = ty;
+        if (nx > 1)
+            tr = std::min(tr, (double)HL_VOTE_RUNS);
+        if (tr < 1.0)
+            continue;
+        const int need_y = (int)ceil(ty / std::min(tr, (double)ty));
+        const int ny = std::min(ty, std::max(need_y, (int)ceil(n_min / nx)));
+        const double gh = std::min(((ty + ny - 1) / ny) * HL_TILE_H, hh);
+        const double cost = (double)nx * ny * (region_rows(e, gw, gh) + 64.0);
+        if (cost < best) {
+            best = cost;
+            *bx = nx;
+            *by = ny;
+            *nwin = 1;
+        }
+        if (nx > 4.0 * n_min + 8 && *nwin)
+            break;
     }
-    const auto heavier = [](const vote_part &a, const vote_part &c) { return a.wt > c.wt; };
-    std::stable_sort(parts.begin(), parts.end(), heavier);
+    if (!*nwin)   /* one tile a region, several windows */
+        *nwin = (int)ceil(region_rows(e, std::min(w, HL_TILE_W), std::min(hh, HL_TILE_H)) / cap);
+}
+
+/* The item of a whole w x hh image whose range exceeds the window, voted with a
+ * sliding window; false where one window holds it or sliding cannot.  A point's
+ * rho relative to the centre's differs from its tile centre's at the middle
+ * theta by at most the tile's half diagonal (66) and the centre distance times
+ * the angle to the middle (16 steps at most), so a band of adv rows needs adv +
+ * 2 e rows; the window moves by adv, at least half of itself, so that moving
+ * the rest down does not overlap. */
+static bool slide_item(const hl_handle *h, const slice_ext &e, int w, int hh, int sl, int cap,
+                       hl_vote_item *it)
+{
+    const int tx = (w + HL_TILE_W - 1) / HL_TILE_W, ty = (hh + HL_TILE_H - 1) / HL_TILE_H;
+    const double irho = 1.0 / h->p.derho;
+    if (region_rows(e, w, hh) <= cap || ty > HL_VOTE_RUNS || irho > 4.0)
+        return false;
+    const double lx = 0.5 * w + HL_TILE_W, ly = 0.5 * hh + HL_TILE_H;
+    const double dist = sqrt(lx * lx + ly * ly) * irho;
+    const int err = (int)ceil(66.0 * irho + dist * 16.0 * h->p.detheta + dist * 1e-5) + 4;
+    const int adv = (cap - 2 * err - 4) / 4 * 4;
+    if (2 * adv < cap)
+        return false;
+    const int km = std::min(sl * HL_SLICE + HL_SLICE / 2, h->T - 1);
+    const double half = ceil(lx * fabs((double)h->h_cos[km]) * irho +
+                             ly * fabs((double)h->h_sin[km]) * irho) + 2.0;
+    memset(it, 0, sizeof(*it));
+    it->slice = sl;
+    it->tx = tx << 16;
+    it->ty = ty << 16;
+    it->slab = -1;
+    it->nseg = (int)ceil(2.0 * half / adv);
+    it->adv = adv;
+    it->off0 = -(int)half - err;
+    it->half = (float)half;
+    return it->nseg > 1;
+}
+
+/* Plans the vote of n images with windows of at most cap rows on ctas
+ * persistent CTAs. */
+static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int ctas,
+                     vote_plan *pl)
+{
+    const int slices = h->Tp / HL_SLICE;
+    std::vector<slice_ext> ext;
+    slice_extents(h, ext);
+    double total = 0.0;
+    for (int i = 0; i < n; i++)
+        for (int sl = 0; sl < slices; sl++)
+            total += (double)im[i].w * im[i].h +
+                     HL_ROW_PIXELS * std::min(region_rows(ext[sl], im[i].w, im[i].h), 4.0 * cap);
+    const double wcap = std::max(total / (HL_PLAN_SHARE * std::max(ctas, 1)), HL_MIN_REGION);
+    std::vector<plan_region> reg;
+    bool slides = false;
+    pl->exact = pl->add = 0;
+    pl->part16 = 1;
+    for (int i = 0; i < n; i++) {
+        const int w = im[i].w, hh = im[i].h;
+        const int tx = (w + HL_TILE_W - 1) / HL_TILE_W, ty = (hh + HL_TILE_H - 1) / HL_TILE_H;
+        if (im[i].R >= (1 << 22))
+            pl->exact = 1;
+        for (int sl = 0; sl < slices; sl++) {
+            const double n_min = std::max(1.0, ceil((double)w * hh / wcap));
+            hl_vote_item whole;
+            if (n_min <= 1.0 && slide_item(h, ext[sl], w, hh, sl, cap, &whole)) {
+                whole.img = i;
+                plan_region r;
+                r.it = whole;
+                r.blk = i * slices + sl;
+                r.wt = (double)w * hh + HL_ROW_PIXELS * region_rows(ext[sl], w, hh);
+                reg.push_back(r);
+                slides = true;
+                continue;
+            }
+            int nx, ny, nw;
+            best_grid(ext[sl], w, hh, cap, n_min, &nx, &ny, &nw);
+            const bool clip = nw > 1;
+            pl->add |= clip;
+            for (int y = 0; y < ny; y++)
+                for (int x = 0; x < nx; x++) {
+                    const int x0 = tx * x / nx, x1 = tx * (x + 1) / nx;
+                    const int y0 = ty * y / ny, y1 = ty * (y + 1) / ny;
+                    const double gw = std::min(x1 * HL_TILE_W, w) - x0 * HL_TILE_W;
+                    const double gh = std::min(y1 * HL_TILE_H, hh) - y0 * HL_TILE_H;
+                    for (int v = 0; v < nw; v++) {
+                        plan_region r;
+                        memset(&r.it, 0, sizeof(r.it));
+                        r.it.img = i;
+                        r.it.slice = sl;
+                        r.it.tx = x0 | ((x1 - x0) << 16);
+                        r.it.ty = y0 | ((y1 - y0) << 16);
+                        r.it.win = v;
+                        r.it.clip = clip;
+                        r.it.nseg = 1;
+                        r.blk = i * slices + sl;
+                        /* a region that the slice's rho 0 crosses votes by the
+                         * sign of each vote, about 1.4 times the time */
+                        const int k0 = sl * HL_SLICE, k1 = std::min(k0 + HL_SLICE, h->T) - 1;
+                        const bool mixed = h->h_cos[k1] < 0.0f &&
+                                           (x0 * h->h_cos[k0] * HL_TILE_W +
+                                                y1 * h->h_sin[k0] * HL_TILE_H > 0.0f) &&
+                                           (x1 * h->h_cos[k1] * HL_TILE_W +
+                                                y0 * h->h_sin[k1] * HL_TILE_H < 0.0f);
+                        r.wt = gw * gh * (mixed ? 1.4 : 1.0) +
+                               HL_ROW_PIXELS * std::min(region_rows(ext[sl], gw, gh), (double)cap);
+                        reg.push_back(r);
+                    }
+                }
+        }
+    }
+    const auto heavier = [](const plan_region &a, const plan_region &c) { return a.wt > c.wt; };
+    std::stable_sort(reg.begin(), reg.end(), heavier);
     {
+        /* the late starters of a list schedule, halved along their longer side */
         typedef std::pair<double, int> slot_t;
         std::priority_queue<slot_t, std::vector<slot_t>, std::greater<slot_t>> free_at;
         for (int c = 0; c < std::max(ctas, 1); c++)
             free_at.push({0.0, c});
-        std::vector<double> start(parts.size());
+        std::vector<double> start(reg.size());
         double makespan = 0.0;
-        for (size_t i = 0; i < parts.size(); i++) {
+        for (size_t i = 0; i < reg.size(); i++) {
             slot_t f = free_at.top();
             free_at.pop();
             start[i] = f.first;
-            makespan = std::max(makespan, f.first + parts[i].wt);
-            free_at.push({f.first + parts[i].wt, f.second});
+            makespan = std::max(makespan, f.first + reg[i].wt);
+            free_at.push({f.first + reg[i].wt, f.second});
         }
-        std::vector<vote_part> out;
-        out.reserve(parts.size() * 2);
-        for (size_t i = 0; i < parts.size(); i++) {
-            const vote_part &p = parts[i];
-            if (start[i] > 0.6 * makespan && p.wt > 0.25 * cap && p.nparts <= 16 &&
-                p.wt >= 2.0 * HL_MIN_PART) {
-                out.push_back({p.wt / 2, p.blk, 2 * p.part, 2 * p.nparts});
-                out.push_back({p.wt / 2, p.blk, 2 * p.part + 1, 2 * p.nparts});
+        const size_t n0 = reg.size();
+        for (size_t i = 0; i < n0; i++) {
+            plan_region r = reg[i];
+            if (!(start[i] > 0.6 * makespan && r.wt > 0.25 * wcap && r.wt >= 2.0 * HL_MIN_REGION &&
+                  !r.it.clip && r.it.nseg == 1))
+                continue;
+            const int txn = r.it.tx >> 16, tyn = r.it.ty >> 16;
+            plan_region a = r, b = r;
+            if (txn * HL_TILE_W >= tyn * HL_TILE_H && txn > 1 && tyn <= HL_VOTE_RUNS) {
+                const int x0 = r.it.tx & 0xffff, m = txn / 2;
+                a.it.tx = x0 | (m << 16);
+                b.it.tx = (x0 + m) | ((txn - m) << 16);
+            } else if (tyn > 1) {
+                const int y0 = r.it.ty & 0xffff, m = tyn / 2;
+                a.it.ty = y0 | (m << 16);
+                b.it.ty = (y0 + m) | ((tyn - m) << 16);
             } else {
-                out.push_back(p);
+                continue;
+            }
+            a.wt = b.wt = 0.6 * r.wt;
+            reg[i] = a;
+            reg.push_back(b);
+        }
+    }
+    std::stable_sort(reg.begin(), reg.end(), heavier);
+    /* slabs and merge blocks of the blocks with several items */
+    std::vector<int> count((size_t)n * slices, 0), first((size_t)n * slices, 0);
+    for (const plan_region &r : reg)
+        count[(size_t)r.blk]++;
+    pl->blocks.clear();
+    int nslab = 0;
+    for (int b = 0; b < n * slices; b++)
+        if (count[(size_t)b] > 1) {
+            first[(size_t)b] = nslab;
+            pl->blocks.push_back({b / slices, b % slices, nslab, count[(size_t)b]});
+            nslab += count[(size_t)b];
+        }
+    pl->slabs.assign((size_t)nslab, make_int2(0, 0));
+    for (const plan_region &r : reg) {
+        const int w = im[r.it.img].w, hh = im[r.it.img].h;
+        pl->part16 &= hl_part16_ok(h->p.derho, std::min((r.it.tx >> 16) * HL_TILE_W, w),
+                                   std::min((r.it.ty >> 16) * HL_TILE_H, hh));
+    }
+    pl->items.resize(reg.size());
+    pl->scratch_units = 0;
+    double most = 8.0;
+    const double irho = 1.0 / h->p.derho;
+    for (size_t i = 0; i < reg.size(); i++) {
+        hl_vote_item it = reg[i].it;
+        const int w = im[it.img].w, hh = im[it.img].h;
+        const int x1 = std::min(((it.tx & 0xffff) + (it.tx >> 16)) * HL_TILE_W, w);
+        const int y1 = std::min(((it.ty & 0xffff) + (it.ty >> 16)) * HL_TILE_H, hh);
+        const double rows = region_rows(ext[it.slice], x1 - (it.tx & 0xffff) * HL_TILE_W,
+                                        y1 - (it.ty & 0xffff) * HL_TILE_H);
+        most = std::max(most, std::min(rows, (double)cap));
+        const size_t b = (size_t)reg[i].blk;
+        it.slab = -1;
+        if (count[b] > 1) {
+            /* a column group's rows: the region's, and what its far corner
+             * sweeps over 7 theta steps */
+            const double far = sqrt((double)x1 * x1 + (double)y1 * y1) * irho;
+            const double grp = std::min(rows, (double)cap) + far * 7.0 * h->p.detheta;
+            it.ncap = (int)(std::min(grp, (double)im[it.img].R) / 4.0) + HL_SLAB_SLACK / 4 + 1;
+            const long long units = hl_slab_units(it.ncap, pl->part16);
+            pl->add |= pl->scratch_units + units > HL_MAX_SCRATCH / 64;
+            if (!pl->add) {
+                it.slab = (int)pl->scratch_units;
+                pl->scratch_units += units;
+                pl->slabs[(size_t)first[b]++] = make_int2(it.slab, it.ncap);
             }
         }
-        parts.swap(out);
+        pl->items[i] = it;
     }
-    std::stable_sort(parts.begin(), parts.end(), heavier);
-    pieces.assign(wt.size(), 0);
-    for (const vote_part &p : parts)
-        pieces[p.blk]++;
-    return parts;
+    if (pl->add) {
+        for (hl_vote_item &it : pl->items)
+            it.slab = -1;
+        pl->blocks.clear();
+        pl->slabs.clear();
+        pl->scratch_units = 0;
+    }
+    pl->win_rows = slides ? cap : std::min(cap, ((int)most + 7) / 8 * 8);
+    return HL_NO_ERROR;
 }
 
-/* Work items of the vote kernel, heaviest first, weighted by
- * block_weights_tiles.  A block heavier than half of one CTA's fair share
- * (total / ctas; a third and a quarter measured slower at 4096 x 4096) is
- * split into parts that each vote a contiguous share of the point stream
- * (at most 16 parts), each voting into its own scratch slot; the merge
- * launch after the vote sums a split block's slots.  Cached per geometry with
- * the list of split blocks; fills va's items and scratch. */
-static int vote_items(hl_handle *h, int w, int hh, int rho_min, int R,
-                      int rows, int nwin, int ctas, hl_vote_args *va)
+/* rows a window may have: the override (at least what one tile needs at a
+ * whole rho step) or what fits next to the staging ring */
+static int plan_cap(const hl_handle *h)
 {
-    const int slices = h->Tp / HL_SLICE;
-    const int nblocks = slices * nwin;
-    if (!(h->order_dev && h->order_w == w && h->order_h == hh &&
-          h->order_rows == rows && h->order_R == R && h->order_T == h->T &&
-          h->order_derho == h->p.derho && h->order_detheta == h->p.detheta &&
-          h->order_ctas == ctas)) {
-        h->masks_dirty = 1;
-        std::vector<double> wt;
-        block_weights_tiles(h, w, hh, rho_min, R, rows, nwin, wt);
-        std::vector<int> pieces;
-        const std::vector<vote_part> parts = plan_parts(wt, ctas, 2.0, pieces);
-        /* scratch slots and merge regions of the split blocks */
-        std::vector<hl_merge_region> merge;
-        std::vector<int> slot0((size_t)nblocks, 0), used((size_t)nblocks, 0);
-        int nslots = 0;
-        for (int b = 0; b < nblocks; b++) {
-            if (pieces[b] <= 1)
-                continue;
-            const int w0 = (b / slices) * rows, k0 = (b % slices) * HL_SLICE;
-            const long long off = (long long)w0 * h->Tp + k0;
-            slot0[b] = nslots;
-            merge.push_back({off / 4, std::min(rows, R - w0), k0, nslots, pieces[b], w0, 0, {0, 0}});
-            nslots += pieces[b];
-        }
-        const int n = (int)parts.size();
-        std::vector<int4> items((size_t)n);
-        for (int i = 0; i < n; i++) {
-            const vote_part &p = parts[i];
-            const int slot = pieces[p.blk] > 1 ? slot0[p.blk] + used[p.blk]++ : 0;
-            items[i] = make_int4(p.blk, p.part | (p.nparts << 16), slot, 0);
-        }
-        int rc = grow((void **)&h->order_dev, &h->cap_order, sizeof(int4) * (size_t)n);
-        if (rc == HL_NO_ERROR && !merge.empty())
-            rc = grow((void **)&h->d_merge, &h->cap_merge,
-                      sizeof(hl_merge_region) * merge.size());
+    const int maxr = hl_vote_max_rows();
+    if (h->win_rows_override <= 0)
+        return maxr;
+    return std::min(maxr, std::max(h->win_rows_override, 168));
+}
+static int vote_threads(const hl_handle *h)
+{
+    return h->threads_override > 0 ? h->threads_override : 1024;
+}
+/* persistent CTAs an SM holds with windows of `rows` rows */
+static int vote_ctas(const hl_handle *h, int rows, int threads)
+{
+    const size_t smem = hl_vote_smem_bytes(rows);
+    const int per_sm = std::max(1, std::min(2048 / threads, (int)((228u * 1024u) / (smem + 1024))));
+    return std::max(h->sms, 1) * per_sm;
+}
+
+/* The handle's plan for a w x hh ROI, uploaded; fills va's items, scratch and
+ * window rows. */
+static size_t plan_bytes(const vote_plan &p)
+{
+    return p.items.size() * sizeof(hl_vote_item) + p.blocks.size() * sizeof(hl_merge_block) +
+           p.slabs.size() * sizeof(int2);
+}
+static void plan_copy(const vote_plan &p, unsigned char *dst)
+{
+    size_t o = p.items.size() * sizeof(hl_vote_item);
+    memcpy(dst, p.items.data(), o);
+    memcpy(dst + o, p.blocks.data(), p.blocks.size() * sizeof(hl_merge_block));
+    o += p.blocks.size() * sizeof(hl_merge_block);
+    memcpy(dst + o, p.slabs.data(), p.slabs.size() * sizeof(int2));
+}
+static void plan_args(const vote_plan &p, const unsigned char *d_plan, unsigned char *scratch,
+                      hl_vote_args *va, hl_merge_args *ma)
+{
+    va->items = reinterpret_cast<const hl_vote_item *>(d_plan);
+    va->nitems = (int)p.items.size();
+    va->win_rows = p.win_rows;
+    va->exact = p.exact;
+    va->part16 = p.part16;
+    va->add = p.add;
+    va->scratch = scratch;
+    size_t o = p.items.size() * sizeof(hl_vote_item);
+    ma->imgs = va->imgs;
+    ma->img0 = va->img0;
+    ma->T = va->T;
+    ma->Tp = va->Tp;
+    ma->scratch = scratch;
+    ma->blocks = reinterpret_cast<const hl_merge_block *>(d_plan + o);
+    ma->nblocks = (int)p.blocks.size();
+    ma->slabs =
+        reinterpret_cast<const int2 *>(d_plan + o + p.blocks.size() * sizeof(hl_merge_block));
+    ma->part16 = p.part16;
+    ma->cand = va->cand;
+}
+
+static int handle_plan(hl_handle *h, int w, int hh, int R)
+{
+    const int cap = plan_cap(h), threads = vote_threads(h);
+    if (!(h->plan && h->plan_w == w && h->plan_h == hh && h->plan_R == R && h->plan_T == h->T &&
+          h->plan_derho == h->p.derho && h->plan_detheta == h->p.detheta && h->plan_cap == cap &&
+          h->plan_thr == threads)) {
+        if (!h->plan && !(h->plan = new (std::nothrow) vote_plan()))
+            return HL_OUT_OF_MEM;
+        h->plan_w = 0;   /* not valid until the upload below */
+        if (h->acc_state == ACC_UNREACHED)
+            h->acc_state = ACC_ANY;
+        const plan_img im = {w, hh, R};
+        int rc = make_plan(h, &im, 1, cap, std::max(h->sms, 1), h->plan);
         if (rc != HL_NO_ERROR)
             return rc;
-        CK(cudaMemcpy(h->order_dev, items.data(), sizeof(int4) * (size_t)n,
-                      cudaMemcpyHostToDevice));
-        if (!merge.empty())
-            CK(cudaMemcpy(h->d_merge, merge.data(), sizeof(hl_merge_region) * merge.size(),
-                          cudaMemcpyHostToDevice));
-        h->order_w = w;
-        h->order_h = hh;
-        h->order_rows = rows;
-        h->order_R = R;
-        h->order_T = h->T;
-        h->order_derho = h->p.derho;
-        h->order_detheta = h->p.detheta;
-        h->order_ctas = ctas;
-        h->order_n = n;
-        h->order_nmerge = (int)merge.size();
-        h->order_nslots = nslots;
+        std::vector<unsigned char> tab(plan_bytes(*h->plan));
+        plan_copy(*h->plan, tab.data());
+        if ((rc = grow((void **)&h->d_plan, &h->cap_plan, tab.size())) != HL_NO_ERROR)
+            return rc;
+        CK(cudaMemcpy(h->d_plan, tab.data(), tab.size(), cudaMemcpyHostToDevice));
+        h->plan_w = w;
+        h->plan_h = hh;
+        h->plan_R = R;
+        h->plan_T = h->T;
+        h->plan_derho = h->p.derho;
+        h->plan_detheta = h->p.detheta;
+        h->plan_cap = cap;
+        h->plan_thr = threads;
     }
     int rc = grow((void **)&h->d_scratch, &h->cap_scratch,
-                  sizeof(int4) * (size_t)std::max(h->order_nslots, 1) * rows * (HL_SLICE / 4));
+                  (size_t)std::max(h->plan->scratch_units, 1LL) * 64);
     if (rc != HL_NO_ERROR)
         return rc;
-    va->items = h->order_dev;
-    va->nitems = h->order_n;
-    va->scratch = h->d_scratch;
-    return HL_NO_ERROR;
+    return grow((void **)&h->d_cand, &h->cap_cand,
+                sizeof(unsigned long long) * (65536 + (size_t)R * h->Tp / 128));
 }
 
 static int ensure_image(hl_handle *h, const hl_geom &g, int w, int hh)
@@ -648,7 +832,7 @@ static int ensure_image(hl_handle *h, const hl_geom &g, int w, int hh)
     return HL_NO_ERROR;
 }
 
-/* Peak candidates (batches): the list and its room; a threshold that only
+/* Peak candidates: the list and its room; a threshold that only
  * peaks-to-be clear leaves a few hundred per image, and past the room the
  * peak pass scans the accumulators instead.  A null list: no noting. */
 static hl_cand_list cand_list(unsigned long long *e, size_t cap_bytes, int *count)
@@ -752,13 +936,11 @@ static int launch_compaction(hl_handle *h, const hl_roi &roi, const hl_geom &g,
     return HL_NO_ERROR;
 }
 
-static int run_ab(hl_handle *h, const hl_roi &roi, const hl_geom &g,
+static int run_ab(hl_handle *h, const hl_roi &roi, const hl_geom &g, bool peaks,
                   cudaStream_t s, int *launches)
 {
     const int ntiles = g.tiles_x * g.tiles_y;
 
-    /* the vote plan first: its split blocks' regions are cleared by the
-     * compaction launch, and its tile masks are computed once per geometry */
     hl_vote_args va;
     memset(&va, 0, sizeof(va));
     va.imgs = nullptr;
@@ -776,36 +958,30 @@ static int run_ab(hl_handle *h, const hl_roi &roi, const hl_geom &g,
     va.sinv = h->d_sin;
     va.T = h->T;
     va.Tp = h->Tp;
-    int threads;
-    vote_shape(h, g.numrho, &va.win_rows, &va.img0.nwin, &threads);
     va.irho = (float)(1.0 / h->p.derho);   /* okano_3_0/HoughLine.cu:107 */
     va.status = h->d_counters + 1;
-    va.part16 = hl_part16_ok(h->p.derho, roi.w, roi.h);
-    /* one image: no candidate list (the peak pass scans the accumulator,
-     * which is still in L2; noting measured slower on the whole step) */
-    va.cand = cand_list(nullptr, 0, nullptr);
-    /* persistent CTAs: as many as fit (one per SM at 1024 threads) */
-    const size_t smem = hl_vote_smem_bytes(va.win_rows);
-    const int per_sm = std::max(1, std::min(2048 / threads,
-                                            (int)((228u * 1024u) / (smem + 1024))));
-    const int ctas = std::max(h->sms, 1) * per_sm;
-    int rc = vote_items(h, roi.w, roi.h, g.rho_min, g.numrho, va.win_rows,
-                        va.img0.nwin, ctas, &va);
+    int rc = handle_plan(h, roi.w, roi.h, g.numrho);
     if (rc != HL_NO_ERROR)
         return rc;
-    const size_t mwords = hl_tile_mask_words(h->Tp / HL_SLICE, va.img0.nwin, ntiles);
-    const void *old_mask = h->d_tmask;
-    if ((rc = grow((void **)&h->d_tmask, &h->cap_tmask, sizeof(unsigned) * mwords)) !=
-        HL_NO_ERROR)
-        return rc;
-    if (h->d_tmask != old_mask)
-        h->masks_dirty = 1;
-    va.img0.tmask = h->d_tmask;
-    if (h->masks_dirty) {
-        CK(hl_launch_tile_masks(&va, 1, mwords, s));
-        (*launches)++;
-        h->masks_dirty = 0;
+    /* bins above the threshold are noted where their final count is known;
+     * the accumulator entry points take no peaks */
+    va.cand = peaks && !h->plan->add
+                  ? cand_list(h->d_cand, h->cap_cand, h->d_counters + 10 + h->cand_par)
+                  : cand_list(nullptr, 0, nullptr);
+    hl_merge_args ma;
+    memset(&ma, 0, sizeof(ma));
+    plan_args(*h->plan, h->d_plan, h->d_scratch, &va, &ma);
+    const int threads = vote_threads(h);
+    const int ctas = vote_ctas(h, va.win_rows, threads);
+    if (h->acc_bytes != h->cap_acc || va.add)
+        h->acc_state = ACC_ANY;
+    if (h->acc_state == ACC_ANY || (peaks && h->acc_state != ACC_ZERO)) {
+        CK(cudaMemsetAsync(h->d_acc, 0, h->cap_acc, s));
+        CK(cudaMemsetAsync(h->d_counters + 10, 0, 2 * sizeof(int), s));
+        h->acc_bytes = h->cap_acc;
     }
+    /* with peaks the tail clears what is stored (set when it is launched) */
+    h->acc_state = peaks || va.add ? ACC_ANY : ACC_UNREACHED;
 
     prof_mark(h, 0, s);
     rc = launch_compaction(h, roi, g, s);
@@ -821,20 +997,8 @@ static int run_ab(hl_handle *h, const hl_roi &roi, const hl_geom &g,
     /* every CTA takes one ticket per item plus one that finds no item */
     h->work_base += (unsigned)(va.nitems + grid);
     (*launches)++;
-    if (h->order_nmerge > 0) {
-        hl_merge_args ma;
-        ma.acc = reinterpret_cast<int4 *>(h->d_acc);
-        ma.pitch4 = h->Tp / 4;
-        ma.T = h->T;
-        ma.scratch = h->d_scratch;
-        ma.slot4 = hl_slot4(va.win_rows, va.part16);
-        ma.regs = h->d_merge;
-        ma.nreg = h->order_nmerge;
-        ma.part16 = va.part16;
-        ma.pimgs = nullptr;
-        ma.thr0 = h->p.threshold;
-        ma.cand = va.cand;
-        CK(hl_launch_merge(&ma, va.win_rows, s));
+    if (ma.nblocks > 0) {
+        CK(hl_launch_merge(&ma, g.numrho, s));
         (*launches)++;
     }
     prof_mark(h, 2, s);
@@ -868,7 +1032,8 @@ static void final_args(hl_handle *h, const hl_geom &g, int linesmax, hl_line *li
     fa->img0.count_out = count_dev;
 }
 
-static int run_c(hl_handle *h, const hl_geom &g, int linesmax,
+/* noted: the vote noted the peak candidates (d_cand) */
+static int run_c(hl_handle *h, const hl_geom &g, bool noted, int linesmax,
                  hl_line *lines_dev, int *count_dev, cudaStream_t s,
                  int *launches)
 {
@@ -890,14 +1055,26 @@ static int run_c(hl_handle *h, const hl_geom &g, int linesmax,
     pa.T = h->T;
     pa.Tp = h->Tp;
     pa.status = h->d_counters + 1;
-    pa.cand = cand_list(nullptr, 0, nullptr);
+    pa.cand = noted ? cand_list(h->d_cand, h->cap_cand, h->d_counters + 10 + h->cand_par)
+                    : cand_list(nullptr, 0, nullptr);
     CK(hl_launch_peaks(&pa, s));
     (*launches)++;
     prof_mark(h, 3, s);
 
     hl_final_args fa;
     final_args(h, g, linesmax, lines_dev, count_dev, &fa);
+    if (noted) {
+        fa.clear = pa.cand;
+        fa.acc = h->d_acc;
+        fa.acc_ints = (long long)g.numrho * h->Tp;
+        fa.Tp = h->Tp;
+        fa.cand_count = h->d_counters + 10 + (h->cand_par ^ 1);
+    }
     CK(hl_launch_finalize(&fa, 1, s));
+    if (noted) {
+        h->cand_par ^= 1;
+        h->acc_state = ACC_ZERO;
+    }
     (*launches)++;
     prof_mark(h, 4, s);
     return HL_NO_ERROR;
@@ -911,6 +1088,7 @@ static void reset_counters(hl_handle *h, cudaStream_t s)
     cudaStreamSynchronize(s);
     h->ticket_base = 0;
     h->work_base = 0;
+    h->acc_state = ACC_ANY;
 }
 
 static int fetch_result(hl_handle *h, int *linesmax, hl_line *lines,
@@ -975,9 +1153,9 @@ static int plain_launch(hl_handle *h, const hl_image_desc *img, int linesmax,
         h->last_launches = 1;
         return HL_NO_ERROR;
     }
-    if ((rc = run_ab(h, roi, g, s, &launches)) != HL_NO_ERROR)
+    if ((rc = run_ab(h, roi, g, true, s, &launches)) != HL_NO_ERROR)
         return rc;
-    rc = run_c(h, g, linesmax, lines_dev, count_dev, s, &launches);
+    rc = run_c(h, g, !h->plan->add, linesmax, lines_dev, count_dev, s, &launches);
     h->last_launches = launches;
     return rc;
 }
@@ -1104,7 +1282,7 @@ extern "C" int hl_accumulator(hl_handle *h, const hl_image_desc *img,
         return rc;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     int launches = 0;
-    if ((rc = run_ab(h, roi, g, s, &launches)) != HL_NO_ERROR)
+    if ((rc = run_ab(h, roi, g, false, s, &launches)) != HL_NO_ERROR)
         return rc;
     CK(hl_launch_to_tight(h->d_acc, g.numrho, h->T, h->Tp, acc_dev, s));
     h->last_launches = launches + 1;
@@ -1129,7 +1307,7 @@ extern "C" int hl_accumulator_ref_layout(hl_handle *h, const hl_image_desc *img,
         return rc;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     int launches = 0;
-    if ((rc = run_ab(h, roi, g, s, &launches)) != HL_NO_ERROR)
+    if ((rc = run_ab(h, roi, g, false, s, &launches)) != HL_NO_ERROR)
         return rc;
     CK(hl_launch_to_ref(h->d_acc, g.numrho, h->T, h->Tp, g.rho_min,
                         g.ref_numrho, ref_dev, s));
@@ -1152,10 +1330,11 @@ extern "C" int hl_lines_from_accumulator(hl_handle *h, const int32_t *acc_dev,
     if ((rc = ensure_acc(h, g.numrho, *linesmax)) != HL_NO_ERROR)
         return rc;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    h->acc_state = ACC_ANY;
     CK(hl_launch_from_tight(acc_dev, g.numrho, h->T, h->Tp, h->d_acc, s));
     h->prof_open = 0;
     int launches = 1;
-    if ((rc = run_c(h, g, *linesmax, nullptr, nullptr, s, &launches)) !=
+    if ((rc = run_c(h, g, false, *linesmax, nullptr, nullptr, s, &launches)) !=
         HL_NO_ERROR)
         return rc;
     h->last_launches = launches;
@@ -1234,10 +1413,11 @@ extern "C" int hl_plain_points(hl_handle *h, const int *xy_dev, int n,
     pa.exact = g.numrho >= (1 << 22);
     pa.irho = (float)(1.0 / h->p.derho);
     pa.acc = h->d_acc;
+    h->acc_state = ACC_ANY;
     CK(hl_launch_vote_points(&pa, std::max(h->sms, 1), s));
     int launches = 2;
     h->prof_open = 0;
-    if ((rc = run_c(h, g, *linesmax, nullptr, nullptr, s, &launches)) !=
+    if ((rc = run_c(h, g, false, *linesmax, nullptr, nullptr, s, &launches)) !=
         HL_NO_ERROR)
         return rc;
     h->last_launches = launches;
@@ -1416,11 +1596,8 @@ struct hl_batch_ws {
     size_t cap_keys;
     unsigned long long *d_cand;    /* noted peak candidates; counter d_cnt[8] */
     size_t cap_cand;
-    int4 *d_scratch;               /* split parts' slots: win_rows x HL_SLICE */
+    unsigned char *d_scratch;      /* the vote items' slabs */
     size_t cap_scratch;
-    unsigned *d_tmask;             /* every image's admitted-tile masks */
-    size_t cap_tmask;
-    int masks_dirty;               /* the plan changed: recompute them */
     int *d_ncand;                  /* per image, zero between calls */
     size_t cap_ncand;
     int *d_cnt;
@@ -1440,20 +1617,15 @@ struct hl_batch_ws {
     /* the plan of the last call (reused while the geometry is the same) */
     std::vector<int> key;
     size_t tab_bytes;
-    size_t off_cimg, off_gimg, off_vimg, off_items, off_pimg, off_chunks,
-        off_fimg, off_merge;
-    int ngroups, ntiles, nitems, nchunks, grid, threads, win_rows;
+    size_t off_cimg, off_gimg, off_vimg, off_plan, off_pimg, off_chunks, off_fimg;
+    int ngroups, ntiles, nchunks, grid, threads, maxR;
     size_t npts_cap, acc_ints, nkeys;
     std::vector<size_t> acc_off, key_off;
     std::vector<size_t> pts_base;  /* each image's first point */
-    std::vector<int> key_cap_i, tile_base, group_base, nwin, rho_min, R,
-        ref_numrho;
-    std::vector<int4> items;
-    std::vector<hl_merge_region> merge; /* the split blocks */
-    int nslots;                    /* scratch slots of their parts */
-    int part16;                    /* 16-bit slots (hl_part16_ok for all) */
-    std::vector<size_t> tmask_off; /* each image's first mask word */
-    size_t tmask_words, max_mask_words;
+    std::vector<int> key_cap_i, tile_base, group_base, rho_min, R, ref_numrho;
+    vote_plan plan;
+    size_t acc_zero;               /* d_acc is zero between calls: its cap_acc,
+                                      or 0 when it is not */
     std::vector<int2> chunks;
     std::vector<int> group_img;
 
@@ -1481,7 +1653,7 @@ static void batch_ws_free(hl_batch_ws *b)
         return;
     void *dp[] = {b->d_pts, b->d_state, b->d_tile_off, b->d_acc, b->d_keys, b->d_cand,
                   b->d_ncand, b->d_cnt, b->d_tab, b->d_lines, b->d_counts,
-                  b->d_scratch, b->d_tmask};
+                  b->d_scratch};
     for (void *q : dp)
         if (q)
             cudaFree(q);
@@ -1515,35 +1687,6 @@ static int grow_host(unsigned char **ptr, size_t *cap, size_t need)
 
 static size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
-/* Per-image rho-window weights of the vote items on an 8 x 8 grid of cell
- * centres (the image's share of points in each (slice, window) block when
- * edges are spread evenly), in units of pixels. */
-static void batch_block_weights(const hl_handle *h, int w, int hh, int rho_min,
-                                int rows, int nwin, std::vector<double> &wt)
-{
-    const int slices = h->Tp / HL_SLICE;
-    wt.assign((size_t)slices * nwin, 0.0);
-    const int G = 8;
-    const double cell = (double)w * hh / (G * G);
-    for (int sl = 0; sl < slices; sl++) {
-        const int k0 = sl * HL_SLICE;
-        const int k1 = std::min(k0 + HL_SLICE, h->T) - 1;
-        if (k0 >= h->T)
-            continue;
-        const double th = 0.5 * (k0 + k1) * h->p.detheta;
-        const double c = cos(th), sn = sin(th);
-        for (int gy = 0; gy < G; gy++) {
-            const double y = (gy + 0.5) * hh / G;
-            for (int gx = 0; gx < G; gx++) {
-                const double x = (gx + 0.5) * w / G;
-                const int row = (int)floor((x * c + y * sn) / h->p.derho) - rho_min;
-                const int wn = std::min(std::max(row / rows, 0), nwin - 1);
-                wt[(size_t)sl + (size_t)slices * wn] += cell;   /* 32 lanes per point */
-            }
-        }
-    }
-}
-
 /* Plan a batch: sizes, offsets, work items, chunks; fills the pinned tables
  * (image pointers and thresholds included).  The geometry part is reused
  * when the sizes and the launch shape equal the previous call's. */
@@ -1551,7 +1694,6 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
                       int nimg, const int *thr, int K, hl_line *lines_dev,
                       int *counts_dev, const hl_roi *rois)
 {
-    const int slices = h->Tp / HL_SLICE;
     int maxR = 1;
     std::vector<hl_geom> gs((size_t)nimg);
     for (int i = 0; i < nimg; i++) {
@@ -1562,26 +1704,17 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
     }
     /* launch shape: the override (autotuner) or the largest window that
      * fits, 1024 threads */
-    const int maxr = hl_vote_max_rows();
-    int rows = h->win_rows_override > 0 ? std::min(h->win_rows_override, maxr)
-                                        : std::min(maxR, maxr);
-    rows = std::max(8, (rows + 7) / 8 * 8);
-    rows = std::min(rows, maxr);
-    const int threads = h->threads_override > 0 ? h->threads_override : 1024;
-    const size_t smem = hl_vote_smem_bytes(rows);
-    const int per_sm = std::max(1, std::min(2048 / threads,
-                                            (int)((228u * 1024u) / (smem + 1024))));
-    const int ctas = std::max(h->sms, 1) * per_sm;
+    const int cap = plan_cap(h), threads = vote_threads(h);
 
     std::vector<int> key;
     key.reserve(2 * (size_t)nimg + 8);
     key.push_back(nimg);
-    key.push_back(rows);
+    key.push_back(cap);
     key.push_back(threads);
     key.push_back(h->T);
-    {   /* derho sets every image's rho range */
+    for (double v : {h->p.derho, h->p.detheta}) {   /* rho range, theta table */
         unsigned long long bits;
-        memcpy(&bits, &h->p.derho, sizeof(bits));
+        memcpy(&bits, &v, sizeof(bits));
         key.push_back((int)(bits & 0xffffffffu));
         key.push_back((int)(bits >> 32));
     }
@@ -1590,15 +1723,14 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
         key.push_back(rois[i].h);
     }
     if (key != b->key) {
-        b->key = key;
-        b->win_rows = rows;
+        b->key.clear();   /* not valid until the plan below is whole */
         b->threads = threads;
+        b->maxR = maxR;
         b->acc_off.assign(nimg, 0);
         b->key_off.assign(nimg, 0);
         b->key_cap_i.assign(nimg, 0);
         b->tile_base.assign(nimg, 0);
         b->group_base.assign(nimg, 0);
-        b->nwin.assign(nimg, 0);
         b->rho_min.assign(nimg, 0);
         b->R.assign(nimg, 0);
         b->ref_numrho.assign(nimg, 0);
@@ -1607,13 +1739,7 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
         size_t acc = 0, keys = 0, pts = 0;
         b->pts_base.assign(nimg, 0);
         int tiles = 0, groups = 0;
-        b->tmask_off.assign(nimg, 0);
-        b->tmask_words = 0;
-        b->max_mask_words = 0;
-        b->masks_dirty = 1;
-        std::vector<double> allw;
-        std::vector<int2> blocks;
-        std::vector<double> wt;
+        std::vector<plan_img> pim((size_t)nimg);
         for (int i = 0; i < nimg; i++) {
             const hl_geom &g = gs[i];
             const int nt = g.tiles_x * g.tiles_y;
@@ -1639,62 +1765,20 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
             b->rho_min[i] = g.rho_min;
             b->R[i] = g.numrho;
             b->ref_numrho[i] = g.ref_numrho;
-            b->nwin[i] = (g.numrho + rows - 1) / rows;
-            {
-                const size_t mw = hl_tile_mask_words(slices, b->nwin[i], nt);
-                b->tmask_off[i] = b->tmask_words;
-                b->tmask_words += mw;
-                b->max_mask_words = std::max(b->max_mask_words, mw);
-            }
+            pim[i] = {rois[i].w, rois[i].h, g.numrho};
             for (int r0 = 0; r0 < g.numrho; r0 += HL_PEAK_ROWS)
                 b->chunks.push_back(make_int2(i, r0));
-            if ((size_t)slices * b->nwin[i] > 0xffff)
-                return HL_OP_OVERFLOW;   /* ... and the block in 16 bits */
-            batch_block_weights(h, rois[i].w, rois[i].h, g.rho_min, rows,
-                                b->nwin[i], wt);
-            for (size_t q = 0; q < wt.size(); q++) {
-                blocks.push_back(make_int2(i, (int)q));
-                allw.push_back(wt[q]);
-            }
         }
         if (nimg > 0xffff)
-            return HL_OP_OVERFLOW;   /* the item packs the image in 16 bits */
-        /* items: plan_parts over every image's blocks (a block heavier
-         * than a third of one CTA's share is split); the parts of a split
-         * block vote into scratch slots, summed into it by the merge
-         * launch */
-        std::vector<int> pieces;
-        const std::vector<vote_part> parts = plan_parts(allw, ctas, 3.0, pieces);
-        b->merge.clear();
-        std::vector<int> slot0(blocks.size(), 0), used(blocks.size(), 0);
-        int nslots = 0;
-        for (size_t q = 0; q < blocks.size(); q++) {
-            if (pieces[q] <= 1)
-                continue;
-            const int im = blocks[q].x, blk = blocks[q].y;
-            const int w0 = (blk / slices) * rows, k0 = (blk % slices) * HL_SLICE;
-            const long long off = (long long)b->acc_off[im] + (long long)w0 * h->Tp + k0;
-            slot0[q] = nslots;
-            b->merge.push_back({off / 4, std::min(rows, b->R[im] - w0), k0, nslots, pieces[q],
-                                w0, im, {0, 0}});
-            nslots += pieces[q];
-        }
-        b->items.resize(parts.size());
-        for (size_t q = 0; q < parts.size(); q++) {
-            const vote_part &p = parts[q];
-            const int slot = pieces[p.blk] > 1 ? slot0[p.blk] + used[p.blk]++ : 0;
-            b->items[q] = make_int4(blocks[p.blk].y | (blocks[p.blk].x << 16),
-                                    p.part | (p.nparts << 16), slot, 0);
-        }
-        b->nslots = nslots;
-        b->part16 = 1;
-        for (int i = 0; i < nimg; i++)
-            b->part16 &= hl_part16_ok(h->p.derho, rois[i].w, rois[i].h);
+            return HL_OP_OVERFLOW;
+        int rc = make_plan(h, pim.data(), nimg, cap, std::max(h->sms, 1), &b->plan);
+        if (rc != HL_NO_ERROR)
+            return rc;
         b->ngroups = groups;
         b->ntiles = tiles;
-        b->nitems = (int)b->items.size();
         b->nchunks = (int)b->chunks.size();
-        b->grid = std::max(1, std::min(b->nitems, ctas));
+        b->grid = std::max(1, std::min((int)b->plan.items.size(),
+                                       vote_ctas(h, b->plan.win_rows, threads)));
         b->npts_cap = pts;
         b->acc_ints = acc;
         b->nkeys = keys;
@@ -1703,12 +1787,12 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
         b->off_cimg = o;   o = align16(o + sizeof(hl_compact_img) * nimg);
         b->off_gimg = o;   o = align16(o + sizeof(int) * (size_t)groups);
         b->off_vimg = o;   o = align16(o + sizeof(hl_vote_img) * nimg);
-        b->off_items = o;  o = align16(o + sizeof(int4) * b->items.size());
-        b->off_merge = o;  o = align16(o + sizeof(hl_merge_region) * b->merge.size());
+        b->off_plan = o;   o = align16(o + plan_bytes(b->plan));
         b->off_pimg = o;   o = align16(o + sizeof(hl_peak_img) * nimg);
         b->off_chunks = o; o = align16(o + sizeof(int2) * b->chunks.size());
         b->off_fimg = o;   o = align16(o + sizeof(hl_final_img) * nimg);
         b->tab_bytes = o;
+        b->key = key;
     }
 
     /* device buffers */
@@ -1725,11 +1809,7 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
                    sizeof(unsigned long long) * b->nkeys)) != HL_NO_ERROR ||
         (rc = grow((void **)&b->d_tab, &b->cap_tab, b->tab_bytes)) != HL_NO_ERROR ||
         (rc = grow((void **)&b->d_scratch, &b->cap_scratch,
-                   sizeof(int4) * (size_t)std::max(b->nslots, 1) * b->win_rows *
-                       (HL_SLICE / 4))) != HL_NO_ERROR ||
-        (rc = grow_tracked((void **)&b->d_tmask, &b->cap_tmask,
-                           sizeof(unsigned) * std::max(b->tmask_words, (size_t)1),
-                           &b->masks_dirty)) != HL_NO_ERROR)
+                   (size_t)std::max(b->plan.scratch_units, 1LL) * 64)) != HL_NO_ERROR)
         return rc;
     if (b->cap_ncand < sizeof(int) * (size_t)nimg || !b->d_ncand) {
         if ((rc = grow((void **)&b->d_ncand, &b->cap_ncand, sizeof(int) * (size_t)nimg)) !=
@@ -1770,9 +1850,8 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
         vi[i].h = rois[i].h;
         vi[i].rho_min = g.rho_min;
         vi[i].R = g.numrho;
-        vi[i].nwin = b->nwin[i];
         vi[i].threshold = thr ? thr[i] : h->p.threshold;
-        vi[i].tmask = b->d_tmask + b->tmask_off[i];
+        vi[i].pad = 0;
         vi[i].acc = b->d_acc + b->acc_off[i];
         pi[i].acc = b->d_acc + b->acc_off[i];
         pi[i].keys = b->d_keys + b->key_off[i];
@@ -1791,9 +1870,7 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
         fi[i].count_out = counts_dev + i;
     }
     memcpy(t + b->off_gimg, b->group_img.data(), sizeof(int) * b->group_img.size());
-    memcpy(t + b->off_items, b->items.data(), sizeof(int4) * b->items.size());
-    if (!b->merge.empty())
-        memcpy(t + b->off_merge, b->merge.data(), sizeof(hl_merge_region) * b->merge.size());
+    plan_copy(b->plan, t + b->off_plan);
     memcpy(t + b->off_chunks, b->chunks.data(), sizeof(int2) * b->chunks.size());
     return HL_NO_ERROR;
 }
@@ -1840,33 +1917,21 @@ static int batch_enqueue_vote_peaks(hl_handle *h, hl_batch_ws *b, cudaStream_t s
     va.sinv = h->d_sin;
     va.T = h->T;
     va.Tp = h->Tp;
-    va.win_rows = b->win_rows;
     va.irho = (float)(1.0 / h->p.derho);   /* okano_3_0/HoughLine.cu:107 */
     va.status = b->d_cnt + 2;
-    va.items = reinterpret_cast<const int4 *>(dt + b->off_items);
-    va.nitems = b->nitems;
-    va.scratch = b->d_scratch;
-    va.part16 = b->part16;
     /* the counter is cleared with the others at the start of every call */
-    va.cand = cand_list(b->d_cand, b->cap_cand, b->d_cnt + 8);
+    va.cand = b->plan.add ? cand_list(nullptr, 0, nullptr)
+                          : cand_list(b->d_cand, b->cap_cand, b->d_cnt + 8);
     va.work = reinterpret_cast<unsigned *>(b->d_cnt + 1);
     va.work_base = 0;
+    hl_merge_args ma;
+    memset(&ma, 0, sizeof(ma));
+    plan_args(b->plan, dt + b->off_plan, b->d_scratch, &va, &ma);
+    if (va.add)
+        CK(cudaMemsetAsync(b->d_acc, 0, sizeof(int32_t) * b->acc_ints, s));
     CK(hl_launch_vote(&va, b->threads, b->grid, s));
-    if (!b->merge.empty()) {
-        hl_merge_args ma;
-        ma.acc = reinterpret_cast<int4 *>(b->d_acc);
-        ma.pitch4 = h->Tp / 4;
-        ma.T = h->T;
-        ma.scratch = b->d_scratch;
-        ma.slot4 = hl_slot4(b->win_rows, b->part16);
-        ma.regs = reinterpret_cast<const hl_merge_region *>(dt + b->off_merge);
-        ma.nreg = (int)b->merge.size();
-        ma.part16 = b->part16;
-        ma.pimgs = reinterpret_cast<const hl_peak_img *>(dt + b->off_pimg);
-        ma.thr0 = 0;
-        ma.cand = va.cand;
-        CK(hl_launch_merge(&ma, b->win_rows, s));
-    }
+    if (ma.nblocks > 0)
+        CK(hl_launch_merge(&ma, b->maxR, s));
     prof_mark(h, 2, s);
 
     hl_peak_args pa;
@@ -1883,8 +1948,9 @@ static int batch_enqueue_vote_peaks(hl_handle *h, hl_batch_ws *b, cudaStream_t s
     return HL_NO_ERROR;
 }
 
-/* rank, merge and write the lines of every image */
-static int batch_enqueue_finalize(hl_handle *h, hl_batch_ws *b, int nimg, int K,
+/* rank, merge and write the lines of every image; voted: clear the bins that
+ * the vote stored */
+static int batch_enqueue_finalize(hl_handle *h, hl_batch_ws *b, int nimg, int K, bool voted,
                                   cudaStream_t s)
 {
     unsigned char *dt = b->d_tab;
@@ -1898,6 +1964,13 @@ static int batch_enqueue_finalize(hl_handle *h, hl_batch_ws *b, int nimg, int K,
     fa.linesmax = K;
     fa.hdr = nullptr;
     fa.status = b->d_cnt + 2;
+    if (voted && !b->plan.add) {
+        fa.clear = cand_list(b->d_cand, b->cap_cand, b->d_cnt + 8);
+        fa.clear_imgs = reinterpret_cast<const hl_peak_img *>(dt + b->off_pimg);
+        fa.acc = b->d_acc;
+        fa.acc_ints = (long long)b->acc_ints;
+        fa.Tp = h->Tp;
+    }
     CK(hl_launch_finalize(&fa, nimg, s));
     prof_mark(h, 4, s);
     return HL_NO_ERROR;
@@ -1910,7 +1983,7 @@ static int batch_enqueue(hl_handle *h, hl_batch_ws *b, int nimg, int K,
     if ((rc = batch_enqueue_compact(h, b, nimg, s)) != HL_NO_ERROR ||
         (rc = batch_enqueue_vote_peaks(h, b, s)) != HL_NO_ERROR)
         return rc;
-    return batch_enqueue_finalize(h, b, nimg, K, s);
+    return batch_enqueue_finalize(h, b, nimg, K, true, s);
 }
 
 static int batch_run_ws(hl_handle *h, hl_batch_ws **pb, const hl_image_desc *imgs,
@@ -1940,23 +2013,9 @@ static int batch_run_ws(hl_handle *h, hl_batch_ws **pb, const hl_image_desc *img
         CK(cudaEventCreateWithFlags(&b->tab_read, cudaEventDisableTiming));
         b->tab_event = 1;
     }
-    if (b->masks_dirty) {
-        /* tile masks of the new plan, outside the (captured) pipeline: the
-         * image table they read is the one the pipeline uploads again */
-        CK(cudaMemcpyAsync(b->d_tab + b->off_vimg, b->h_tab + b->off_vimg,
-                           sizeof(hl_vote_img) * (size_t)nimg, cudaMemcpyHostToDevice, s));
-        hl_vote_args va;
-        memset(&va, 0, sizeof(va));
-        va.imgs = reinterpret_cast<const hl_vote_img *>(b->d_tab + b->off_vimg);
-        va.cosv = h->d_cos;
-        va.sinv = h->d_sin;
-        va.T = h->T;
-        va.Tp = h->Tp;
-        va.win_rows = b->win_rows;
-        va.irho = (float)(1.0 / h->p.derho);
-        CK(hl_launch_tile_masks(&va, nimg, b->max_mask_words, s));
-        b->masks_dirty = 0;
-    }
+    if (b->acc_zero != b->cap_acc && !b->plan.add)   /* outside the (captured) pipeline */
+        CK(cudaMemsetAsync(b->d_acc, 0, b->cap_acc, s));
+    b->acc_zero = 0;
     prof_mark(h, 0, s);
     if (!h->batch_graph || h->prof) {
         rc = batch_enqueue(h, b, nimg, K, s);
@@ -1971,7 +2030,6 @@ static int batch_run_ws(hl_handle *h, hl_batch_ws **pb, const hl_image_desc *img
         gk.push_back((long long)(uintptr_t)b->d_tab);
         gk.push_back((long long)(uintptr_t)b->h_tab);
         gk.push_back((long long)(uintptr_t)b->d_keys);
-        gk.push_back((long long)(uintptr_t)b->d_tmask);
         gk.push_back((long long)(uintptr_t)b->d_scratch);
         gk.push_back((long long)(uintptr_t)b->d_cand);
         if (!b->gexec || gk != b->gkey) {
@@ -2003,8 +2061,10 @@ static int batch_run_ws(hl_handle *h, hl_batch_ws **pb, const hl_image_desc *img
         CK(cudaGraphLaunch(b->gexec, s));
         h->last_launches = 4;
     }
-    if (rc == HL_NO_ERROR)
+    if (rc == HL_NO_ERROR) {
+        b->acc_zero = b->plan.add ? 0 : b->cap_acc;   /* the tail clears what is stored */
         CK(cudaEventRecord(b->tab_read, s));
+    }
     return rc;
 }
 
@@ -2405,7 +2465,7 @@ extern "C" int hl_proposal_batch(hl_handle *h, hl_net *net,
     wa.status = pw->d_cnt + 1;
     wa.nk_fast = nk_fast;
     CK(hl_launch_window_vote(&wa, (int)max_bins, std::max(1, h->sms) * 6, s));
-    if ((rc = batch_enqueue_finalize(h, b, nimg, K, s)) != HL_NO_ERROR)
+    if ((rc = batch_enqueue_finalize(h, b, nimg, K, false, s)) != HL_NO_ERROR)
         return rc;
     CK(cudaEventRecord(b->tab_read, s));
 

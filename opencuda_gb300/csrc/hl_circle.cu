@@ -278,7 +278,7 @@ hl_circle_tile_kernel(hl_circle_tile_args a0)
                             hi = mid - 1;
                     }
                     const float2 pt = a.pts[sm.start[lo] + (i - sm.pre[lo])];
-                    /* the compaction's sentinel of an odd tile is 1e30 */
+                    /* the compaction's sentinel of an odd tile is infinite */
                     if (pt.x < 1.0e29f) {
                         const int px = (int)pt.x, py = (int)pt.y;
                         ok = px >= hx0 && px <= hx1 && py >= hy0 && py <= hy1;

@@ -160,75 +160,73 @@ __device__ __forceinline__ void diag_table(DiagTab &t, const float *cs, const fl
     }
 }
 
-/* The 8 steps of one point (x, y) on this lane.  rho per the vote rule
- * (okano_3_0/HoughLine.cu:115-121), the row relative to the window clamped
- * to the dump row `lim`; float -> integer by the magic constant (CV_FLOOR /
- * CV_CEIL, CV_SIGN, see RHO_MAGIC) or by the exact conversion (CV_EXACT). */
+/* rho of one point for the lane's columns of steps 2i and 2i + 1, per the
+ * vote rule (okano_3_0/HoughLine.cu:115-121), as the bit patterns of the
+ * magic-constant sums (see RHO_MAGIC): floor, ceil, or truncation by the sign */
+template <bool UNIT, int CV>
+__device__ __forceinline__ void diag_bits(f2x X, f2x Y, const f2x &c, const f2x &s, f2x ir,
+                                          unsigned &r0, unsigned &r1)
+{
+    const f2x M = f2_pack(RHO_MAGIC, RHO_MAGIC);
+    f2x a = f2_mul(X, c), b = f2_mul(Y, s);
+    if (!UNIT) {
+        a = f2_mul(a, ir);
+        b = f2_mul(b, ir);
+    }
+    const f2x v = f2_add(a, b);
+    if (CV == CV_FLOOR) {
+        f2_unpack(f2_add_rz(v, M), r0, r1);
+    } else if (CV == CV_CEIL) {
+        f2_unpack(f2_add_rp(v, M), r0, r1);
+    } else {
+        unsigned u0, u1, f0, f1, c0, c1;
+        f2_unpack(v, u0, u1);
+        f2_unpack(f2_add_rz(v, M), f0, f1);
+        f2_unpack(f2_add_rp(v, M), c0, c1);
+        const unsigned s0 = (unsigned)((int)u0 >> 31), s1 = (unsigned)((int)u1 >> 31);
+        r0 = (c0 & s0) | (f0 & ~s0);
+        r1 = (c1 & s1) | (f1 & ~s1);
+    }
+}
+
+/* The 8 steps of one point (x, y) on this lane; the row relative to the window
+ * (`base` is the magic constant's bits plus the rho of row 0) clamped to the
+ * dump row `lim`, or by the exact conversion (CV_EXACT, `base` the rho). */
 template <bool UNIT, int CV>
 __device__ __forceinline__ void diag_point(float x, float y, const DiagTab &t, f2x ir,
                                            int base, unsigned lim)
 {
     const f2x X = f2_pack(x, x), Y = f2_pack(y, y);
-    const f2x M = f2_pack(RHO_MAGIC, RHO_MAGIC);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        f2x a = f2_mul(X, t.c[i]), b = f2_mul(Y, t.s[i]);
-        if (!UNIT) {
-            a = f2_mul(a, ir);
-            b = f2_mul(b, ir);
-        }
-        const f2x v = f2_add(a, b);
         unsigned r0, r1;
-        if (CV == CV_FLOOR) {
-            f2_unpack(f2_add_rz(v, M), r0, r1);
-        } else if (CV == CV_CEIL) {
-            f2_unpack(f2_add_rp(v, M), r0, r1);
-        } else if (CV == CV_SIGN) {
-            unsigned u0, u1, f0, f1, c0, c1;
-            f2_unpack(v, u0, u1);
-            f2_unpack(f2_add_rz(v, M), f0, f1);
-            f2_unpack(f2_add_rp(v, M), c0, c1);
-            const unsigned s0 = (unsigned)((int)u0 >> 31), s1 = (unsigned)((int)u1 >> 31);
-            r0 = (c0 & s0) | (f0 & ~s0);
-            r1 = (c1 & s1) | (f1 & ~s1);
-        } else {
+        if (CV == CV_EXACT) {
+            f2x a = f2_mul(X, t.c[i]), b = f2_mul(Y, t.s[i]);
+            if (!UNIT) {
+                a = f2_mul(a, ir);
+                b = f2_mul(b, ir);
+            }
             unsigned u0, u1;
-            f2_unpack(v, u0, u1);
+            f2_unpack(f2_add(a, b), u0, u1);
             r0 = (unsigned)__float2int_rz(__uint_as_float(u0));
             r1 = (unsigned)__float2int_rz(__uint_as_float(u1));
+        } else {
+            diag_bits<UNIT, CV>(X, Y, t.c[i], t.s[i], ir, r0, r1);
         }
         red_smem(t.col[2 * i] + 128u * min(r0 - (unsigned)base, lim));
         red_smem(t.col[2 * i + 1] + 128u * min(r1 - (unsigned)base, lim));
     }
 }
 
-
-/* Notes the bins of one int4 of counts whose bit is set in bits (bin
- * idx0 + j for bit j, j < 4) as peak candidates of image img; once the list
- * is full (the peak pass then scans every accumulator) a bin costs one
- * load. */
-__device__ __forceinline__ void note_cands(const hl_cand_list &c, int img, unsigned idx0,
-                                           unsigned bits)
+/* Notes bin idx of image img as a peak candidate; once the list is full (the
+ * peak pass then scans every accumulator) a bin costs one load. */
+__device__ __forceinline__ void note_cand(const hl_cand_list &c, int img, unsigned idx)
 {
     if (*(volatile int *)c.count >= c.cap)
         return;
-    while (bits) {
-        const int j = __ffs(bits) - 1;
-        bits &= bits - 1;
-        const int pos = atomicAdd(c.count, 1);
-        if (pos < c.cap)
-            c.e[pos] = ((unsigned long long)(unsigned)img << 32) | (idx0 + (unsigned)j);
-    }
-}
-
-/* bits of the bins of v above thr, bins kq + j >= T (padding) left out */
-__device__ __forceinline__ unsigned above4(const int4 &v, int thr, int kq, int T)
-{
-    unsigned b = (unsigned)(v.x > thr) | ((unsigned)(v.y > thr) << 1) |
-                 ((unsigned)(v.z > thr) << 2) | ((unsigned)(v.w > thr) << 3);
-    if (kq + 3 >= T)
-        b &= (T > kq) ? (1u << (T - kq)) - 1u : 0u;
-    return b;
+    const int pos = atomicAdd(c.count, 1);
+    if (pos < c.cap)
+        c.e[pos] = ((unsigned long long)(unsigned)img << 32) | idx;
 }
 
 #endif

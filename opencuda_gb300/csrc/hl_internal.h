@@ -83,27 +83,65 @@ typedef struct hl_compact_args {
 typedef struct hl_vote_img {
     const float2 *pts;        /* (x, y) of every edge point, tile-major */
     const int *tile_off;      /* the image's [ntiles + 1] tile offsets */
-    /* admitted tiles of every (slice, window) block: bit t % 32 of word
-     * [block][t / 32] (hl_launch_tile_masks; they depend on the geometry
-     * only) */
-    unsigned *tmask;
     int ntiles, tiles_x;
-    int w, h;                 /* ROI size (tile clipping) */
+    int w, h;                 /* ROI size */
     int rho_min, R;
-    int nwin;                 /* rho windows of win_rows rows */
     int threshold;            /* peak threshold: bins above it are noted */
-    int32_t *acc;             /* [R][Tp] */
+    int pad;
+    /* [R][Tp], zero at the launch: with a candidate list the bins above the
+     * threshold are stored, without one every row that a vote can reach */
+    int32_t *acc;
 } hl_vote_img;
+
+/* One work item of the vote: a rectangle of an image's compaction tiles (a
+ * region) voted for one theta slice.  Every theta's window of rows starts at
+ * the lowest rho the rectangle reaches, so `rows` of them hold every vote.
+ * win > 0 or clip: a rectangle of one tile whose range needs several windows
+ * (rho steps far below a pixel); votes outside the window are dropped. */
+typedef struct hl_vote_item {
+    int img, slice;
+    int tx, ty;               /* first tile | tiles << 16 */
+    int slab;                 /* scratch slab, 64-byte units; -1: the block's
+                                 only item (or hl_vote_args.add) */
+    int ncap;                 /* the slab's row groups per column group */
+    int win, clip;
+    /* nseg > 1: a whole image whose range does not fit one window, voted in
+     * nseg segments with the window sliding by adv rows after each: segment j
+     * holds the tiles whose centre lies, at the slice's middle theta, [j adv,
+     * (j + 1) adv) above -half from the image's centre; column k's row 0 is
+     * floor(rho of the centre at theta_k) + off0 + j adv */
+    int nseg, adv, off0;
+    float half;
+} hl_vote_item;
+
+/* A slab of scratch: the counts of an item as its block's merge reads them.
+ * Four groups of 8 columns; group g holds the accumulator rows [4 b[g],
+ * 4 (b[g] + n[g])) in row groups of four, [row group][column][4 rows], 16-bit
+ * counts (64 bytes a row group) or 32-bit ones (128).  The header comes
+ * first, 64 bytes. */
+typedef struct hl_slab_hdr {
+    int b[4], n[4];
+    int pad[8];
+} hl_slab_hdr;
+static inline long long hl_slab_units(int ncap, int part16)
+{
+    return 1 + 4LL * ncap * (part16 ? 1 : 2);
+}
+/* rows and angles of slack a slab's capacity needs past its rows: a group's
+ * base is rounded down to four rows */
+#define HL_SLAB_SLACK 8
 
 /* Peak candidates of a launch: every accumulator bin above its image's
  * threshold, noted as image << 32 | (row * T + theta) when its final count
- * is stored (the vote's block store, the merge of a split block).  A
- * counter past cap means some were not noted: the peak pass then scans
- * every accumulator instead.  The counter is zero at the vote's start (the
- * batch clears it with its other counters); e == NULL: nothing is noted. */
+ * is stored (the vote's block store, the merge of a split block); the other
+ * bins stay zero.  A counter past cap means some were not noted: the peak pass
+ * then scans every accumulator instead.  The counter is zero at the vote's
+ * start (a batch clears it with its other counters; single images alternate
+ * between two, and a call's tail clears the next one's); e == NULL: nothing is
+ * noted and whole accumulators are stored. */
 typedef struct hl_cand_list {
     unsigned long long *e;
-    int *count;               /* cleared by the compaction launch */
+    int *count;
     int cap;
     int pad;
 } hl_cand_list;
@@ -113,84 +151,65 @@ typedef struct hl_vote_args {
     hl_vote_img img0;
     const float *cosv, *sinv; /* [theta_pad] */
     int T, Tp;
-    int win_rows;             /* rho window per work item */
+    int win_rows;             /* rows of a window in shared memory */
     float irho;
+    int exact;                /* |rho| may reach 2^22: convert exactly */
     int *status;
-    /* persistent scheduling: work items are taken in the order items[]
-     * (heaviest first) from a monotonically increasing counter.  An item is
-     * one part of a (slice, window) block of one image: .x = block | image
-     * << 16 with block = slice + nslices * window, .y = part | nparts << 16,
-     * .z = the part's scratch slot when nparts > 1, .w = 0.  A whole block
-     * is stored into the accumulator; a part of a split block stores its
-     * counts to its slot, and hl_merge_kernel adds the parts' slots into the
-     * block afterwards. */
-    const int4 *items;
+    /* persistent scheduling: items are taken in order (heaviest first) from a
+     * monotonically increasing counter */
+    const hl_vote_item *items;
     int nitems;
     unsigned *work;           /* counter */
     unsigned work_base;       /* its value at launch */
-    int4 *scratch;            /* slots of win_rows x HL_SLICE counts */
-    /* nonzero: a slot holds 16-bit counts (two per word; the host sets it
-     * when no bin can reach 2^16 votes, see hl_part16_ok), half the bytes */
-    int part16;
+    unsigned char *scratch;   /* slabs, 64-byte units */
+    int part16;               /* slabs hold 16-bit counts (hl_part16_ok) */
+    int add;                  /* no slabs: items add to the cleared accumulator */
     hl_cand_list cand;
 } hl_vote_args;
 
-/* A split vote block: its accumulator region (rows x 8 int4 from off4, rows
- * pitch4 apart, first theta k0) is the sum of nparts scratch slots from
- * slot0 on. */
-typedef struct hl_merge_region {
-    long long off4;
-    int rows, k0;
-    int slot0, nparts;
-    int w0;                   /* first row of the block in its image */
-    int img;                  /* its image */
-    int pad[2];
-} hl_merge_region;
-
-struct hl_peak_img;
+/* A block (an image's theta slice) voted in several items: its accumulator
+ * columns are the sum of the slabs [first, first + n) of the slab list. */
+typedef struct hl_merge_block {
+    int img, slice;
+    int first, n;
+} hl_merge_block;
 
 typedef struct hl_merge_args {
-    int4 *acc;
-    int pitch4;
-    int T;
-    const int4 *scratch;
-    long long slot4;          /* int4 per scratch slot */
-    const hl_merge_region *regs;
-    int nreg;
-    int part16;               /* slots hold 16-bit counts (hl_vote_args) */
-    /* the peak threshold of region r: pimgs[r.img].threshold, or thr0 */
-    const struct hl_peak_img *pimgs;
-    int thr0;
+    const hl_vote_img *imgs;  /* as in hl_vote_args */
+    hl_vote_img img0;
+    int T, Tp;
+    const unsigned char *scratch;
+    const hl_merge_block *blocks;
+    int nblocks;
+    unsigned chunks;          /* CTAs a block (set by the launcher) */
+    const int2 *slabs;        /* {slab, ncap} */
+    int part16;
     hl_cand_list cand;
 } hl_merge_args;
 
-/* Can a split part's counts be kept in 16 bits?  A bin of one rho bin width
+struct hl_peak_img;
+
+/* Can an item's counts be kept in 16 bits?  A bin of one rho bin width
  * derho (the rho-0 bin spans two, truncation toward zero) holds the pixels of
- * a strip of width <= 2 derho across the ROI: fewer than (2 derho + 2)(w + h)
- * of them. */
+ * a strip of width <= 2 derho across the region: fewer than (2 derho + 2)
+ * (w + h) of them. */
 static inline int hl_part16_ok(double derho, int w, int h)
 {
     return (2.0 * derho + 2.0) * ((double)w + (double)h) < 65535.0;
-}
-/* int4 per scratch slot of a launch */
-#ifdef __CUDACC__
-__host__ __device__
-#endif
-static inline long long hl_slot4(int win_rows, int part16)
-{
-    return (long long)win_rows * (HL_SLICE / 4) / (part16 ? 2 : 1);
 }
 
 /* Tiles the allocation-free compaction entry point can serve. */
 #define HL_NOALLOC_MAX_TILES 65536
 
-/* Vote-kernel staging: points per consumer warp per batch, points per ring
- * slot (at most 31 consumer warps), ring slots, tiles per coarse-filter
- * group. */
-#define HL_VOTE_PPW 64
-#define HL_VOTE_CHUNK (HL_VOTE_PPW * 32)
-#define HL_VOTE_SLOTS 3
-#define HL_VOTE_TG 4096
+/* Vote-kernel staging: points per ring slot, ring slots; tile rows of a region
+ * at most (unless it spans the image's width: then its points are one run). */
+#ifndef HL_VOTE_CHUNK
+#define HL_VOTE_CHUNK 2048
+#endif
+#ifndef HL_VOTE_SLOTS
+#define HL_VOTE_SLOTS 2
+#endif
+#define HL_VOTE_RUNS 128
 /* largest rho window (rows) one CTA can hold next to its staging */
 int hl_vote_max_rows(void);
 
@@ -247,6 +266,15 @@ typedef struct hl_final_args {
     int linesmax;
     hl_result_hdr *hdr;       /* out (one image), or NULL */
     int *status;              /* read; reset to 0 when hdr is set */
+    /* the bins that the vote stored above the threshold, cleared again (the
+     * whole accumulator when they did not all fit the list); e NULL: none */
+    hl_cand_list clear;
+    const hl_peak_img *clear_imgs;   /* per image, or NULL: acc */
+    int32_t *acc;                    /* acc_ints of them */
+    long long acc_ints;
+    int Tp;
+    int *cand_count;          /* another call's candidate counter, reset to 0
+                                 for the next one (or NULL) */
 } hl_final_args;
 
 /* The whole plain path of one small image in one cluster launch (see
@@ -371,16 +399,7 @@ cudaError_t hl_launch_compact(const hl_compact_args *a, cudaStream_t s);
  * one to the ticket word */
 int hl_compact_persist_ctas(int ntiles, int sms);
 cudaError_t hl_launch_compact_persist(const hl_compact_args *a, int nct, cudaStream_t s);
-/* Tile masks of every image of a vote launch (nimg images: a->imgs, or
- * a->img0 when it is NULL); the vote kernel reads them. */
-cudaError_t hl_launch_tile_masks(const hl_vote_args *a, int nimg,
-                                 size_t max_words, cudaStream_t s);
-/* words of an image's tile mask */
-static inline size_t hl_tile_mask_words(int nslices, int nwin, int ntiles)
-{
-    return (size_t)nslices * nwin * ((ntiles + 31) / 32);
-}
-cudaError_t hl_launch_merge(const hl_merge_args *a, int max_rows, cudaStream_t s);
+cudaError_t hl_launch_merge(hl_merge_args *a, int max_R, cudaStream_t s);
 cudaError_t hl_launch_vote(const hl_vote_args *a, int threads, int grid,
                            cudaStream_t s);
 size_t hl_vote_smem_bytes(int win_rows);

@@ -394,10 +394,10 @@ hl_compact_kernel(hl_compact_args a)
         }
     }
 #undef CT_TILE_XY
-    /* the sentinel (1e30, 0) never votes inside an accumulator: its rho is
-     * 1e30 * cos(theta_k), and cosf of a float angle is never 0 */
+    /* the sentinel (+infinity, 0) never votes inside an accumulator: its rho is
+     * infinity * cos(theta_k), and cosf of a float angle is never 0 */
     if (a.pts_f2 && tid < CT_GROUP && (s_tcnt[tid] & 1))
-        a.pts_f2[s_im.pts_base + s_tbase[tid] + s_tcnt[tid]] = make_float2(1.0e30f, 0.0f);
+        a.pts_f2[s_im.pts_base + s_tbase[tid] + s_tcnt[tid]] = make_float2(__int_as_float(0x7f800000), 0.0f);
 }
 
 /* Single-image compaction with few, large CTAs: CTA c of nct takes tiles [ntiles c / nct, ntiles (c + 1) / nct) -- at most CP_MAXT --
@@ -632,12 +632,12 @@ hl_compact_persist_kernel(hl_compact_args a, int nct)
             pos++;
         }
     }
-    /* the sentinel (1e30, 0) of an odd float2 tile never votes inside an
+    /* the sentinel (+infinity, 0) of an odd float2 tile never votes inside an
      * accumulator (see hl_compact_kernel) */
     if (pad && tid < nt) {
         const int cq = s_tstart[tid + 1] - s_tstart[tid];
         if (cq & 1)
-            a.pts_f2[excl + s_tbase[tid] + cq] = make_float2(1.0e30f, 0.0f);
+            a.pts_f2[excl + s_tbase[tid] + cq] = make_float2(__int_as_float(0x7f800000), 0.0f);
     }
 }
 

@@ -7,8 +7,9 @@
  * arrays to the host and ranks / merges there (:781-948).  Here:
  *   hl_peaks_kernel   -- bounds-checked peak rule, peaks appended as
  *                        64-bit keys (votes << 32 | ~index): over the bins
- *                        the vote noted above the threshold (batches), or one
- *                        read of acc[R][Tp] (one image; HBM / L2 bound);
+ *                        the vote noted above the threshold, or one read of
+ *                        acc[R][Tp] (more of them than the list holds, or a
+ *                        given accumulator; HBM / L2 bound);
  *   hl_finalize_kernel -- one CTA: top-M selection (MSD radix select when the
  *                        peaks exceed one 1024-key chunk), rank sort of the
  *                        chunk (keys are unique), the reference's float
@@ -460,6 +461,8 @@ __device__ void finalize_report(const hl_final_args &a, const hl_final_img &im, 
     if (im.count_out)
         *im.count_out = cnt;
     *im.ncand = 0;
+    if (a.cand_count)
+        *a.cand_count = 0;
     if (ncand_raw > im.cap)
         atomicOr(a.status, HL_ST_CAND_OVERFLOW);
     if (a.hdr) {   /* one image: report and clear the status word */
@@ -583,17 +586,45 @@ __device__ void finalize_cta(const hl_final_args &a, const hl_final_img &im, flo
         finalize_report(a, im, S, ncand_raw);
 }
 
+/* Clears the accumulator bins that the vote stored, part `part` of `parts`: the
+ * listed ones, or everything when the list overflowed.  The peak pass is over. */
+__device__ __forceinline__ void clear_bins(const hl_final_args &a, int part, int parts)
+{
+    const int nc = *a.clear.count;
+    if (nc <= a.clear.cap) {
+        for (int j = part * FIN_THREADS + threadIdx.x; j < nc; j += parts * FIN_THREADS) {
+            const unsigned long long e = a.clear.e[j];
+            const unsigned idx = (unsigned)e;
+            const unsigned row = idx / (unsigned)a.T, k = idx % (unsigned)a.T;
+            int32_t *acc = a.clear_imgs ? const_cast<int32_t *>(a.clear_imgs[e >> 32].acc) : a.acc;
+            acc[(size_t)row * a.Tp + k] = 0;
+        }
+    } else {
+        int4 *p = reinterpret_cast<int4 *>(a.acc);
+        for (long long i = (long long)part * FIN_THREADS + threadIdx.x; i < a.acc_ints / 4;
+             i += (long long)parts * FIN_THREADS)
+            p[i] = make_int4(0, 0, 0, 0);
+    }
+}
+
 __global__ void __launch_bounds__(FIN_THREADS)
-hl_finalize_kernel(hl_final_args a, float scale)
+hl_finalize_kernel(hl_final_args a, int nimg, float scale)
 {
     extern __shared__ __align__(16) unsigned char fin_raw[];
     FinSmem &sm = *reinterpret_cast<FinSmem *>(fin_raw);
     hl_pdl_begin();
+    if (a.clear.e)
+        clear_bins(a, blockIdx.x, gridDim.x);
+    if ((int)blockIdx.x >= nimg)
+        return;
     const hl_final_img im = a.imgs ? a.imgs[blockIdx.x] : a.img0;  /* CTA = image */
     finalize_cta(a, im, scale, sm);
 }
 
 #define FIN_CLUSTER 8
+/* CTAs of a tail that clears bins at least: only an overflowing list (a
+ * threshold that does not separate) needs them all */
+#define FIN_CLEAR_CTAS 128
 
 /* One image on a cluster of FIN_CLUSTER CTAs (one per SM) when its peaks
  * fit one chunk: every CTA loads the keys, ranks an eighth of them into
@@ -611,6 +642,10 @@ hl_finalize_cluster_kernel(hl_final_args a, float scale)
     const int rank = (int)cl.block_rank();
     const int tid = threadIdx.x;
     hl_pdl_begin();
+    if (blockIdx.x >= FIN_CLUSTER) {   /* the other clusters clear, the first ranks */
+        clear_bins(a, (int)blockIdx.x - FIN_CLUSTER, (int)gridDim.x - FIN_CLUSTER);
+        return;
+    }
     const hl_final_img im = a.img0;
     const int ncand_raw = *im.ncand;
     const int n = min(ncand_raw, im.cap);
@@ -668,15 +703,17 @@ cudaError_t hl_launch_finalize(const hl_final_args *a, int nimg, cudaStream_t s)
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess)
             return e;
-        return hl_launch_pdl(hl_finalize_cluster_kernel, dim3(FIN_CLUSTER), dim3(FIN_THREADS),
+        return hl_launch_pdl(hl_finalize_cluster_kernel,
+                             dim3(a->clear.e ? FIN_CLEAR_CTAS : FIN_CLUSTER), dim3(FIN_THREADS),
                              smem, s, false, *a, scale);
     }
     e = cudaFuncSetAttribute(hl_finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
     if (e != cudaSuccess)
         return e;
-    return hl_launch_pdl(hl_finalize_kernel, dim3(nimg), dim3(FIN_THREADS), smem, s, false, *a,
-                         scale);
+    return hl_launch_pdl(hl_finalize_kernel,
+                         dim3(a->clear.e ? std::max(nimg, FIN_CLEAR_CTAS) : nimg),
+                         dim3(FIN_THREADS), smem, s, false, *a, nimg, scale);
 }
 
 /* ---- one small image in one launch ----------------------------------------

@@ -8,47 +8,65 @@
  * toward zero (the reference's +-0.5 step after the (int) cast is a no-op),
  * and cos_k/sin_k come from the GPU-evaluated table.
  *
- * Work decomposition.  A work item is one (theta slice, rho window) block of
- * the accumulator, held in shared memory as acc[row][column]: 32 thetas x
- * win_rows rho bins.  A warp votes 8 points at a time on the diagonal
- * schedule (DiagTab): at every step its 32 lanes add to 32 different theta
- * columns -- 32 different banks -- so every shared-memory reduction is
- * conflict-free and no two lanes ever hit one address (the aggregation a
- * warp-aggregated atomic would buy is built into the layout).
+ * Work decomposition.  A work item is one theta slice (32 thetas) of one
+ * region of the image, a rectangle of compaction tiles.  Its counts live in
+ * shared memory as acc[row][column], where each column's rows start at the
+ * lowest rho the rectangle reaches at that theta: over the slice the windows
+ * follow the rectangle's sinusoid, so about its diagonal's number of rows holds
+ * every vote of its points.  No vote falls outside and none is executed twice
+ * -- fixed rho windows over all points executed 1.4 to 1.6 votes a useful one,
+ * a tile being voted by every window its rho range over the slice meets.
+ * A warp votes 8 points at a time on the diagonal schedule (DiagTab): at every
+ * step its 32 lanes add to 32 different theta columns -- 32 different banks --
+ * so every shared-memory reduction is conflict-free and no two lanes ever hit
+ * one address.
  *
  * Pipeline.  Persistent CTAs of one producer warp and consumer warps that
  * meet only on mbarriers.  The producer takes items heaviest-first from a
- * global counter.  For an item it reads the block's tile mask -- the 128x32
- * compaction tiles whose rho interval over the slice meets the window,
- * computed once per geometry by hl_tile_mask_kernel -- and turns it into
- * runs of tiles: contiguous ranges of the tile-major point list, 16-byte
- * aligned because the compaction pads every tile to an even number of
- * float2 entries.  The runs, laid end to end, form the item's point stream.
- * It publishes the item as a segment (double-buffered descriptor) and
- * streams it: a batch is HL_VOTE_PPW points per consumer warp, batch b the stream
- * range [b*B, (b+1)*B); the producer's lanes each copy one run's part of it
- * into a ring of HL_VOTE_SLOTS shared-memory slots with cp.async.bulk (TMA
- * bulk copies completing on the slot's full barrier), so a slot holds its
- * batch gap-free; consumer warp i votes points [PPW i, PPW i + PPW) of the slot
- * straight from shared memory and arrives on the slot's empty barrier, which
- * the producer waits on before refilling it.  The producer moves on to the
- * next item as soon as the current one is issued, so its setup and first
- * copies overlap the consumers' last batches.
- * When an item is voted the consumers store the block with coalesced
- * 128-byte rows into acc[R][Tp] (a part of a split block: into its scratch
- * slot, summed into the block by hl_merge_kernel) and clear it; every bin is
- * written exactly once, so the accumulator needs no clearing.
+ * global counter.  For an item it evaluates the vote rule at the rectangle's
+ * corners (every rounded step is monotone in x and in y, so they bound every
+ * point's rho exactly), reads the point offsets of the rectangle's tile rows
+ * -- contiguous ranges of the tile-major point list, 16-byte aligned because
+ * the compaction pads every tile to an even number of float2 entries -- and
+ * publishes it as a segment (double-buffered descriptor).  The runs, laid end
+ * to end, form the item's point stream: it is copied in batches into a ring of
+ * HL_VOTE_SLOTS shared-memory slots with cp.async.bulk (completing on the slot's
+ * full barrier); the consumer warps take blocks of 32 points of a slot in turn,
+ * vote them straight from shared memory and arrive on the slot's empty barrier,
+ * which the producer waits on before refilling it.  The producer moves on to
+ * the next item as soon as the current one is issued.
+ * When an item is voted the consumers read it and clear what they read.  The
+ * only item of its block is final: when peaks are wanted, its bins above the
+ * threshold go to the accumulator, which is zero otherwise (the peak rule needs
+ * no others, and the tail clears them again), and onto the candidate list --
+ * writing whole accumulators cost a batch of 256 images 670 MB and a fifth of
+ * its vote kernel; when the accumulator itself is wanted, all of it.  Other
+ * items go to a scratch slab that hl_merge_kernel sums.
+ * A whole image that one CTA votes alone (batches) but whose range exceeds the
+ * window is voted in segments of a sliding window: tiles are taken in bands
+ * across the slice's middle normal, the rows that no later band reaches are
+ * stored, and the rest moves down.
  *
- * Per vote: one packed multiply of x and one of y (two thetas per f32x2
- * instruction, so half of each), half a packed add, half a packed
- * magic-constant add (the float -> integer, see RHO_MAGIC), one clamp to the
- * dump row, one address add and one red.shared -- about five issue slots --
- * plus an eighth of a point load (the diagonal schedule, see DiagTab); no
- * branch per vote.
+ * Per vote: half a packed multiply of x and of y each for two thetas, half a
+ * packed add and half a packed magic-constant add (the float -> integer, see
+ * RHO_MAGIC), one shift-and-add (the column's address, window base and the
+ * constant's bits are one register) and one red.shared, plus an eighth of a
+ * point load; no clamp and no branch per vote.
  *
- * Bounds: every vote's row is clamped to the window's dump row, one row past
- * the window in every column; the padding columns (thetas >= T) are stored
- * as zero.
+ * Bound by instruction issue: 5 instructions a warp-vote in the loop, 1.6 of an
+ * SM's cycles against the 1.13 of the shared-memory atomics alone, and the
+ * items' edges (first copies, store, barriers) about a quarter of the time.
+ * 4096 x 4096, T = 720: 101 us (fixed rho windows 122 us); the whole call with
+ * slab merge 160 -> 148 us.  256 images of 256..2048 a side, T = 360: 890 us
+ * (1295), the call 1596 -> 1186 us.  2048 points a slot: 1024 make every warp
+ * wait on a barrier for every block it votes (4096 x 4096 158 against 153 us,
+ * the batch 1364 against 1318).
+ *
+ * Bounds: every voted point lies in the item's rectangle (or band), whose rows
+ * the window holds; the list's sentinel (+infinity pads an odd tile) and stale
+ * ring data vote 0 at the place of a real point; items whose window may be too
+ * small test every row.  A launch whose compaction reported an error votes
+ * nothing.
  * After the start there is no block-wide barrier, and every mbarrier wait is
  * bounded: a time-out sets a status bit that the host reads with the result
  * and an abort flag on which every other waiting warp gives up too; the
@@ -120,27 +138,119 @@ __device__ __forceinline__ bool mbar_wait_sleep(unsigned long long *bar,
     return false;
 }
 
-/* A consumer warp's share of a slot: points [0, m) of pts, m <= HL_VOTE_PPW,
- * 8 per round.  Entries past m (stale ring data) vote as the sentinel
- * (1e30, 0), whose rows lie outside every window and go to the dump row. */
+/* An item as the producer hands it to the consumers, or the end of the work
+ * (item < 0). */
+struct VoteSeg {
+    int32_t *acc;                      /* the image's accumulator */
+    int item;                          /* its index, or -1 */
+    int img, k0;                       /* image, first theta of the slice */
+    int mode;                          /* CV_* (CV_EXACT: every row tested) */
+    int total;                         /* points of its stream */
+    int rho_min, R, thr;               /* the image's */
+    int slab, ncap;                    /* see hl_vote_item */
+    int last, adv;                     /* the item's last segment; rows to slide */
+    int rows;                          /* rows its votes can reach */
+    float margin;                      /* one rho bin in pixels */
+    float c[HL_SLICE], s[HL_SLICE];    /* cos / sin of the slice's thetas */
+    int base[HL_SLICE];                /* rho of each column's row 0 */
+    int gb[4], gn[4];                  /* the slab's header */
+};
+
+/* The lane's tables of an item: cos / sin of its columns as f2x pairs of
+ * consecutive steps (DiagTab's order), and key[i] with 128 * bits + key[i] the
+ * shared address of the vote at step i (bits: the magic-constant sum). */
+struct VoteTab {
+    f2x c[4], s[4];
+    unsigned key[8];
+};
+
+/* 32 points from pts on, 8 a round, 8 votes of each a lane. */
 template <bool UNIT, int CV>
-__device__ __forceinline__ void vote_share(const float2 *pts, int m, const DiagTab &t,
-                                           f2x ir, int base, unsigned lim, int p)
+__device__ __forceinline__ void vote_rounds(const float2 *pts, const VoteTab &t, f2x ir)
 {
-    if (m >= HL_VOTE_PPW) {
-#pragma unroll 2
-        for (int r = 0; r < HL_VOTE_PPW; r += 8) {
-            const float2 q = pts[r + p];
-            diag_point<UNIT, CV>(q.x, q.y, t, ir, base, lim);
-        }
-    } else {
-        for (int r = 0; r < m; r += 8) {
-            float2 q = pts[r + p];
-            if (r + p >= m)
-                q = make_float2(1e30f, 0.0f);
-            diag_point<UNIT, CV>(q.x, q.y, t, ir, base, lim);
+    pts += threadIdx.x & 7;
+#pragma unroll
+    for (int r = 0; r < 32; r += 8) {
+        const float2 q = pts[r];
+        const f2x X = f2_pack(q.x, q.x), Y = f2_pack(q.y, q.y);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            unsigned r0, r1;
+            diag_bits<UNIT, CV>(X, Y, t.c[i], t.s[i], ir, r0, r1);
+            red_smem(128u * r0 + t.key[2 * i]);
+            red_smem(128u * r1 + t.key[2 * i + 1]);
         }
     }
+}
+
+/* Points that a clipped item's window may not hold, or whose |rho| may reach
+ * 2^22: point by point, a lane a theta, by the conversion instruction, every
+ * row tested. */
+template <bool UNIT>
+__device__ __noinline__ void vote_clipped(const float2 *pts, unsigned real, const VoteSeg &g,
+                                          int rows, int *acc, float irho)
+{
+    const int lane = threadIdx.x & 31;
+    const float c = g.c[lane], s = g.s[lane];
+    const int base = g.base[lane];
+    for (; real; real &= real - 1) {
+        const float2 q = pts[__ffs(real) - 1];
+        const int row = rho_of<UNIT>(q.x, q.y, c, s, irho) - base;
+        if ((unsigned)row < (unsigned)rows)
+            atomicAdd(acc + row * HL_SLICE + lane, 1);
+    }
+}
+
+/* A warp's block of a slot: 32 places, n of them filled.  They are looked at
+ * once, a lane a place: the ones with no point (past the end, or the list's
+ * sentinel) are filled with one of the block's points, whose surplus votes the
+ * warp takes off again, so that no vote needs a test; and which blocks lie on
+ * one side of rho 0 over the whole slice (a sinusoid has at most one zero in
+ * it, so its ends tell, with a bin to spare).  Blocks on one side vote by floor
+ * or by ceil, the others by the sign of each vote.  Conflict-free red.shared
+ * alone take 1.13 cycles a warp-vote an SM; the floor 1.5, truncation by sign
+ * 2.15 (micro-benchmark, 31 warps). */
+template <bool UNIT>
+__device__ __forceinline__ void vote_block(float2 *pts, int n, int mode, const VoteTab &t,
+                                           f2x ir, const VoteSeg &g, int rows, int *acc,
+                                           float irho)
+{
+    const int lane = threadIdx.x & 31;
+    const float2 q = pts[lane];
+    const bool there = lane < n && q.x < 1.0e29f;
+    const unsigned real = __ballot_sync(FULL, there);
+    if (mode == CV_EXACT) {   /* a clipped item, or the exact conversion */
+        vote_clipped<UNIT>(pts, real, g, rows, acc, irho);
+        return;
+    }
+    if (real != FULL) {
+        if (!real)
+            return;
+        const float2 f = pts[__ffs(real) - 1];
+        if (!there) {
+            pts[lane] = f;
+            /* the slot is refilled by the async proxy */
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        const int row = rho_of<UNIT>(f.x, f.y, g.c[lane], g.s[lane], irho) - g.base[lane];
+        atomicSub(acc + row * HL_SLICE + lane, 32 - __popc(real));
+        __syncwarp();
+    }
+    int cv = mode;
+    if (mode == CV_SIGN) {
+        const float v0 = q.x * g.c[0] + q.y * g.s[0];
+        const float v1 = q.x * g.c[HL_SLICE - 1] + q.y * g.s[HL_SLICE - 1];
+        if (__all_sync(FULL, !there || fminf(v0, v1) > g.margin))
+            cv = CV_FLOOR;
+        else if (__all_sync(FULL, !there || fmaxf(v0, v1) < -g.margin))
+            cv = CV_CEIL;
+    }
+    if (cv == CV_FLOOR)
+        vote_rounds<UNIT, CV_FLOOR>(pts, t, ir);
+    else if (cv == CV_CEIL)
+        vote_rounds<UNIT, CV_CEIL>(pts, t, ir);
+    else
+        vote_rounds<UNIT, CV_SIGN>(pts, t, ir);
 }
 
 /* Bounded wait that also gives up as soon as another warp of the CTA has
@@ -170,318 +280,278 @@ __device__ __forceinline__ bool mbar_wait_ab(unsigned long long *bar,
     return false;
 }
 
-/* One segment of the producer's stream: one tile group (HL_VOTE_TG tiles)
- * of a work item, or the end of the work (item < 0). */
-struct VoteSeg {
-    int32_t *acc;                      /* the image's accumulator */
-    int item;                          /* slice + nslices * window, or -1 */
-    int part, nparts, slot;            /* see hl_vote_args.items */
-    int rho_min, R;                    /* the image's rho range */
-    int total;                         /* points in the segment's runs */
-    int b_lo, b_hi;                    /* this part's batches of them */
-    int first, last;                   /* first / last segment of the item */
-    float c[HL_SLICE], s[HL_SLICE];    /* cos / sin of the slice's thetas */
-    int img;                           /* the image (in the tail padding: the
-                                          layout measured fastest is kept) */
-};
-
 struct VoteSmem {
     unsigned long long full[HL_VOTE_SLOTS];
     unsigned long long empty[HL_VOTE_SLOTS];
     unsigned long long seg_full[2];    /* producer -> consumers */
     unsigned long long seg_empty[2];   /* consumers -> producer */
-    unsigned long long cbar;           /* barrier of the consumer threads */
+    unsigned long long cbar;           /* barrier of the consumer warps */
     int abort;                         /* a warp gave up waiting */
     VoteSeg seg[2];
-    int run_s[HL_VOTE_TG / 2];         /* producer: the segment's runs */
-    int run_e[HL_VOTE_TG / 2];
-    int rpre[HL_VOTE_TG / 2];          /* stream position of each run */
+    int run_s[HL_VOTE_RUNS];           /* producer: the runs' first points */
+    int rpre[HL_VOTE_RUNS + 1];        /* their stream positions */
     alignas(16) float2 raw[HL_VOTE_SLOTS][SLOT_CAP];
 };
 
 #define VOTE_FIXED ((sizeof(VoteSmem) + 127) / 128 * 128)
 
-/* the window's rows plus the dump row */
 size_t hl_vote_smem_bytes(int win_rows)
 {
-    return VOTE_FIXED + (size_t)(win_rows + 1) * HL_SLICE * sizeof(int);
+    return VOTE_FIXED + (size_t)win_rows * HL_SLICE * sizeof(int);
 }
 
 int hl_vote_max_rows(void)
 {
     const size_t cap = 227u * 1024u;
-    return (int)((cap - VOTE_FIXED) / (HL_SLICE * sizeof(int)) - 1) & ~7;
+    return (int)((cap - VOTE_FIXED) / (HL_SLICE * sizeof(int))) & ~7;
 }
 
-/* Admitted tiles of every (slice, window) block of an image: one warp per
- * mask word, lane = tile (tile_hits; every tile when the image has a single
- * window).  They depend on the geometry only, so callers compute them once
- * per geometry. */
-__global__ void hl_tile_mask_kernel(hl_vote_args a)
-{
-    const hl_vote_img im = a.imgs ? a.imgs[blockIdx.y] : a.img0;
-    const int words = (im.ntiles + 31) >> 5;
-    const int nslices = a.Tp / HL_SLICE;
-    const long long nw = (long long)nslices * im.nwin * words;
-    const int lane = threadIdx.x & 31;
-    const long long wstep = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long wd = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-         wd < nw; wd += wstep) {
-        const int blk = (int)(wd / words), wi = (int)(wd % words);
-        const int slice = blk % nslices, win = blk / nslices;
-        const int k0 = slice * HL_SLICE;
-        const int klast = min(k0 + HL_SLICE - 1, a.T - 1);
-        const int w0 = win * a.win_rows;
-        const int rows = min(a.win_rows, im.R - w0);
-        const int t = wi * 32 + lane;
-        bool hit = false;
-        if (t < im.ntiles)
-            hit = im.nwin <= 1 ||
-                  tile_hits(t, im.tiles_x, im.w, im.h, a.cosv[k0], a.sinv[k0],
-                            a.cosv[klast], a.sinv[klast],
-                            (float)(im.rho_min + w0),
-                            (float)(im.rho_min + w0 + rows - 1), a.irho);
-        const unsigned m = __ballot_sync(FULL, hit);
-        if (lane == 0)
-            im.tmask[wd] = m;
-    }
-}
-
-/* barrier of the consumer threads (every one arrives; bounded wait) */
+/* barrier of the consumer warps (bounded wait): one arrival a warp, after its
+ * lanes' accesses -- an arrival a thread serialises a thousand of them on one
+ * shared-memory word */
 __device__ __forceinline__ bool cons_sync(VoteSmem &sm, unsigned &par,
                                           int *status)
 {
-    mbar_arrive(&sm.cbar);
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0)
+        mbar_arrive(&sm.cbar);
     const bool ok = mbar_wait_ab(&sm.cbar, par, &sm.abort, status);
     par ^= 1u;
     return ok;
 }
 
-/* Producer warp: takes items, turns each tile group of an item into a
- * segment (runs of admitted tiles -> point ranges -> batches), publishes the
- * segment and streams its batches into the ring.  It runs ahead of the
- * consumers by up to the ring's depth, so the next item's setup and first
- * copies overlap the current item's last votes. */
-template <bool NOTE>
-__device__ __forceinline__ void vote_producer(const hl_vote_args &a,
-                                              VoteSmem &sm, int batch)
+/* minimum / maximum over the 8 lanes of a column group */
+__device__ __forceinline__ int group_min(int v)
+{
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1)
+        v = min(v, __shfl_xor_sync(FULL, v, o));
+    return v;
+}
+
+/* Producer warp: takes items, publishes each as a segment and streams its
+ * points into the ring.  It runs ahead of the consumers by up to the ring's
+ * depth, so the next item's setup and first copies overlap the current item's
+ * last votes. */
+__device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &sm)
 {
     const int lane = threadIdx.x & 31;
-    const int nslices = a.Tp / HL_SLICE;
     unsigned seq = 0;    /* batches issued */
     unsigned nseg = 0;   /* segments published */
     bool ok = true;
+    /* nothing is voted after a failed compaction: its offsets are not valid */
+    const bool skip = *(volatile int *)a.status != 0;
     while (ok) {
+        /* in order of arrival, the first item too: under programmatic launch
+         * some CTAs start late */
         unsigned t = 0;
         if (lane == 0)
             t = atomicAdd(a.work, 1u) - a.work_base;
         t = __shfl_sync(FULL, t, 0);
         const bool have = t < (unsigned)a.nitems;
-        int4 it = make_int4(-1, 0, 0, 0);
+        hl_vote_item it = {};
         hl_vote_img im = a.img0;
         if (have) {
             it = a.items[t];
             if (a.imgs)
-                im = a.imgs[(unsigned)it.x >> 16];
+                im = a.imgs[it.img];
         }
-        const int item = have ? (it.x & 0xffff) : -1;
-        const int part = it.y & 0xffff, nparts = max(it.y >> 16, 1);
-        const int k0 = have ? (item % nslices) * HL_SLICE : 0;
-        const float cl = have ? a.cosv[k0 + lane] : 0.0f;
-        const float sl = have ? a.sinv[k0 + lane] : 0.0f;
-        const int ntiles = have ? im.ntiles : 0;
-        const int words = (ntiles + 31) >> 5;
-        const unsigned *mk = have ? im.tmask + (size_t)item * words : nullptr;
-        int tg = 0;
-        do {
-            const int tg_n = min(HL_VOTE_TG, ntiles - tg);
-            int total = 0, nruns = 0;
-            if (have) {
-                /* runs of the group's mask words, four words per lane */
-                constexpr int WPL = HL_VOTE_TG / 32 / 32;
-                unsigned m[WPL], st[WPL], en[WPL];
-                int cs = 0, ce = 0;
+        const int tx0 = it.tx & 0xffff, txn = it.tx >> 16;
+        const int ty0 = it.ty & 0xffff, tyn = it.ty >> 16;
+        /* the columns past T vote like the last theta: their counts are
+         * cleared with the others' and stored as zero */
+        const int k = min(it.slice * HL_SLICE + lane, a.T - 1);
+        const float cl = a.cosv[k], sl = a.sinv[k];
+        /* rho range of each theta over the rectangle */
+        float lo = 3.0e38f, hi = -3.0e38f;
 #pragma unroll
-                for (int q = 0; q < WPL; q++) {
-                    const int wd = lane * WPL + q;
-                    m[q] = wd * 32 < tg_n ? mk[(tg >> 5) + wd] : 0u;
-                }
-                unsigned prev = __shfl_up_sync(FULL, m[WPL - 1], 1);
-                unsigned next = __shfl_down_sync(FULL, m[0], 1);
-                if (lane == 0)
-                    prev = 0u;
-                if (lane == 31)
-                    next = 0u;
-#pragma unroll
-                for (int q = 0; q < WPL; q++) {
-                    const unsigned pv = q > 0 ? m[q - 1] : prev;
-                    const unsigned nx = q + 1 < WPL ? m[q + 1] : next;
-                    st[q] = m[q] & ~((m[q] << 1) | (pv >> 31));
-                    en[q] = m[q] & ~((m[q] >> 1) | ((nx & 1u) << 31));
-                    cs += __popc(st[q]);
-                    ce += __popc(en[q]);
-                }
-                int is = cs, ie = ce;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t1 = __shfl_up_sync(FULL, is, o);
-                    const int t2 = __shfl_up_sync(FULL, ie, o);
-                    if (lane >= o) {
-                        is += t1;
-                        ie += t2;
-                    }
-                }
-                nruns = __shfl_sync(FULL, is, 31);
-                is -= cs;
-                ie -= ce;
-                /* tile indices of the run ends, then their point offsets
-                 * (four loads in flight per lane) */
-#pragma unroll
-                for (int q = 0; q < WPL; q++) {
-                    const int base = (lane * WPL + q) * 32;
-                    for (unsigned x = st[q]; x; x &= x - 1)
-                        sm.run_s[is++] = base + __ffs(x) - 1;
-                    for (unsigned x = en[q]; x; x &= x - 1)
-                        sm.run_e[ie++] = base + __ffs(x);
-                }
-                __syncwarp();
-                const int *toff = im.tile_off + tg;
-                for (int r0 = 0; r0 < nruns; r0 += 128) {
-                    int vs[4], ve[4];
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const int r = r0 + 32 * u + lane;
-                        if (r < nruns) {
-                            vs[u] = toff[sm.run_s[r]];
-                            ve[u] = toff[sm.run_e[r]];
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const int r = r0 + 32 * u + lane;
-                        if (r < nruns) {
-                            sm.run_s[r] = vs[u];
-                            sm.run_e[r] = ve[u];
-                        }
-                    }
-                }
-                __syncwarp();
-                /* stream positions: a chunk of runs per lane, warp scan */
-                const int per = (nruns + 31) / 32;
-                const int ra = min(nruns, lane * per), rb = min(nruns, ra + per);
-                int sum = 0;
-                for (int r = ra; r < rb; r++)
-                    sum += sm.run_e[r] - sm.run_s[r];
-                int incl = sum;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t1 = __shfl_up_sync(FULL, incl, o);
-                    if (lane >= o)
-                        incl += t1;
-                }
-                int pos = incl - sum;
-                for (int r = ra; r < rb; r++) {
-                    sm.rpre[r] = pos;
-                    pos += sm.run_e[r] - sm.run_s[r];
-                }
-                total = __shfl_sync(FULL, incl, 31);
-                __syncwarp();
-            }
-            const int nb_all = (total + batch - 1) / batch;
-            const int b_lo = (int)((long long)nb_all * part / nparts);
-            const int b_hi = (int)((long long)nb_all * (part + 1) / nparts);
+        for (int i = 0; i < 4; i++) {
+            const float x = (float)((i & 1) ? min((tx0 + txn) * HL_TILE_W, im.w) - 1
+                                            : tx0 * HL_TILE_W);
+            const float y = (float)((i & 2) ? min((ty0 + tyn) * HL_TILE_H, im.h) - 1
+                                            : ty0 * HL_TILE_H);
+            const float v = rho_f<false>(x, y, cl, sl, a.irho);
+            lo = fminf(lo, v);
+            hi = fmaxf(hi, v);
+        }
+        const bool slide = it.nseg > 1;
+        const float ctx = 0.5f * (float)(im.w - 1), cty = 0.5f * (float)(im.h - 1);
+        int base = slide ? __float2int_rd(rho_f<false>(ctx, cty, cl, sl, a.irho)) + it.off0
+                         : __float2int_rz(lo) + it.win * a.win_rows;
+        int top = __float2int_rz(hi);
+        if (have && !slide && !it.clip && __any_sync(FULL, top - base >= a.win_rows)) {
+            if (lane == 0)   /* the plan promised more rows than there are */
+                atomicOr(a.status, HL_ST_RHO_OUT_OF_RANGE);
+            it.clip = 1;
+        }
+        if (!slide)
+            top = min(top, base + a.win_rows - 1);
+        int mode = a.exact ? CV_EXACT
+                           : (!__any_sync(FULL, lo < 0.0f)
+                                  ? CV_FLOOR
+                                  : (!__any_sync(FULL, hi > 0.0f) ? CV_CEIL : CV_SIGN));
+        const bool mixed = mode == CV_SIGN;
+        /* the slab's column groups: rows of the columns that reach the window */
+        const bool in = top >= base;
+        const int glo = group_min(in ? base - im.rho_min : 0x7fffffff) >> 2;
+        const int ghi = -group_min(in ? -(top - im.rho_min) : 0x7fffffff);
+        int gn = glo < 0x1fffffff ? (ghi >> 2) - glo + 1 : 0;
+        if (have && it.slab >= 0 && gn > it.ncap) {
+            atomicOr(a.status, HL_ST_RHO_OUT_OF_RANGE);
+            gn = it.ncap;
+        }
+        /* sliding: the middle theta's normal in rho units a tile */
+        const int km = min(it.slice * HL_SLICE + HL_SLICE / 2, a.T - 1);
+        const float sm_ = slide ? a.sinv[km] * a.irho : 0.0f;
+        float cm = slide ? a.cosv[km] * a.irho : 0.0f;
+        cm = copysignf(fmaxf(fabsf(cm), 1.0e-9f), cm);
+        const float icm = 1.0f / (cm * HL_TILE_W);
+        const bool wide = txn == im.tiles_x && !slide;
+        const int nsegs = have ? max(it.nseg, 1) : 1;
 
-            /* publish the segment once the consumers are done with the one
-             * that last used its slot */
-            const int ds = (int)(nseg & 1u);
-            if (nseg >= 2 &&
-                !mbar_wait_ab(&sm.seg_empty[ds], ((nseg >> 1) - 1u) & 1u, &sm.abort,
+        for (int sj = 0; sj < nsegs && ok; sj++, base += it.adv) {
+        const int rows = __reduce_max_sync(FULL, max(min(top, base + a.win_rows - 1) - base + 1, 0));
+        if (it.clip)
+            mode = CV_EXACT;   /* every row tested */
+        if (slide && mixed)   /* by the segment's own rows */
+            mode = !__any_sync(FULL, base < 0)
+                       ? CV_FLOOR
+                       : (!__any_sync(FULL, base + a.win_rows > 0) ? CV_CEIL : CV_SIGN);
+        /* the runs, four per lane: one a tile row, or one for a rectangle as
+         * wide as the image */
+        const int nruns = have && !skip ? (wide ? 1 : min(tyn, HL_VOTE_RUNS)) : 0;
+        int st[4], ln[4], sum = 0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int r = 4 * lane + q;
+            st[q] = ln[q] = 0;
+            if (r < nruns) {
+                int ta = 0, tb = txn;   /* the run's tiles, from tx0 */
+                if (slide) {
+                    /* first tile past the band's near and far edge: monotone
+                     * in x, so the bands' edges split the row */
+                    const float yk = ((float)((ty0 + r) * HL_TILE_H + HL_TILE_H / 2) - cty) * sm_;
+                    const float k0 = (float)(sj * it.adv) - it.half - yk;
+                    const float e0 = ceilf(k0 * icm + (ctx - HL_TILE_W / 2) * (1.0f / HL_TILE_W));
+                    const float e1 = ceilf((k0 + (float)it.adv) * icm +
+                                           (ctx - HL_TILE_W / 2) * (1.0f / HL_TILE_W));
+                    const int i0 = (int)fminf(fmaxf(e0, 0.0f), (float)txn);
+                    const int i1 = (int)fminf(fmaxf(e1, 0.0f), (float)txn);
+                    const bool fst = sj == 0, lst = sj == nsegs - 1;
+                    ta = cm > 0.0f ? (fst ? 0 : i0) : (lst ? 0 : i1);
+                    tb = cm > 0.0f ? (lst ? txn : i1) : (fst ? txn : i0);
+                }
+                if (tb > ta) {
+                    const int t0 = (ty0 + r) * im.tiles_x + tx0;
+                    st[q] = im.tile_off[t0 + ta];
+                    ln[q] = im.tile_off[wide ? (ty0 + tyn) * im.tiles_x : t0 + tb] - st[q];
+                }
+            }
+            sum += ln[q];
+        }
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t1 = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o)
+                incl += t1;
+        }
+        const int total = __shfl_sync(FULL, incl, 31);
+        int pos = incl - sum;
+        __syncwarp();   /* the previous segment's runs are no longer read */
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int r = 4 * lane + q;
+            if (r < nruns) {
+                sm.run_s[r] = st[q];
+                sm.rpre[r] = pos;
+                pos += ln[q];
+                if (r == nruns - 1)
+                    sm.rpre[nruns] = pos;
+            }
+        }
+
+        /* publish the segment once the consumers are done with the one that
+         * last used its slot */
+        const int ds = (int)(nseg & 1u);
+        if (nseg >= 2 && !mbar_wait_ab(&sm.seg_empty[ds], ((nseg >> 1) - 1u) & 1u, &sm.abort,
+                                       a.status)) {
+            ok = false;
+            break;
+        }
+        VoteSeg &g = sm.seg[ds];
+        g.c[lane] = cl;
+        g.s[lane] = sl;
+        g.base[lane] = base;
+        if ((lane & 7) == 0) {
+            g.gb[lane >> 3] = glo;
+            g.gn[lane >> 3] = gn;
+        }
+        if (lane == 0) {
+            g.acc = im.acc;
+            g.item = have ? (int)t : -1;
+            g.img = it.img;
+            g.k0 = it.slice * HL_SLICE;
+            g.mode = mode;
+            g.margin = 1.0f / a.irho;
+            g.total = total;
+            g.rho_min = im.rho_min;
+            g.R = im.R;
+            g.thr = im.threshold;
+            g.slab = it.slab;
+            g.ncap = it.ncap;
+            g.last = sj == nsegs - 1;
+            g.adv = it.adv;
+            g.rows = rows;
+        }
+        __syncwarp();
+        if (lane == 0)
+            mbar_arrive(&sm.seg_full[ds]);
+        nseg++;
+
+        /* batch b is stream range [b * SLOT_CAP, ...): lane i copies the part
+         * of run r0 + i overlapping it; a ballot finds the first run of the
+         * next batch */
+        const int nb = (total + SLOT_CAP - 1) / SLOT_CAP;
+        int r0 = 0;
+        for (int b = 0; b < nb && ok; b++) {
+            const int slot = (int)(seq % HL_VOTE_SLOTS);
+            if (seq >= HL_VOTE_SLOTS &&
+                !mbar_wait_ab(&sm.empty[slot], ((seq / HL_VOTE_SLOTS) - 1u) & 1u, &sm.abort,
                               a.status)) {
                 ok = false;
                 break;
             }
-            VoteSeg &g = sm.seg[ds];
-            g.c[lane] = cl;
-            g.s[lane] = sl;
-            if (lane == 0) {
-                g.acc = im.acc;
-                g.item = item;
-                g.part = part;
-                g.nparts = nparts;
-                g.slot = it.z;
-                if (NOTE)
-                    g.img = a.imgs ? (int)((unsigned)it.x >> 16) : 0;
-                g.rho_min = im.rho_min;
-                g.R = im.R;
-                g.total = total;
-                g.b_lo = b_lo;
-                g.b_hi = b_hi;
-                g.first = tg == 0;
-                g.last = tg + HL_VOTE_TG >= ntiles;
-            }
-            __syncwarp();
+            const int s0 = b * SLOT_CAP;
+            const int e0 = min(total, s0 + SLOT_CAP);
             if (lane == 0)
-                mbar_arrive(&sm.seg_full[ds]);
-            nseg++;
-            if (!have)
-                break;
-
-            /* batch b is stream range [b * batch, ...): lane i copies the
-             * part of run r0 + i overlapping it; a ballot finds the first run
-             * of the next batch */
-            int r0 = 0;
-            {
-                const int s_first = b_lo * batch;
-                int lo = 0, hi = max(nruns - 1, 0);
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if (sm.rpre[mid] + (sm.run_e[mid] - sm.run_s[mid]) <= s_first)
-                        lo = mid + 1;
-                    else
-                        hi = mid;
+                mbar_expect_tx(&sm.full[slot], (unsigned)(e0 - s0) * 8u);
+            __syncwarp();
+            /* runs from r0 on: every run ending at or before e0 lies wholly in
+             * this batch; the first one reaching past e0 is shared with the
+             * next batch and ends the scan */
+            int nextr = nruns;
+            for (int rb = r0; rb < nruns; rb += 32) {
+                const int r = rb + lane;
+                bool past = false;
+                if (r < nruns) {
+                    const int rs = sm.rpre[r], re = sm.rpre[r + 1];
+                    const int ps = max(s0, rs), pe = min(e0, re);
+                    if (pe > ps)
+                        bulk_g2s(&sm.raw[slot][ps - s0], im.pts + sm.run_s[r] + (ps - rs),
+                                 (unsigned)(pe - ps) * 8u, &sm.full[slot]);
+                    past = re > e0;
                 }
-                r0 = lo;
-            }
-            for (int b = b_lo; b < b_hi && ok; b++) {
-                const int slot = (int)(seq % HL_VOTE_SLOTS);
-                if (seq >= HL_VOTE_SLOTS &&
-                    !mbar_wait_ab(&sm.empty[slot], ((seq / HL_VOTE_SLOTS) - 1u) & 1u,
-                                  &sm.abort, a.status)) {
-                    ok = false;
+                const unsigned pm = __ballot_sync(FULL, past);
+                if (pm) {
+                    nextr = rb + __ffs(pm) - 1;
                     break;
                 }
-                const int s0 = b * batch;
-                const int e0 = min(total, s0 + batch);
-                if (lane == 0)
-                    mbar_expect_tx(&sm.full[slot], (unsigned)(e0 - s0) * 8u);
-                __syncwarp();
-                /* runs from r0 on: every run ending at or before e0 lies
-                 * wholly in this batch; the first one reaching past e0 is
-                 * shared with the next batch and ends the scan */
-                int nextr = nruns;
-                for (int rb = r0; rb < nruns; rb += 32) {
-                    const int r = rb + lane;
-                    bool past = false;
-                    if (r < nruns) {
-                        const int rs = sm.rpre[r];
-                        const int re = rs + (sm.run_e[r] - sm.run_s[r]);
-                        const int ps = max(s0, rs), pe = min(e0, re);
-                        if (pe > ps)
-                            bulk_g2s(&sm.raw[slot][ps - s0], im.pts + sm.run_s[r] + (ps - rs),
-                                     (unsigned)(pe - ps) * 8u, &sm.full[slot]);
-                        past = re > e0;
-                    }
-                    const unsigned pm = __ballot_sync(FULL, past);
-                    if (pm) {
-                        nextr = rb + __ffs(pm) - 1;
-                        break;
-                    }
-                }
-                r0 = nextr;
-                seq++;
             }
-            tg += HL_VOTE_TG;
-        } while (ok && tg < ntiles);
+            r0 = nextr;
+            seq++;
+        }
+        }
         if (!have)
             break;
     }
@@ -493,9 +563,7 @@ __device__ __forceinline__ void vote_producer(const hl_vote_args &a,
     }
 }
 
-/* NOTE: note the bins above the threshold as peak candidates (a.cand);
- * without, the code is the plain vote and store */
-template <bool UNIT, bool NOTE>
+template <bool UNIT>
 __global__ void __launch_bounds__(1024, 1)
 hl_vote_kernel(hl_vote_args a)
 {
@@ -505,16 +573,11 @@ hl_vote_kernel(hl_vote_args a)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nthr = blockDim.x, nwarps = nthr >> 5;
     const int ncons = nwarps - 1;               /* consumer warps 1..nwarps-1 */
-    /* points per batch: HL_VOTE_PPW per consumer warp (at most SLOT_CAP) */
-    const int batch = HL_VOTE_PPW * ncons;
-    const int nslices = a.Tp / HL_SLICE;
-
-    /* the block and its dump row start at zero (before the wait for the
-     * previous launch: shared memory only); after each item the consumers
-     * clear what it used */
+    /* the window starts at zero (before the wait for the previous launch:
+     * shared memory only); after each item the consumers clear what it used */
     {
         int4 *z = reinterpret_cast<int4 *>(s_acc);
-        for (int i = tid; i < (a.win_rows + 1) * (HL_SLICE / 4); i += nthr)
+        for (int i = tid; i < a.win_rows * (HL_SLICE / 4); i += nthr)
             z[i] = make_int4(0, 0, 0, 0);
     }
     hl_pdl_begin();
@@ -527,7 +590,7 @@ hl_vote_kernel(hl_vote_args a)
             mbar_init(&sm.seg_full[i], 1);
             mbar_init(&sm.seg_empty[i], (unsigned)ncons);
         }
-        mbar_init(&sm.cbar, (unsigned)(32 * ncons));
+        mbar_init(&sm.cbar, (unsigned)ncons);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         sm.abort = 0;
     }
@@ -535,269 +598,312 @@ hl_vote_kernel(hl_vote_args a)
      * consumers meet on mbarriers, every wait bounded */
     __syncthreads();
     if (warp == 0) {
-        vote_producer<NOTE>(a, sm, batch);
+        vote_producer(a, sm);
         return;
     }
 
     const int cw = warp - 1;
-    const int ctid = tid - 32, nct = nthr - 32;
     const unsigned acc_base = smem_u32(s_acc);
     const f2x ir = f2_pack(a.irho, a.irho);
-    const int pl = lane & 7;
-    int4 *src4 = reinterpret_cast<int4 *>(s_acc);
     unsigned seq = 0, nseg = 0, cpar = 0;
-    /* the current item */
-    DiagTab tab;
-    diag_table(tab, a.cosv, a.sinv, acc_base, lane);
-    int cv = CV_EXACT, vbase = 0, rows = 0, w0 = 0, k0 = 0;
-    unsigned lrows = 0;
-    int32_t *acc_g = nullptr;
-    int nparts = 1, pslot = 0;
-    int img = 0;   /* the item's image (noting candidates only) */
     while (true) {
         const int ds = (int)(nseg & 1u);
         if (!mbar_wait_ab(&sm.seg_full[ds], (nseg >> 1) & 1u, &sm.abort, a.status))
             return;
         nseg++;
         const VoteSeg &g = sm.seg[ds];
-        const int item = g.item;
-        const int total = g.total, b_lo = g.b_lo, b_hi = g.b_hi;
-        const bool last = g.last;
-        if (item >= 0 && g.first) {
-            const int slice = item % nslices, win = item / nslices;
-            k0 = slice * HL_SLICE;
-            diag_table(tab, g.c, g.s, acc_base, lane);
-            w0 = win * a.win_rows;
-            rows = min(a.win_rows, g.R - w0);
-            const int row_base = g.rho_min + w0;   /* rho bin of local row 0 */
-            /* every column's dump row is row `rows`; the padding columns
-             * (thetas >= T, cos = sin = 0) vote there or into their own
-             * column, which the store writes as zero */
-            lrows = (unsigned)rows;
-            cv = row_base >= 1 ? CV_FLOOR
-                               : (row_base + rows - 1 <= -1 ? CV_CEIL : CV_EXACT);
-            vbase = cv == CV_EXACT ? row_base : RHO_MAGIC_BITS + row_base;
-            acc_g = g.acc;
-            nparts = g.nparts;
-            pslot = g.slot;
-            if (NOTE)
-                img = g.img;
-        }
-        __syncwarp();
-        if (lane == 0)
-            mbar_arrive(&sm.seg_empty[ds]);
-        if (item < 0)
+        if (g.item < 0)
             return;
-
-        /* vote every point of the segment's batches, freeing each slot */
-        for (int b = b_lo; b < b_hi; b++) {
-            const int slot = (int)(seq % HL_VOTE_SLOTS);
-            if (!mbar_wait_ab(&sm.full[slot], (seq / HL_VOTE_SLOTS) & 1u, &sm.abort,
-                              a.status))
-                return;
-            seq++;
-            /* this warp's share: points [PPW cw, PPW cw + PPW) */
-            const int m = min(HL_VOTE_PPW, total - b * batch - HL_VOTE_PPW * cw);
-            const float2 *pts = sm.raw[slot] + HL_VOTE_PPW * cw;
-            if (cv == CV_FLOOR)
-                vote_share<UNIT, CV_FLOOR>(pts, m, tab, ir, vbase, lrows, pl);
-            else if (cv == CV_CEIL)
-                vote_share<UNIT, CV_CEIL>(pts, m, tab, ir, vbase, lrows, pl);
-            else
-                vote_share<UNIT, CV_EXACT>(pts, m, tab, ir, vbase, lrows, pl);
-            __syncwarp();
-            if (lane == 0)
-                mbar_arrive(&sm.empty[slot]);
-        }
-        if (!last)
-            continue;
-
-        /* the item is voted: store the block, row i of the window ->
-         * acc[(w0 + i) * Tp + k0 ..], then clear it for the next item */
-        if (!cons_sync(sm, cpar, a.status))
-            return;
-        /* a whole block goes to acc (the padding columns, thetas >= T,
-         * hold dumped votes and are stored as zero; bins above the
-         * image's threshold are noted as peak candidates), a part of a
-         * split block to its scratch slot as it is; each thread stores and
-         * clears the same elements */
-        const int tp4 = a.Tp >> 2;
-        const int n4 = rows * (HL_SLICE / 4);
-        int4 *dst4 = nparts == 1 ? reinterpret_cast<int4 *>(acc_g) + (size_t)w0 * tp4 + (k0 >> 2)
-                                 : a.scratch + (size_t)pslot * hl_slot4(a.win_rows, a.part16);
-        const bool pack = nparts > 1 && a.part16;
-        /* the image's peak threshold, read once (noting candidates only) */
-        const int thr = NOTE ? (a.imgs ? a.imgs[img].threshold : a.img0.threshold) : 0;
-        for (int i = ctid; i < n4 + HL_SLICE / 4; i += nct) {
-            if (i < n4) {
-                const int rr = i >> 3, q = i & 7;
-                int4 v = src4[i];
-                if (nparts == 1) {
-                    if (k0 + 4 * q + 3 >= a.T) {
-                        const int kq = k0 + 4 * q;
-                        if (kq >= a.T) v.x = 0;
-                        if (kq + 1 >= a.T) v.y = 0;
-                        if (kq + 2 >= a.T) v.z = 0;
-                        if (kq + 3 >= a.T) v.w = 0;
-                    }
-                    dst4[(size_t)rr * tp4 + q] = v;
-                    if (NOTE) {
-                        const unsigned bits = above4(v, thr, k0 + 4 * q, a.T);
-                        if (bits)
-                            note_cands(a.cand, img,
-                                       (unsigned)(w0 + rr) * (unsigned)a.T +
-                                           (unsigned)(k0 + 4 * q),
-                                       bits);
-                    }
-                } else if (pack) {
-                    reinterpret_cast<int2 *>(dst4)[i] =
-                        make_int2((v.x & 0xffff) | (v.y << 16), (v.z & 0xffff) | (v.w << 16));
-                } else {
-                    dst4[i] = v;
+        const int total = g.total, mode = g.mode;
+        {
+            VoteTab tab;
+            {
+                const int p = lane & 7, j = lane >> 3;
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) {
+                    const int c0 = 8 * j + ((p + i) & 7), c1 = 8 * j + ((p + i + 1) & 7);
+                    tab.c[i / 2] = f2_pack(g.c[c0], g.c[c1]);
+                    tab.s[i / 2] = f2_pack(g.s[c0], g.s[c1]);
+                    tab.key[i] = acc_base + 4u * (unsigned)c0 -
+                                 128u * (unsigned)(RHO_MAGIC_BITS + g.base[c0]);
+                    tab.key[i + 1] = acc_base + 4u * (unsigned)c1 -
+                                     128u * (unsigned)(RHO_MAGIC_BITS + g.base[c1]);
                 }
             }
-            src4[i] = make_int4(0, 0, 0, 0);
+            /* vote the item's blocks in turn, freeing each slot */
+            int i = 32 * cw;   /* the warp's next point of the slot */
+            for (int b = 0; b * SLOT_CAP < total; b++) {
+                const int slot = (int)(seq % HL_VOTE_SLOTS);
+                if (!mbar_wait_ab(&sm.full[slot], (seq / HL_VOTE_SLOTS) & 1u, &sm.abort,
+                                  a.status))
+                    return;
+                seq++;
+                const int n = min(SLOT_CAP, total - b * SLOT_CAP);
+                for (; i < n; i += 32 * ncons)
+                    vote_block<UNIT>(sm.raw[slot] + i, n - i, mode, tab, ir, g, a.win_rows,
+                                     s_acc, a.irho);
+                i -= n;
+                __syncwarp();
+                if (lane == 0)
+                    mbar_arrive(&sm.empty[slot]);
+            }
+        }
+
+        /* the item is voted: store it and clear what is read, lane = column */
+        if (!cons_sync(sm, cpar, a.status))
+            return;
+        const int k = g.k0 + lane;
+        const bool kvalid = k < a.T;
+        const int rb = g.base[lane] - g.rho_min;   /* the accumulator row of row 0 */
+        int *col = s_acc + lane;
+        if (g.slab < 0) {
+            /* the rows that are final: all of them, or those below the next
+             * segment's window */
+            const bool last = g.last;
+            const int nr = last ? g.rows : g.adv;
+            if (a.add) {   /* several items of a block, no slabs */
+                for (int i = cw; i < nr; i += ncons) {
+                    const int v = col[i * HL_SLICE];
+                    if (v) {
+                        col[i * HL_SLICE] = 0;
+                        if (kvalid && (unsigned)(i + rb) < (unsigned)g.R)
+                            atomicAdd(g.acc + (size_t)(i + rb) * a.Tp + k, v);
+                    }
+                }
+            } else if (a.cand.e) {
+                /* only bins above the threshold matter (the peak rule compares
+                 * them with each other): they go to the accumulator, which is
+                 * zero otherwise, and onto the candidate list.  Four columns
+                 * of a row a lane, as the window lies in shared memory. */
+                const int thr = max(g.thr, 0);
+                int4 *w = reinterpret_cast<int4 *>(s_acc);
+                for (int i = 32 * cw + lane; i < nr * (HL_SLICE / 4); i += 32 * ncons) {
+                    const int4 v = w[i];
+                    w[i] = make_int4(0, 0, 0, 0);
+                    if (max(max(v.x, v.y), max(v.z, v.w)) > thr) {
+                        const int x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const int c = 4 * (i & 7) + e;
+                            const int r = (i >> 3) + g.base[c] - g.rho_min;
+                            if (x[e] > thr && g.k0 + c < a.T && (unsigned)r < (unsigned)g.R) {
+                                g.acc[(size_t)r * a.Tp + g.k0 + c] = x[e];
+                                note_cand(a.cand, g.img,
+                                          (unsigned)r * (unsigned)a.T + (unsigned)(g.k0 + c));
+                            }
+                        }
+                    }
+                }
+            } else {
+                /* the whole accumulator is asked for: row by row, the shear
+                 * undone by each lane's own offset.  Rows that no vote reaches
+                 * stay as they are, zero. */
+                const int lo = __reduce_min_sync(FULL, rb);
+                const int hi = __reduce_max_sync(FULL, rb) + nr;
+                for (int r = max(lo, 0) + cw; r < min(hi, g.R); r += ncons) {
+                    const unsigned i = (unsigned)(r - rb);
+                    if (i < (unsigned)nr) {
+                        g.acc[(size_t)r * a.Tp + k] = kvalid ? col[i * HL_SLICE] : 0;
+                        col[i * HL_SLICE] = 0;
+                    }
+                }
+            }
+            if (!last) {
+                /* rows [adv, win_rows) move to the window's start (the plan
+                 * keeps adv at least half the window) */
+                if (!cons_sync(sm, cpar, a.status))
+                    return;
+                int4 *w = reinterpret_cast<int4 *>(s_acc), *f = w + nr * (HL_SLICE / 4);
+                for (int i = 32 * cw + lane; i < (a.win_rows - nr) * (HL_SLICE / 4);
+                     i += 32 * ncons) {
+                    w[i] = f[i];
+                    f[i] = make_int4(0, 0, 0, 0);
+                }
+            }
+        } else {
+            unsigned char *slab = a.scratch + (size_t)g.slab * 64u;
+            const int grp = lane >> 3, cc = lane & 7;
+            if (cw == 0 && cc == 0) {
+                reinterpret_cast<hl_slab_hdr *>(slab)->b[grp] = g.gb[grp];
+                reinterpret_cast<hl_slab_hdr *>(slab)->n[grp] = g.gn[grp];
+            }
+            const int gb = g.gb[grp], gn = g.gn[grp];
+            const int most = max(max(g.gn[0], g.gn[1]), max(g.gn[2], g.gn[3]));
+            const size_t at = (size_t)grp * g.ncap * 8 + cc;
+            for (int q = cw; q < most; q += ncons) {
+                int v[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const unsigned i = (unsigned)(4 * (gb + q) + u - rb);
+                    v[u] = 0;
+                    if (q < gn && i < (unsigned)a.win_rows) {
+                        v[u] = col[i * HL_SLICE];
+                        col[i * HL_SLICE] = 0;
+                    }
+                }
+                if (q < gn) {
+                    if (a.part16)
+                        reinterpret_cast<uint2 *>(slab + 64)[at + (size_t)q * 8] =
+                            make_uint2((unsigned)v[0] | ((unsigned)v[1] << 16),
+                                       (unsigned)v[2] | ((unsigned)v[3] << 16));
+                    else
+                        reinterpret_cast<int4 *>(slab + 64)[at + (size_t)q * 8] =
+                            make_int4(v[0], v[1], v[2], v[3]);
+                }
+            }
         }
         if (!cons_sync(sm, cpar, a.status))
             return;
+        if (lane == 0)
+            mbar_arrive(&sm.seg_empty[ds]);
     }
 }
 
-/* The blocks voted in parts: block region = sum of its parts' scratch
- * slots, the padding columns (thetas >= T) stored as zero, the bins above
- * the image's threshold noted as peak candidates.  A
- * thread takes 16 bytes of every part of its region (grid.y = region): two
- * output int4 when the parts hold 16-bit counts, one otherwise; every slot
- * is read once, from L2 where the vote launch just wrote it; the parts'
- * loads go four at a time, all in flight. */
-template <bool NOTE>
+/* Blocks voted in several items: accumulator columns = sum of their slabs.  As
+ * in hl_vote_kernel the bins above the image's threshold are stored and noted
+ * as peak candidates, or every bin is stored (padding columns, thetas >= T,
+ * zero).  A thread takes four rows of two columns: one
+ * 16-byte load of every slab whose rows overlap (two with 32-bit counts), from
+ * L2 where the vote launch just wrote them, eight in flight. */
+#define MERGE_HDRS 64
+template <bool P16>
 __global__ void __launch_bounds__(256)
 hl_merge_kernel(hl_merge_args a)
 {
+    __shared__ int4 s_b[MERGE_HDRS], s_n[MERGE_HDRS];
+    __shared__ const unsigned char *s_p[MERGE_HDRS];
+    __shared__ int s_cap[MERGE_HDRS];
+    __shared__ int s_hits;
+    const int tid = threadIdx.x;
     hl_pdl_begin();
-    const hl_merge_region r = a.regs[blockIdx.y];
-    const int n4 = r.rows * (HL_SLICE / 4);   /* output int4 of the region */
-    int4 v0 = make_int4(0, 0, 0, 0), v1 = make_int4(0, 0, 0, 0);
-    int o;   /* first output int4 of this thread */
-    if (a.part16) {
-        /* one 16-byte load per part: eight 16-bit counts, output int4 o and
-         * o + 1 (a row holds 8, so both lie in one row); the parts' loads
-         * four at a time, all four in flight (the last group predicated) */
-        const int j = blockIdx.x * 256 + threadIdx.x;
-        o = 2 * j;
-        if (o >= n4)
-            return;
-        const int4 *src = a.scratch + (size_t)r.slot0 * a.slot4 + j;
-        for (int p = 0; p < r.nparts; p += 4) {
-            int4 q[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-                q[u] = p + u < r.nparts ? __ldcg(src + (size_t)(p + u) * a.slot4)
-                                        : make_int4(0, 0, 0, 0);
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                v0.x += q[u].x & 0xffff;
-                v0.y += (unsigned)q[u].x >> 16;
-                v0.z += q[u].y & 0xffff;
-                v0.w += (unsigned)q[u].y >> 16;
-                v1.x += q[u].z & 0xffff;
-                v1.y += (unsigned)q[u].z >> 16;
-                v1.z += q[u].w & 0xffff;
-                v1.w += (unsigned)q[u].w >> 16;
+    const unsigned bi = blockIdx.x / a.chunks, chunk = blockIdx.x - bi * a.chunks;
+    const hl_merge_block blk = a.blocks[bi];
+    const hl_vote_img &im = a.imgs ? a.imgs[blk.img] : a.img0;
+    const int R = im.R;
+    const int c0 = (int)chunk * 16;                /* the CTA's first row group */
+    if (4 * c0 >= R)
+        return;
+    const int rg = c0 + (tid >> 4);                /* the thread's */
+    const int g = (tid >> 2) & 3, cp = tid & 3;
+    int v[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    int hits = 0;
+    for (int j0 = 0; j0 < blk.n; j0 += MERGE_HDRS) {
+        /* the slabs that reach the CTA's rows */
+        __syncthreads();
+        if (tid == 0)
+            s_hits = 0;
+        __syncthreads();
+        if (tid < MERGE_HDRS && j0 + tid < blk.n) {
+            const int2 sl = a.slabs[blk.first + j0 + tid];
+            const unsigned char *p = a.scratch + (size_t)sl.x * 64u;
+            const int4 hb = __ldcg(reinterpret_cast<const int4 *>(p));
+            const int4 hn = __ldcg(reinterpret_cast<const int4 *>(p) + 1);
+            const int lo = min(min(hb.x, hb.y), min(hb.z, hb.w));
+            const int hi = max(max(hb.x + hn.x, hb.y + hn.y), max(hb.z + hn.z, hb.w + hn.w));
+            if (lo < c0 + 16 && hi > c0) {
+                const int at = atomicAdd(&s_hits, 1);
+                s_b[at] = hb;
+                s_n[at] = hn;
+                s_p[at] = p + 64;
+                s_cap[at] = sl.y;
             }
         }
-    } else {
-        o = blockIdx.x * 256 + threadIdx.x;
-        if (o >= n4)
-            return;
-        const int4 *src = a.scratch + (size_t)r.slot0 * a.slot4 + o;
-        for (int p = 0; p < r.nparts; p += 4) {
-            int4 q[4];
+        __syncthreads();
+        const int nj = s_hits;
+        hits |= nj;
+        /* the slabs' loads eight at a time (four with 32-bit counts) */
+        constexpr int U = P16 ? 8 : 4;
+        for (int j = 0; j < nj; j += U) {
+            uint4 q[8];
 #pragma unroll
-            for (int u = 0; u < 4; u++)
-                q[u] = p + u < r.nparts ? __ldcg(src + (size_t)(p + u) * a.slot4)
-                                        : make_int4(0, 0, 0, 0);
+            for (int u = 0; u < U; u++) {
+                const int jj = min(j + u, nj - 1);
+                const int rel = rg - reinterpret_cast<const int *>(&s_b[jj])[g];
+                const bool ok = j + u < nj &&
+                                (unsigned)rel < (unsigned)reinterpret_cast<const int *>(&s_n[jj])[g];
+                const size_t at = ((size_t)g * s_cap[jj] + rel) * 8 + 2 * cp;
+                if (P16) {
+                    q[u] = ok ? __ldcg(reinterpret_cast<const uint4 *>(
+                                    reinterpret_cast<const uint2 *>(s_p[jj]) + at))
+                              : make_uint4(0u, 0u, 0u, 0u);
+                } else {
+                    const uint4 *p = reinterpret_cast<const uint4 *>(s_p[jj]) + at;
+                    q[2 * u] = ok ? __ldcg(p) : make_uint4(0u, 0u, 0u, 0u);
+                    q[2 * u + 1] = ok ? __ldcg(p + 1) : make_uint4(0u, 0u, 0u, 0u);
+                }
+            }
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                v0.x += q[u].x;
-                v0.y += q[u].y;
-                v0.z += q[u].z;
-                v0.w += q[u].w;
+            for (int u = 0; u < U; u++) {
+                if (P16) {
+                    v[0][0] += q[u].x & 0xffffu;
+                    v[0][1] += q[u].x >> 16;
+                    v[0][2] += q[u].y & 0xffffu;
+                    v[0][3] += q[u].y >> 16;
+                    v[1][0] += q[u].z & 0xffffu;
+                    v[1][1] += q[u].z >> 16;
+                    v[1][2] += q[u].w & 0xffffu;
+                    v[1][3] += q[u].w >> 16;
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        v[e][0] += (int)q[2 * u + e].x;
+                        v[e][1] += (int)q[2 * u + e].y;
+                        v[e][2] += (int)q[2 * u + e].z;
+                        v[e][3] += (int)q[2 * u + e].w;
+                    }
+                }
             }
         }
     }
-    const int nout = a.part16 ? 2 : 1;
-    for (int e = 0; e < nout; e++) {
-        int4 v = e ? v1 : v0;
-        const int oi = o + e;
-        const int rr = oi >> 3, q = oi & 7;
-        if (r.k0 + 4 * q + 3 >= a.T) {
-            const int kq = r.k0 + 4 * q;
-            if (kq >= a.T) v.x = 0;
-            if (kq + 1 >= a.T) v.y = 0;
-            if (kq + 2 >= a.T) v.z = 0;
-            if (kq + 3 >= a.T) v.w = 0;
-        }
-        a.acc[r.off4 + (size_t)rr * a.pitch4 + q] = v;
-        if (NOTE) {
-            const unsigned bits =
-                above4(v, a.pimgs ? a.pimgs[r.img].threshold : a.thr0, r.k0 + 4 * q, a.T);
-            if (bits)
-                note_cands(a.cand, r.img,
-                           (unsigned)(r.w0 + rr) * (unsigned)a.T + (unsigned)(r.k0 + 4 * q), bits);
-        }
+    /* rows that no slab reaches stay zero (see hl_vote_kernel) */
+    if (!hits)
+        return;
+    const int k = blk.slice * HL_SLICE + 8 * g + 2 * cp;
+    const bool k0v = k < a.T, k1v = k + 1 < a.T;
+    int32_t *dst = im.acc + k;
+    if (!a.cand.e) {   /* the whole accumulator is asked for */
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (4 * rg + u < R)
+                *reinterpret_cast<int2 *>(dst + (size_t)(4 * rg + u) * a.Tp) =
+                    make_int2(k0v ? v[0][u] : 0, k1v ? v[1][u] : 0);
+        return;
     }
+    const int thr = max(im.threshold, 0);
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+        if (max(v[0][u], v[1][u]) > thr && 4 * rg + u < R)
+#pragma unroll
+            for (int e = 0; e < 2; e++)
+                if (v[e][u] > thr && (e ? k1v : k0v)) {
+                    dst[(size_t)(4 * rg + u) * a.Tp + e] = v[e][u];
+                    note_cand(a.cand, blk.img,
+                              (unsigned)(4 * rg + u) * (unsigned)a.T + (unsigned)(k + e));
+                }
 }
 
-cudaError_t hl_launch_merge(const hl_merge_args *a, int max_rows, cudaStream_t s)
+cudaError_t hl_launch_merge(hl_merge_args *a, int max_R, cudaStream_t s)
 {
-    if (a->nreg <= 0)
+    if (a->nblocks <= 0)
         return cudaSuccess;
-    const int per_thread = a->part16 ? 2 : 1;   /* output int4 per thread */
-    const unsigned gx =
-        (unsigned)((max_rows * (HL_SLICE / 4) / per_thread + 255) / 256);
-    if (a->cand.e)
-        return hl_launch_pdl(hl_merge_kernel<true>, dim3(gx, (unsigned)a->nreg), dim3(256), 0, s,
-                             false, *a);
-    return hl_launch_pdl(hl_merge_kernel<false>, dim3(gx, (unsigned)a->nreg), dim3(256), 0, s,
-                         false, *a);
-}
-
-cudaError_t hl_launch_tile_masks(const hl_vote_args *a, int nimg, size_t max_words,
-                                 cudaStream_t s)
-{
-    if (nimg <= 0 || max_words == 0)
-        return cudaSuccess;
-    size_t blocks = (max_words * 32 + 255) / 256;
-    if (blocks > 4096)
-        blocks = 4096;
-    hl_tile_mask_kernel<<<dim3((unsigned)blocks, (unsigned)nimg), 256, 0, s>>>(*a);
-    return cudaGetLastError();
-}
-
-template <bool UNIT, bool NOTE>
-static cudaError_t launch_vote_t(const hl_vote_args *a, int threads, int grid, size_t smem,
-                                 cudaStream_t s)
-{
-    const cudaError_t e = cudaFuncSetAttribute(hl_vote_kernel<UNIT, NOTE>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem);
-    if (e != cudaSuccess)
-        return e;
-    return hl_launch_pdl(hl_vote_kernel<UNIT, NOTE>, dim3(grid), dim3(threads), smem, s, false,
-                         *a);
+    a->chunks = (unsigned)((max_R + 63) / 64);   /* 64 rows of a block a CTA */
+    const unsigned long long grid = (unsigned long long)a->chunks * (unsigned)a->nblocks;
+    if (grid > 0x7fffffffull)
+        return cudaErrorInvalidConfiguration;
+    return hl_launch_pdl(a->part16 ? hl_merge_kernel<true> : hl_merge_kernel<false>,
+                         dim3((unsigned)grid), dim3(256), 0, s, false, *a);
 }
 
 cudaError_t hl_launch_vote(const hl_vote_args *a, int threads, int grid,
                            cudaStream_t s)
 {
     const size_t smem = hl_vote_smem_bytes(a->win_rows);
-    const bool note = a->cand.e != nullptr;
-    if (a->irho == 1.0f)
-        return note ? launch_vote_t<true, true>(a, threads, grid, smem, s)
-                    : launch_vote_t<true, false>(a, threads, grid, smem, s);
-    return note ? launch_vote_t<false, true>(a, threads, grid, smem, s)
-                : launch_vote_t<false, false>(a, threads, grid, smem, s);
+    const auto kernel = a->irho == 1.0f ? hl_vote_kernel<true> : hl_vote_kernel<false>;
+    const cudaError_t e = cudaFuncSetAttribute(
+        kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess)
+        return e;
+    return hl_launch_pdl(kernel, dim3(grid), dim3(threads), smem, s, false, *a);
 }
 
 /* ---- voting over a coordinate list ------------------------------------------
