@@ -898,7 +898,18 @@ static int roi_of(const hl_image_desc *img, hl_roi *roi)
     return HL_NO_ERROR;
 }
 
-/* stages (a) + (b) into h->d_acc ([R][Tp]) */
+/* hl_launch_compact on a ticket counter of its own (the number of tickets a
+ * launch takes is not known) */
+static cudaError_t launch_compact_groups(hl_handle *h, hl_compact_args *ca, cudaStream_t s)
+{
+    const cudaError_t e = cudaMemsetAsync(h->d_counters + 12, 0, sizeof(unsigned), s);
+    if (e != cudaSuccess)
+        return e;
+    ca->ticket = reinterpret_cast<unsigned *>(h->d_counters + 12);
+    ca->ticket_base = 0;
+    return hl_launch_compact(ca, s);
+}
+
 /* Stage (a) of one image's ROI into h->d_pts (float2, tile-major, odd tiles
  * padded), h->d_tile_off and the point count h->d_counters[2]: about one
  * CTA per SM when they fit at once, else one CTA per 4-tile group. */
@@ -930,12 +941,12 @@ static int launch_compaction(hl_handle *h, const hl_roi &roi, const hl_geom &g,
         CK(hl_launch_compact_persist(&ca, nct, s));
         h->ticket_base += (unsigned)nct;
     } else {
-        CK(hl_launch_compact(&ca, s));
-        h->ticket_base += (unsigned)((ntiles + HL_COMPACT_GROUP - 1) / HL_COMPACT_GROUP);
+        CK(launch_compact_groups(h, &ca, s));
     }
     return HL_NO_ERROR;
 }
 
+/* stages (a) + (b) into h->d_acc ([R][Tp]) */
 static int run_ab(hl_handle *h, const hl_roi &roi, const hl_geom &g, bool peaks,
                   cudaStream_t s, int *launches)
 {
@@ -1256,8 +1267,7 @@ extern "C" int hl_compact(hl_handle *h, const hl_image_desc *img,
             CK(hl_launch_compact_persist(&ca, nct, s));
             h->ticket_base += (unsigned)nct;
         } else {
-            CK(hl_launch_compact(&ca, s));
-            h->ticket_base += (unsigned)((ntiles + HL_COMPACT_GROUP - 1) / HL_COMPACT_GROUP);
+            CK(launch_compact_groups(h, &ca, s));
         }
     }
     h->last_launches = 1;

@@ -3,16 +3,13 @@
  *
  * Compaction replaces the flag / ScanArray / scatter chain of
  * ImgConvert::imgConvertToCst (okano_3_0/ImgConvert.cu:142-353,
- * okano_3_0/ScanArray.cu:1351+) with ONE pass: every CTA reads a group of
- * four 128 x 32 tiles with 16-byte vector loads (all four issued before any
- * is used), counts their 255-pixels with one packed block scan, obtains the
- * group's exclusive prefix by decoupled look-back over its predecessors'
- * published aggregates, and scatters packed coordinates.  The predicate is
- * the vote kernel's `pixel == 255` (okano_3_0/HoughLine.cu:125), not
+ * okano_3_0/ScanArray.cu:1351+) with ONE pass over the image: tiles of 128 x 32
+ * pixels are read with 16-byte loads, their 255-pixels counted, the counts
+ * published, the predecessors' summed and the coordinates written, by
+ * persistent CTAs that pipeline groups of four tiles (batches, images of more
+ * than 20 M pixels) or by one large CTA per SM (single images).  The predicate
+ * is the vote kernel's `pixel == 255` (okano_3_0/HoughLine.cu:125), not
  * ImgConvert's `>= 128`.
- *
- * HBM-bound: each image byte is read once (w*h bytes) and each edge point is
- * written once (4 bytes).
  */
 #include <algorithm>
 
@@ -45,21 +42,23 @@ cudaError_t hl_launch_trig(float *cosv, float *sinv, int T, int Tp,
     return cudaGetLastError();
 }
 
-/* 4-bit mask of the bytes of w equal to 0xFF (bit i = byte i). */
-__device__ __forceinline__ uint32_t eq255x4(uint32_t w)
-{
-    uint32_t m = __vcmpeq4(w, 0xffffffffu) & 0x80808080u;
-    return (m * 0x00204081u) >> 28;
-}
-
-/* The same mask by exact SWAR arithmetic: a byte of ~w is zero exactly when
- * the byte of w is 0xFF; (b & 0x7F) + 0x7F sets the high bit of every
- * nonzero low part with no carry between bytes, OR b keeps the rest. */
-__device__ __forceinline__ uint32_t ff_nibble(uint32_t w)
+/* 0x80 in the bytes of w equal to 0xFF, by exact SWAR arithmetic: a byte of ~w
+ * is zero exactly when the byte of w is 0xFF; (b & 0x7F) + 0x7F sets the high
+ * bit of every nonzero low part with no carry between bytes, OR b keeps the
+ * rest. */
+__device__ __forceinline__ uint32_t ff_flags(uint32_t w)
 {
     const uint32_t t = ~w;
-    const uint32_t nz = (((t & 0x7f7f7f7fu) + 0x7f7f7f7fu) | t) & 0x80808080u;
-    return ((~nz & 0x80808080u) * 0x00204081u) >> 28;
+    return ~(((t & 0x7f7f7f7fu) + 0x7f7f7f7fu) | t) & 0x80808080u;
+}
+
+/* 16-bit mask of the bytes of v equal to 0xFF (bit i = byte i): the flags times
+ * the bits' weights, summed by byte dot products (128 times the mask) */
+__device__ __forceinline__ uint32_t ff_mask16(const uint4 &v)
+{
+    const uint32_t lo = __dp4a(ff_flags(v.y), 0x80402010u, __dp4a(ff_flags(v.x), 0x08040201u, 0u));
+    const uint32_t hi = __dp4a(ff_flags(v.w), 0x80402010u, __dp4a(ff_flags(v.z), 0x08040201u, 0u));
+    return (lo >> 7) + (hi << 1);
 }
 
 /* Look-back state word: epoch (30 bits) | flag (2 bits) | value (32 bits).
@@ -93,21 +92,17 @@ __device__ __forceinline__ unsigned long long lb_load(
     return v;
 }
 
-/* Warp-wide decoupled look-back (all 32 lanes of warp 0 call it).  Returns
- * the exclusive prefix of `tile`.  Waits are bounded: past LB_SPIN_LIMIT
+/* Warp-wide decoupled look-back (all 32 lanes of warp 0 call it) of a tile
+ * whose own total is published already (as a prefix when it is the first).
+ * Returns the exclusive prefix of `tile`.  Waits are bounded: past LB_SPIN_LIMIT
  * polls the status word gets HL_ST_LOOKBACK_TIMEOUT and the partial sum is
  * used, so the kernel always ends. */
 __device__ int lookback(unsigned long long *state, int tile, int total,
                         unsigned epoch, int *status)
 {
     const int lane = threadIdx.x & 31;
-    if (tile == 0) {
-        if (lane == 0)
-            lb_store(&state[0], lb_pack(epoch, LB_PRE, (unsigned)total));
+    if (tile == 0)
         return 0;
-    }
-    if (lane == 0)
-        lb_store(&state[tile], lb_pack(epoch, LB_AGG, (unsigned)total));
     int excl = 0;
     int top = tile - 1;
     int spins = 0;
@@ -161,12 +156,10 @@ __device__ int lookback(unsigned long long *state, int tile, int total,
 
 /* Exclusive prefix of group g as the plain sum of every predecessor's own
  * count (all threads of the CTA call it; each group publishes only its count,
- * flag AGG, and never an inclusive prefix).  With every group of a launch
- * resident at once -- a 4096 x 4096 image has 1024 groups -- the chained
- * look-back forwards inclusive prefixes only 32 groups per memory round
- * trip; here a group waits just for its slowest predecessor to publish, and
- * 256 threads read up to 1024 predecessors in one round trip.  Waits are
- * bounded as in lookback(). */
+ * flag AGG, and never an inclusive prefix): a group waits just for its slowest
+ * predecessor to publish, and 256 threads read up to 1024 predecessors in one
+ * round trip, where the chained look-back forwards inclusive prefixes only 32
+ * groups per memory round trip.  Waits are bounded as in lookback(). */
 template <int NT>
 __device__ int prefix_all(const unsigned long long *state, int g, unsigned epoch,
                           int *status, int *s_red)
@@ -176,7 +169,13 @@ __device__ int prefix_all(const unsigned long long *state, int g, unsigned epoch
     while (true) {
         int sum = 0;
         bool bad = false;
-        for (int j0 = 0; j0 < g; j0 += 4 * NT) {
+        if (g <= NT) {
+            if (tid < g) {
+                const unsigned long long st = lb_load(&state[tid]);
+                bad = (unsigned)(st >> 34) != epoch || ((st >> 32) & 3u) == 0u;
+                sum = (int)(unsigned)st;
+            }
+        } else for (int j0 = 0; j0 < g; j0 += 4 * NT) {
             unsigned long long st[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
@@ -194,17 +193,14 @@ __device__ int prefix_all(const unsigned long long *state, int g, unsigned epoch
                 }
             }
         }
+        sum = __reduce_add_sync(FULL, sum);
+        if ((tid & 31) == 0)
+            s_red[tid >> 5] = sum;
         if (!__syncthreads_or(bad)) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-                sum += __shfl_xor_sync(FULL, sum, o);
-            if ((tid & 31) == 0)
-                s_red[tid >> 5] = sum;
-            __syncthreads();
             int t = 0;
+#pragma unroll
             for (int w = 0; w < NT / 32; w++)
                 t += s_red[w];
-            __syncthreads();
             return t;
         }
         bool quit = ++spins > LB_SPIN_LIMIT;
@@ -219,185 +215,319 @@ __device__ int prefix_all(const unsigned long long *state, int g, unsigned epoch
     }
 }
 
-/* Tiles per CTA: one look-back and four 16-byte loads in flight per thread
- * for every 16 KB of image. */
+/* A group of CT_GROUP consecutive tiles, four 16-byte loads a thread. */
 #define CT_GROUP HL_COMPACT_GROUP
+#define CT_CTAS_PER_SM 5
+#define CT_PAD 0xffffu
 
-__global__ void __launch_bounds__(HL_COMPACT_THREADS, 8)
+struct CompactGroup {
+    hl_compact_img im;
+    int g;                        /* group in the batch, or -1: no more */
+    int whole;                    /* four whole tiles of 16-byte aligned rows */
+    int x0[CT_GROUP], y0[CT_GROUP];
+    const uint8_t *p[CT_GROUP];   /* the tiles' first pixels */
+};
+
+/* Compaction of many groups (batches; images too large for the cooperative
+ * kernel below) by persistent CTAs, two groups in flight each: while the
+ * counts of group i are published, the image bytes of group i + 1 are on their
+ * way and group i - 1, whose predecessors have had a stage's time to publish,
+ * gets its prefix and is scattered.  A ticket orders the groups, so a group
+ * waits only for groups that were taken before it: of the unpublished ones the
+ * first never waits for another, and every wait ends.  Tickets, image numbers
+ * and image records are fetched two to four groups ahead by one warp, a hop a
+ * stage.
+ * The points go through shared memory, so that the divergent loop over mask
+ * bits is short and the list is written in whole lines.
+ * 256 images, 340 MB: 137 us (243 us with a CTA a group: ticket, records, bytes,
+ * prefix and scatter in one chain of 13 us, the bytes on their way for a tenth
+ * of it).  Bound by instruction issue (about two thirds of the slots) and the
+ * barriers of a stage; 4, 5 and 6 CTAs an SM 1095, 1097, 1109 us for the whole
+ * batch call. */
+__global__ void __launch_bounds__(HL_COMPACT_THREADS, CT_CTAS_PER_SM)
 hl_compact_kernel(hl_compact_args a)
 {
-    __shared__ int s_grp;
-    __shared__ hl_compact_img s_im;
-    __shared__ unsigned long long s_wsum[HL_COMPACT_THREADS / 32];
-    __shared__ int s_tbase[CT_GROUP];
-    __shared__ int s_tcnt[CT_GROUP];
-    __shared__ unsigned long long s_tot4;
+    constexpr int NW = HL_COMPACT_THREADS / 32;
+    __shared__ CompactGroup s_grp[4];             /* group i in slot i & 3 */
+    /* group i - 1's points: tile << 12 | row << 7 | column; CT_PAD: a sentinel */
+    __shared__ unsigned short s_out[CT_GROUP * (HL_TILE_W * HL_TILE_H + 1)];
+    __shared__ unsigned long long s_wsum[2][NW];  /* warps' counts, then offsets */
+    __shared__ int s_tb[2][CT_GROUP + 1];         /* tile bases in the group */
+    __shared__ int s_cnt[2][CT_GROUP];            /* tile counts */
+    __shared__ int s_red[NW];
     __shared__ int s_excl;
-    __shared__ int s_red[HL_COMPACT_THREADS / 32];
+    /* the fetching warp's: tickets of the slots i + 2 and i + 3, i + 2's image */
+    __shared__ int s_t2, s_t3, s_i2;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ngroups = a.imgs ? a.ngroups : (a.ntiles + CT_GROUP - 1) / CT_GROUP;
+    const int pad = a.pts_f2 ? 1 : 0;
     hl_pdl_begin();
 
-    /* Groups are taken in ticket order, so every predecessor of a group is
-     * already resident when the group looks back: the waits always end. */
-    if (tid == 0) {
-        const int g = (int)(atomicAdd(a.ticket, 1u) - a.ticket_base);
-        s_grp = g;
-        if (!a.imgs) {
-            s_im.roi = a.roi;
-            s_im.tiles_x = a.tiles_x;
-            s_im.ntiles = a.ntiles;
-            s_im.tile_base = 0;
-            s_im.group_base = 0;
-            s_im.ngroups = ngroups;
-            s_im.pts_base = 0;
-        } else if (g >= 0 && g < ngroups) {
-            s_im = a.imgs[a.group_img[g]];
+    const bool fetch = warp == NW - 1;
+    const auto ticket = [&](int prev) {
+        int t = -1;
+        if (prev >= 0 && lane == 0) {
+            t = (int)(atomicAdd(a.ticket, 1u) - a.ticket_base);
+            if (t >= ngroups)
+                t = -1;
+        }
+        return t;   /* lane 0's */
+    };
+    const auto image_of = [&](int t) { return a.imgs && lane == 0 && t >= 0 ? a.group_img[t] : 0; };
+    /* the record's words, a lane each */
+    const auto record = [&](int gi) {
+        gi = __shfl_sync(FULL, gi, 0);   /* lane 0's */
+        return a.imgs && lane < (int)(sizeof(hl_compact_img) / 4)
+                   ? reinterpret_cast<const int *>(a.imgs + gi)[lane]
+                   : 0;
+    };
+    const auto publish_slot = [&](int slot, int t, int word) {
+        CompactGroup &s = s_grp[slot];
+        if (a.imgs) {
+            if (lane < (int)(sizeof(hl_compact_img) / 4))
+                reinterpret_cast<int *>(&s.im)[lane] = word;
+        } else if (lane == 0) {
+            s.im.roi = a.roi;
+            s.im.tiles_x = a.tiles_x;
+            s.im.ntiles = a.ntiles;
+            s.im.tile_base = 0;
+            s.im.group_base = 0;
+            s.im.ngroups = ngroups;
+            s.im.pts_base = 0;
+        }
+        t = __shfl_sync(FULL, t, 0);     /* lane 0's */
+        __syncwarp();
+        bool in = true;
+        if (lane < CT_GROUP && t >= 0) {
+            const int tile = (t - s.im.group_base) * CT_GROUP + lane;
+            const int ty = tile / s.im.tiles_x;
+            const int x = (tile - ty * s.im.tiles_x) * HL_TILE_W;
+            /* tiles past the last one lie below the image */
+            const int y = tile < s.im.ntiles ? ty * HL_TILE_H : s.im.roi.h;
+            const uint8_t *p = s.im.roi.base + (size_t)y * (size_t)s.im.roi.pitch + x;
+            s.x0[lane] = x;
+            s.y0[lane] = y;
+            s.p[lane] = p;
+            in = y + HL_TILE_H <= s.im.roi.h && x + HL_TILE_W <= s.im.roi.w &&
+                 (((uintptr_t)p | (uintptr_t)s.im.roi.pitch) & 15u) == 0;
+        }
+        in = __all_sync(FULL, in);
+        if (lane == 0) {
+            s.g = t;
+            s.whole = in;
+        }
+    };
+    if (fetch) {
+        /* one ticket after the other: a CTA that took several at once would
+         * hold groups that the next CTAs' first ones wait for */
+        const int t0 = ticket(0);
+        const int i0 = image_of(t0), t1 = ticket(t0);
+        const int w0 = record(i0), i1 = image_of(t1), t2 = ticket(t1);
+        publish_slot(0, t0, w0);
+        const int w1 = record(i1), i2 = image_of(t2), t3 = ticket(t2);
+        publish_slot(1, t1, w1);
+        if (lane == 0) {
+            s_t2 = t2;
+            s_t3 = t3;
+            s_i2 = i2;
         }
     }
     __syncthreads();
-    const int ggrp = s_grp;              /* group in the batch (look-back) */
-    if (ggrp < 0 || ggrp >= ngroups)
-        return;
-    const int grp = ggrp - s_im.group_base;   /* group in its image */
-    const int r = tid >> 3, ch = tid & 7;
 
-    /* this thread's 16 pixels of tile q: row ty*32 + r, columns
-     * tx*128 + 16*ch .. +15 (recomputed where needed, to keep the live
-     * registers low enough for eight CTAs per SM) */
-    const int tx0 = (grp * CT_GROUP) % s_im.tiles_x, ty0 = (grp * CT_GROUP) / s_im.tiles_x;
-#define CT_TILE_XY(q, xx, yy)                                                  \
-    const int xx = ((tx0 + (q)) % s_im.tiles_x) * HL_TILE_W + ch * 16;         \
-    const int yy = (ty0 + (tx0 + (q)) / s_im.tiles_x) * HL_TILE_H + r
-    /* all loads first */
+    const int r = tid >> 3, ch = tid & 7;
+    /* this thread's 16 pixels of tile q: row y0 + r, columns x0 + 16 ch .. + 15 */
     uint4 v[CT_GROUP];
+    const auto load = [&](const CompactGroup &s) {
+        const size_t off = (size_t)r * (size_t)s.im.roi.pitch + ch * 16;
+        if (s.whole) {
 #pragma unroll
-    for (int q = 0; q < CT_GROUP; q++) {
-        CT_TILE_XY(q, xq, yq);
-        const bool any = grp * CT_GROUP + q < s_im.ntiles && yq < s_im.roi.h && xq < s_im.roi.w;
-        const uint8_t *p = s_im.roi.base + (size_t)yq * (size_t)s_im.roi.pitch + xq;
-        const bool vec = any && xq + 16 <= s_im.roi.w && (((uintptr_t)p) & 15u) == 0;
-        v[q] = vec ? __ldcs((const uint4 *)p) : make_uint4(0, 0, 0, 0);
-    }
-    uint32_t m[CT_GROUP];
-    unsigned long long cnt4 = 0;   /* four 16-bit counts, tile q in bits 16q */
-#pragma unroll
-    for (int q = 0; q < CT_GROUP; q++) {
-        CT_TILE_XY(q, xq, yq);
-        const bool any = grp * CT_GROUP + q < s_im.ntiles && yq < s_im.roi.h && xq < s_im.roi.w;
-        const uint8_t *p = s_im.roi.base + (size_t)yq * (size_t)s_im.roi.pitch + xq;
-        const bool vec = any && xq + 16 <= s_im.roi.w && (((uintptr_t)p) & 15u) == 0;
-        uint32_t mm = 0;
-        if (vec) {
-            mm = eq255x4(v[q].x) | (eq255x4(v[q].y) << 4) |
-                 (eq255x4(v[q].z) << 8) | (eq255x4(v[q].w) << 12);
-        } else if (any) {
-            const int lim = min(16, s_im.roi.w - xq);
-            for (int i = 0; i < lim; i++)
-                mm |= (uint32_t)(p[i] == 255) << i;
+            for (int q = 0; q < CT_GROUP; q++)
+                v[q] = __ldcs(reinterpret_cast<const uint4 *>(s.p[q] + off));
+            return;
         }
-        m[q] = mm;
-        cnt4 |= (unsigned long long)__popc(mm) << (16 * q);
-    }
-    /* block scan of the packed counts (no field exceeds 4096) */
-    unsigned long long incl = cnt4;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long t = __shfl_up_sync(FULL, incl, o);
-        if (lane >= o)
-            incl += t;
-    }
-    if (lane == 31)
-        s_wsum[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        const int nw = HL_COMPACT_THREADS / 32;
-        const unsigned long long ws = lane < nw ? s_wsum[lane] : 0ull;
-        unsigned long long wi = ws;
-#pragma unroll
-        for (int o = 1; o < nw; o <<= 1) {
-            const unsigned long long t = __shfl_up_sync(FULL, wi, o);
-            if (lane >= o)
-                wi += t;
-        }
-        const unsigned long long tot4 = __shfl_sync(FULL, wi, nw - 1);
-        if (lane < nw)
-            s_wsum[lane] = wi - ws;
-        /* float2 output: every tile holds an even number of entries (one
-         * sentinel pads an odd count), so runs of tiles start and end on
-         * 16-byte boundaries */
-        const int pad = a.pts_f2 ? 1 : 0;
-        int total = 0;
 #pragma unroll
         for (int q = 0; q < CT_GROUP; q++) {
-            const int cq = (int)((tot4 >> (16 * q)) & 0xffffu);
-            total += cq + (cq & pad);
+            const int x = s.x0[q] + ch * 16, y = s.y0[q] + r;
+            const uint8_t *p = s.p[q] + off;
+            const bool vec = y < s.im.roi.h && x + 16 <= s.im.roi.w && (((uintptr_t)p) & 15u) == 0;
+            v[q] = vec ? __ldcs(reinterpret_cast<const uint4 *>(p)) : make_uint4(0, 0, 0, 0);
         }
-        /* the prefix runs over the image's own groups */
-        unsigned long long *st = a.tile_state + s_im.group_base;
-        if (s_im.ngroups > LB_FULL_MAX) {
-            const int excl = lookback(st, grp, total, a.epoch, a.status);
-            if (lane == 0)
-                s_excl = excl;
-        } else if (lane == 0) {
-            lb_store(&st[grp], lb_pack(a.epoch, LB_AGG, (unsigned)total));
+    };
+    if (s_grp[0].g >= 0)
+        load(s_grp[0]);
+    uint32_t pm[CT_GROUP / 2] = {0u, 0u};   /* group i - 1: masks, offsets in the warp */
+    unsigned long long pex = 0;
+    for (int i = 0;; i++) {
+        const CompactGroup &cur = s_grp[i & 3];
+        const bool have = cur.g >= 0;
+        const int par = i & 1;
+        /* fetches for the slots i + 2 .. i + 4 */
+        int w2 = 0, i3 = 0, t4 = -1;
+        if (fetch) {
+            w2 = record(s_i2);
+            i3 = image_of(s_t3);
+            t4 = ticket(s_t3);
         }
-        if (lane == 0)
-            s_tot4 = tot4;
-    }
-    __syncthreads();
-    if (s_im.ngroups <= LB_FULL_MAX) {
-        const int excl = prefix_all<HL_COMPACT_THREADS>(a.tile_state + s_im.group_base, grp,
-                                                        a.epoch, a.status, s_red);
-        if (tid == 0)
-            s_excl = excl;
-        __syncthreads();
-    }
-    {
-        const int pad = a.pts_f2 ? 1 : 0;
-        const unsigned long long tot4 = s_tot4;
-        if (tid == 0) {
-            int run = s_excl;
+        uint32_t m[CT_GROUP / 2] = {0u, 0u};
+        unsigned long long ex = 0;
+        if (have) {
+            unsigned long long cnt4 = 0;   /* four 16-bit counts, tile q in bits 16q */
 #pragma unroll
             for (int q = 0; q < CT_GROUP; q++) {
-                const int tile = grp * CT_GROUP + q;
-                const int cq = (int)((tot4 >> (16 * q)) & 0xffffu);
-                s_tbase[q] = run;
-                s_tcnt[q] = cq;
-                if (tile < s_im.ntiles)
-                    a.tile_off[s_im.tile_base + tile] = run;
-                run += cq + (cq & pad);
+                uint32_t mm = ff_mask16(v[q]);
+                if (!cur.whole) {
+                    const int x = cur.x0[q] + ch * 16;
+                    if (cur.y0[q] + r < cur.im.roi.h && x < cur.im.roi.w) {
+                        const uint8_t *p = cur.p[q] + (size_t)r * (size_t)cur.im.roi.pitch + ch * 16;
+                        if (x + 16 > cur.im.roi.w || (((uintptr_t)p) & 15u) != 0) {
+                            const int lim = min(16, cur.im.roi.w - x);
+                            for (int b = 0; b < lim; b++)
+                                mm |= (uint32_t)(p[b] == 255) << b;
+                        }
+                    }
+                }
+                m[q >> 1] |= mm << (16 * (q & 1));
+                cnt4 |= (unsigned long long)__popc(mm) << (16 * q);
             }
-            /* the image's end (equal to the next image's start) */
-            if (grp == s_im.ngroups - 1)
-                a.tile_off[s_im.tile_base + s_im.ntiles] = run;
-            if (ggrp == ngroups - 1)
-                *a.count = run;
-        }
-    }
-    __syncthreads();
-    const unsigned long long ex4 = s_wsum[warp] + incl - cnt4;
+            /* warp scan of the packed counts (no field exceeds 4096) */
+            unsigned long long incl = cnt4;
 #pragma unroll
-    for (int q = 0; q < CT_GROUP; q++) {
-        CT_TILE_XY(q, xq, yq);
-        uint32_t mm = m[q];
-        int pos = s_tbase[q] + (int)((ex4 >> (16 * q)) & 0xffffu);
-        const uint32_t yy = (uint32_t)yq << 16;
-        while (mm) {
-            const int bb = __ffs(mm) - 1;
-            mm &= mm - 1;
-            if (a.pts_f2)
-                a.pts_f2[s_im.pts_base + pos] = make_float2((float)(xq + bb), (float)yq);
-            else
-                a.pts[s_im.pts_base + pos] = (uint32_t)(xq + bb) | yy;
-            pos++;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long t = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o)
+                    incl += t;
+            }
+            ex = incl - cnt4;
+            if (lane == 31)
+                s_wsum[par][warp] = incl;
         }
+        const CompactGroup &nxt = s_grp[(i + 1) & 3];
+        if (have && nxt.g >= 0)
+            load(nxt);
+        __syncthreads();
+        if (have && warp == 0) {
+            const unsigned long long ws = lane < NW ? s_wsum[par][lane] : 0ull;
+            unsigned long long wi = ws;
+#pragma unroll
+            for (int o = 1; o < NW; o <<= 1) {
+                const unsigned long long t = __shfl_up_sync(FULL, wi, o);
+                if (lane >= o)
+                    wi += t;
+            }
+            const unsigned long long tot4 = __shfl_sync(FULL, wi, NW - 1);
+            if (lane < NW)
+                s_wsum[par][lane] = wi - ws;
+            if (lane == 0) {
+                /* float2 output: every tile holds an even number of entries
+                 * (one sentinel pads an odd count), so runs of tiles start and
+                 * end on 16-byte boundaries */
+                int run = 0;
+#pragma unroll
+                for (int q = 0; q < CT_GROUP; q++) {
+                    const int cq = (int)((tot4 >> (16 * q)) & 0xffffu);
+                    s_tb[par][q] = run;
+                    s_cnt[par][q] = cq;
+                    run += cq + (cq & pad);
+                }
+                s_tb[par][CT_GROUP] = run;
+                /* the prefix runs over the image's own groups; the chained one
+                 * starts from the first group's */
+                const int grp = cur.g - cur.im.group_base;
+                const bool first = grp == 0 && cur.im.ngroups > LB_FULL_MAX;
+                lb_store(a.tile_state + cur.g, lb_pack(a.epoch, first ? LB_PRE : LB_AGG,
+                                                       (unsigned)run));
+            }
+        }
+        if (fetch) {
+            publish_slot((i + 2) & 3, s_t2, w2);
+            if (lane == 0) {
+                s_t2 = s_t3;
+                s_t3 = t4;
+                s_i2 = i3;
+            }
+            __syncwarp();
+        }
+        if (i == 0) {
+            __syncthreads();
+        } else {
+            /* group i - 1: prefix and scatter */
+            const CompactGroup &pr = s_grp[(i - 1) & 3];
+            const int pp = par ^ 1;
+            const int grp = pr.g - pr.im.group_base;
+            /* the points' places in the group, two tiles' 32 pixels at a time:
+             * a tile's first place less the thread's points before it, in 16
+             * bits (a tile's base counts them), plus the point's number */
+            {
+                unsigned long long e4 = s_wsum[pp][warp] + pex;
+                int before = 0;
+#pragma unroll
+                for (int q = 0; q < CT_GROUP; q++) {
+                    e4 += (unsigned long long)(s_tb[pp][q] - before) << (16 * q);
+                    before += __popc((pm[q >> 1] >> (16 * (q & 1))) & 0xffffu);
+                }
+                int n = 0;
+#pragma unroll
+                for (int hf = 0; hf < CT_GROUP / 2; hf++) {
+                    const unsigned e2 = (unsigned)(e4 >> (32 * hf));
+                    const unsigned code = ((2u * hf) << 12) | (unsigned)(r << 7) | (unsigned)(ch * 16);
+                    for (uint32_t mm = pm[hf]; mm; mm &= mm - 1, n++) {
+                        const unsigned b = (unsigned)__ffs(mm) - 1u;
+                        /* bit 4 of b is the tile: from there to bit 12 */
+                        s_out[((e2 >> (b & 16u)) & 0xffffu) + n] =
+                            (unsigned short)(code + b + (b & 16u) * 255u);
+                    }
+                }
+                /* the sentinel (+infinity, 0) of an odd tile never votes inside
+                 * an accumulator: its rho is infinity * cos(theta_k), and cosf
+                 * of a float angle is never 0 */
+                if (pad && tid < CT_GROUP && (s_cnt[pp][tid] & 1))
+                    s_out[s_tb[pp][tid] + s_cnt[pp][tid]] = CT_PAD;
+            }
+            unsigned long long *st = a.tile_state + pr.im.group_base;
+            int excl;
+            if (pr.im.ngroups <= LB_FULL_MAX) {
+                excl = prefix_all<HL_COMPACT_THREADS>(st, grp, a.epoch, a.status, s_red);
+            } else {
+                if (warp == 0) {
+                    const int e = lookback(st, grp, s_tb[pp][CT_GROUP], a.epoch, a.status);
+                    if (lane == 0)
+                        s_excl = e;
+                }
+                __syncthreads();
+                excl = s_excl;
+            }
+            if (tid < CT_GROUP) {
+                const int tile = grp * CT_GROUP + tid;
+                if (tile < pr.im.ntiles)
+                    a.tile_off[pr.im.tile_base + tile] = excl + s_tb[pp][tid];
+            } else if (tid == CT_GROUP) {
+                /* the image's end (equal to the next image's start) */
+                const int end = excl + s_tb[pp][CT_GROUP];
+                if (grp == pr.im.ngroups - 1)
+                    a.tile_off[pr.im.tile_base + pr.im.ntiles] = end;
+                if (pr.g == ngroups - 1)
+                    *a.count = end;
+            }
+            /* the points, in order, as the group's stretch of the list */
+            const long long first = pr.im.pts_base + excl;
+            for (int j = tid; j < s_tb[pp][CT_GROUP]; j += HL_COMPACT_THREADS) {
+                const unsigned e = s_out[j], q = e >> 12;
+                const unsigned x = (e & 127u) + pr.x0[q & 3], y = ((e >> 7) & 31u) + pr.y0[q & 3];
+                if (!a.pts_f2)
+                    a.pts[first + j] = x | (y << 16);
+                else if (e == CT_PAD)
+                    a.pts_f2[first + j] = make_float2(__int_as_float(0x7f800000), 0.0f);
+                else
+                    a.pts_f2[first + j] = make_float2((float)x, (float)y);
+            }
+        }
+        if (!have)
+            break;
+#pragma unroll
+        for (int q = 0; q < CT_GROUP / 2; q++)
+            pm[q] = m[q];
+        pex = ex;
     }
-#undef CT_TILE_XY
-    /* the sentinel (+infinity, 0) never votes inside an accumulator: its rho is
-     * infinity * cos(theta_k), and cosf of a float angle is never 0 */
-    if (a.pts_f2 && tid < CT_GROUP && (s_tcnt[tid] & 1))
-        a.pts_f2[s_im.pts_base + s_tbase[tid] + s_tcnt[tid]] = make_float2(__int_as_float(0x7f800000), 0.0f);
 }
 
 /* Single-image compaction with few, large CTAs: CTA c of nct takes tiles [ntiles c / nct, ntiles (c + 1) / nct) -- at most CP_MAXT --
@@ -489,8 +619,7 @@ hl_compact_persist_kernel(hl_compact_args a, int nct)
             if (y < a.roi.h && x < a.roi.w) {
                 const uint8_t *p = a.roi.base + (size_t)y * (size_t)a.roi.pitch + x;
                 if (x + 16 <= a.roi.w && (((uintptr_t)p) & 15u) == 0) {
-                    mm = ff_nibble(v[k].x) | (ff_nibble(v[k].y) << 4) |
-                         (ff_nibble(v[k].z) << 8) | (ff_nibble(v[k].w) << 12);
+                    mm = ff_mask16(v[k]);
                 } else {
                     const int lim = min(16, a.roi.w - x);
                     for (int i = 0; i < lim; i++)
@@ -661,11 +790,19 @@ cudaError_t hl_launch_compact_persist(const hl_compact_args *a, int nct, cudaStr
                          *a, nct);
 }
 
+static int compact_ctas(int ngroups)
+{
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return std::max(1, std::min(ngroups, std::max(sms, 1) * CT_CTAS_PER_SM));
+}
+
 cudaError_t hl_launch_compact(const hl_compact_args *a, cudaStream_t s)
 {
     const int ngroups = a->imgs ? a->ngroups : (a->ntiles + CT_GROUP - 1) / CT_GROUP;
-    return hl_launch_pdl(hl_compact_kernel, dim3(ngroups), dim3(HL_COMPACT_THREADS), 0, s,
-                         false, *a);
+    return hl_launch_pdl(hl_compact_kernel, dim3(compact_ctas(ngroups)),
+                         dim3(HL_COMPACT_THREADS), 0, s, false, *a);
 }
 
 /* Bounding box of an interleaved (x, y) list: bbox = {xmin, ymin, xmax, ymax}
