@@ -85,6 +85,9 @@ struct hl_handle {
     /* HoughCircle: candidate keys, [ncand, status] counters, results; the
      * workspace of circle batches */
     struct hl_cb_ws *cb;
+    int *d_ctab;             /* the circles' offsets (hl_circle_table) */
+    uint32_t *d_cbits;       /* an image's edge map */
+    size_t cap_cbits;
     unsigned long long *d_ckeys;
     int *d_ccnt;
     unsigned char *d_cres;
@@ -253,7 +256,8 @@ extern "C" int hl_destroy(hl_handle *h)
     void *ptrs[] = {h->d_cos, h->d_sin, h->d_pts, h->d_tile_state,
                     h->d_tile_off, h->d_acc, h->d_keys, h->d_aux,
                     h->d_result, h->d_counters, h->d_plan, h->d_scratch, h->d_cand,
-                    h->d_ckeys, h->d_ccnt, h->d_cres, h->d_bbox};
+                    h->d_ckeys, h->d_ccnt, h->d_cres, h->d_bbox, h->d_ctab,
+                    h->d_cbits};
     for (void *q : ptrs)
         if (q)
             cudaFree(q);
@@ -2616,7 +2620,40 @@ static int circle_prepare(hl_handle *h, const hl_image_desc *img, const hl_circl
     return ensure_image(h, *g, roi->w, roi->h);
 }
 
-/* the compaction, then one tile-kernel launch: the accumulator written to acc
+/* radii of [radius_min, radius_max] that are counted on bit planes: the smallest */
+static int circle_dense(const hl_circle_params *p)
+{
+    return std::max(0, std::min(p->radius_max, HL_CIRCLE_DENSE_R) - p->radius_min + 1);
+}
+
+/* the table of circle offsets, made once a handle; sets the kernel's pointers */
+static int circle_table(hl_handle *h, hl_circle_bits_args *ba)
+{
+    if (!h->d_ctab) {
+        std::vector<int> t(hl_circle_table_bytes() / sizeof(int));
+        hl_circle_table(t.data());
+        int *d = nullptr;
+        CK(cudaMalloc(&d, hl_circle_table_bytes()));
+        const cudaError_t e =
+            cudaMemcpy(d, t.data(), hl_circle_table_bytes(), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) {
+            cudaFree(d);
+            return map_err(e);
+        }
+        h->d_ctab = d;
+    }
+    ba->table = h->d_ctab;
+    ba->count = h->d_ctab + hl_circle_table_bytes() / sizeof(int) - (HL_CIRCLE_DENSE_R + 1);
+    return HL_NO_ERROR;
+}
+
+static long long circle_bits_blocks(const hl_circle_bits_img &b)
+{
+    return ((long long)b.pitch * b.h + 255) / 256;
+}
+
+/* The smaller radii on bit planes of the edge map; the larger ones by the
+ * compaction and one tile-kernel launch: the accumulator written to acc
  * ([nr][h][w]) when it is given, the local maxima appended to the handle's
  * candidate keys when peaks is set */
 static int circle_run(hl_handle *h, const hl_roi &roi, const hl_geom &g,
@@ -2629,9 +2666,40 @@ static int circle_run(hl_handle *h, const hl_roi &roi, const hl_geom &g,
     ta.nty = (roi.h + HL_CIRCLE_TH - 1) / HL_CIRCLE_TH;
     if ((long long)ta.ntx * ta.nty * nr > 0x7fffffffLL)
         return HL_OP_OVERFLOW;   /* more CTAs than one launch takes */
-    int rc = launch_compaction(h, roi, g, s);
-    if (rc != HL_NO_ERROR)
+    int rc;
+    const int nd = circle_dense(p);
+    if (nd > 0) {
+        hl_circle_bits_args ba;
+        memset(&ba, 0, sizeof(ba));
+        hl_circle_bits_img &b = ba.img0;
+        b.roi = roi;
+        b.w = roi.w;
+        b.h = roi.h;
+        hl_circle_bits_tiles(&b);
+        if ((rc = circle_table(h, &ba)) != HL_NO_ERROR ||
+            (rc = grow((void **)&h->d_cbits, &h->cap_cbits,
+                       sizeof(uint32_t) * (size_t)b.pitch * (size_t)b.h)) != HL_NO_ERROR)
+            return rc;
+        b.bits = h->d_cbits;
+        ba.nimg = 1;
+        ba.rmin = p->radius_min;
+        ba.nr = nd;
+        ba.acc = acc;
+        ba.threshold = p->threshold;
+        if (peaks) {
+            ba.keys = h->d_ckeys;
+            ba.ncand = h->d_ccnt;
+            ba.cap = HL_CIRCLE_MAXCAND;
+            ba.status = h->d_ccnt + 1;
+        }
+        CK(hl_launch_edge_bits(nullptr, &b, 1, circle_bits_blocks(b), s));
+        CK(hl_launch_circle_bits(&ba, (long long)b.ntx * b.nty * nd, b.twu, s));
+    }
+    if (nd == nr)
+        return HL_NO_ERROR;
+    if ((rc = launch_compaction(h, roi, g, s)) != HL_NO_ERROR)
         return rc;
+    ta.nz = nr - nd;
     ta.pts = reinterpret_cast<const float2 *>(h->d_pts);
     ta.tile_off = h->d_tile_off;
     ta.ctiles_x = g.tiles_x;
@@ -2754,6 +2822,8 @@ struct hl_cb_ws {
     size_t cap_toff;
     unsigned long long *d_state;
     size_t cap_state;
+    uint32_t *d_bits;
+    size_t cap_bits;
     unsigned char *d_tab;
     size_t cap_tab;
     unsigned char *h_tab;
@@ -2773,7 +2843,7 @@ static void circle_batch_free(hl_handle *h)
     hl_cb_ws *c = h->cb;
     if (!c)
         return;
-    void *dp[] = {c->d_pts, c->d_toff, c->d_state, c->d_tab, c->d_keys, c->d_cnt, c->d_res};
+    void *dp[] = {c->d_pts, c->d_toff, c->d_state, c->d_bits, c->d_tab, c->d_keys, c->d_cnt, c->d_res};
     for (void *q : dp)
         if (q)
             cudaFree(q);
@@ -2809,7 +2879,11 @@ extern "C" int hl_circles_batch(hl_handle *h, const hl_image_desc *imgs, int nim
     std::vector<long long> pts_base((size_t)nimg);
     std::vector<int> tile_base((size_t)nimg), group_base((size_t)nimg), cta_base((size_t)nimg);
     std::vector<int> group_img;
-    long long pts = 0, ctas = 0, tiles = 0, groups = 0;
+    long long pts = 0, ctas = 0, blocks = 0, tiles = 0, groups = 0;
+    const int nd = circle_dense(p);
+    std::vector<hl_circle_bits_img> bi((size_t)nimg);
+    long long bctas = 0, bblocks = 0;
+    int twu_min = 8;
     for (int i = 0; i < nimg; i++) {
         int rc = roi_of(&imgs[i], &rois[i]);
         if (rc != HL_NO_ERROR)
@@ -2833,8 +2907,18 @@ extern "C" int hl_circles_batch(hl_handle *h, const hl_image_desc *imgs, int nim
         const long long ntx = (rois[i].w + HL_CIRCLE_TW - 1) / HL_CIRCLE_TW;
         const long long nty = (rois[i].h + HL_CIRCLE_TH - 1) / HL_CIRCLE_TH;
         cta_base[i] = (int)std::min(ctas, (long long)0x7fffffff);
-        ctas += ntx * nty * nr;
-        if (ctas > 0x7fffffffLL || tiles > 0x7fffffffLL || groups > 0x7fffffffLL)
+        ctas += ntx * nty * (nr - nd);
+        blocks += ntx * nty * nr;
+        bi[i].roi = rois[i];
+        bi[i].w = rois[i].w;
+        bi[i].h = rois[i].h;
+        hl_circle_bits_tiles(&bi[i]);
+        bi[i].cta_base = bctas;
+        bctas += (long long)bi[i].ntx * bi[i].nty * nd;
+        bi[i].blk_base = (int)std::min(bblocks, (long long)0x7fffffff);
+        bblocks += circle_bits_blocks(bi[i]);
+        twu_min = std::min(twu_min, bi[i].twu);
+        if (blocks > 0x7fffffffLL || bblocks > 0x7fffffffLL || tiles > 0x7fffffffLL || groups > 0x7fffffffLL)
             return HL_OP_OVERFLOW;
     }
     if (!h->cb && !(h->cb = new (std::nothrow) hl_cb_ws()))
@@ -2845,13 +2929,19 @@ extern "C" int hl_circles_batch(hl_handle *h, const hl_image_desc *imgs, int nim
     const size_t off_cimg = 0;
     const size_t off_gimg = align16(sizeof(hl_compact_img) * (size_t)nimg);
     const size_t off_circ = align16(off_gimg + sizeof(int) * (size_t)groups);
-    const size_t tab_bytes = align16(off_circ + sizeof(hl_circle_img) * (size_t)nimg);
+    const size_t off_bits = align16(off_circ + sizeof(hl_circle_img) * (size_t)nimg);
+    const size_t tab_bytes = align16(off_bits + sizeof(hl_circle_bits_img) * (size_t)nimg);
     const size_t ncnt = 4 + 2 * (size_t)nimg;   /* ticket, count, status, pad, per ROI */
     int rc;
-    if ((rc = grow((void **)&c->d_pts, &c->cap_pts, sizeof(float2) * (size_t)pts)) != HL_NO_ERROR ||
-        (rc = grow((void **)&c->d_toff, &c->cap_toff, sizeof(int) * (size_t)tiles)) != HL_NO_ERROR ||
-        (rc = grow((void **)&c->d_state, &c->cap_state,
-                   sizeof(unsigned long long) * (size_t)(groups + 1))) != HL_NO_ERROR ||
+    if ((nr > nd &&
+         ((rc = grow((void **)&c->d_pts, &c->cap_pts, sizeof(float2) * (size_t)pts)) !=
+              HL_NO_ERROR ||
+          (rc = grow((void **)&c->d_toff, &c->cap_toff, sizeof(int) * (size_t)tiles)) !=
+              HL_NO_ERROR ||
+          (rc = grow((void **)&c->d_state, &c->cap_state,
+                     sizeof(unsigned long long) * (size_t)(groups + 1))) != HL_NO_ERROR)) ||
+        (rc = grow((void **)&c->d_bits, &c->cap_bits,
+                   sizeof(uint32_t) * 256 * (size_t)bblocks)) != HL_NO_ERROR ||
         (rc = grow((void **)&c->d_tab, &c->cap_tab, tab_bytes)) != HL_NO_ERROR ||
         (rc = grow_host(&c->h_tab, &c->cap_htab, tab_bytes)) != HL_NO_ERROR ||
         (rc = grow((void **)&c->d_keys, &c->cap_keys,
@@ -2889,39 +2979,61 @@ extern "C" int hl_circles_batch(hl_handle *h, const hl_image_desc *imgs, int nim
         im[i].ncand = c->d_cnt + 4 + 2 * i;
         im[i].hdr = reinterpret_cast<hl_result_hdr *>(c->d_res + rstride * i);
         im[i].out = reinterpret_cast<hl_circle *>(c->d_res + rstride * i + sizeof(hl_result_hdr));
+        bi[i].bits = c->d_bits + 256 * (size_t)bi[i].blk_base;
+        bi[i].keys = im[i].keys;
+        bi[i].ncand = im[i].ncand;
     }
+    memcpy(c->h_tab + off_bits, bi.data(), sizeof(hl_circle_bits_img) * (size_t)nimg);
     memcpy(c->h_tab + off_gimg, group_img.data(), sizeof(int) * group_img.size());
     unsigned char *dt = c->d_tab;
     CK(cudaMemsetAsync(c->d_cnt, 0, sizeof(int) * ncnt, s));
-    CK(cudaMemsetAsync(c->d_state, 0, sizeof(unsigned long long) * (size_t)(groups + 1), s));
     CK(cudaMemcpyAsync(dt, c->h_tab, tab_bytes, cudaMemcpyHostToDevice, s));
-    hl_compact_args ca;
-    memset(&ca, 0, sizeof(ca));
-    ca.imgs = reinterpret_cast<const hl_compact_img *>(dt + off_cimg);
-    ca.group_img = reinterpret_cast<const int *>(dt + off_gimg);
-    ca.nimg = nimg;
-    ca.ngroups = (int)groups;
-    ca.tile_state = c->d_state;
-    ca.ticket = reinterpret_cast<unsigned *>(c->d_cnt + 0);
-    ca.ticket_base = 0;
-    ca.epoch = 1;
-    ca.pts = nullptr;
-    ca.pts_f2 = c->d_pts;
-    ca.tile_off = c->d_toff;
-    ca.count = c->d_cnt + 1;
-    ca.status = c->d_cnt + 2;
-    CK(hl_launch_compact(&ca, s));
-    hl_circle_tile_args ta;
-    memset(&ta, 0, sizeof(ta));
-    ta.imgs = reinterpret_cast<const hl_circle_img *>(dt + off_circ);
-    ta.nimg = nimg;
-    ta.nctas = (int)ctas;
-    ta.rmin = p->radius_min;
-    ta.nr = nr;
-    ta.acc = nullptr;
-    ta.threshold = p->threshold;
-    ta.cap = HL_CIRCLE_MAXCAND;
-    CK(hl_launch_circle_tiles(&ta, s));
+    if (nd > 0) {
+        hl_circle_bits_args ba;
+        memset(&ba, 0, sizeof(ba));
+        if ((rc = circle_table(h, &ba)) != HL_NO_ERROR)
+            return rc;
+        ba.imgs = reinterpret_cast<const hl_circle_bits_img *>(dt + off_bits);
+        ba.nimg = nimg;
+        ba.rmin = p->radius_min;
+        ba.nr = nd;
+        ba.threshold = p->threshold;
+        ba.keys = c->d_keys;   /* each image's own: see imgs */
+        ba.cap = HL_CIRCLE_MAXCAND;
+        CK(hl_launch_edge_bits(ba.imgs, &ba.img0, nimg, bblocks, s));
+        CK(hl_launch_circle_bits(&ba, bctas, twu_min, s));
+    }
+    if (nr > nd) {
+        CK(cudaMemsetAsync(c->d_state, 0, sizeof(unsigned long long) * (size_t)(groups + 1), s));
+        hl_compact_args ca;
+        memset(&ca, 0, sizeof(ca));
+        ca.imgs = reinterpret_cast<const hl_compact_img *>(dt + off_cimg);
+        ca.group_img = reinterpret_cast<const int *>(dt + off_gimg);
+        ca.nimg = nimg;
+        ca.ngroups = (int)groups;
+        ca.tile_state = c->d_state;
+        ca.ticket = reinterpret_cast<unsigned *>(c->d_cnt + 0);
+        ca.ticket_base = 0;
+        ca.epoch = 1;
+        ca.pts = nullptr;
+        ca.pts_f2 = c->d_pts;
+        ca.tile_off = c->d_toff;
+        ca.count = c->d_cnt + 1;
+        ca.status = c->d_cnt + 2;
+        CK(hl_launch_compact(&ca, s));
+        hl_circle_tile_args ta;
+        memset(&ta, 0, sizeof(ta));
+        ta.imgs = reinterpret_cast<const hl_circle_img *>(dt + off_circ);
+        ta.nimg = nimg;
+        ta.nctas = (int)ctas;
+        ta.rmin = p->radius_min;
+        ta.nr = nr;
+        ta.nz = nr - nd;
+        ta.acc = nullptr;
+        ta.threshold = p->threshold;
+        ta.cap = HL_CIRCLE_MAXCAND;
+        CK(hl_launch_circle_tiles(&ta, s));
+    }
     hl_circle_final_args fa;
     memset(&fa, 0, sizeof(fa));
     fa.imgs = reinterpret_cast<const hl_circle_img *>(dt + off_circ);

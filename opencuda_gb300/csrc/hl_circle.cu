@@ -1,9 +1,10 @@
 /*
  * hl_circle.cu -- HoughCircle on the HoughLine engine (the image path of
- * HoughCircle::houghcircle, okano_3_0/HoughCircle.cu:927-1165): the edge
- * pixels come from the same compaction, votes are counted in (radius, row,
- * column) accumulator tiles in shared memory, the local maxima taken in the
- * same pass, then a one-CTA tail.
+ * HoughCircle::houghcircle, okano_3_0/HoughCircle.cu:927-1165) for radii past
+ * HL_CIRCLE_DENSE_R, and the tail of all radii: the edge pixels come from the
+ * same compaction, votes are counted in (radius, row, column) accumulator tiles
+ * in shared memory, the local maxima taken in the same pass, then a one-CTA
+ * tail.
  *
  *   hl_circle_tile_kernel -- one CTA per (accumulator tile, radius), largest
  *       radius first.  The CTA counts its tile and a one-cell apron: every
@@ -520,7 +521,7 @@ cudaError_t hl_launch_circle_tiles(const hl_circle_tile_args *a, cudaStream_t s)
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess)
         return e;
-    const long long grid = a->imgs ? (long long)a->nctas : (long long)a->ntx * a->nty * a->nr;
+    const long long grid = a->imgs ? (long long)a->nctas : (long long)a->ntx * a->nty * a->nz;
     if (grid <= 0 || grid > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
     return hl_launch_pdl(hl_circle_tile_kernel, dim3((unsigned)grid), dim3(CT_THREADS), smem, s,

@@ -14,6 +14,7 @@
 #include <algorithm>
 
 #include "hl_internal.h"
+#include "hl_device.cuh"
 
 #define FULL 0xffffffffu
 
@@ -40,25 +41,6 @@ cudaError_t hl_launch_trig(float *cosv, float *sinv, int T, int Tp,
 {
     hl_trig_kernel<<<(Tp + 127) / 128, 128, 0, s>>>(cosv, sinv, T, Tp, detheta);
     return cudaGetLastError();
-}
-
-/* 0x80 in the bytes of w equal to 0xFF, by exact SWAR arithmetic: a byte of ~w
- * is zero exactly when the byte of w is 0xFF; (b & 0x7F) + 0x7F sets the high
- * bit of every nonzero low part with no carry between bytes, OR b keeps the
- * rest. */
-__device__ __forceinline__ uint32_t ff_flags(uint32_t w)
-{
-    const uint32_t t = ~w;
-    return ~(((t & 0x7f7f7f7fu) + 0x7f7f7f7fu) | t) & 0x80808080u;
-}
-
-/* 16-bit mask of the bytes of v equal to 0xFF (bit i = byte i): the flags times
- * the bits' weights, summed by byte dot products (128 times the mask) */
-__device__ __forceinline__ uint32_t ff_mask16(const uint4 &v)
-{
-    const uint32_t lo = __dp4a(ff_flags(v.y), 0x80402010u, __dp4a(ff_flags(v.x), 0x08040201u, 0u));
-    const uint32_t hi = __dp4a(ff_flags(v.w), 0x80402010u, __dp4a(ff_flags(v.z), 0x08040201u, 0u));
-    return (lo >> 7) + (hi << 1);
 }
 
 /* Look-back state word: epoch (30 bits) | flag (2 bits) | value (32 bits).
