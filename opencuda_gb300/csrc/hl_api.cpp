@@ -416,8 +416,9 @@ extern "C" int hl_last_launch_count(const hl_handle *h)
 struct vote_plan {
     std::vector<hl_vote_item> items;
     std::vector<hl_merge_block> blocks;
-    std::vector<int2> slabs;
-    long long scratch_units;   /* 64 bytes each */
+    std::vector<hl_slab> slabs;
+    long long scratch_units;   /* row groups of slabs */
+    unsigned chunks;           /* of a merge launch */
     int part16, win_rows, exact;
     /* the blocks' items add to the accumulator instead of going through slabs:
      * where a tile needs several windows (rho steps below 0.1 pixels) or the
@@ -428,10 +429,14 @@ struct vote_plan {
     int add;
 };
 #define HL_MAX_SCRATCH (1LL << 30)
+static size_t plan_scratch(const vote_plan &p)
+{
+    return (size_t)std::max(p.scratch_units, 1LL) * (p.part16 ? 64 : 128);
+}
 static void plan_free(vote_plan *p) { delete p; }
 
 struct plan_img {
-    int w, h, R;
+    int w, h, R, rho_min;
 };
 
 /* max|cos| and max|sin| of a slice's thetas times irho, with a little slack
@@ -543,6 +548,47 @@ static bool slide_item(const hl_handle *h, const slice_ext &e, int w, int hh, in
     return it->nseg > 1;
 }
 
+/* The rows that the votes of an item's four column groups can fall into, in
+ * groups of four rows (sl's b, n, lo and hi).  A corner's rho is a sinusoid over
+ * the group's thetas: no lower than at its ends less the distance times 1 -
+ * cos(half the span), and as much higher; a row and 2^-20 of the value more for
+ * the vote rule's floats. */
+static void slab_groups(const hl_handle *h, const plan_img &im, const hl_vote_item &it, int x1,
+                        int y1, hl_slab *sl)
+{
+    const double irho = 1.0 / h->p.derho;
+    const int R4 = (im.R + 3) / 4;
+    const double xs[2] = {(double)((it.tx & 0xffff) * HL_TILE_W), x1 - 1.0};
+    const double ys[2] = {(double)((it.ty & 0xffff) * HL_TILE_H), y1 - 1.0};
+    const double far = sqrt(xs[1] * xs[1] + ys[1] * ys[1]) * irho;
+    sl->lo = 0x7fffffff;
+    sl->hi = 0;
+    for (int g = 0; g < 4; g++) {
+        /* columns past the last theta vote like it, and are cleared alike */
+        const int k0 = std::min(it.slice * HL_SLICE + 8 * g, h->T - 1);
+        const int k1 = std::min(it.slice * HL_SLICE + 8 * g + 7, h->T - 1);
+        double lo = 1e300, hi = -1e300;
+        for (int e = 0; e < 8; e++) {
+            const int k = e & 4 ? k1 : k0;
+            const double v = (xs[e & 1] * (double)h->h_cos[k] +
+                              ys[(e >> 1) & 1] * (double)h->h_sin[k]) * irho;
+            lo = std::min(lo, v);
+            hi = std::max(hi, v);
+        }
+        const double half = std::min(0.5 * (k1 - k0) * h->p.detheta, M_PI);
+        const double slack = far * (1.0 - cos(half)) + far * (1.0 / (1 << 20)) + 1.0;
+        const double r0 = floor(lo - slack) - im.rho_min, r1 = ceil(hi + slack) - im.rho_min;
+        const int b = (int)std::min(std::max(floor(r0 / 4.0), 0.0), (double)R4);
+        const int e = (int)std::min(std::max(floor(r1 / 4.0) + 1.0, (double)b), (double)R4);
+        sl->b[g] = b;
+        sl->n[g] = e - b;
+        if (e > b) {
+            sl->lo = std::min(sl->lo, b);
+            sl->hi = std::max(sl->hi, e);
+        }
+    }
+}
+
 /* Plans the vote of n images with windows of at most cap rows on ctas
  * persistent CTAs. */
 static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int ctas,
@@ -557,6 +603,12 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
             total += (double)im[i].w * im[i].h +
                      HL_ROW_PIXELS * std::min(region_rows(ext[sl], im[i].w, im[i].h), 4.0 * cap);
     const double wcap = std::max(total / (HL_PLAN_SHARE * std::max(ctas, 1)), HL_MIN_REGION);
+    /* A block heavier than that is one item all the same, one such a CTA, if it is
+     * no more than a CTA's share: the rest, split, fill what is left.  A whole block
+     * needs no slabs: 21 images of 2048 x 2048, T = 360, voted 271 and merged 18 us
+     * instead of 278 and 50 with every block in two or more regions. */
+    const double share = total / std::max(ctas, 1);
+    int big = 0;
     std::vector<plan_region> reg;
     bool slides = false;
     pl->exact = pl->add = 0;
@@ -567,8 +619,15 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
         if (im[i].R >= (1 << 22))
             pl->exact = 1;
         for (int sl = 0; sl < slices; sl++) {
-            const double n_min = std::max(1.0, ceil((double)w * hh / wcap));
+            double n_min = std::max(1.0, ceil((double)w * hh / wcap));
             hl_vote_item whole;
+            if (n_min > 1.0 && big < ctas &&
+                (double)w * hh + HL_ROW_PIXELS * region_rows(ext[sl], w, hh) <= share &&
+                (region_rows(ext[sl], w, hh) <= cap ||
+                 slide_item(h, ext[sl], w, hh, sl, cap, &whole))) {
+                n_min = 1.0;
+                big++;
+            }
             if (n_min <= 1.0 && slide_item(h, ext[sl], w, hh, sl, cap, &whole)) {
                 whole.img = i;
                 plan_region r;
@@ -659,6 +718,7 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
     std::stable_sort(reg.begin(), reg.end(), heavier);
     /* slabs and merge blocks of the blocks with several items */
     std::vector<int> count((size_t)n * slices, 0), first((size_t)n * slices, 0);
+    std::vector<int> at((size_t)n * slices, -1);   /* in pl->blocks */
     for (const plan_region &r : reg)
         count[(size_t)r.blk]++;
     pl->blocks.clear();
@@ -666,10 +726,11 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
     for (int b = 0; b < n * slices; b++)
         if (count[(size_t)b] > 1) {
             first[(size_t)b] = nslab;
-            pl->blocks.push_back({b / slices, b % slices, nslab, count[(size_t)b]});
+            at[(size_t)b] = (int)pl->blocks.size();
+            pl->blocks.push_back({b / slices, b % slices, nslab, count[(size_t)b], 0x7fffffff, 0});
             nslab += count[(size_t)b];
         }
-    pl->slabs.assign((size_t)nslab, make_int2(0, 0));
+    pl->slabs.assign((size_t)nslab, hl_slab{});
     for (const plan_region &r : reg) {
         const int w = im[r.it.img].w, hh = im[r.it.img].h;
         pl->part16 &= hl_part16_ok(h->p.derho, std::min((r.it.tx >> 16) * HL_TILE_W, w),
@@ -690,17 +751,24 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
         const size_t b = (size_t)reg[i].blk;
         it.slab = -1;
         if (count[b] > 1) {
-            /* a column group's rows: the region's, and what its far corner
-             * sweeps over 7 theta steps */
-            const double far = sqrt((double)x1 * x1 + (double)y1 * y1) * irho;
-            const double grp = std::min(rows, (double)cap) + far * 7.0 * h->p.detheta;
-            it.ncap = (int)(std::min(grp, (double)im[it.img].R) / 4.0) + HL_SLAB_SLACK / 4 + 1;
-            const long long units = hl_slab_units(it.ncap, pl->part16);
-            pl->add |= pl->scratch_units + units > HL_MAX_SCRATCH / 64;
+            hl_slab sl = {};
+            slab_groups(h, im[it.img], it, x1, y1, &sl);
+            long long units = 0;
+            for (int g = 0; g < 4; g++) {
+                sl.o[g] = (int)units;
+                units += sl.n[g];
+                it.gb[g] = sl.b[g];
+                it.gn[g] = sl.n[g];
+                it.go[g] = sl.o[g];
+            }
+            pl->add |= pl->scratch_units + units > HL_MAX_SCRATCH / (pl->part16 ? 64 : 128);
             if (!pl->add) {
-                it.slab = (int)pl->scratch_units;
+                it.slab = sl.at = (int)pl->scratch_units;
                 pl->scratch_units += units;
-                pl->slabs[(size_t)first[b]++] = make_int2(it.slab, it.ncap);
+                hl_merge_block &mb = pl->blocks[(size_t)at[b]];
+                mb.lo = std::min(mb.lo, sl.lo);
+                mb.hi = std::max(mb.hi, sl.hi);
+                pl->slabs[(size_t)first[b]++] = sl;
             }
         }
         pl->items[i] = it;
@@ -712,6 +780,9 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
         pl->slabs.clear();
         pl->scratch_units = 0;
     }
+    pl->chunks = 1;
+    for (const hl_merge_block &mb : pl->blocks)
+        pl->chunks = std::max(pl->chunks, (unsigned)(mb.hi - mb.lo + 15) / 16);
     pl->win_rows = slides ? cap : std::min(cap, ((int)most + 7) / 8 * 8);
     return HL_NO_ERROR;
 }
@@ -742,27 +813,34 @@ static int vote_ctas(const hl_handle *h, int rows, int threads)
 static size_t plan_bytes(const vote_plan &p)
 {
     return p.items.size() * sizeof(hl_vote_item) + p.blocks.size() * sizeof(hl_merge_block) +
-           p.slabs.size() * sizeof(int2);
+           p.slabs.size() * sizeof(hl_slab);
 }
+/* slabs (read in 16-byte pieces), items, blocks */
 static void plan_copy(const vote_plan &p, unsigned char *dst)
 {
-    size_t o = p.items.size() * sizeof(hl_vote_item);
-    memcpy(dst, p.items.data(), o);
-    memcpy(dst + o, p.blocks.data(), p.blocks.size() * sizeof(hl_merge_block));
-    o += p.blocks.size() * sizeof(hl_merge_block);
-    memcpy(dst + o, p.slabs.data(), p.slabs.size() * sizeof(int2));
+    size_t o = 0;
+    const auto put = [&](const void *src, size_t n) {
+        if (n)
+            memcpy(dst + o, src, n);
+        o += n;
+    };
+    put(p.slabs.data(), p.slabs.size() * sizeof(hl_slab));
+    put(p.items.data(), p.items.size() * sizeof(hl_vote_item));
+    put(p.blocks.data(), p.blocks.size() * sizeof(hl_merge_block));
 }
 static void plan_args(const vote_plan &p, const unsigned char *d_plan, unsigned char *scratch,
                       hl_vote_args *va, hl_merge_args *ma)
 {
-    va->items = reinterpret_cast<const hl_vote_item *>(d_plan);
+    size_t o = p.slabs.size() * sizeof(hl_slab);
+    ma->slabs = reinterpret_cast<const hl_slab *>(d_plan);
+    va->items = reinterpret_cast<const hl_vote_item *>(d_plan + o);
     va->nitems = (int)p.items.size();
     va->win_rows = p.win_rows;
     va->exact = p.exact;
     va->part16 = p.part16;
     va->add = p.add;
     va->scratch = scratch;
-    size_t o = p.items.size() * sizeof(hl_vote_item);
+    o += p.items.size() * sizeof(hl_vote_item);
     ma->imgs = va->imgs;
     ma->img0 = va->img0;
     ma->T = va->T;
@@ -770,13 +848,12 @@ static void plan_args(const vote_plan &p, const unsigned char *d_plan, unsigned 
     ma->scratch = scratch;
     ma->blocks = reinterpret_cast<const hl_merge_block *>(d_plan + o);
     ma->nblocks = (int)p.blocks.size();
-    ma->slabs =
-        reinterpret_cast<const int2 *>(d_plan + o + p.blocks.size() * sizeof(hl_merge_block));
+    ma->chunks = p.chunks;
     ma->part16 = p.part16;
     ma->cand = va->cand;
 }
 
-static int handle_plan(hl_handle *h, int w, int hh, int R)
+static int handle_plan(hl_handle *h, int w, int hh, int R, int rho_min)
 {
     const int cap = plan_cap(h), threads = vote_threads(h);
     if (!(h->plan && h->plan_w == w && h->plan_h == hh && h->plan_R == R && h->plan_T == h->T &&
@@ -787,7 +864,7 @@ static int handle_plan(hl_handle *h, int w, int hh, int R)
         h->plan_w = 0;   /* not valid until the upload below */
         if (h->acc_state == ACC_UNREACHED)
             h->acc_state = ACC_ANY;
-        const plan_img im = {w, hh, R};
+        const plan_img im = {w, hh, R, rho_min};
         int rc = make_plan(h, &im, 1, cap, std::max(h->sms, 1), h->plan);
         if (rc != HL_NO_ERROR)
             return rc;
@@ -806,7 +883,7 @@ static int handle_plan(hl_handle *h, int w, int hh, int R)
         h->plan_thr = threads;
     }
     int rc = grow((void **)&h->d_scratch, &h->cap_scratch,
-                  (size_t)std::max(h->plan->scratch_units, 1LL) * 64);
+                  plan_scratch(*h->plan));
     if (rc != HL_NO_ERROR)
         return rc;
     return grow((void **)&h->d_cand, &h->cap_cand,
@@ -975,7 +1052,7 @@ static int run_ab(hl_handle *h, const hl_roi &roi, const hl_geom &g, bool peaks,
     va.Tp = h->Tp;
     va.irho = (float)(1.0 / h->p.derho);   /* okano_3_0/HoughLine.cu:107 */
     va.status = h->d_counters + 1;
-    int rc = handle_plan(h, roi.w, roi.h, g.numrho);
+    int rc = handle_plan(h, roi.w, roi.h, g.numrho, g.rho_min);
     if (rc != HL_NO_ERROR)
         return rc;
     /* bins above the threshold are noted where their final count is known;
@@ -1013,7 +1090,7 @@ static int run_ab(hl_handle *h, const hl_roi &roi, const hl_geom &g, bool peaks,
     h->work_base += (unsigned)(va.nitems + grid);
     (*launches)++;
     if (ma.nblocks > 0) {
-        CK(hl_launch_merge(&ma, g.numrho, s));
+        CK(hl_launch_merge(&ma, s));
         (*launches)++;
     }
     prof_mark(h, 2, s);
@@ -1632,7 +1709,7 @@ struct hl_batch_ws {
     std::vector<int> key;
     size_t tab_bytes;
     size_t off_cimg, off_gimg, off_vimg, off_plan, off_pimg, off_chunks, off_fimg;
-    int ngroups, ntiles, nchunks, grid, threads, maxR;
+    int ngroups, ntiles, nchunks, grid, threads;
     size_t npts_cap, acc_ints, nkeys;
     std::vector<size_t> acc_off, key_off;
     std::vector<size_t> pts_base;  /* each image's first point */
@@ -1708,13 +1785,11 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
                       int nimg, const int *thr, int K, hl_line *lines_dev,
                       int *counts_dev, const hl_roi *rois)
 {
-    int maxR = 1;
     std::vector<hl_geom> gs((size_t)nimg);
     for (int i = 0; i < nimg; i++) {
         int rc = hl_geometry(h, rois[i].w, rois[i].h, &gs[i]);
         if (rc != HL_NO_ERROR)
             return rc;
-        maxR = std::max(maxR, gs[i].numrho);
     }
     /* launch shape: the override (autotuner) or the largest window that
      * fits, 1024 threads */
@@ -1739,7 +1814,6 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
     if (key != b->key) {
         b->key.clear();   /* not valid until the plan below is whole */
         b->threads = threads;
-        b->maxR = maxR;
         b->acc_off.assign(nimg, 0);
         b->key_off.assign(nimg, 0);
         b->key_cap_i.assign(nimg, 0);
@@ -1779,7 +1853,7 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
             b->rho_min[i] = g.rho_min;
             b->R[i] = g.numrho;
             b->ref_numrho[i] = g.ref_numrho;
-            pim[i] = {rois[i].w, rois[i].h, g.numrho};
+            pim[i] = {rois[i].w, rois[i].h, g.numrho, g.rho_min};
             for (int r0 = 0; r0 < g.numrho; r0 += HL_PEAK_ROWS)
                 b->chunks.push_back(make_int2(i, r0));
         }
@@ -1823,7 +1897,7 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
                    sizeof(unsigned long long) * b->nkeys)) != HL_NO_ERROR ||
         (rc = grow((void **)&b->d_tab, &b->cap_tab, b->tab_bytes)) != HL_NO_ERROR ||
         (rc = grow((void **)&b->d_scratch, &b->cap_scratch,
-                   (size_t)std::max(b->plan.scratch_units, 1LL) * 64)) != HL_NO_ERROR)
+                   plan_scratch(b->plan))) != HL_NO_ERROR)
         return rc;
     if (b->cap_ncand < sizeof(int) * (size_t)nimg || !b->d_ncand) {
         if ((rc = grow((void **)&b->d_ncand, &b->cap_ncand, sizeof(int) * (size_t)nimg)) !=
@@ -1945,7 +2019,7 @@ static int batch_enqueue_vote_peaks(hl_handle *h, hl_batch_ws *b, cudaStream_t s
         CK(cudaMemsetAsync(b->d_acc, 0, sizeof(int32_t) * b->acc_ints, s));
     CK(hl_launch_vote(&va, b->threads, b->grid, s));
     if (ma.nblocks > 0)
-        CK(hl_launch_merge(&ma, b->maxR, s));
+        CK(hl_launch_merge(&ma, s));
     prof_mark(h, 2, s);
 
     hl_peak_args pa;

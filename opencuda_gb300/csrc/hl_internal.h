@@ -101,9 +101,9 @@ typedef struct hl_vote_img {
 typedef struct hl_vote_item {
     int img, slice;
     int tx, ty;               /* first tile | tiles << 16 */
-    int slab;                 /* scratch slab, 64-byte units; -1: the block's
-                                 only item (or hl_vote_args.add) */
-    int ncap;                 /* the slab's row groups per column group */
+    int slab;                 /* its slab's first row group in scratch; -1: the
+                                 block's only item (or hl_vote_args.add) */
+    int gb[4], gn[4], go[4];  /* the slab's column groups: see hl_slab */
     int win, clip;
     /* nseg > 1: a whole image whose range does not fit one window, voted in
      * nseg segments with the window sliding by adv rows after each: segment j
@@ -116,20 +116,15 @@ typedef struct hl_vote_item {
 
 /* A slab of scratch: the counts of an item as its block's merge reads them.
  * Four groups of 8 columns; group g holds the accumulator rows [4 b[g],
- * 4 (b[g] + n[g])) in row groups of four, [row group][column][4 rows], 16-bit
- * counts (64 bytes a row group) or 32-bit ones (128).  The header comes
- * first, 64 bytes. */
-typedef struct hl_slab_hdr {
-    int b[4], n[4];
-    int pad[8];
-} hl_slab_hdr;
-static inline long long hl_slab_units(int ncap, int part16)
-{
-    return 1 + 4LL * ncap * (part16 ? 1 : 2);
-}
-/* rows and angles of slack a slab's capacity needs past its rows: a group's
- * base is rounded down to four rows */
-#define HL_SLAB_SLACK 8
+ * 4 (b[g] + n[g])), which every vote of the group falls into, in row groups of
+ * four, [row group][column][4 rows], 16-bit counts (64 bytes a row group) or
+ * 32-bit ones (128), from row group o[g] of the slab on. */
+typedef struct hl_slab {
+    int at;                   /* its first row group in scratch */
+    int lo, hi;               /* row groups that some column group holds */
+    int pad;
+    int b[4], n[4], o[4];
+} hl_slab;
 
 /* Peak candidates of a launch: every accumulator bin above its image's
  * threshold, noted as image << 32 | (row * T + theta) when its final count
@@ -161,7 +156,7 @@ typedef struct hl_vote_args {
     int nitems;
     unsigned *work;           /* counter */
     unsigned work_base;       /* its value at launch */
-    unsigned char *scratch;   /* slabs, 64-byte units */
+    unsigned char *scratch;   /* slabs: row groups */
     int part16;               /* slabs hold 16-bit counts (hl_part16_ok) */
     int add;                  /* no slabs: items add to the cleared accumulator */
     hl_cand_list cand;
@@ -172,6 +167,7 @@ typedef struct hl_vote_args {
 typedef struct hl_merge_block {
     int img, slice;
     int first, n;
+    int lo, hi;               /* row groups that some slab holds */
 } hl_merge_block;
 
 typedef struct hl_merge_args {
@@ -181,8 +177,8 @@ typedef struct hl_merge_args {
     const unsigned char *scratch;
     const hl_merge_block *blocks;
     int nblocks;
-    unsigned chunks;          /* CTAs a block (set by the launcher) */
-    const int2 *slabs;        /* {slab, ncap} */
+    unsigned chunks;          /* CTAs a block: 16 row groups each */
+    const hl_slab *slabs;
     int part16;
     hl_cand_list cand;
 } hl_merge_args;
@@ -437,7 +433,7 @@ cudaError_t hl_launch_compact(const hl_compact_args *a, cudaStream_t s);
  * one to the ticket word */
 int hl_compact_persist_ctas(int ntiles, int sms);
 cudaError_t hl_launch_compact_persist(const hl_compact_args *a, int nct, cudaStream_t s);
-cudaError_t hl_launch_merge(hl_merge_args *a, int max_R, cudaStream_t s);
+cudaError_t hl_launch_merge(const hl_merge_args *a, cudaStream_t s);
 cudaError_t hl_launch_vote(const hl_vote_args *a, int threads, int grid,
                            cudaStream_t s);
 size_t hl_vote_smem_bytes(int win_rows);

@@ -147,13 +147,13 @@ struct VoteSeg {
     int mode;                          /* CV_* (CV_EXACT: every row tested) */
     int total;                         /* points of its stream */
     int rho_min, R, thr;               /* the image's */
-    int slab, ncap;                    /* see hl_vote_item */
+    int slab;                          /* see hl_vote_item */
     int last, adv;                     /* the item's last segment; rows to slide */
     int rows;                          /* rows its votes can reach */
     float margin;                      /* one rho bin in pixels */
     float c[HL_SLICE], s[HL_SLICE];    /* cos / sin of the slice's thetas */
     int base[HL_SLICE];                /* rho of each column's row 0 */
-    int gb[4], gn[4];                  /* the slab's header */
+    int gb[4], gn[4], go[4];           /* the slab's column groups */
 };
 
 /* The lane's tables of an item: cos / sin of its columns as f2x pairs of
@@ -320,15 +320,6 @@ __device__ __forceinline__ bool cons_sync(VoteSmem &sm, unsigned &par,
     return ok;
 }
 
-/* minimum / maximum over the 8 lanes of a column group */
-__device__ __forceinline__ int group_min(int v)
-{
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1)
-        v = min(v, __shfl_xor_sync(FULL, v, o));
-    return v;
-}
-
 /* Producer warp: takes items, publishes each as a segment and streams its
  * points into the ring.  It runs ahead of the consumers by up to the ring's
  * depth, so the next item's setup and first copies overlap the current item's
@@ -391,15 +382,6 @@ __device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &s
                                   ? CV_FLOOR
                                   : (!__any_sync(FULL, hi > 0.0f) ? CV_CEIL : CV_SIGN));
         const bool mixed = mode == CV_SIGN;
-        /* the slab's column groups: rows of the columns that reach the window */
-        const bool in = top >= base;
-        const int glo = group_min(in ? base - im.rho_min : 0x7fffffff) >> 2;
-        const int ghi = -group_min(in ? -(top - im.rho_min) : 0x7fffffff);
-        int gn = glo < 0x1fffffff ? (ghi >> 2) - glo + 1 : 0;
-        if (have && it.slab >= 0 && gn > it.ncap) {
-            atomicOr(a.status, HL_ST_RHO_OUT_OF_RANGE);
-            gn = it.ncap;
-        }
         /* sliding: the middle theta's normal in rho units a tile */
         const int km = min(it.slice * HL_SLICE + HL_SLICE / 2, a.T - 1);
         const float sm_ = slide ? a.sinv[km] * a.irho : 0.0f;
@@ -483,10 +465,6 @@ __device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &s
         g.c[lane] = cl;
         g.s[lane] = sl;
         g.base[lane] = base;
-        if ((lane & 7) == 0) {
-            g.gb[lane >> 3] = glo;
-            g.gn[lane >> 3] = gn;
-        }
         if (lane == 0) {
             g.acc = im.acc;
             g.item = have ? (int)t : -1;
@@ -499,7 +477,12 @@ __device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &s
             g.R = im.R;
             g.thr = im.threshold;
             g.slab = it.slab;
-            g.ncap = it.ncap;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                g.gb[q] = it.gb[q];
+                g.gn[q] = it.gn[q];
+                g.go[q] = it.go[q];
+            }
             g.last = sj == nsegs - 1;
             g.adv = it.adv;
             g.rows = rows;
@@ -721,15 +704,10 @@ hl_vote_kernel(hl_vote_args a)
                 }
             }
         } else {
-            unsigned char *slab = a.scratch + (size_t)g.slab * 64u;
             const int grp = lane >> 3, cc = lane & 7;
-            if (cw == 0 && cc == 0) {
-                reinterpret_cast<hl_slab_hdr *>(slab)->b[grp] = g.gb[grp];
-                reinterpret_cast<hl_slab_hdr *>(slab)->n[grp] = g.gn[grp];
-            }
             const int gb = g.gb[grp], gn = g.gn[grp];
             const int most = max(max(g.gn[0], g.gn[1]), max(g.gn[2], g.gn[3]));
-            const size_t at = (size_t)grp * g.ncap * 8 + cc;
+            const size_t at = ((size_t)g.slab + g.go[grp]) * 8 + cc;
             for (int q = cw; q < most; q += ncons) {
                 int v[4];
 #pragma unroll
@@ -743,11 +721,11 @@ hl_vote_kernel(hl_vote_args a)
                 }
                 if (q < gn) {
                     if (a.part16)
-                        reinterpret_cast<uint2 *>(slab + 64)[at + (size_t)q * 8] =
+                        reinterpret_cast<uint2 *>(a.scratch)[at + (size_t)q * 8] =
                             make_uint2((unsigned)v[0] | ((unsigned)v[1] << 16),
                                        (unsigned)v[2] | ((unsigned)v[3] << 16));
                     else
-                        reinterpret_cast<int4 *>(slab + 64)[at + (size_t)q * 8] =
+                        reinterpret_cast<int4 *>(a.scratch)[at + (size_t)q * 8] =
                             make_int4(v[0], v[1], v[2], v[3]);
                 }
             }
@@ -764,48 +742,46 @@ hl_vote_kernel(hl_vote_args a)
  * as peak candidates, or every bin is stored (padding columns, thetas >= T,
  * zero).  A thread takes four rows of two columns: one
  * 16-byte load of every slab whose rows overlap (two with 32-bit counts), from
- * L2 where the vote launch just wrote them, eight in flight. */
+ * L2 where the vote launch just wrote them, eight in flight.  Bound by latency:
+ * a block's slab list, then the slabs; where the slabs lie is the plan's, so no
+ * header is read between.  4096 x 4096, T = 720: 18 us (23 us with headers that
+ * the vote wrote, and CTAs for rows that no slab holds); 1913 x 1077, T = 360:
+ * 8 us (13 us). */
 #define MERGE_HDRS 64
 template <bool P16>
 __global__ void __launch_bounds__(256)
 hl_merge_kernel(hl_merge_args a)
 {
-    __shared__ int4 s_b[MERGE_HDRS], s_n[MERGE_HDRS];
-    __shared__ const unsigned char *s_p[MERGE_HDRS];
-    __shared__ int s_cap[MERGE_HDRS];
+    __shared__ int4 s_b[MERGE_HDRS], s_n[MERGE_HDRS], s_o[MERGE_HDRS];   /* o: in scratch */
     __shared__ int s_hits;
     const int tid = threadIdx.x;
     hl_pdl_begin();
     const unsigned bi = blockIdx.x / a.chunks, chunk = blockIdx.x - bi * a.chunks;
     const hl_merge_block blk = a.blocks[bi];
+    const int c0 = blk.lo + (int)chunk * 16;       /* the CTA's first row group */
+    if (c0 >= blk.hi)
+        return;
     const hl_vote_img &im = a.imgs ? a.imgs[blk.img] : a.img0;
     const int R = im.R;
-    const int c0 = (int)chunk * 16;                /* the CTA's first row group */
-    if (4 * c0 >= R)
-        return;
     const int rg = c0 + (tid >> 4);                /* the thread's */
     const int g = (tid >> 2) & 3, cp = tid & 3;
     int v[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
     int hits = 0;
     for (int j0 = 0; j0 < blk.n; j0 += MERGE_HDRS) {
         /* the slabs that reach the CTA's rows */
-        __syncthreads();
+        if (j0)
+            __syncthreads();
         if (tid == 0)
             s_hits = 0;
         __syncthreads();
         if (tid < MERGE_HDRS && j0 + tid < blk.n) {
-            const int2 sl = a.slabs[blk.first + j0 + tid];
-            const unsigned char *p = a.scratch + (size_t)sl.x * 64u;
-            const int4 hb = __ldcg(reinterpret_cast<const int4 *>(p));
-            const int4 hn = __ldcg(reinterpret_cast<const int4 *>(p) + 1);
-            const int lo = min(min(hb.x, hb.y), min(hb.z, hb.w));
-            const int hi = max(max(hb.x + hn.x, hb.y + hn.y), max(hb.z + hn.z, hb.w + hn.w));
-            if (lo < c0 + 16 && hi > c0) {
+            const int4 *sl = reinterpret_cast<const int4 *>(a.slabs + blk.first + j0 + tid);
+            const int4 h = sl[0], b = sl[1], n = sl[2], o = sl[3];
+            if (h.y < c0 + 16 && h.z > c0) {
                 const int at = atomicAdd(&s_hits, 1);
-                s_b[at] = hb;
-                s_n[at] = hn;
-                s_p[at] = p + 64;
-                s_cap[at] = sl.y;
+                s_b[at] = b;
+                s_n[at] = n;
+                s_o[at] = make_int4(h.x + o.x, h.x + o.y, h.x + o.z, h.x + o.w);
             }
         }
         __syncthreads();
@@ -821,13 +797,14 @@ hl_merge_kernel(hl_merge_args a)
                 const int rel = rg - reinterpret_cast<const int *>(&s_b[jj])[g];
                 const bool ok = j + u < nj &&
                                 (unsigned)rel < (unsigned)reinterpret_cast<const int *>(&s_n[jj])[g];
-                const size_t at = ((size_t)g * s_cap[jj] + rel) * 8 + 2 * cp;
+                const size_t at = ((size_t)reinterpret_cast<const int *>(&s_o[jj])[g] + rel) * 8 +
+                                  2 * cp;
                 if (P16) {
                     q[u] = ok ? __ldcg(reinterpret_cast<const uint4 *>(
-                                    reinterpret_cast<const uint2 *>(s_p[jj]) + at))
+                                    reinterpret_cast<const uint2 *>(a.scratch) + at))
                               : make_uint4(0u, 0u, 0u, 0u);
                 } else {
-                    const uint4 *p = reinterpret_cast<const uint4 *>(s_p[jj]) + at;
+                    const uint4 *p = reinterpret_cast<const uint4 *>(a.scratch) + at;
                     q[2 * u] = ok ? __ldcg(p) : make_uint4(0u, 0u, 0u, 0u);
                     q[2 * u + 1] = ok ? __ldcg(p + 1) : make_uint4(0u, 0u, 0u, 0u);
                 }
@@ -882,11 +859,10 @@ hl_merge_kernel(hl_merge_args a)
                 }
 }
 
-cudaError_t hl_launch_merge(hl_merge_args *a, int max_R, cudaStream_t s)
+cudaError_t hl_launch_merge(const hl_merge_args *a, cudaStream_t s)
 {
     if (a->nblocks <= 0)
         return cudaSuccess;
-    a->chunks = (unsigned)((max_R + 63) / 64);   /* 64 rows of a block a CTA */
     const unsigned long long grid = (unsigned long long)a->chunks * (unsigned)a->nblocks;
     if (grid > 0x7fffffffull)
         return cudaErrorInvalidConfiguration;

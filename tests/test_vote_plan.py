@@ -98,3 +98,18 @@ def test_batches_reuse_their_accumulators(hl_mod, det, derho):
             assert rc == 0
             for im, t, got in zip(imgs, thr, res):
                 assert [l.astuple() for l in got] == _want(hl, im, t, 16, det, derho), im.shape
+
+
+def test_blocks_whole_and_split_in_one_batch(hl_mod):
+    """More blocks than CTAs, each most of a CTA's share: some are voted whole,
+    the rest in regions that fill the gaps."""
+    HoughLine, Image = hl_mod
+    det = math.pi / 300
+    hl = HoughLine(detheta=det)
+    imgs = [_scene(640, 480, 100 + i) for i in range(20)]
+    dev = [Image.from_host(im) for im in imgs]
+    for thr in (300, 25):
+        rc, res = hl.houghLineBatch(dev, 16, [thr] * len(imgs))
+        assert rc == 0
+        for im, got in zip(imgs, res):
+            assert [l.astuple() for l in got] == _want(hl, im, thr, 16, det, 1.0)
