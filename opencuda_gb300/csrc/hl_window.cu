@@ -28,6 +28,10 @@
 #define FULL 0xffffffffu
 
 #define NCELL (HL_COARSE_T * HL_COARSE_R)
+#define SEL_THREADS 1024
+#define SEL_WARPS (SEL_THREADS / 32)
+#define SEL_STEPS 24
+#define SEL_VALS ((NCELL + SEL_THREADS - 1) / SEL_THREADS)
 
 /* Is coarse cell i a local maximum of the logits (3 x 3 neighbourhood, ties
  * to the earlier cell in raster order)? */
@@ -35,6 +39,12 @@ __device__ __forceinline__ bool local_max(const float *z, int i)
 {
     const int t = i / HL_COARSE_R, r = i % HL_COARSE_R;
     const float v = z[i];
+    if (t > 0 && t < HL_COARSE_T - 1 && r > 0 && r < HL_COARSE_R - 1) {
+        const float *a = z + i - HL_COARSE_R, *b = z + i + HL_COARSE_R;
+        const float before = fmaxf(fmaxf(a[-1], a[0]), fmaxf(a[1], z[i - 1]));
+        const float after = fmaxf(fmaxf(b[-1], b[0]), fmaxf(b[1], z[i + 1]));
+        return !(before >= v) && !(after > v);
+    }
     for (int dt = -1; dt <= 1; dt++) {
         const int tt = t + dt;
         if (tt < 0 || tt >= HL_COARSE_T)
@@ -52,51 +62,90 @@ __device__ __forceinline__ bool local_max(const float *z, int i)
     return true;
 }
 
-/* Value level with at least `target` of the n candidate values cv above it
- * (bisection on the value; the block's threads count in parallel).  Returns
- * -inf when there are at most `target` candidates. */
-__device__ float level_for(const float *cv, int n, int target, float *red, int *s_cnt)
+/* Value levels with at least target and target + 1 of the n candidate values cv
+ * above them (bisections on the value: the same steps until they part; the
+ * block's threads hold the values and count in parallel, one barrier a step).
+ * -inf when there are at most as many candidates. */
+__device__ __forceinline__ float2 levels_for(const float *cv, int n, int target, float *red,
+                                             int *s_cnt)
 {
-    if (n <= target)
-        return -3.0e38f;
-    float mn = 3.0e38f, mx = -3.0e38f;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        mn = fminf(mn, cv[i]);
-        mx = fmaxf(mx, cv[i]);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float v[SEL_VALS], mn = 3.0e38f, mx = -3.0e38f;
+#pragma unroll
+    for (int u = 0; u < SEL_VALS; u++) {
+        const int i = threadIdx.x + u * SEL_THREADS;
+        /* a value past the last is above no level */
+        v[u] = i < n ? cv[i] : __int_as_float(0x7fc00000);
+        mn = fminf(mn, v[u]);
+        mx = fmaxf(mx, v[u]);
     }
     for (int o = 16; o > 0; o >>= 1) {
         mn = fminf(mn, __shfl_xor_sync(FULL, mn, o));
         mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, o));
     }
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) {
-        red[threadIdx.x >> 5] = mn;
-        red[16 + (threadIdx.x >> 5)] = mx;
+    if (threadIdx.x < 2 * SEL_STEPS)
+        s_cnt[threadIdx.x] = 0;
+    if (lane == 0) {
+        red[warp] = mn;
+        red[SEL_WARPS + warp] = mx;
     }
     __syncthreads();
-    float lo = red[0], hi = red[16];
-    for (int w = 1; w < (int)(blockDim.x >> 5); w++) {
-        lo = fminf(lo, red[w]);
-        hi = fmaxf(hi, red[16 + w]);
+    float lo0 = red[lane], hi0 = red[SEL_WARPS + lane];
+    for (int o = 16; o > 0; o >>= 1) {
+        lo0 = fminf(lo0, __shfl_xor_sync(FULL, lo0, o));
+        hi0 = fmaxf(hi0, __shfl_xor_sync(FULL, hi0, o));
     }
-    lo -= 1.0f;   /* count(cv > lo) = n >= target */
-    for (int it = 0; it < 24; it++) {
-        const float mid = 0.5f * (lo + hi);
+    lo0 -= 1.0f;   /* count(cv > lo) = n */
+    float lo1 = lo0, hi1 = hi0;
+    /* the thread's values above the lower and the upper bounds */
+    int from0 = 0, above0 = 0;
+#pragma unroll
+    for (int u = 0; u < SEL_VALS; u++)
+        from0 += v[u] > lo0;
+    int from1 = from0, above1 = above0;
+    for (int it = 0; it < SEL_STEPS; it++) {
+        const float m0 = 0.5f * (lo0 + hi0), m1 = 0.5f * (lo1 + hi1);
+        /* a warp without values between its bounds counts as at the upper one */
+        int c0 = above0, c1 = above1;
+        if (__any_sync(FULL, from0 != above0)) {
+            c0 = 0;
+#pragma unroll
+            for (int u = 0; u < SEL_VALS; u++)
+                c0 += v[u] > m0;
+        }
+        if (m1 == m0) {
+            c1 = c0;
+        } else if (__any_sync(FULL, from1 != above1)) {
+            c1 = 0;
+#pragma unroll
+            for (int u = 0; u < SEL_VALS; u++)
+                c1 += v[u] > m1;
+        }
+        /* both counts of a warp in one word: at most 32 * SEL_VALS each */
+        int c = c0 | (c1 << 16);
+        for (int o = 16; o > 0; o >>= 1)
+            c += __shfl_xor_sync(FULL, c, o);
+        if (lane == 0 && c) {
+            atomicAdd(&s_cnt[2 * it], c & 0xffff);
+            atomicAdd(&s_cnt[2 * it + 1], c >> 16);
+        }
         __syncthreads();
-        if (threadIdx.x == 0)
-            *s_cnt = 0;
-        __syncthreads();
-        int c = 0;
-        for (int i = threadIdx.x; i < n; i += blockDim.x)
-            c += cv[i] > mid;
-        atomicAdd(s_cnt, c);
-        __syncthreads();
-        if (*s_cnt >= target)
-            lo = mid;
-        else
-            hi = mid;
+        if (s_cnt[2 * it] >= target) {
+            lo0 = m0;
+            from0 = c0;
+        } else {
+            hi0 = m0;
+            above0 = c0;
+        }
+        if (s_cnt[2 * it + 1] >= target + 1) {
+            lo1 = m1;
+            from1 = c1;
+        } else {
+            hi1 = m1;
+            above1 = c1;
+        }
     }
-    return lo;
+    return make_float2(n <= target ? -3.0e38f : lo0, n <= target + 1 ? -3.0e38f : lo1);
 }
 
 /* One CTA per image.  Candidates are the coarse cells (with nms: the local
@@ -105,89 +154,120 @@ __device__ float level_for(const float *cv, int n, int target, float *red, int *
  * The image falls back to the plain method when more than max_props
  * candidates clear the cutoff (a cluttered scene), or -- the confidence
  * test -- when the best candidate left out of the top_m is itself above
- * zconf: the network sees more likely lines than the budget covers. */
-__global__ void __launch_bounds__(512)
+ * zconf: the network sees more likely lines than the budget covers.
+ * A CTA an image, bound by its own instructions and barriers: 26 us for 32 images
+ * (49 us with two bisections, a shared atomic a thread and three barriers a step,
+ * and the windows marked and numbered cell by cell with atomics). */
+__global__ void __launch_bounds__(SEL_THREADS)
 hl_select_kernel(hl_select_args a)
 {
     extern __shared__ float zs[];          /* [NCELL] logits, [NCELL] candidate values */
     float *cv = zs + NCELL;
-    __shared__ unsigned mark[NCELL / 32];
-    __shared__ int cnt, ncand, s_cnt;
-    __shared__ float red[32];
-    const int b = blockIdx.x;
+    __shared__ unsigned sel[NCELL / 32];
+    __shared__ int cnt, ncand, s_cnt[2 * SEL_STEPS], nrun, ncell, first;
+    __shared__ float red[2 * SEL_WARPS];
+    const int b = blockIdx.x, lane = threadIdx.x & 31;
     const float *z = a.logits + (size_t)b * NCELL;
     for (int i = threadIdx.x; i < NCELL; i += blockDim.x)
         zs[i] = z[i];
-    for (int i = threadIdx.x; i < NCELL / 32; i += blockDim.x)
-        mark[i] = 0u;
     if (threadIdx.x == 0) {
         cnt = 0;
         ncand = 0;
+        nrun = ncell = 0;
     }
     __syncthreads();
     int mine = 0;
-    for (int i = threadIdx.x; i < NCELL; i += blockDim.x) {
-        if (a.nms && !local_max(zs, i))
-            continue;
-        cv[atomicAdd(&ncand, 1)] = zs[i];
-        mine += zs[i] > a.zcut;
+    for (int i0 = 0; i0 < NCELL; i0 += SEL_THREADS) {
+        const int i = i0 + threadIdx.x;
+        const bool is = i < NCELL && (!a.nms || local_max(zs, i));
+        const unsigned m = __ballot_sync(FULL, is);
+        int at = 0;
+        if (lane == 0 && m)
+            at = atomicAdd(&ncand, __popc(m));
+        at = __shfl_sync(FULL, at, 0) + __popc(m & ((1u << lane) - 1u));
+        if (is) {
+            cv[at] = zs[i];
+            mine += zs[i] > a.zcut;
+        }
     }
-    atomicAdd(&cnt, mine);
+    mine = __reduce_add_sync(FULL, mine);
+    if (lane == 0)
+        atomicAdd(&cnt, mine);
     __syncthreads();
     const int nc = ncand;
     int fb = (cnt > a.max_props || a.force_fallback) ? 1 : 0;
     float level = a.zcut;
     if (!fb && a.top_m > 0) {
-        level = fminf(level, level_for(cv, nc, a.top_m, red, &s_cnt));
-        if (a.use_conf && nc > a.top_m) {
-            /* the (top_m + 1)-th candidate lies above this level */
-            const float next = level_for(cv, nc, a.top_m + 1, red, &s_cnt);
-            if (next >= a.zconf)
-                fb = 2;
-        }
+        const float2 lv = levels_for(cv, nc, a.top_m, red, s_cnt);
+        level = fminf(level, lv.x);
+        /* the (top_m + 1)-th candidate lies above this level */
+        if (a.use_conf && nc > a.top_m && lv.y >= a.zconf)
+            fb = 2;
     }
     if (threadIdx.x == 0)
         a.fallback[b] = fb;
     if (fb)
         return;
-    for (int i = threadIdx.x; i < NCELL; i += blockDim.x) {
-        if (!(zs[i] > level) || (a.nms && !local_max(zs, i)))
-            continue;
-        const int t = i / HL_COARSE_R, r = i % HL_COARSE_R;
-        for (int dt = -a.dil_t; dt <= a.dil_t; dt++) {
-            const int tt = t + dt;
-            if (tt < 0 || tt >= HL_COARSE_T)
-                continue;
-            for (int dr = -a.dil_r; dr <= a.dil_r; dr++) {
-                const int rr = r + dr;
-                if (rr < 0 || rr >= HL_COARSE_R)
-                    continue;
-                const int c = tt * HL_COARSE_R + rr;
-                atomicOr(&mark[c >> 5], 1u << (c & 31));
+    /* the selected cells' mask (a word is 32 consecutive rho cells of one theta
+     * cell), then grown by the dilation, a thread a word */
+    for (int i0 = 0; i0 < NCELL; i0 += SEL_THREADS) {
+        const int i = i0 + threadIdx.x;
+        const bool is = i < NCELL && zs[i] > level && (!a.nms || local_max(zs, i));
+        const unsigned m = __ballot_sync(FULL, is);
+        if (lane == 0 && i < NCELL)
+            sel[i >> 5] = m;
+    }
+    __syncthreads();
+    static_assert(NCELL / 32 <= SEL_THREADS && HL_COARSE_R % 32 == 0, "a thread a mask word");
+    unsigned word = 0;
+    if (threadIdx.x < NCELL / 32) {
+        constexpr int RW = HL_COARSE_R / 32;
+        const int t = threadIdx.x / RW, w = threadIdx.x % RW;
+        for (int tt = max(t - a.dil_t, 0); tt <= min(t + a.dil_t, HL_COARSE_T - 1); tt++) {
+            const unsigned *row = sel + tt * RW;
+            for (int dr = -min(a.dil_r, HL_COARSE_R); dr <= min(a.dil_r, HL_COARSE_R); dr++) {
+                /* bits dr further along the row */
+                const int q = w + (dr >> 5);
+                const unsigned lo = q >= 0 && q < RW ? row[q] : 0u;
+                const unsigned hi = q + 1 >= 0 && q + 1 < RW ? row[q + 1] : 0u;
+                word |= __funnelshift_r(lo, hi, dr & 31);
             }
         }
     }
-    __syncthreads();
     /* one window per run of marked cells along rho at one theta (a mask
      * word holds 32 consecutive rho cells of one theta cell), at most
      * HL_WIN_RUN cells: the run's points are read once for all its cells */
-    for (int wd = threadIdx.x; wd < NCELL / 32; wd += blockDim.x) {
-        unsigned m = mark[wd];
-        if (m)
-            atomicAdd(a.ncells, __popc(m));
-        while (m) {
-            const int bit = __ffs(m) - 1;
-            const unsigned ones = ~(m >> bit);            /* the run ends at its first 0 */
-            const int len = min(ones ? __ffs(ones) - 1 : 32 - bit, HL_WIN_RUN);
-            m &= ~(((len == 32 ? 0u : (1u << len)) - 1u) << bit);
-            const int c = wd * 32 + bit;
-            const int q = atomicAdd(a.nwin, 1);
-            if (q < a.cap)
-                a.win[q] = make_int4(b, c / HL_COARSE_R, c % HL_COARSE_R,
-                                     c % HL_COARSE_R + len - 1);
-            else
-                atomicOr(a.status, HL_ST_CAND_OVERFLOW);
-        }
+    /* the windows' places: one global reservation a CTA */
+    int runs = 0;
+    for (unsigned m = word; m; runs++) {
+        const int bit = __ffs(m) - 1;
+        const unsigned ones = ~(m >> bit);            /* the run ends at its first 0 */
+        const int len = min(ones ? __ffs(ones) - 1 : 32 - bit, HL_WIN_RUN);
+        m &= ~(((len == 32 ? 0u : (1u << len)) - 1u) << bit);
+    }
+    int at = runs ? atomicAdd(&nrun, runs) : 0;
+    const int cells = __reduce_add_sync(FULL, __popc(word));
+    if (lane == 0 && cells)
+        atomicAdd(&ncell, cells);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        first = nrun ? atomicAdd(a.nwin, nrun) : 0;
+        if (ncell)
+            atomicAdd(a.ncells, ncell);
+    }
+    __syncthreads();
+    at += first;
+    for (unsigned m = word; m; at++) {
+        const int bit = __ffs(m) - 1;
+        const unsigned ones = ~(m >> bit);
+        const int len = min(ones ? __ffs(ones) - 1 : 32 - bit, HL_WIN_RUN);
+        m &= ~(((len == 32 ? 0u : (1u << len)) - 1u) << bit);
+        const int c = threadIdx.x * 32 + bit;
+        if (at < a.cap)
+            a.win[at] = make_int4(b, c / HL_COARSE_R, c % HL_COARSE_R,
+                                  c % HL_COARSE_R + len - 1);
+        else
+            atomicOr(a.status, HL_ST_CAND_OVERFLOW);
     }
 }
 
@@ -198,7 +278,7 @@ cudaError_t hl_launch_select(const hl_select_args *a, int nimg, cudaStream_t s)
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess)
         return e;
-    hl_select_kernel<<<nimg, 512, smem, s>>>(*a);
+    hl_select_kernel<<<nimg, SEL_THREADS, smem, s>>>(*a);
     return cudaGetLastError();
 }
 
