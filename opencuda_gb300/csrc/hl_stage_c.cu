@@ -35,7 +35,7 @@ namespace cg = cooperative_groups;
 
 #define FULL 0xffffffffu
 #define FIN_THREADS 1024
-#define FIN_CHUNK 1024
+#define FIN_CHUNK 1024         /* a key a thread */
 #define FIN_SCACHE 1024
 
 /* The peak rule (okano_3_0/HoughLine.cu:195-199, bounds-checked: zero
@@ -258,7 +258,8 @@ __device__ __forceinline__ void decode(unsigned long long key, int T,
 /* Predecessor bitmask of a sorted, decoded chunk of m candidates: bit j of
  * pred[i][j / 32] <=> j < i and similar(j, i).  Only the words holding some
  * j < i are built: entry (i, wd) for 32 wd < i, enumerated word by word.
- * Four adjacent threads share an entry (8 tests each, OR-ed by shuffles);
+ * Four adjacent threads share an entry (8 tests each, OR-ed by shuffles; a warp
+ * without entries leaves, so a few candidates cost a few warps' instructions);
  * the threads of a warp mostly share wd and read the word's candidates with
  * broadcast loads.  Of nsub CTAs (a cluster) CTA sub takes every nsub-th
  * entry, so the CTAs share the work evenly; pred may be another CTA's
@@ -276,6 +277,8 @@ __device__ __forceinline__ void build_pred(const FinSmem &sm, int m, const hl_fi
     /* a whole number of passes: every lane of a warp runs the same trips */
     const int span = (nent + estep - 1) / estep * estep;
     for (int en = (int)(threadIdx.x >> 2) * nsub + sub; en < span; en += estep) {
+        if (!__any_sync(FULL, en < nent))
+            break;   /* a warp without entries: most of them when candidates are few */
         unsigned bits = 0u;
         int i = 0, wd = 0, jn = 0;
         if (en < nent) {
@@ -287,32 +290,32 @@ __device__ __forceinline__ void build_pred(const FinSmem &sm, int m, const hl_fi
             i = 32 * wd + 1 + rem;
             jn = min(32, i - (wd << 5));
         }
-        {
-            /* every lane runs the same 8 tests (invalid ones masked
-             * afterwards), so the rare exact wrap-around test is a
-             * warp-uniform branch */
-            const int j0 = wd << 5;
-            const float ai = sm.ang[i];
-            const int di = sm.dist[i];
+        /* every lane runs the same 8 tests, all in flight at once (invalid ones
+         * masked); the rare pairs whose wrap-around test needs the exact form
+         * are settled afterwards */
+        const int j0 = (wd << 5) + 8 * q;
+        const float ai = sm.ang[i];
+        const int di = sm.dist[i];
+        unsigned amb = 0u;
 #pragma unroll
-            for (int b = 8 * q; b < 8 * q + 8; b++) {
-                const int j = min(j0 + b, m - 1);
-                const float aj = sm.ang[j];
-                const int dj = sm.dist[j];
-                const bool same = (abs(dj - di) < a.thresdis) &
-                                  (fabsf(__fsub_rn(aj, ai)) < a.thresang);
-                const bool near = abs(dj + di) < a.thresdis;
-                const float est = fabsf(__fsub_rn(__fsub_rn(3.14159265f, aj), ai));
-                const bool lo = est < a.thresang - 1e-6f;
-                const bool hi = est > a.thresang + 1e-6f;
-                bool wrap = near & lo;
-                const bool amb = near & !lo & !hi & (b < jn);
-                if (__any_sync(FULL, amb)) {
-                    if (amb)
-                        wrap = wrap_exact(aj, ai, a.thresang);
-                }
-                bits |= (unsigned)((same | wrap) & (b < jn)) << b;
-            }
+        for (int b = 0; b < 8; b++) {
+            const int j = min(j0 + b, m - 1);
+            const float aj = sm.ang[j];
+            const int dj = sm.dist[j];
+            const bool same = (abs(dj - di) < a.thresdis) &
+                              (fabsf(__fsub_rn(aj, ai)) < a.thresang);
+            const bool near = abs(dj + di) < a.thresdis;
+            const float est = fabsf(__fsub_rn(__fsub_rn(3.14159265f, aj), ai));
+            const bool lo = est < a.thresang - 1e-6f;
+            const bool hi = est > a.thresang + 1e-6f;
+            const bool in = 8 * q + b < jn;
+            bits |= (unsigned)((same | (near & lo)) & in) << (8 * q + b);
+            amb |= (unsigned)(near & !lo & !hi & !same & in) << b;
+        }
+        for (; amb; amb &= amb - 1) {
+            const int b = __ffs(amb) - 1;
+            if (wrap_exact(sm.ang[j0 + b], ai, a.thresang))
+                bits |= 1u << (8 * q + b);
         }
         bits |= __shfl_xor_sync(FULL, bits, 1);
         bits |= __shfl_xor_sync(FULL, bits, 2);
@@ -389,7 +392,12 @@ __device__ int greedy_chunk(FinSmem &sm, const hl_final_img &im, int m, int K, i
             unsigned kill = valid ? (sm.removed[w] >> lane) & 1u : 1u;
             unsigned pin = 0u;
             if (valid) {
-                for (int v = 0; v < w; v++)
+                int v = 0;
+                for (; v + 4 <= w; v += 4)
+                    kill |= (sm.pred[i][v] & sm.alive[v]) | (sm.pred[i][v + 1] & sm.alive[v + 1]) |
+                            (sm.pred[i][v + 2] & sm.alive[v + 2]) |
+                            (sm.pred[i][v + 3] & sm.alive[v + 3]);
+                for (; v < w; v++)
                     kill |= sm.pred[i][v] & sm.alive[v];
                 /* the in-word entry holds bits below the lane only (none
                  * was built for lane 0) */
@@ -482,6 +490,8 @@ __device__ void finalize_cta(const hl_final_args &a, const hl_final_img &im, flo
                              FinSmem &sm)
 {
     const int tid = threadIdx.x;
+    /* the first keys are on their way while their number is read */
+    const unsigned long long key0 = tid < min(im.cap, FIN_CHUNK) ? __ldcg(im.keys + tid) : 0ull;
     const int ncand_raw = *im.ncand;
     const int n = min(ncand_raw, im.cap);
     const int K = a.linesmax;
@@ -493,8 +503,8 @@ __device__ void finalize_cta(const hl_final_args &a, const hl_final_img &im, flo
     while (taken < n && S < K) {
         const int m = min(FIN_CHUNK, n - taken);
         if (n <= FIN_CHUNK) {
-            for (int i = tid; i < m; i += blockDim.x)
-                sm.keys[i] = im.keys[i];
+            if (tid < m)
+                sm.keys[tid] = key0;
         } else {
             /* MSD radix select of the m-th largest key below `upper` */
             unsigned long long prefix = 0, pmask = 0;
@@ -626,6 +636,11 @@ hl_finalize_kernel(hl_final_args a, int nimg, float scale)
  * threshold that does not separate) needs them all */
 #define FIN_CLEAR_CTAS 128
 
+/* Peaks that CTA 0 ranks alone: up to here its sort and bitmask take less than
+ * the two cluster barriers.  27 peaks (2048 x 2048, lines drawn): 64.7 us alone,
+ * 66.0 on the cluster; 306 (4096 x 4096, T = 720): 147.2 and 140.6 us. */
+#define FIN_ALONE 128
+
 /* One image on a cluster of FIN_CLUSTER CTAs (one per SM) when its peaks
  * fit one chunk: every CTA loads the keys, ranks an eighth of them into
  * every CTA's sorted[] (distributed shared memory), decodes all of them and
@@ -647,17 +662,18 @@ hl_finalize_cluster_kernel(hl_final_args a, float scale)
         return;
     }
     const hl_final_img im = a.img0;
+    const unsigned long long key0 = tid < min(im.cap, FIN_CHUNK) ? __ldcg(im.keys + tid) : 0ull;
     const int ncand_raw = *im.ncand;
     const int n = min(ncand_raw, im.cap);
     const int K = a.linesmax;
-    if (n > FIN_CHUNK || n == 0 || K <= 0) {
+    if (n > FIN_CHUNK || n <= FIN_ALONE || K <= 0) {
         if (rank == 0)
             finalize_cta(a, im, scale, sm);
         return;
     }
     const int m = n;
-    for (int i = tid; i < m; i += blockDim.x)
-        sm.keys[i] = im.keys[i];
+    if (tid < m)
+        sm.keys[tid] = key0;
     __syncthreads();
     {
         unsigned long long *dst[FIN_CLUSTER];
