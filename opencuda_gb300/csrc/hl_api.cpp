@@ -422,10 +422,10 @@ struct vote_plan {
     int part16, win_rows, exact;
     /* the blocks' items add to the accumulator instead of going through slabs:
      * where a tile needs several windows (rho steps below 0.1 pixels) or the
-     * slabs would take more than HL_MAX_SCRATCH (images of 32 K and more a
-     * side, or a handful of angles: a slab's column groups are as tall as their
-     * thetas lie apart).  Dense: the accumulator is cleared before and scanned
-     * after */
+     * slabs would take more than HL_MAX_SCRATCH and twice the accumulators (images
+     * of 32 K and more a side, or a handful of angles: a slab's column groups are
+     * as tall as their thetas lie apart).  Dense: the accumulator is cleared
+     * before and scanned after */
     int add;
 };
 #define HL_MAX_SCRATCH (1LL << 30)
@@ -738,6 +738,11 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
     }
     pl->items.resize(reg.size());
     pl->scratch_units = 0;
+    long long max_scratch = 0;
+    for (int i = 0; i < n; i++)
+        max_scratch += 8LL * im[i].R * h->Tp;
+    /* slabs are numbered in 31 bits */
+    max_scratch = std::min(std::max(max_scratch, HL_MAX_SCRATCH), 64LL * 0x7fffffff);
     double most = 8.0;
     const double irho = 1.0 / h->p.derho;
     for (size_t i = 0; i < reg.size(); i++) {
@@ -761,7 +766,7 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
                 it.gn[g] = sl.n[g];
                 it.go[g] = sl.o[g];
             }
-            pl->add |= pl->scratch_units + units > HL_MAX_SCRATCH / (pl->part16 ? 64 : 128);
+            pl->add |= pl->scratch_units + units > max_scratch / (pl->part16 ? 64 : 128);
             if (!pl->add) {
                 it.slab = sl.at = (int)pl->scratch_units;
                 pl->scratch_units += units;
@@ -2576,7 +2581,7 @@ extern "C" int hl_proposal_batch(hl_handle *h, hl_net *net,
     CK(cudaEventRecord(b->tab_read, s));
 
     /* fall-back and judged images run the plain method on the points that are
-     * there already (32 x 2048 x 2048, 21 of them: 754 us, 785 with their own
+     * there already (32 x 2048 x 2048, 21 of them: 757 us, 792 with their own
      * compaction) */
     int st_host[5] = {0, 0, 0, 0, 0};
     CK(cudaMemcpyAsync(pw->h_fb, pw->d_fb, sizeof(int) * nimg, cudaMemcpyDeviceToHost, s));
