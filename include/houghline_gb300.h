@@ -110,8 +110,8 @@ int hl_last_status(hl_handle *h, int *status, void *stream);
 
 /* Batched plain HoughLine: nimg independent DEVICE images (each with its own
  * size and ROI) through one compaction, one persistent vote launch over the
- * (image, theta slice, rho window) work queue, one peak pass and one
- * finalize CTA per image.  Every image gets the result hl_plain would give
+ * (image, theta slice, region) work queue, the merge of split slices, one peak
+ * pass and one finalize CTA per image.  Every image gets the result hl_plain would give
  * it (same vote rule, its own rho range, the handle's theta step, thresdis
  * and thresang); thresholds[i] replaces the handle's vote threshold for
  * image i when thresholds is not NULL.  The reference has no batched entry
@@ -216,8 +216,8 @@ int hl_lines_from_accumulator(hl_handle *h, const int32_t *acc_dev, int w,
                               int h_, int *linesmax, hl_line *lines,
                               void *stream);
 
-/* Vote-kernel launch shape: rows of the rho window held per CTA (0 = auto)
- * and threads per CTA (0 = auto). */
+/* Vote-kernel launch shape: rows of the rho window held per CTA at most (0 =
+ * auto; at least 168 are) and threads per CTA (0 = auto). */
 int hl_set_vote_shape(hl_handle *h, int window_rows, int threads);
 
 /* Shared-memory int32 atomicAdd ceiling of this GPU: conflict-free atomics

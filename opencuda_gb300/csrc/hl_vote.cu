@@ -56,9 +56,8 @@
  * Bound by instruction issue: 5 instructions a warp-vote in the loop, 1.6 of an
  * SM's cycles against the 1.13 of the shared-memory atomics alone, and the
  * items' edges (first copies, store, barriers) about a quarter of the time.
- * 4096 x 4096, T = 720: 101 us (fixed rho windows 122 us); the whole call with
- * slab merge 160 -> 148 us.  256 images of 256..2048 a side, T = 360: 890 us
- * (1295), the call 1596 -> 1186 us.  2048 points a slot: 1024 make every warp
+ * 4096 x 4096, T = 720: 92 us (fixed rho windows 118 us), with the slab merge 109
+ * (128).  256 images of 256..2048 a side, T = 360: 854 us (1267).  2048 points a slot: 1024 make every warp
  * wait on a barrier for every block it votes (4096 x 4096 158 against 153 us,
  * the batch 1364 against 1318).
  *
