@@ -85,7 +85,7 @@ struct hl_handle {
     /* HoughCircle: candidate keys, [ncand, status] counters, results; the
      * workspace of circle batches */
     struct hl_cb_ws *cb;
-    int *d_ctab;             /* the circles' offsets (hl_circle_table) */
+    int *d_ctab;             /* the circles' offsets (hl_circle_table_kernel) */
     uint32_t *d_cbits;       /* an image's edge map */
     size_t cap_cbits;
     unsigned long long *d_ckeys;
@@ -2714,9 +2714,7 @@ static int circle_prepare(hl_handle *h, const hl_image_desc *img, const hl_circl
     int rc = roi_of(img, roi);
     if (rc != HL_NO_ERROR)
         return rc;
-    if ((rc = hl_geometry(h, roi->w, roi->h, g)) != HL_NO_ERROR)
-        return rc;
-    return ensure_image(h, *g, roi->w, roi->h);
+    return hl_geometry(h, roi->w, roi->h, g);
 }
 
 /* radii of [radius_min, radius_max] that are counted on bit planes: the smallest */
@@ -2725,16 +2723,16 @@ static int circle_dense(const hl_circle_params *p)
     return std::max(0, std::min(p->radius_max, HL_CIRCLE_DENSE_R) - p->radius_min + 1);
 }
 
-/* the table of circle offsets, made once a handle; sets the kernel's pointers */
-static int circle_table(hl_handle *h, hl_circle_bits_args *ba)
+/* the table of circle offsets, made once a handle and waited for, so that later
+ * calls may come on other streams; sets the kernel's pointers */
+static int circle_table(hl_handle *h, hl_circle_bits_args *ba, cudaStream_t s)
 {
     if (!h->d_ctab) {
-        std::vector<int> t(hl_circle_table_bytes() / sizeof(int));
-        hl_circle_table(t.data());
         int *d = nullptr;
         CK(cudaMalloc(&d, hl_circle_table_bytes()));
-        const cudaError_t e =
-            cudaMemcpy(d, t.data(), hl_circle_table_bytes(), cudaMemcpyHostToDevice);
+        cudaError_t e = hl_launch_circle_table(d, s);
+        if (e == cudaSuccess)
+            e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
             cudaFree(d);
             return map_err(e);
@@ -2775,7 +2773,7 @@ static int circle_run(hl_handle *h, const hl_roi &roi, const hl_geom &g,
         b.w = roi.w;
         b.h = roi.h;
         hl_circle_bits_tiles(&b);
-        if ((rc = circle_table(h, &ba)) != HL_NO_ERROR ||
+        if ((rc = circle_table(h, &ba, s)) != HL_NO_ERROR ||
             (rc = grow((void **)&h->d_cbits, &h->cap_cbits,
                        sizeof(uint32_t) * (size_t)b.pitch * (size_t)b.h)) != HL_NO_ERROR)
             return rc;
@@ -2796,7 +2794,8 @@ static int circle_run(hl_handle *h, const hl_roi &roi, const hl_geom &g,
     }
     if (nd == nr)
         return HL_NO_ERROR;
-    if ((rc = launch_compaction(h, roi, g, s)) != HL_NO_ERROR)
+    if ((rc = ensure_image(h, g, roi.w, roi.h)) != HL_NO_ERROR ||
+        (rc = launch_compaction(h, roi, g, s)) != HL_NO_ERROR)
         return rc;
     ta.nz = nr - nd;
     ta.pts = reinterpret_cast<const float2 *>(h->d_pts);
@@ -2954,10 +2953,11 @@ static void circle_batch_free(hl_handle *h)
     h->cb = nullptr;
 }
 
-/* Circles of many ROIs (of one image or several) in one pipeline: one
- * compaction over every ROI (the batch form of the compaction kernel, each
- * ROI its own point region and tile offsets), one tile launch over every
- * ROI's (tile, radius) CTAs, one tail CTA per ROI, one copy of the results. */
+/* Circles of many ROIs (of one image or several) in one pipeline: the edge maps
+ * of every ROI and one bit-plane launch over their (tile, radius) CTAs, for the
+ * larger radii one compaction over every ROI (the batch form of the compaction
+ * kernel, each ROI its own point region and tile offsets) and one tile launch,
+ * then one tail CTA per ROI, one copy of the results. */
 extern "C" int hl_circles_batch(hl_handle *h, const hl_image_desc *imgs, int nimg,
                                 const hl_circle_params *p, int circlemax, hl_circle *out,
                                 int *counts, void *stream)
@@ -3090,7 +3090,7 @@ extern "C" int hl_circles_batch(hl_handle *h, const hl_image_desc *imgs, int nim
     if (nd > 0) {
         hl_circle_bits_args ba;
         memset(&ba, 0, sizeof(ba));
-        if ((rc = circle_table(h, &ba)) != HL_NO_ERROR)
+        if ((rc = circle_table(h, &ba, s)) != HL_NO_ERROR)
             return rc;
         ba.imgs = reinterpret_cast<const hl_circle_bits_img *>(dt + off_bits);
         ba.nimg = nimg;

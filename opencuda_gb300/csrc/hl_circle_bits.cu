@@ -12,6 +12,7 @@
  * the bit planes too: v above the threshold, above the left and upper
  * neighbours and at least the right and lower ones, zero outside the ROI.
  *
+ *   hl_circle_table_kernel -- the circles' offsets, once a handle.
  *   hl_edge_bits_kernel   -- the edge map: a bit a pixel (pixel == 255).
  *   hl_circle_bits_kernel -- a CTA a (tile, radius), largest radius first.
  *
@@ -42,6 +43,52 @@
 /* A row of the shared edge map: word 4 q + m at CB_Q m + q, so that threads on
  * consecutive units read consecutive words whatever the column distance. */
 #define CB_Q 10
+
+/* ---- the offsets ---------------------------------------------------------- */
+
+/* The offsets of the radii 0 .. HL_CIRCLE_DENSE_R, a CTA a radius, sorted by
+ * columns and then rows: the row distance << 16, the group << 8 (32 column
+ * distances, the first from -96) and the distance in the group.  A column's
+ * offsets come in pairs of rows +-i, so a group has an even number of them and two
+ * neighbours of an even place are of one group.  Made once a handle, by rank: the
+ * entries below an entry are counted.  Latency only.  Sorting the 22 K entries on the
+ * host took 1.16 ms: the first call of a new handle, 1024 x 1024, radii 5 to 50, is
+ * 200 us instead of 1346. */
+__global__ void __launch_bounds__(CB_TAB) hl_circle_table_kernel(int *table)
+{
+    __shared__ int s_y[CB_TAB / 8], s_key[CB_TAB], s_m;
+    const int tid = threadIdx.x, r = blockIdx.x;
+    if (tid == 0) {   /* the walk, okano_3_0/HoughCircle.cu:214-243 */
+        int m = 0;
+        for (int y = r, d = 3 - 2 * r; m < y && m < CB_TAB / 8; m++) {
+            s_y[m] = y;
+            const bool up = d < y;
+            d += up ? 4 * m + 6 : 4 * (m - y) + 10;
+            y -= up ? 0 : 1;
+        }
+        s_m = m;
+    }
+    __syncthreads();
+    const int n = 8 * s_m;
+    int row = 0, col = 0, key = 0;
+    if (tid < n) {
+        const int x = tid >> 3, y = s_y[x];
+        row = (tid & 1 ? x : y) * (tid & 2 ? -1 : 1);
+        col = (tid & 1 ? y : x) * (tid & 4 ? -1 : 1);
+        key = ((col + 128) * 256 + row + 128) * CB_TAB + tid;   /* no two alike */
+        s_key[tid] = key;
+    }
+    __syncthreads();
+    if (tid < n) {
+        int rank = 0;
+        for (int i = 0; i < n; i++)
+            rank += s_key[i] < key;
+        table[r * CB_TAB + rank] =
+            (int)((unsigned)row << 16) | (((col + 96) >> 5) << 8) | (col & 31);
+    }
+    if (tid == 0)
+        table[(HL_CIRCLE_DENSE_R + 1) * CB_TAB + r] = n;
+}
 
 /* ---- the edge map --------------------------------------------------------- */
 
@@ -407,47 +454,16 @@ hl_circle_bits_kernel(hl_circle_bits_args a)
 
 /* ---- host ------------------------------------------------------------------ */
 
-/* The offsets of the radii 0 .. HL_CIRCLE_DENSE_R, by groups of column distances
- * of 32, then rows: the row distance << 16, the group << 8 and the distance in
- * it.  A group has an even number of entries: an odd one takes one of the next
- * group's first column, at distance 32.  table: CB_TAB ints a radius, then a
- * count a radius. */
+/* table: CB_TAB entries a radius, then a count a radius */
 size_t hl_circle_table_bytes(void)
 {
     return (HL_CIRCLE_DENSE_R + 1) * (CB_TAB + 1) * sizeof(int);
 }
 
-void hl_circle_table(int *table)
+cudaError_t hl_launch_circle_table(int *table, cudaStream_t s)
 {
-    int *count = table + (HL_CIRCLE_DENSE_R + 1) * CB_TAB;
-    for (int r = 0; r <= HL_CIRCLE_DENSE_R; r++) {
-        /* votes of the walk (okano_3_0/HoughCircle.cu:214-243) by row and column */
-        static thread_local unsigned char cell[2 * HL_CIRCLE_DENSE_R + 1][2 * HL_CIRCLE_DENSE_R + 1];
-        for (int i = -r; i <= r; i++)
-            for (int j = -r; j <= r; j++)
-                cell[i + r][j + r] = 0;
-        for (int x = 0, y = r, d = 3 - 2 * r; x < y; x++) {
-            for (int s = 0; s < 4; s++) {
-                const int sx = s & 1 ? -1 : 1, sy = s & 2 ? -1 : 1;
-                cell[r + sy * y][r + sx * x]++;
-                cell[r + sy * x][r + sx * y]++;
-            }
-            const bool up = d < y;
-            d += up ? 4 * x + 6 : 4 * (x - y) + 10;
-            y -= up ? 0 : 1;
-        }
-        int n = 0;
-        for (int k = 0; k < 6; k++) {
-            const int j0 = 32 * (k - 3);
-            for (int j = std::max(-r, j0); j <= std::min(r, j0 + 32); j++)
-                for (int i = -r; i <= r; i++)
-                    while (cell[i + r][j + r] && (j < j0 + 32 || (n & 1))) {
-                        cell[i + r][j + r]--;
-                        table[r * CB_TAB + n++] = (int)((unsigned)i << 16) | (k << 8) | (j - j0);
-                    }
-        }
-        count[r] = n;
-    }
+    hl_circle_table_kernel<<<HL_CIRCLE_DENSE_R + 1, CB_TAB, 0, s>>>(table);
+    return cudaGetLastError();
 }
 
 /* the tiles of a w x h image: sets its pitch, twu, ntx and nty */

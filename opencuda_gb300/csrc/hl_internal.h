@@ -350,7 +350,7 @@ typedef struct hl_circle_bits_args {
     hl_circle_bits_img img0;
     int nimg;
     int rmin, nr;             /* rmin + nr - 1 <= HL_CIRCLE_DENSE_R */
-    const int *table, *count; /* hl_circle_table */
+    const int *table, *count; /* hl_circle_table_kernel */
     int32_t *acc;             /* [nr][h][w], or NULL */
     int threshold;
     unsigned long long *keys; /* one image: votes << 32 | ~index, or NULL */
@@ -359,7 +359,7 @@ typedef struct hl_circle_bits_args {
     int *status;
 } hl_circle_bits_args;
 size_t hl_circle_table_bytes(void);
-void hl_circle_table(int *table);
+cudaError_t hl_launch_circle_table(int *table, cudaStream_t s);
 void hl_circle_bits_tiles(hl_circle_bits_img *im);
 cudaError_t hl_launch_edge_bits(const hl_circle_bits_img *dev, const hl_circle_bits_img *im0,
                                 int nimg, long long blocks, cudaStream_t s);

@@ -66,3 +66,11 @@ def test_batches_of_uneven_sizes(mod, rmin, rmax, thr):
     for im, got in zip(imgs, per):
         want, n = O.houghcircle(im, rmin, rmax, thr, 4.0, 3, 12)
         assert n <= 4096 and [c.astuple() for c in got] == list(want), im.shape
+
+
+@pytest.mark.parametrize("rmin,rmax", [(0, 44), (45, 89)])
+def test_offsets_of_every_radius(mod, rmin, rmax):
+    HoughCircle, Image = mod
+    img = _noise(203, 190, 0.3, rmax)
+    got = HoughCircle(rmin, rmax).accumulator(Image.from_host(img)).cpu().numpy()
+    assert np.array_equal(got, O.circle_vote(img, rmin, rmax))
