@@ -2197,6 +2197,8 @@ static int batch_last_status(hl_handle *h, int *status, cudaStream_t s)
     CK(cudaMemcpyAsync(&st, b->d_cnt + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     *status = st;
+    if (st != 0)
+        b->acc_zero = 0;   /* a launch that gave up may have left bins */
     return HL_NO_ERROR;
 }
 
@@ -2281,8 +2283,10 @@ extern "C" int hl_batch(hl_handle *h, const hl_image_desc *imgs, int nimg,
     if (lbytes)
         CK(cudaMemcpyAsync(b->h_res, b->d_lines, lbytes, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    if (h_counts[nimg] != 0)
+    if (h_counts[nimg] != 0) {
+        b->acc_zero = 0;   /* a launch that gave up may have left bins */
         return HL_CUDA_ERROR;
+    }
     for (int i = 0; i < nimg; i++) {
         const int c = std::max(0, std::min(h_counts[i], linesmax));
         counts[i] = c;
