@@ -412,6 +412,16 @@ extern "C" int hl_last_launch_count(const hl_handle *h)
  * then cost more than its votes.  1913 x 1077, T = 360: 64 K, 128 K, 192 K pixels
  * 45.6, 45.5, 43.1 us; 2048 x 2048, T = 360, lines drawn: 72.6, 73.6, 67.9 us. */
 #define HL_MIN_REGION (192.0 * 1024.0)
+/* At rho steps below 1 regions of one window get small and the rows that they
+ * store many; a stored and merged row costs about this many pixels then (16 images
+ * of 1000 x 900, T = 180, step 0.1: 32 M rows, 1.5 ms).  If regions of several
+ * windows come to less than three quarters of that over a launch, they are taken.
+ * A call, T = 180, with one window a region in brackets: 16 images of 1000 x 900,
+ * step 0.1 1380 us (1724), 0.05 2121 (3421); one of 2048 x 2048, 0.1 359 (497),
+ * 0.05 462 (743).  At 0.25 one window is the cheaper: 222 us for the 16 images, 711
+ * with several. */
+#define HL_SLAB_PIXELS 384.0
+#define HL_CLIP_COST 2.5
 
 struct vote_plan {
     std::vector<hl_vote_item> items;
@@ -421,7 +431,7 @@ struct vote_plan {
     unsigned chunks;           /* of a merge launch */
     int part16, win_rows, exact;
     /* the blocks' items add to the accumulator instead of going through slabs:
-     * where a tile needs several windows (rho steps below 0.1 pixels) or the
+     * where a region has several windows (fine rho steps, HL_SLAB_PIXELS) or the
      * slabs would take more than HL_MAX_SCRATCH and twice the accumulators (images
      * of 32 K and more a side, or a handful of angles: a slab's column groups are
      * as tall as their thetas lie apart).  Dense: the accumulator is cleared
@@ -511,6 +521,39 @@ static void best_grid(const slice_ext &e, int w, int hh, int cap, double n_min, 
     }
     if (!*nwin)   /* one tile a region, several windows */
         *nwin = (int)ceil(region_rows(e, std::min(w, HL_TILE_W), std::min(hh, HL_TILE_H)) / cap);
+}
+
+/* The same with several windows a region where that is cheaper: every window
+ * tests all votes of its region (HL_CLIP_COST plain votes each), rows are stored
+ * once a region.  Returns the cost in pixels; *grid is best_grid's. */
+static double window_grid(const slice_ext &e, int w, int hh, int cap, double n_min, int *bx,
+                          int *by, int *nwin, double *grid)
+{
+    const int tx = (w + HL_TILE_W - 1) / HL_TILE_W, ty = (hh + HL_TILE_H - 1) / HL_TILE_H;
+    const auto cost = [&](int nx, int ny, int nw) {
+        const double gw = std::min(((tx + nx - 1) / nx) * HL_TILE_W, w);
+        const double gh = std::min(((ty + ny - 1) / ny) * HL_TILE_H, hh);
+        return (double)nx * ny * (gw * gh * nw * (nw > 1 ? HL_CLIP_COST : 1.0) +
+                                  HL_SLAB_PIXELS * std::min(region_rows(e, gw, gh),
+                                                            (double)nw * cap));
+    };
+    best_grid(e, w, hh, cap, n_min, bx, by, nwin);
+    double best = *grid = cost(*bx, *by, *nwin);
+    for (int nx = 1; nx <= std::min(tx, 8); nx *= 2)
+        for (int ny = 1; ny <= std::min(ty, 16); ny *= 2) {
+            if (nx > 1 && (ty + ny - 1) / ny > HL_VOTE_RUNS)
+                continue;
+            const double gw = std::min(((tx + nx - 1) / nx) * HL_TILE_W, w);
+            const double gh = std::min(((ty + ny - 1) / ny) * HL_TILE_H, hh);
+            const int nw = (int)ceil(region_rows(e, gw, gh) / cap);
+            if (cost(nx, ny, nw) < best) {
+                best = cost(nx, ny, nw);
+                *bx = nx;
+                *by = ny;
+                *nwin = nw;
+            }
+        }
+    return best;
 }
 
 /* The item of a whole w x hh image whose range exceeds the window, voted with a
@@ -611,6 +654,22 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
     int big = 0;
     std::vector<plan_region> reg;
     bool slides = false;
+    bool windows = false;   /* several a region: see HL_SLAB_PIXELS */
+    if (h->p.derho < 1.0) {
+        double in_windows = 0.0, in_grids = 0.0;
+        for (int i = 0; i < n; i++)
+            for (int sl = 0; sl < slices; sl++) {
+                const double n_min = std::max(1.0, ceil((double)im[i].w * im[i].h / wcap));
+                hl_vote_item it;
+                int nx, ny, nw;
+                double g;
+                if (n_min <= 1.0 && slide_item(h, ext[sl], im[i].w, im[i].h, sl, cap, &it))
+                    continue;
+                in_windows += window_grid(ext[sl], im[i].w, im[i].h, cap, n_min, &nx, &ny, &nw, &g);
+                in_grids += g;
+            }
+        windows = in_windows < 0.75 * in_grids;
+    }
     pl->exact = pl->add = 0;
     pl->part16 = 1;
     for (int i = 0; i < n; i++) {
@@ -639,7 +698,11 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
                 continue;
             }
             int nx, ny, nw;
-            best_grid(ext[sl], w, hh, cap, n_min, &nx, &ny, &nw);
+            double grid;
+            if (windows)
+                window_grid(ext[sl], w, hh, cap, n_min, &nx, &ny, &nw, &grid);
+            else
+                best_grid(ext[sl], w, hh, cap, n_min, &nx, &ny, &nw);
             const bool clip = nw > 1;
             pl->add |= clip;
             for (int y = 0; y < ny; y++)

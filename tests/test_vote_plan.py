@@ -113,3 +113,23 @@ def test_blocks_whole_and_split_in_one_batch(hl_mod):
         assert rc == 0
         for im, got in zip(imgs, res):
             assert [l.astuple() for l in got] == _want(hl, im, thr, 16, det, 1.0)
+
+
+@pytest.mark.parametrize("derho", [0.5, 0.25, 0.1, 0.03])
+def test_fine_rho_steps(hl_mod, derho):
+    """Regions of one window and of several, for one image and for a batch."""
+    HoughLine, Image = hl_mod
+    det = math.pi / 60
+    hl = HoughLine(detheta=det, derho=derho)
+    imgs = [_scene(w, h, w) for w, h in ((611, 507), (130, 900), (1000, 33))]
+    dev = [Image.from_host(im) for im in imgs]
+    c, s = hl.trig_table()
+    for im, d in zip(imgs, dev):
+        acc, rho_min = hl.accumulator(d)
+        want, wmin, _ = O.vote_image(im, c, s, derho)
+        assert rho_min == wmin and np.array_equal(acc.cpu().numpy(), want)
+    thr = [max(im.shape) // 2 for im in imgs]
+    rc, res = hl.houghLineBatch(dev, 16, thr)
+    assert rc == 0
+    for im, t, got in zip(imgs, thr, res):
+        assert [l.astuple() for l in got] == _want(hl, im, t, 16, det, derho), im.shape
