@@ -72,6 +72,7 @@
  * producer then waits (bounded) for its copies in flight before exiting.
  */
 #include "hl_internal.h"
+#include "hl_band.h"
 #include "hl_device.cuh"
 
 #include <algorithm>
@@ -387,6 +388,7 @@ __device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &s
         float cm = slide ? a.cosv[km] * a.irho : 0.0f;
         cm = copysignf(fmaxf(fabsf(cm), 1.0e-9f), cm);
         const float icm = 1.0f / (cm * HL_TILE_W);
+        const float x0 = __fmul_rn(ctx - HL_TILE_W / 2, 1.0f / HL_TILE_W);
         const bool wide = txn == im.tiles_x && !slide;
         const int nsegs = have ? max(it.nseg, 1) : 1;
 
@@ -409,18 +411,9 @@ __device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &s
             if (r < nruns) {
                 int ta = 0, tb = txn;   /* the run's tiles, from tx0 */
                 if (slide) {
-                    /* first tile past the band's near and far edge: monotone
-                     * in x, so the bands' edges split the row */
-                    const float yk = ((float)((ty0 + r) * HL_TILE_H + HL_TILE_H / 2) - cty) * sm_;
-                    const float k0 = (float)(sj * it.adv) - it.half - yk;
-                    const float e0 = ceilf(k0 * icm + (ctx - HL_TILE_W / 2) * (1.0f / HL_TILE_W));
-                    const float e1 = ceilf((k0 + (float)it.adv) * icm +
-                                           (ctx - HL_TILE_W / 2) * (1.0f / HL_TILE_W));
-                    const int i0 = (int)fminf(fmaxf(e0, 0.0f), (float)txn);
-                    const int i1 = (int)fminf(fmaxf(e1, 0.0f), (float)txn);
-                    const bool fst = sj == 0, lst = sj == nsegs - 1;
-                    ta = cm > 0.0f ? (fst ? 0 : i0) : (lst ? 0 : i1);
-                    tb = cm > 0.0f ? (lst ? txn : i1) : (fst ? txn : i0);
+                    const float yk = __fmul_rn(
+                        (float)((ty0 + r) * HL_TILE_H + HL_TILE_H / 2) - cty, sm_);
+                    hl_band_tiles(sj, nsegs, it.adv, it.half, yk, cm, icm, x0, txn, &ta, &tb);
                 }
                 if (tb > ta) {
                     const int t0 = (ty0 + r) * im.tiles_x + tx0;
