@@ -78,6 +78,10 @@ struct hl_handle {
     double plan_detheta, plan_derho;
     unsigned char *d_plan;   /* items, merge blocks, slab list */
     size_t cap_plan;
+    unsigned char *h_plan;   /* its pinned staging copy ... */
+    size_t cap_hplan;
+    cudaEvent_t plan_read;   /* ... and the last upload's end */
+    int plan_event;
     unsigned char *d_scratch;
     size_t cap_scratch;
     unsigned long long *d_cand;   /* noted peak candidates */
@@ -160,6 +164,21 @@ static int grow(void **ptr, size_t *cap, size_t need_bytes)
         *ptr = nullptr;
         return e == cudaErrorMemoryAllocation ? HL_OUT_OF_MEM : HL_CUDA_ERROR;
     }
+    *cap = nb;
+    return HL_NO_ERROR;
+}
+
+static int grow_host(unsigned char **ptr, size_t *cap, size_t need)
+{
+    if (*cap >= need && *ptr)
+        return HL_NO_ERROR;
+    size_t nb = std::max(need, (size_t)4096);
+    nb += nb / 4;
+    if (*ptr)
+        cudaFreeHost(*ptr);
+    *ptr = nullptr;
+    *cap = 0;
+    CK(cudaMallocHost(ptr, nb));
     *cap = nb;
     return HL_NO_ERROR;
 }
@@ -267,6 +286,10 @@ extern "C" int hl_destroy(hl_handle *h)
         cudaFreeHost(h->h_cres);
     if (h->h_bbox)
         cudaFreeHost(h->h_bbox);
+    if (h->h_plan)
+        cudaFreeHost(h->h_plan);
+    if (h->plan_event)
+        cudaEventDestroy(h->plan_read);
     free(h->h_cos);
     free(h->h_sin);
     if (h->prof_ev) {
@@ -876,8 +899,6 @@ static int vote_ctas(const hl_handle *h, int rows, int threads)
     return std::max(h->sms, 1) * per_sm;
 }
 
-/* The handle's plan for a w x hh ROI, uploaded; fills va's items, scratch and
- * window rows. */
 static size_t plan_bytes(const vote_plan &p)
 {
     return p.items.size() * sizeof(hl_vote_item) + p.blocks.size() * sizeof(hl_merge_block) +
@@ -921,7 +942,35 @@ static void plan_args(const vote_plan &p, const unsigned char *d_plan, unsigned 
     ma->cand = va->cand;
 }
 
-static int handle_plan(hl_handle *h, int w, int hh, int R, int rho_min)
+/* Uploads the handle's plan on s, behind whatever there still reads the previous
+ * one; the staging copy is rewritten once the previous upload has read it.  A
+ * stream under capture is refused: a replay would read the staging copy as later
+ * calls leave it. */
+static int plan_upload(hl_handle *h, cudaStream_t s)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone)
+        return HL_CUDA_ERROR;
+    const size_t bytes = plan_bytes(*h->plan);
+    if (!h->plan_event) {
+        CK(cudaEventCreateWithFlags(&h->plan_read, cudaEventDisableTiming));
+        h->plan_event = 1;
+    }
+    CK(cudaEventSynchronize(h->plan_read));
+    int rc;
+    if ((rc = grow_host(&h->h_plan, &h->cap_hplan, bytes)) != HL_NO_ERROR ||
+        (rc = grow((void **)&h->d_plan, &h->cap_plan, bytes)) != HL_NO_ERROR)
+        return rc;
+    plan_copy(*h->plan, h->h_plan);
+    CK(cudaMemcpyAsync(h->d_plan, h->h_plan, bytes, cudaMemcpyHostToDevice, s));
+    CK(cudaEventRecord(h->plan_read, s));
+    return HL_NO_ERROR;
+}
+
+/* The handle's plan for a w x hh ROI, uploaded, and room for its slabs and noted
+ * candidates. */
+static int handle_plan(hl_handle *h, int w, int hh, int R, int rho_min, cudaStream_t s)
 {
     const int cap = plan_cap(h), threads = vote_threads(h);
     if (!(h->plan && h->plan_w == w && h->plan_h == hh && h->plan_R == R && h->plan_T == h->T &&
@@ -936,11 +985,8 @@ static int handle_plan(hl_handle *h, int w, int hh, int R, int rho_min)
         int rc = make_plan(h, &im, 1, cap, std::max(h->sms, 1), h->plan);
         if (rc != HL_NO_ERROR)
             return rc;
-        std::vector<unsigned char> tab(plan_bytes(*h->plan));
-        plan_copy(*h->plan, tab.data());
-        if ((rc = grow((void **)&h->d_plan, &h->cap_plan, tab.size())) != HL_NO_ERROR)
+        if ((rc = plan_upload(h, s)) != HL_NO_ERROR)
             return rc;
-        CK(cudaMemcpy(h->d_plan, tab.data(), tab.size(), cudaMemcpyHostToDevice));
         h->plan_w = w;
         h->plan_h = hh;
         h->plan_R = R;
@@ -1120,7 +1166,7 @@ static int run_ab(hl_handle *h, const hl_roi &roi, const hl_geom &g, bool peaks,
     va.Tp = h->Tp;
     va.irho = (float)(1.0 / h->p.derho);   /* okano_3_0/HoughLine.cu:107 */
     va.status = h->d_counters + 1;
-    int rc = handle_plan(h, roi.w, roi.h, g.numrho, g.rho_min);
+    int rc = handle_plan(h, roi.w, roi.h, g.numrho, g.rho_min, s);
     if (rc != HL_NO_ERROR)
         return rc;
     /* bins above the threshold are noted where their final count is known;
@@ -1827,21 +1873,6 @@ static void batch_ws_free(hl_batch_ws *b)
     if (b->cap_stream)
         cudaStreamDestroy(b->cap_stream);
     delete b;
-}
-
-static int grow_host(unsigned char **ptr, size_t *cap, size_t need)
-{
-    if (*cap >= need && *ptr)
-        return HL_NO_ERROR;
-    size_t nb = std::max(need, (size_t)4096);
-    nb += nb / 4;
-    if (*ptr)
-        cudaFreeHost(*ptr);
-    *ptr = nullptr;
-    *cap = 0;
-    CK(cudaMallocHost(ptr, nb));
-    *cap = nb;
-    return HL_NO_ERROR;
 }
 
 static size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
