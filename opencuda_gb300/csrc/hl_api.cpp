@@ -1004,19 +1004,21 @@ static int handle_plan(hl_handle *h, int w, int hh, int R, int rho_min, cudaStre
                 sizeof(unsigned long long) * (65536 + (size_t)R * h->Tp / 128));
 }
 
-static int ensure_image(hl_handle *h, const hl_geom &g, int w, int hh)
+/* New buffers are cleared on the call's stream: the default stream's order does not
+ * reach a non-blocking one. */
+static int ensure_image(hl_handle *h, const hl_geom &g, int w, int hh, cudaStream_t s)
 {
     int rc;
     size_t ntiles = (size_t)g.tiles_x * g.tiles_y;
     if ((rc = grow((void **)&h->d_pts, &h->cap_pts,
                    sizeof(float2) * ((size_t)w * hh + 16))) != HL_NO_ERROR)
         return rc;
-    if (h->cap_tiles < ntiles + 1 || !h->d_tile_state) {
+    if (h->cap_tiles < ntiles + 1 || !h->d_tile_state || !h->d_tile_off) {
         size_t cap = 0;
         if ((rc = grow((void **)&h->d_tile_state, &cap,
                        sizeof(unsigned long long) * (ntiles + 1))) != HL_NO_ERROR)
             return rc;
-        CK(cudaMemset(h->d_tile_state, 0, cap));
+        CK(cudaMemsetAsync(h->d_tile_state, 0, cap, s));
         size_t cap2 = 0;
         if ((rc = grow((void **)&h->d_tile_off, &cap2,
                        sizeof(int) * (ntiles + 1))) != HL_NO_ERROR)
@@ -1331,7 +1333,7 @@ static int plain_launch(hl_handle *h, const hl_image_desc *img, int linesmax,
         return rc;
     if (ref_numrho_override > 0)
         g.ref_numrho = ref_numrho_override;
-    if ((rc = ensure_image(h, g, roi.w, roi.h)) != HL_NO_ERROR)
+    if ((rc = ensure_image(h, g, roi.w, roi.h, s)) != HL_NO_ERROR)
         return rc;
     if ((rc = ensure_acc(h, g.numrho, linesmax)) != HL_NO_ERROR)
         return rc;
@@ -1421,6 +1423,7 @@ extern "C" int hl_compact(hl_handle *h, const hl_image_desc *img,
 {
     if (!h || !img || !pts_dev || !tile_off_dev || !count_dev)
         return HL_NULL_POINTER;
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     hl_roi roi;
     int rc = roi_of(img, &roi);
     if (rc != HL_NO_ERROR)
@@ -1428,9 +1431,8 @@ extern "C" int hl_compact(hl_handle *h, const hl_image_desc *img,
     hl_geom g;
     if ((rc = hl_geometry(h, roi.w, roi.h, &g)) != HL_NO_ERROR)
         return rc;
-    if ((rc = ensure_image(h, g, roi.w, roi.h)) != HL_NO_ERROR)
+    if ((rc = ensure_image(h, g, roi.w, roi.h, s)) != HL_NO_ERROR)
         return rc;
-    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const int ntiles = g.tiles_x * g.tiles_y;
     hl_compact_args ca;
     memset(&ca, 0, sizeof(ca));
@@ -1474,6 +1476,7 @@ extern "C" int hl_accumulator(hl_handle *h, const hl_image_desc *img,
 {
     if (!h || !img || !acc_dev)
         return HL_NULL_POINTER;
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     hl_roi roi;
     int rc = roi_of(img, &roi);
     if (rc != HL_NO_ERROR)
@@ -1481,11 +1484,10 @@ extern "C" int hl_accumulator(hl_handle *h, const hl_image_desc *img,
     hl_geom g;
     if ((rc = hl_geometry(h, roi.w, roi.h, &g)) != HL_NO_ERROR)
         return rc;
-    if ((rc = ensure_image(h, g, roi.w, roi.h)) != HL_NO_ERROR)
+    if ((rc = ensure_image(h, g, roi.w, roi.h, s)) != HL_NO_ERROR)
         return rc;
     if ((rc = ensure_acc(h, g.numrho, 1)) != HL_NO_ERROR)
         return rc;
-    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     int launches = 0;
     if ((rc = run_ab(h, roi, g, false, s, &launches)) != HL_NO_ERROR)
         return rc;
@@ -1499,6 +1501,7 @@ extern "C" int hl_accumulator_ref_layout(hl_handle *h, const hl_image_desc *img,
 {
     if (!h || !img || !ref_dev)
         return HL_NULL_POINTER;
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     hl_roi roi;
     int rc = roi_of(img, &roi);
     if (rc != HL_NO_ERROR)
@@ -1506,11 +1509,10 @@ extern "C" int hl_accumulator_ref_layout(hl_handle *h, const hl_image_desc *img,
     hl_geom g;
     if ((rc = hl_geometry(h, roi.w, roi.h, &g)) != HL_NO_ERROR)
         return rc;
-    if ((rc = ensure_image(h, g, roi.w, roi.h)) != HL_NO_ERROR)
+    if ((rc = ensure_image(h, g, roi.w, roi.h, s)) != HL_NO_ERROR)
         return rc;
     if ((rc = ensure_acc(h, g.numrho, 1)) != HL_NO_ERROR)
         return rc;
-    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     int launches = 0;
     if ((rc = run_ab(h, roi, g, false, s, &launches)) != HL_NO_ERROR)
         return rc;
@@ -1883,7 +1885,7 @@ static size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
  * points are another workspace's, image i's those of its image src_img[i]. */
 static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
                       int nimg, const int *thr, int K, hl_line *lines_dev,
-                      int *counts_dev, const hl_roi *rois,
+                      int *counts_dev, const hl_roi *rois, cudaStream_t s,
                       const hl_batch_ws *src = nullptr, const int *src_img = nullptr)
 {
     std::vector<hl_geom> gs((size_t)nimg);
@@ -2006,7 +2008,7 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
         if ((rc = grow((void **)&b->d_ncand, &b->cap_ncand, sizeof(int) * (size_t)nimg)) !=
             HL_NO_ERROR)
             return rc;
-        CK(cudaMemset(b->d_ncand, 0, b->cap_ncand));
+        CK(cudaMemsetAsync(b->d_ncand, 0, b->cap_ncand, s));   /* not the default stream's */
     }
     if (!b->d_cnt)
         CK(cudaMalloc(&b->d_cnt, BW_NCNT * sizeof(int)));
@@ -2208,8 +2210,8 @@ static int batch_run_ws(hl_handle *h, hl_batch_ws **pb, const hl_image_desc *img
         if (rc != HL_NO_ERROR)
             return rc;
     }
-    int rc = batch_plan(h, b, imgs, nimg, thr, K, lines_dev, counts_dev, rois.data(), src,
-                        src_img);
+    int rc = batch_plan(h, b, imgs, nimg, thr, K, lines_dev, counts_dev, rois.data(), s,
+                        src, src_img);
     if (rc != HL_NO_ERROR)
         return rc;
     h->last_batch = 1;
@@ -2568,7 +2570,7 @@ extern "C" int hl_proposal_batch(hl_handle *h, hl_net *net,
         if ((rc = roi_of(&imgs[i], &rois[i])) != HL_NO_ERROR)
             return rc;
     if ((rc = batch_plan(h, b, imgs, nimg, thresholds, K, lines_dev, counts_dev,
-                         rois.data())) != HL_NO_ERROR)
+                         rois.data(), s)) != HL_NO_ERROR)
         return rc;
     h->last_batch = 1;
 
@@ -2892,7 +2894,7 @@ static int circle_run(hl_handle *h, const hl_roi &roi, const hl_geom &g,
     }
     if (nd == nr)
         return HL_NO_ERROR;
-    if ((rc = ensure_image(h, g, roi.w, roi.h)) != HL_NO_ERROR ||
+    if ((rc = ensure_image(h, g, roi.w, roi.h, s)) != HL_NO_ERROR ||
         (rc = launch_compaction(h, roi, g, s)) != HL_NO_ERROR)
         return rc;
     ta.nz = nr - nd;
@@ -2963,7 +2965,7 @@ extern "C" int hl_circles(hl_handle *h, const hl_image_desc *img, const hl_circl
     if (!h->d_ckeys) {
         CK(cudaMalloc(&h->d_ckeys, sizeof(unsigned long long) * HL_CIRCLE_MAXCAND));
         CK(cudaMalloc(&h->d_ccnt, 2 * sizeof(int)));
-        CK(cudaMemset(h->d_ccnt, 0, 2 * sizeof(int)));
+        CK(cudaMemsetAsync(h->d_ccnt, 0, 2 * sizeof(int), s));
     }
     /* results: header + room for circlemax circles, pinned mirror */
     static const size_t kResCap = sizeof(hl_result_hdr) + sizeof(hl_circle) * 4096;

@@ -53,3 +53,36 @@ def test_geometries_alternate_on_one_stream(cuda):
         ang = got[i, :m, 0].copy().view(np.float32)
         assert [(float(a), int(d), int(v)) for a, d, v in
                 zip(ang, got[i, :m, 1], got[i, :m, 2])] == want[i % 2], i
+
+
+def test_first_calls_beside_a_busy_default_stream(cuda):
+    """A new handle's first batch and first circles on a non-blocking stream while
+    the default stream is busy: their fresh counters are cleared in order."""
+    import torch
+    from opencuda_gb300 import _lib
+    from opencuda_gb300.houghcircle import HoughCircle
+    from opencuda_gb300.houghline import HoughLine, Image
+    L = _lib.load()
+    det, K = math.pi / 180, 16
+    imgs = [_image(700 + 60 * i, 500 + 90 * i, i) for i in range(4)]
+    dev = [Image.from_host(im) for im in imgs]
+    ref, hl = HoughLine(detheta=det, threshold=150), HoughLine(detheta=det, threshold=150)
+    rc, want = ref.houghLineBatch(dev, K)
+    assert rc == 0
+    circ = [HoughCircle(), HoughCircle()]
+    wantc = circ[0].houghcircle(dev[0], None, 8)
+    # dirty memory for the buffers to come
+    dirt = [torch.full((1 << 18,), 0x01010101, dtype=torch.int32, device=cuda) for _ in range(64)]
+    torch.cuda.synchronize()
+    del dirt
+    torch.cuda.empty_cache()
+    st = torch.cuda.Stream()
+    a = torch.randn((8192, 8192), dtype=torch.bfloat16, device=cuda)
+    for _ in range(40):
+        b = a @ a
+    rc, got = hl.houghLineBatch(dev, K, stream=st)
+    assert rc == 0 and got == want
+    gotc = circ[1].houghcircle(dev[0], None, 8, stream=st)
+    assert gotc == wantc
+    torch.cuda.synchronize()
+    del b
