@@ -2229,16 +2229,16 @@ static int batch_run_ws(hl_handle *h, hl_batch_ws **pb, const hl_image_desc *img
     } else {
         /* graph key: the plan key plus what the captured nodes hold */
         std::vector<long long> gk(b->key.begin(), b->key.end());
-        gk.push_back((long long)(uintptr_t)lines_dev);
-        gk.push_back((long long)(uintptr_t)counts_dev);
+        const void *held[] = {lines_dev, counts_dev, h->d_cos, h->d_sin, b->d_acc, b->d_pts,
+                              b->d_state, b->d_tile_off, b->d_tab, b->h_tab, b->d_keys,
+                              b->d_ncand, b->d_cnt, b->d_scratch, b->d_cand};
+        for (const void *p : held)
+            gk.push_back((long long)(uintptr_t)p);
+        unsigned ang;
+        memcpy(&ang, &h->p.thresang, sizeof(ang));
         gk.push_back(K);
-        gk.push_back((long long)(uintptr_t)b->d_acc);
-        gk.push_back((long long)(uintptr_t)b->d_pts);
-        gk.push_back((long long)(uintptr_t)b->d_tab);
-        gk.push_back((long long)(uintptr_t)b->h_tab);
-        gk.push_back((long long)(uintptr_t)b->d_keys);
-        gk.push_back((long long)(uintptr_t)b->d_scratch);
-        gk.push_back((long long)(uintptr_t)b->d_cand);
+        gk.push_back(h->p.thresdis);
+        gk.push_back((long long)ang);
         if (!b->gexec || gk != b->gkey) {
             if (b->gexec) {
                 cudaGraphExecDestroy(b->gexec);
