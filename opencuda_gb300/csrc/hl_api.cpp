@@ -132,10 +132,13 @@ static void prof_mark(hl_handle *h, int st, cudaStream_t s)
     }
 }
 
+/* An error is reported once: the runtime keeps a failed call's as the last error,
+ * which the check after the next launch would take for that launch's. */
 static int map_err(cudaError_t e)
 {
     if (e == cudaSuccess)
         return HL_NO_ERROR;
+    cudaGetLastError();
     if (e == cudaErrorMemoryAllocation)
         return HL_OUT_OF_MEM;
     return HL_CUDA_ERROR;
@@ -162,7 +165,7 @@ static int grow(void **ptr, size_t *cap, size_t need_bytes)
     cudaError_t e = cudaMalloc(ptr, nb);
     if (e != cudaSuccess) {
         *ptr = nullptr;
-        return e == cudaErrorMemoryAllocation ? HL_OUT_OF_MEM : HL_CUDA_ERROR;
+        return map_err(e);
     }
     *cap = nb;
     return HL_NO_ERROR;

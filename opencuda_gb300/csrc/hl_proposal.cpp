@@ -22,6 +22,7 @@ static int cnn_err(cudaError_t e)
 {
     if (e == cudaSuccess)
         return HL_NO_ERROR;
+    cudaGetLastError();   /* reported once: see map_err in hl_api.cpp */
     return e == cudaErrorMemoryAllocation ? HL_OUT_OF_MEM : HL_CUDA_ERROR;
 }
 
