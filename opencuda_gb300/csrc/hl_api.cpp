@@ -72,8 +72,7 @@ struct hl_handle {
      * the persistent-CTA counter base */
     struct vote_plan *plan;
     int plan_w, plan_h, plan_R, plan_T, plan_cap, plan_thr;
-    int acc_state;           /* what is known of d_acc (ACC_*) ... */
-    size_t acc_bytes;        /* ... as long as cap_acc is still this */
+    int acc_state;           /* what is known of d_acc (ACC_*) */
     int cand_par;            /* the noted candidates' counter: [10 + cand_par] */
     double plan_detheta, plan_derho;
     unsigned char *d_plan;   /* items, merge blocks, slab list */
@@ -1049,6 +1048,8 @@ static int ensure_acc(hl_handle *h, int R, int linesmax)
 {
     int rc;
     size_t bins = (size_t)R * h->Tp;
+    if (h->cap_acc < sizeof(int32_t) * bins)
+        h->acc_state = ACC_ANY;   /* another buffer, also after a failed allocation */
     if ((rc = grow((void **)&h->d_acc, &h->cap_acc, sizeof(int32_t) * bins)) !=
         HL_NO_ERROR)
         return rc;
@@ -1184,12 +1185,11 @@ static int run_ab(hl_handle *h, const hl_roi &roi, const hl_geom &g, bool peaks,
     plan_args(*h->plan, h->d_plan, h->d_scratch, &va, &ma);
     const int threads = vote_threads(h);
     const int ctas = vote_ctas(h, va.win_rows, threads);
-    if (h->acc_bytes != h->cap_acc || va.add)
+    if (va.add)
         h->acc_state = ACC_ANY;
     if (h->acc_state == ACC_ANY || (peaks && h->acc_state != ACC_ZERO)) {
         CK(cudaMemsetAsync(h->d_acc, 0, h->cap_acc, s));
         CK(cudaMemsetAsync(h->d_counters + 10, 0, 2 * sizeof(int), s));
-        h->acc_bytes = h->cap_acc;
     }
     /* with peaks the tail clears what is stored (set when it is launched) */
     h->acc_state = peaks || va.add ? ACC_ANY : ACC_UNREACHED;
@@ -1834,8 +1834,7 @@ struct hl_batch_ws {
     std::vector<size_t> pts_base;  /* each image's first point */
     std::vector<int> key_cap_i, tile_base, group_base, rho_min, R, ref_numrho;
     vote_plan plan;
-    size_t acc_zero;               /* d_acc is zero between calls: its cap_acc,
-                                      or 0 when it is not */
+    bool acc_zero;                 /* d_acc is zero between calls */
     std::vector<int2> chunks;
     std::vector<int> group_img;
 
@@ -1991,6 +1990,8 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
 
     /* device buffers */
     int rc;
+    if (b->cap_acc < sizeof(int32_t) * b->acc_ints)
+        b->acc_zero = false;   /* another buffer, also after a failed allocation */
     if ((!src &&
          ((rc = grow((void **)&b->d_pts, &b->cap_pts, sizeof(float2) * b->npts_cap)) !=
               HL_NO_ERROR ||
@@ -2223,9 +2224,9 @@ static int batch_run_ws(hl_handle *h, hl_batch_ws **pb, const hl_image_desc *img
         CK(cudaEventCreateWithFlags(&b->tab_read, cudaEventDisableTiming));
         b->tab_event = 1;
     }
-    if (b->acc_zero != b->cap_acc && !b->plan.add)   /* outside the (captured) pipeline */
+    if (!b->acc_zero && !b->plan.add)   /* outside the (captured) pipeline */
         CK(cudaMemsetAsync(b->d_acc, 0, b->cap_acc, s));
-    b->acc_zero = 0;
+    b->acc_zero = false;
     prof_mark(h, 0, s);
     if (!h->batch_graph || h->prof || src) {
         rc = batch_enqueue(h, b, nimg, K, s, src);
@@ -2272,7 +2273,7 @@ static int batch_run_ws(hl_handle *h, hl_batch_ws **pb, const hl_image_desc *img
         h->last_launches = 4;
     }
     if (rc == HL_NO_ERROR) {
-        b->acc_zero = b->plan.add ? 0 : b->cap_acc;   /* the tail clears what is stored */
+        b->acc_zero = !b->plan.add;   /* the tail clears what is stored */
         CK(cudaEventRecord(b->tab_read, s));
     }
     return rc;
@@ -2297,7 +2298,7 @@ static int batch_last_status(hl_handle *h, int *status, cudaStream_t s)
     CK(cudaStreamSynchronize(s));
     *status = st;
     if (st != 0)
-        b->acc_zero = 0;   /* a launch that gave up may have left bins */
+        b->acc_zero = false;   /* a launch that gave up may have left bins */
     return HL_NO_ERROR;
 }
 
@@ -2383,7 +2384,7 @@ extern "C" int hl_batch(hl_handle *h, const hl_image_desc *imgs, int nimg,
         CK(cudaMemcpyAsync(b->h_res, b->d_lines, lbytes, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     if (h_counts[nimg] != 0) {
-        b->acc_zero = 0;   /* a launch that gave up may have left bins */
+        b->acc_zero = false;   /* a launch that gave up may have left bins */
         return HL_CUDA_ERROR;
     }
     for (int i = 0; i < nimg; i++) {

@@ -15,6 +15,14 @@ def _image(w, h, seed=0):
     return img
 
 
+def _dirty(torch, nbytes, n):
+    """n freed blocks of about nbytes, full of ones."""
+    keep = [torch.full((nbytes // 4,), 1, dtype=torch.int32, device="cuda") for _ in range(n)]
+    torch.cuda.synchronize()
+    del keep
+    torch.cuda.empty_cache()
+
+
 def _too_large(hl):
     """A batch whose accumulators need 400 GB."""
     from opencuda_gb300 import _lib
@@ -35,3 +43,19 @@ def test_a_failed_allocation_is_reported_once(cuda):
     _too_large(hl)
     assert hl.setDeTheta(math.pi / 180) == 0 and hl.setDeRho(1.0) == 0
     assert hl.houghLine(dev, None, 16) == want
+
+
+def test_accumulators_after_a_failed_allocation(cuda):
+    """A batch that is too large, then the batch before it again: its accumulators
+    are as large as they were, and not the ones that were left zero."""
+    import torch
+    from opencuda_gb300.houghline import HoughLine, Image
+    dev = [Image.from_host(_image(500 + 30 * i, 640 - 20 * i, i)) for i in range(8)]
+    hl = HoughLine(detheta=math.pi / 180, threshold=40)
+    want = hl.houghLineBatch(dev, 32)
+    assert want[0] == 0 and hl.houghLineBatch(dev, 32) == want
+    _too_large(hl)
+    assert hl.setDeTheta(math.pi / 180) == 0 and hl.setDeRho(1.0) == 0
+    acc = sum(4 * hl.geometry(d.width, d.height).numrho * 192 for d in dev)
+    _dirty(torch, acc + acc // 4, 16)
+    assert hl.houghLineBatch(dev, 32) == want
