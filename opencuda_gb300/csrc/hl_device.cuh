@@ -218,11 +218,13 @@ __device__ __forceinline__ void diag_point(float x, float y, const DiagTab &t, f
     }
 }
 
-/* Notes bin idx of image img as a peak candidate; once the list is full (the
- * peak pass then scans every accumulator) a bin costs one load. */
+/* Notes bin idx of image img as a peak candidate; once the counter is past the
+ * list's room (the peak pass then scans every accumulator) a bin costs one load.  A
+ * full list alone does not end the noting: its counter would say that nothing is
+ * missing. */
 __device__ __forceinline__ void note_cand(const hl_cand_list &c, int img, unsigned idx)
 {
-    if (*(volatile int *)c.count >= c.cap)
+    if (*(volatile int *)c.count > c.cap)
         return;
     const int pos = atomicAdd(c.count, 1);
     if (pos < c.cap)
