@@ -2286,6 +2286,15 @@ static int batch_run(hl_handle *h, const hl_image_desc *imgs, int nimg,
     return batch_run_ws(h, &h->bw, imgs, nimg, thr, K, lines_dev, counts_dev, s);
 }
 
+/* Every reader of a batch's status word comes here: after an error (a launch that
+ * gave up) the accumulators are cleared before the next call relies on them. */
+static int batch_status(hl_batch_ws *b, int status)
+{
+    if (status != 0)
+        b->acc_zero = false;
+    return status;
+}
+
 static int batch_last_status(hl_handle *h, int *status, cudaStream_t s)
 {
     hl_batch_ws *b = h->bw;
@@ -2296,9 +2305,7 @@ static int batch_last_status(hl_handle *h, int *status, cudaStream_t s)
     int st = 0;
     CK(cudaMemcpyAsync(&st, b->d_cnt + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    *status = st;
-    if (st != 0)
-        b->acc_zero = false;   /* a launch that gave up may have left bins */
+    *status = batch_status(b, st);
     return HL_NO_ERROR;
 }
 
@@ -2383,10 +2390,8 @@ extern "C" int hl_batch(hl_handle *h, const hl_image_desc *imgs, int nimg,
     if (lbytes)
         CK(cudaMemcpyAsync(b->h_res, b->d_lines, lbytes, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    if (h_counts[nimg] != 0) {
-        b->acc_zero = false;   /* a launch that gave up may have left bins */
+    if (batch_status(b, h_counts[nimg]) != 0)
         return HL_CUDA_ERROR;
-    }
     for (int i = 0; i < nimg; i++) {
         const int c = std::max(0, std::min(h_counts[i], linesmax));
         counts[i] = c;
@@ -2765,7 +2770,7 @@ extern "C" int hl_proposal_batch(hl_handle *h, hl_net *net,
             }
         }
         CK(cudaStreamSynchronize(s));
-        if (fst != 0)
+        if (batch_status(h->bw_fb, fst) != 0)
             return HL_CUDA_ERROR;
         if (nj > 0 && K > 0) {
             for (int q = 0; q < ns; q++) {
