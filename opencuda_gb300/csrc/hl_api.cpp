@@ -459,7 +459,7 @@ struct vote_plan {
      * where a region has several windows (fine rho steps, HL_SLAB_PIXELS) or the
      * slabs would take more than HL_MAX_SCRATCH and twice the accumulators (images
      * of 32 K and more a side, or a handful of angles: a slab's column groups are
-     * as tall as their thetas lie apart).  Dense: the accumulator is cleared
+     * as tall as their thetas lie apart), or could not be allocated.  Dense: the accumulator is cleared
      * before and scanned after */
     int add;
 };
@@ -658,9 +658,9 @@ static void slab_groups(const hl_handle *h, const plan_img &im, const hl_vote_it
 }
 
 /* Plans the vote of n images with windows of at most cap rows on ctas
- * persistent CTAs. */
+ * persistent CTAs; slabs: there is memory for them. */
 static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int ctas,
-                     vote_plan *pl)
+                     bool slabs, vote_plan *pl)
 {
     const int slices = h->Tp / HL_SLICE;
     std::vector<slice_ext> ext;
@@ -695,7 +695,8 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
             }
         windows = in_windows < 0.75 * in_grids;
     }
-    pl->exact = pl->add = 0;
+    pl->exact = 0;
+    pl->add = !slabs;
     pl->part16 = 1;
     for (int i = 0; i < n; i++) {
         const int w = im[i].w, hh = im[i].h;
@@ -984,7 +985,7 @@ static int handle_plan(hl_handle *h, int w, int hh, int R, int rho_min, cudaStre
         if (h->acc_state == ACC_UNREACHED)
             h->acc_state = ACC_ANY;
         const plan_img im = {w, hh, R, rho_min};
-        int rc = make_plan(h, &im, 1, cap, std::max(h->sms, 1), h->plan);
+        int rc = make_plan(h, &im, 1, cap, std::max(h->sms, 1), true, h->plan);
         if (rc != HL_NO_ERROR)
             return rc;
         if ((rc = plan_upload(h, s)) != HL_NO_ERROR)
@@ -998,8 +999,17 @@ static int handle_plan(hl_handle *h, int w, int hh, int R, int rho_min, cudaStre
         h->plan_cap = cap;
         h->plan_thr = threads;
     }
-    int rc = grow((void **)&h->d_scratch, &h->cap_scratch,
-                  plan_scratch(*h->plan));
+    int rc = grow((void **)&h->d_scratch, &h->cap_scratch, plan_scratch(*h->plan));
+    if (rc == HL_OUT_OF_MEM && !h->plan->add) {
+        /* no room for the slabs: the form without them */
+        const plan_img im = {w, hh, R, rho_min};
+        h->plan_w = 0;
+        if ((rc = make_plan(h, &im, 1, cap, std::max(h->sms, 1), false, h->plan)) != HL_NO_ERROR ||
+            (rc = plan_upload(h, s)) != HL_NO_ERROR)
+            return rc;
+        h->plan_w = w;
+        rc = grow((void **)&h->d_scratch, &h->cap_scratch, plan_scratch(*h->plan));
+    }
     if (rc != HL_NO_ERROR)
         return rc;
     return grow((void **)&h->d_cand, &h->cap_cand,
@@ -1881,6 +1891,22 @@ static void batch_ws_free(hl_batch_ws *b)
 
 static size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
+/* the launch's grid and the places of its tables */
+static void batch_layout(const hl_handle *h, hl_batch_ws *b, int nimg)
+{
+    b->grid = std::max(1, std::min((int)b->plan.items.size(),
+                                   vote_ctas(h, b->plan.win_rows, b->threads)));
+    size_t o = 0;
+    b->off_cimg = o;   o = align16(o + sizeof(hl_compact_img) * nimg);
+    b->off_gimg = o;   o = align16(o + sizeof(int) * (size_t)b->ngroups);
+    b->off_vimg = o;   o = align16(o + sizeof(hl_vote_img) * nimg);
+    b->off_plan = o;   o = align16(o + plan_bytes(b->plan));
+    b->off_pimg = o;   o = align16(o + sizeof(hl_peak_img) * nimg);
+    b->off_chunks = o; o = align16(o + sizeof(int2) * b->chunks.size());
+    b->off_fimg = o;   o = align16(o + sizeof(hl_final_img) * nimg);
+    b->tab_bytes = o;
+}
+
 /* Plan a batch: sizes, offsets, work items, chunks; fills the pinned tables
  * (image pointers and thresholds included).  The geometry part is reused
  * when the sizes and the launch shape equal the previous call's.  src: the
@@ -1964,27 +1990,16 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
         }
         if (nimg > 0xffff)
             return HL_OP_OVERFLOW;
-        int rc = make_plan(h, pim.data(), nimg, cap, std::max(h->sms, 1), &b->plan);
+        int rc = make_plan(h, pim.data(), nimg, cap, std::max(h->sms, 1), true, &b->plan);
         if (rc != HL_NO_ERROR)
             return rc;
         b->ngroups = groups;
         b->ntiles = tiles;
         b->nchunks = (int)b->chunks.size();
-        b->grid = std::max(1, std::min((int)b->plan.items.size(),
-                                       vote_ctas(h, b->plan.win_rows, threads)));
         b->npts_cap = pts;
         b->acc_ints = acc;
         b->nkeys = keys;
-        /* table layout */
-        size_t o = 0;
-        b->off_cimg = o;   o = align16(o + sizeof(hl_compact_img) * nimg);
-        b->off_gimg = o;   o = align16(o + sizeof(int) * (size_t)groups);
-        b->off_vimg = o;   o = align16(o + sizeof(hl_vote_img) * nimg);
-        b->off_plan = o;   o = align16(o + plan_bytes(b->plan));
-        b->off_pimg = o;   o = align16(o + sizeof(hl_peak_img) * nimg);
-        b->off_chunks = o; o = align16(o + sizeof(int2) * b->chunks.size());
-        b->off_fimg = o;   o = align16(o + sizeof(hl_final_img) * nimg);
-        b->tab_bytes = o;
+        batch_layout(h, b, nimg);
         b->key = key;
     }
 
@@ -2004,9 +2019,23 @@ static int batch_plan(hl_handle *h, hl_batch_ws *b, const hl_image_desc *imgs,
                    sizeof(unsigned long long) * (65536 + b->acc_ints / 128))) != HL_NO_ERROR ||
         (rc = grow((void **)&b->d_keys, &b->cap_keys,
                    sizeof(unsigned long long) * b->nkeys)) != HL_NO_ERROR ||
-        (rc = grow((void **)&b->d_tab, &b->cap_tab, b->tab_bytes)) != HL_NO_ERROR ||
-        (rc = grow((void **)&b->d_scratch, &b->cap_scratch,
-                   plan_scratch(b->plan))) != HL_NO_ERROR)
+        (rc = grow((void **)&b->d_tab, &b->cap_tab, b->tab_bytes)) != HL_NO_ERROR)
+        return rc;
+    rc = grow((void **)&b->d_scratch, &b->cap_scratch, plan_scratch(b->plan));
+    if (rc == HL_OUT_OF_MEM && !b->plan.add) {
+        /* no room for the slabs: the form without them, whose tables are smaller */
+        std::vector<plan_img> pim((size_t)nimg);
+        for (int i = 0; i < nimg; i++)
+            pim[i] = {rois[i].w, rois[i].h, b->R[i], b->rho_min[i]};
+        b->key.clear();
+        if ((rc = make_plan(h, pim.data(), nimg, cap, std::max(h->sms, 1), false, &b->plan)) !=
+            HL_NO_ERROR)
+            return rc;
+        batch_layout(h, b, nimg);
+        b->key = key;
+        rc = grow((void **)&b->d_scratch, &b->cap_scratch, plan_scratch(b->plan));
+    }
+    if (rc != HL_NO_ERROR)
         return rc;
     if (b->cap_ncand < sizeof(int) * (size_t)nimg || !b->d_ncand) {
         if ((rc = grow((void **)&b->d_ncand, &b->cap_ncand, sizeof(int) * (size_t)nimg)) !=

@@ -59,3 +59,40 @@ def test_accumulators_after_a_failed_allocation(cuda):
     acc = sum(4 * hl.geometry(d.width, d.height).numrho * 192 for d in dev)
     _dirty(torch, acc + acc // 4, 16)
     assert hl.houghLineBatch(dev, 32) == want
+
+
+@pytest.mark.parametrize("n", [1, 2])
+def test_no_room_for_slabs(cuda, n):
+    """With memory for everything but the slabs of a split vote (over 100 MB),
+    the items add to the accumulator instead: four launches, the same lines."""
+    import torch
+    from opencuda_gb300.houghline import HoughLine, Image
+    g = torch.Generator(device="cuda").manual_seed(5)
+    buf = (torch.rand((8192, 8192), generator=g, device="cuda") < 0.002).to(torch.uint8) * 255
+    buf[2000, :] = 255
+    buf[:, 5000] = 255
+    dev = [Image(buf, (0, 0, 8192, 8192 - 100 * i)) for i in range(n)]
+
+    def call():
+        hl = HoughLine(detheta=math.pi / 32, threshold=1000)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        got = hl.houghLine(dev[0], None, 16) if n == 1 else hl.houghLineBatch(dev, 16)
+        torch.cuda.synchronize()
+        used = free - torch.cuda.mem_get_info()[0]
+        return got, used, hl.last_launch_count()
+
+    call()
+    want, used, launches = call()
+    assert want[0] == 0 and launches == (5 if n == 1 else 4)
+    torch.cuda.empty_cache()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - used + (60 << 20), dtype=torch.uint8,
+                      device="cuda")
+    try:
+        got, less, launches = call()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert got == want and launches == 4 and less < used
+    # with the memory back a new handle has its slabs again
+    assert call()[0] == want
