@@ -59,7 +59,7 @@ def _newer(target: Path, deps: list[Path]) -> bool:
 def build_library(force: bool = False, verbose: bool = False) -> Path:
     BUILD.mkdir(parents=True, exist_ok=True)
     out = BUILD / LIBNAME
-    headers = list(CSRC.glob("*.h")) + list(INCLUDE.glob("*.h"))
+    headers = list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + list(INCLUDE.glob("*.h"))
     srcs = [CSRC / s for s in CU_SOURCES + CXX_SOURCES + C_SOURCES
             if (CSRC / s).exists()]
     if not force and _newer(out, srcs + headers + [Path(__file__)]):
