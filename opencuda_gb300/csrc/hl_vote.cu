@@ -581,6 +581,7 @@ hl_vote_kernel(hl_vote_args a)
     const unsigned acc_base = smem_u32(s_acc);
     const f2x ir = f2_pack(a.irho, a.irho);
     unsigned seq = 0, nseg = 0, cpar = 0;
+    bool full = false;   /* the candidate list */
     while (true) {
         const int ds = (int)(nseg & 1u);
         if (!mbar_wait_ab(&sm.seg_full[ds], (nseg >> 1) & 1u, &sm.abort, a.status))
@@ -650,24 +651,29 @@ hl_vote_kernel(hl_vote_args a)
                  * them with each other): they go to the accumulator, which is
                  * zero otherwise, and onto the candidate list.  Four columns
                  * of a row a lane, as the window lies in shared memory. */
-                const int thr = max(g.thr, 0);
+                const int thr = max(g.thr, 0), n4 = nr * (HL_SLICE / 4);
                 int4 *w = reinterpret_cast<int4 *>(s_acc);
-                for (int i = 32 * cw + lane; i < nr * (HL_SLICE / 4); i += 32 * ncons) {
-                    const int4 v = w[i];
-                    w[i] = make_int4(0, 0, 0, 0);
+                for (int i0 = 32 * cw; i0 < n4; i0 += 32 * ncons) {
+                    const int i = i0 + lane, c = 4 * (i & 7);
+                    unsigned bits = 0;
+                    int4 v = make_int4(0, 0, 0, 0);
+                    if (i < n4) {
+                        v = w[i];
+                        w[i] = make_int4(0, 0, 0, 0);
+                    }
+                    const auto row = [&](int e) { return (i >> 3) + g.base[c + e] - g.rho_min; };
                     if (max(max(v.x, v.y), max(v.z, v.w)) > thr) {
                         const int x[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const int c = 4 * (i & 7) + e;
-                            const int r = (i >> 3) + g.base[c] - g.rho_min;
-                            if (x[e] > thr && g.k0 + c < a.T && (unsigned)r < (unsigned)g.R) {
-                                g.acc[(size_t)r * a.Tp + g.k0 + c] = x[e];
-                                note_cand(a.cand, g.img,
-                                          (unsigned)r * (unsigned)a.T + (unsigned)(g.k0 + c));
+                        for (int e = 0; e < 4; e++)
+                            if (x[e] > thr && g.k0 + c + e < a.T && (unsigned)row(e) < (unsigned)g.R) {
+                                g.acc[(size_t)row(e) * a.Tp + g.k0 + c + e] = x[e];
+                                bits |= 1u << e;
                             }
-                        }
                     }
+                    note_warp(a.cand, g.img, bits, full, [&](int e) {
+                        return (unsigned)row(e) * (unsigned)a.T + (unsigned)(g.k0 + c + e);
+                    });
                 }
             } else {
                 /* the whole accumulator is asked for: row by row, the shear
@@ -839,6 +845,7 @@ hl_merge_kernel(hl_merge_args a)
         return;
     }
     const int thr = max(im.threshold, 0);
+    unsigned bits = 0;   /* bit 2 u + e */
 #pragma unroll
     for (int u = 0; u < 4; u++)
         if (max(v[0][u], v[1][u]) > thr && 4 * rg + u < R)
@@ -846,9 +853,12 @@ hl_merge_kernel(hl_merge_args a)
             for (int e = 0; e < 2; e++)
                 if (v[e][u] > thr && (e ? k1v : k0v)) {
                     dst[(size_t)(4 * rg + u) * a.Tp + e] = v[e][u];
-                    note_cand(a.cand, blk.img,
-                              (unsigned)(4 * rg + u) * (unsigned)a.T + (unsigned)(k + e));
+                    bits |= 1u << (2 * u + e);
                 }
+    bool full = false;
+    note_warp(a.cand, blk.img, bits, full, [&](int b) {
+        return (unsigned)(4 * rg + (b >> 1)) * (unsigned)a.T + (unsigned)(k + (b & 1));
+    });
 }
 
 cudaError_t hl_launch_merge(const hl_merge_args *a, cudaStream_t s)
