@@ -437,16 +437,27 @@ extern "C" int hl_last_launch_count(const hl_handle *h)
  * then cost more than its votes.  1913 x 1077, T = 360: 64 K, 128 K, 192 K pixels
  * 45.6, 45.5, 43.1 us; 2048 x 2048, T = 360, lines drawn: 72.6, 73.6, 67.9 us. */
 #define HL_MIN_REGION (192.0 * 1024.0)
-/* At rho steps below 1 regions of one window get small and the rows that they
- * store many; a stored and merged row costs about this many pixels then (16 images
- * of 1000 x 900, T = 180, step 0.1: 32 M rows, 1.5 ms).  If regions of several
- * windows come to less than three quarters of that over a launch, they are taken.
- * A call, T = 180, with one window a region in brackets: 16 images of 1000 x 900,
- * step 0.1 1380 us (1724), 0.05 2121 (3421); one of 2048 x 2048, 0.1 359 (497),
- * 0.05 462 (743).  At 0.25 one window is the cheaper: 222 us for the 16 images, 711
- * with several. */
-#define HL_SLAB_PIXELS 384.0
-#define HL_CLIP_COST 2.5
+/* A block may also be voted in windows: an item votes the image's points that may
+ * reach its rows, and each window is final.  It needs no slabs and no merge, but
+ * tests every vote and votes a point once a window that its tile may reach.  It is
+ * the form for rho steps below 1, whose regions get small and store many rows, and
+ * for launches too small to be worth a merge.  Windows that outweigh a CTA's share
+ * are split into parts of their points, which go through slabs like regions.
+ * The form is chosen by estimates in pixels as above.  A tested vote costs
+ * HL_WINDOW_VOTE plain ones, an item's start and end HL_ITEM_PIXELS, a row of a slab
+ * HL_SLAB_PIXELS more than another row, a merge launch HL_MERGE_PIXELS: fitted to
+ * single images and batches of 512 x 512 to 4096 x 4096 at steps 1 to 0.05 in every
+ * form.  At rho steps from 1 on only launches of less than HL_SMALL_PIXELS and two
+ * blocks a CTA are looked at: in others regions win.
+ * T = 180, a call by fixed windows of rows, which this replaced / by regions alone /
+ * now: 16 images of 1000 x 900, step 0.1 229 / 1368 / 193 us, 0.05 380 / 2088 / 287,
+ * 0.25 149 / 217 / 139; one of 2048 x 2048, 0.1 95 / 362 / 113, 0.05 142 / 467 / 122;
+ * 512 x 512, 0.1 45 / 171 / 48; 16 of 512 x 512, step 1 58 / 66 / 58. */
+#define HL_WINDOW_VOTE 2.0
+#define HL_ITEM_PIXELS 120e3
+#define HL_SLAB_PIXELS 100.0
+#define HL_MERGE_PIXELS 60e3
+#define HL_SMALL_PIXELS 400e3
 
 struct vote_plan {
     std::vector<hl_vote_item> items;
@@ -454,10 +465,9 @@ struct vote_plan {
     std::vector<hl_slab> slabs;
     long long scratch_units;   /* row groups of slabs */
     unsigned chunks;           /* of a merge launch */
-    int part16, win_rows, exact;
+    int part16, win_rows, exact, win;
     /* the blocks' items add to the accumulator instead of going through slabs:
-     * where a region has several windows (fine rho steps, HL_SLAB_PIXELS) or the
-     * slabs would take more than HL_MAX_SCRATCH and twice the accumulators (images
+     * where these would take more than HL_MAX_SCRATCH and twice the accumulators (images
      * of 32 K and more a side, or a handful of angles: a slab's column groups are
      * as tall as their thetas lie apart), or could not be allocated.  Dense: the accumulator is cleared
      * before and scanned after */
@@ -505,16 +515,13 @@ struct plan_region {
     int blk;
 };
 
-/* the grid of regions of one (image, slice): nx x ny; nwin windows each (more
- * than one only where a single tile needs it) */
-static void best_grid(const slice_ext &e, int w, int hh, int cap, double n_min, int *bx, int *by,
-                      int *nwin)
+/* the grid of regions of one (image, slice): nx x ny; false where not even a tile's
+ * rows fit a window */
+static bool best_grid(const slice_ext &e, int w, int hh, int cap, double n_min, int *bx, int *by)
 {
     const int tx = (w + HL_TILE_W - 1) / HL_TILE_W, ty = (hh + HL_TILE_H - 1) / HL_TILE_H;
     double best = 1e300;
-    *bx = tx;
-    *by = ty;
-    *nwin = 0;
+    bool found = false;
     for (int nx = 1; nx <= tx; nx++) {
         const int gtx = (tx + nx - 1) / nx;
         if (nx > 1 && gtx == (tx + nx - 2) / (nx - 1))
@@ -539,46 +546,66 @@ static void best_grid(const slice_ext &e, int w, int hh, int cap, double n_min, 
             best = cost;
             *bx = nx;
             *by = ny;
-            *nwin = 1;
+            found = true;
         }
-        if (nx > 4.0 * n_min + 8 && *nwin)
+        if (nx > 4.0 * n_min + 8 && found)
             break;
     }
-    if (!*nwin)   /* one tile a region, several windows */
-        *nwin = (int)ceil(region_rows(e, std::min(w, HL_TILE_W), std::min(hh, HL_TILE_H)) / cap);
+    return found;
 }
 
-/* The same with several windows a region where that is cheaper: every window
- * tests all votes of its region (HL_CLIP_COST plain votes each), rows are stored
- * once a region.  Returns the cost in pixels; *grid is best_grid's. */
-static double window_grid(const slice_ext &e, int w, int hh, int cap, double n_min, int *bx,
-                          int *by, int *nwin, double *grid)
+/* The band of rows of one (image, slice) that windows share out, and what
+ * hl_vote_item needs of it.  Relative to the centre's at the same theta a point's rho
+ * is u cos d + v sin d, u and v its distances from the centre across and along the
+ * middle theta's lines, d the angle to the middle. */
+struct plan_band {
+    int first;                /* off0 of the first window; the last one ends at -first */
+    double out, tang;         /* pixels that a window's ends are moved outwards */
+    double a, b, reach;       /* half widths of u's two parts; tang times the mean |v| */
+};
+static plan_band block_band(const hl_handle *h, int w, int hh, int sl)
 {
-    const int tx = (w + HL_TILE_W - 1) / HL_TILE_W, ty = (hh + HL_TILE_H - 1) / HL_TILE_H;
-    const auto cost = [&](int nx, int ny, int nw) {
-        const double gw = std::min(((tx + nx - 1) / nx) * HL_TILE_W, w);
-        const double gh = std::min(((ty + ny - 1) / ny) * HL_TILE_H, hh);
-        return (double)nx * ny * (gw * gh * nw * (nw > 1 ? HL_CLIP_COST : 1.0) +
-                                  HL_SLAB_PIXELS * std::min(region_rows(e, gw, gh),
-                                                            (double)nw * cap));
-    };
-    best_grid(e, w, hh, cap, n_min, bx, by, nwin);
-    double best = *grid = cost(*bx, *by, *nwin);
-    for (int nx = 1; nx <= std::min(tx, 8); nx *= 2)
-        for (int ny = 1; ny <= std::min(ty, 16); ny *= 2) {
-            if (nx > 1 && (ty + ny - 1) / ny > HL_VOTE_RUNS)
-                continue;
-            const double gw = std::min(((tx + nx - 1) / nx) * HL_TILE_W, w);
-            const double gh = std::min(((ty + ny - 1) / ny) * HL_TILE_H, hh);
-            const int nw = (int)ceil(region_rows(e, gw, gh) / cap);
-            if (cost(nx, ny, nw) < best) {
-                best = cost(nx, ny, nw);
-                *bx = nx;
-                *by = ny;
-                *nwin = nw;
-            }
-        }
-    return best;
+    const int k0 = sl * HL_SLICE, k1 = std::min(k0 + HL_SLICE, h->T) - 1;
+    const int km = std::min(k0 + HL_SLICE / 2, h->T - 1);
+    const double irho = 1.0 / h->p.derho;
+    const double x = 0.5 * w, y = 0.5 * hh;
+    double half = 0.0, tile = 0.0;   /* pixels across that the image and a tile reach */
+    for (int k = k0; k <= k1; k++) {
+        const double c = fabs((double)h->h_cos[k]), s = fabs((double)h->h_sin[k]);
+        half = std::max(half, x * c + y * s);
+        tile = std::max(tile, 0.5 * HL_TILE_W * c + 0.5 * HL_TILE_H * s);
+    }
+    /* rows for the centre's floor, the votes' truncation, floats */
+    const double slack = 4.0 + sqrt(4.0 * (x * x + y * y)) * irho * (1.0 / (1 << 19));
+    const double d = std::max(k1 - km, km - k0) * h->p.detheta;
+    const double c = fabs((double)h->h_cos[km]), s = fabs((double)h->h_sin[km]);
+    plan_band p;
+    p.first = -(int)ceil(half * irho + slack);
+    /* the curvature: a tile's centre lies up to a tile outside the image */
+    p.out = tile + (1.0 - cos(std::min(d, M_PI))) * ((x + HL_TILE_W) * c + (y + HL_TILE_H) * s) +
+            2.0 + slack * h->p.derho;
+    p.tang = d < 0.5 * M_PI ? sin(d) : 1.0;
+    p.a = x * c;
+    p.b = y * s;
+    p.reach = p.tang * 0.5 * (x * s + y * c);
+    return p;
+}
+/* its windows of at most cap rows: their number; *rows: rows of one */
+static int band_windows(const plan_band &p, int cap, int *rows)
+{
+    const int total = 1 - 2 * p.first, n = (total + cap - 1) / cap;
+    *rows = (total + n - 1) / n;
+    return n;
+}
+
+/* the part of a rectangle's area that lies below u = v: u is the sum of two uniform
+ * distances, in [-a, a] and [-b, b] */
+static double area_below(double a, double b, double v)
+{
+    a = std::max(a, 1e-3);
+    b = std::max(b, 1e-3);
+    const auto sq = [](double t) { return t > 0.0 ? t * t : 0.0; };
+    return (sq(v + a + b) - sq(v + a - b) - sq(v - a + b) + sq(v - a - b)) / (8.0 * a * b);
 }
 
 /* The item of a whole w x hh image whose range exceeds the window, voted with a
@@ -616,6 +643,19 @@ static bool slide_item(const hl_handle *h, const slice_ext &e, int w, int hh, in
     return it->nseg > 1;
 }
 
+/* column group g holds the rows r0 to r1 of R4 groups of four */
+static void slab_rows(hl_slab *sl, int g, double r0, double r1, int R4)
+{
+    const int b = (int)std::min(std::max(floor(r0 / 4.0), 0.0), (double)R4);
+    const int e = (int)std::min(std::max(floor(r1 / 4.0) + 1.0, (double)b), (double)R4);
+    sl->b[g] = b;
+    sl->n[g] = e - b;
+    if (e > b) {
+        sl->lo = std::min(sl->lo, b);
+        sl->hi = std::max(sl->hi, e);
+    }
+}
+
 /* The rows that the votes of an item's four column groups can fall into, in
  * groups of four rows (sl's b, n, lo and hi).  A corner's rho is a sinusoid over
  * the group's thetas: no lower than at its ends less the distance times 1 -
@@ -645,31 +685,108 @@ static void slab_groups(const hl_handle *h, const plan_img &im, const hl_vote_it
         }
         const double half = std::min(0.5 * (k1 - k0) * h->p.detheta, M_PI);
         const double slack = far * (1.0 - cos(half)) + far * (1.0 / (1 << 20)) + 1.0;
-        const double r0 = floor(lo - slack) - im.rho_min, r1 = ceil(hi + slack) - im.rho_min;
-        const int b = (int)std::min(std::max(floor(r0 / 4.0), 0.0), (double)R4);
-        const int e = (int)std::min(std::max(floor(r1 / 4.0) + 1.0, (double)b), (double)R4);
-        sl->b[g] = b;
-        sl->n[g] = e - b;
-        if (e > b) {
-            sl->lo = std::min(sl->lo, b);
-            sl->hi = std::max(sl->hi, e);
-        }
+        slab_rows(sl, g, floor(lo - slack) - im.rho_min, ceil(hi + slack) - im.rho_min, R4);
     }
 }
 
-/* Plans the vote of n images with windows of at most cap rows on ctas
- * persistent CTAs; slabs: there is memory for them. */
-static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int ctas,
-                     bool slabs, vote_plan *pl)
+/* the same for an item of one window: the rows that its columns hold (a row and 2^-20
+ * of the value more for the device's floats) */
+static void window_groups(const hl_handle *h, const plan_img &im, const hl_vote_item &it,
+                          hl_slab *sl)
+{
+    const double irho = 1.0 / h->p.derho, x = 0.5 * (im.w - 1), y = 0.5 * (im.h - 1);
+    const double slack = sqrt(x * x + y * y) * irho * (1.0 / (1 << 20)) + 2.0;
+    const int R4 = (im.R + 3) / 4;
+    sl->lo = 0x7fffffff;
+    sl->hi = 0;
+    for (int g = 0; g < 4; g++) {
+        double lo = 1e300, hi = -1e300;
+        for (int c = 0; c < 8; c++) {
+            const int k = std::min(it.slice * HL_SLICE + 8 * g + c, h->T - 1);
+            const double v = (x * (double)h->h_cos[k] + y * (double)h->h_sin[k]) * irho;
+            lo = std::min(lo, v);
+            hi = std::max(hi, v);
+        }
+        slab_rows(sl, g, floor(lo - slack) + it.off0 - im.rho_min,
+                  ceil(hi + slack) + it.off0 + it.adv - im.rho_min, R4);
+    }
+}
+
+/* pixels of window j of rows rows */
+static double window_weight(const hl_handle *h, const plan_band &p, double area, int j, int rows)
+{
+    const double lo = (p.first + (double)j * rows) * h->p.derho - p.out - p.reach;
+    const double hi = (p.first + (double)(j + 1) * rows) * h->p.derho + p.out + p.reach;
+    return area * HL_WINDOW_VOTE * (area_below(p.a, p.b, hi) - area_below(p.a, p.b, lo)) +
+           HL_ROW_PIXELS * rows;
+}
+/* parts of a window's points, of target pixels at most (0: any) */
+static int window_parts(double wt, double target)
+{
+    return target > 0.0 ? (int)std::min(64.0, std::max(1.0, ceil(wt / target))) : 1;
+}
+
+/* The items of one block's windows. */
+static void block_windows(const hl_handle *h, const plan_img &im, int img, int sl, int cap,
+                          double target, std::vector<plan_region> &reg)
+{
+    const plan_band p = block_band(h, im.w, im.h, sl);
+    const int tx = (im.w + HL_TILE_W - 1) / HL_TILE_W, ty = (im.h + HL_TILE_H - 1) / HL_TILE_H;
+    int rows;
+    const int n = band_windows(p, cap, &rows);
+    for (int j = 0; j < n; j++) {
+        plan_region r;
+        memset(&r.it, 0, sizeof(r.it));
+        r.it.img = img;
+        r.it.slice = sl;
+        r.it.tx = tx << 16;
+        r.it.ty = ty << 16;
+        r.it.slab = -1;
+        r.it.win = 1;
+        r.it.nseg = (ty + HL_VOTE_RUNS / 2 - 1) / (HL_VOTE_RUNS / 2);
+        r.it.adv = rows;
+        r.it.off0 = p.first + j * rows;
+        r.it.lo = (float)(r.it.off0 * h->p.derho - p.out);
+        r.it.hi = (float)((r.it.off0 + rows) * h->p.derho + p.out);
+        r.it.tang = (float)p.tang;
+        r.blk = img * (h->Tp / HL_SLICE) + sl;
+        r.wt = window_weight(h, p, (double)im.w * im.h, j, rows);
+        r.it.nparts = window_parts(r.wt, target);
+        r.wt /= r.it.nparts;
+        for (r.it.part = 0; r.it.part < r.it.nparts; r.it.part++)
+            reg.push_back(r);
+    }
+}
+
+static bool heavier(const plan_region &a, const plan_region &c) { return a.wt > c.wt; }
+
+/* A list schedule of the items, heaviest first: when each starts; the end. */
+static double plan_schedule(std::vector<plan_region> &reg, int ctas, std::vector<double> &start)
+{
+    std::stable_sort(reg.begin(), reg.end(), heavier);
+    std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+    double makespan = 0.0;
+    start.resize(reg.size());
+    for (size_t i = 0; i < reg.size(); i++) {
+        start[i] = 0.0;
+        if ((int)i >= std::max(ctas, 1)) {
+            start[i] = free_at.top();
+            free_at.pop();
+        }
+        makespan = std::max(makespan, start[i] + reg[i].wt);
+        free_at.push(start[i] + reg[i].wt);
+    }
+    return makespan;
+}
+
+/* The plan of regions: whole images where they fit a window or can slide and weigh
+ * no more than a CTA's share, else grids of regions (windows where not even a tile's
+ * rows fit one). */
+static void plan_regions(const hl_handle *h, const plan_img *im, int n, int cap, int ctas,
+                           const std::vector<slice_ext> &ext, double total,
+                           std::vector<plan_region> &reg)
 {
     const int slices = h->Tp / HL_SLICE;
-    std::vector<slice_ext> ext;
-    slice_extents(h, ext);
-    double total = 0.0;
-    for (int i = 0; i < n; i++)
-        for (int sl = 0; sl < slices; sl++)
-            total += (double)im[i].w * im[i].h +
-                     HL_ROW_PIXELS * std::min(region_rows(ext[sl], im[i].w, im[i].h), 4.0 * cap);
     const double wcap = std::max(total / (HL_PLAN_SHARE * std::max(ctas, 1)), HL_MIN_REGION);
     /* A block heavier than that is one item all the same, one such a CTA, if it is
      * no more than a CTA's share: the rest, split, fill what is left.  A whole block
@@ -677,32 +794,9 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
      * instead of 278 and 50 with every block in two or more regions. */
     const double share = total / std::max(ctas, 1);
     int big = 0;
-    std::vector<plan_region> reg;
-    bool slides = false;
-    bool windows = false;   /* several a region: see HL_SLAB_PIXELS */
-    if (h->p.derho < 1.0) {
-        double in_windows = 0.0, in_grids = 0.0;
-        for (int i = 0; i < n; i++)
-            for (int sl = 0; sl < slices; sl++) {
-                const double n_min = std::max(1.0, ceil((double)im[i].w * im[i].h / wcap));
-                hl_vote_item it;
-                int nx, ny, nw;
-                double g;
-                if (n_min <= 1.0 && slide_item(h, ext[sl], im[i].w, im[i].h, sl, cap, &it))
-                    continue;
-                in_windows += window_grid(ext[sl], im[i].w, im[i].h, cap, n_min, &nx, &ny, &nw, &g);
-                in_grids += g;
-            }
-        windows = in_windows < 0.75 * in_grids;
-    }
-    pl->exact = 0;
-    pl->add = !slabs;
-    pl->part16 = 1;
     for (int i = 0; i < n; i++) {
         const int w = im[i].w, hh = im[i].h;
         const int tx = (w + HL_TILE_W - 1) / HL_TILE_W, ty = (hh + HL_TILE_H - 1) / HL_TILE_H;
-        if (im[i].R >= (1 << 22))
-            pl->exact = 1;
         for (int sl = 0; sl < slices; sl++) {
             double n_min = std::max(1.0, ceil((double)w * hh / wcap));
             hl_vote_item whole;
@@ -720,96 +814,246 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
                 r.blk = i * slices + sl;
                 r.wt = (double)w * hh + HL_ROW_PIXELS * region_rows(ext[sl], w, hh);
                 reg.push_back(r);
-                slides = true;
                 continue;
             }
-            int nx, ny, nw;
-            double grid;
-            if (windows)
-                window_grid(ext[sl], w, hh, cap, n_min, &nx, &ny, &nw, &grid);
-            else
-                best_grid(ext[sl], w, hh, cap, n_min, &nx, &ny, &nw);
-            const bool clip = nw > 1;
-            pl->add |= clip;
+            int nx, ny;
+            if (!best_grid(ext[sl], w, hh, cap, n_min, &nx, &ny)) {
+                block_windows(h, im[i], i, sl, cap, 0.0, reg);
+                continue;
+            }
             for (int y = 0; y < ny; y++)
                 for (int x = 0; x < nx; x++) {
                     const int x0 = tx * x / nx, x1 = tx * (x + 1) / nx;
                     const int y0 = ty * y / ny, y1 = ty * (y + 1) / ny;
                     const double gw = std::min(x1 * HL_TILE_W, w) - x0 * HL_TILE_W;
                     const double gh = std::min(y1 * HL_TILE_H, hh) - y0 * HL_TILE_H;
-                    for (int v = 0; v < nw; v++) {
-                        plan_region r;
-                        memset(&r.it, 0, sizeof(r.it));
-                        r.it.img = i;
-                        r.it.slice = sl;
-                        r.it.tx = x0 | ((x1 - x0) << 16);
-                        r.it.ty = y0 | ((y1 - y0) << 16);
-                        r.it.win = v;
-                        r.it.clip = clip;
-                        r.it.nseg = 1;
-                        r.blk = i * slices + sl;
-                        /* a region that the slice's rho 0 crosses votes by the
-                         * sign of each vote, about 1.4 times the time */
-                        const int k0 = sl * HL_SLICE, k1 = std::min(k0 + HL_SLICE, h->T) - 1;
-                        const bool mixed = h->h_cos[k1] < 0.0f &&
-                                           (x0 * h->h_cos[k0] * HL_TILE_W +
-                                                y1 * h->h_sin[k0] * HL_TILE_H > 0.0f) &&
-                                           (x1 * h->h_cos[k1] * HL_TILE_W +
-                                                y0 * h->h_sin[k1] * HL_TILE_H < 0.0f);
-                        r.wt = gw * gh * (mixed ? 1.4 : 1.0) +
-                               HL_ROW_PIXELS * std::min(region_rows(ext[sl], gw, gh), (double)cap);
-                        reg.push_back(r);
-                    }
+                    plan_region r;
+                    memset(&r.it, 0, sizeof(r.it));
+                    r.it.img = i;
+                    r.it.slice = sl;
+                    r.it.tx = x0 | ((x1 - x0) << 16);
+                    r.it.ty = y0 | ((y1 - y0) << 16);
+                    r.it.nseg = 1;
+                    r.blk = i * slices + sl;
+                    /* a region that the slice's rho 0 crosses votes by the
+                     * sign of each vote, about 1.4 times the time */
+                    const int k0 = sl * HL_SLICE, k1 = std::min(k0 + HL_SLICE, h->T) - 1;
+                    const bool mixed = h->h_cos[k1] < 0.0f &&
+                                       (x0 * h->h_cos[k0] * HL_TILE_W +
+                                            y1 * h->h_sin[k0] * HL_TILE_H > 0.0f) &&
+                                       (x1 * h->h_cos[k1] * HL_TILE_W +
+                                            y0 * h->h_sin[k1] * HL_TILE_H < 0.0f);
+                    r.wt = gw * gh * (mixed ? 1.4 : 1.0) +
+                           HL_ROW_PIXELS * region_rows(ext[sl], gw, gh);
+                    reg.push_back(r);
                 }
         }
     }
-    const auto heavier = [](const plan_region &a, const plan_region &c) { return a.wt > c.wt; };
-    std::stable_sort(reg.begin(), reg.end(), heavier);
-    {
-        /* the late starters of a list schedule, halved along their longer side */
-        typedef std::pair<double, int> slot_t;
-        std::priority_queue<slot_t, std::vector<slot_t>, std::greater<slot_t>> free_at;
-        for (int c = 0; c < std::max(ctas, 1); c++)
-            free_at.push({0.0, c});
-        std::vector<double> start(reg.size());
-        double makespan = 0.0;
-        for (size_t i = 0; i < reg.size(); i++) {
-            slot_t f = free_at.top();
-            free_at.pop();
-            start[i] = f.first;
-            makespan = std::max(makespan, f.first + reg[i].wt);
-            free_at.push({f.first + reg[i].wt, f.second});
+    /* the late starters of a list schedule, halved along their longer side */
+    std::vector<double> start;
+    double makespan = plan_schedule(reg, ctas, start);
+    const size_t n0 = reg.size();
+    for (size_t i = 0; i < n0; i++) {
+        plan_region r = reg[i];
+        if (!(start[i] > 0.6 * makespan && r.wt > 0.25 * wcap && r.wt >= 2.0 * HL_MIN_REGION &&
+              !r.it.win && r.it.nseg == 1))
+            continue;
+        const int txn = r.it.tx >> 16, tyn = r.it.ty >> 16;
+        plan_region a = r, b = r;
+        if (txn * HL_TILE_W >= tyn * HL_TILE_H && txn > 1 && tyn <= HL_VOTE_RUNS) {
+            const int x0 = r.it.tx & 0xffff, m = txn / 2;
+            a.it.tx = x0 | (m << 16);
+            b.it.tx = (x0 + m) | ((txn - m) << 16);
+        } else if (tyn > 1) {
+            const int y0 = r.it.ty & 0xffff, m = tyn / 2;
+            a.it.ty = y0 | (m << 16);
+            b.it.ty = (y0 + m) | ((tyn - m) << 16);
+        } else {
+            continue;
         }
-        const size_t n0 = reg.size();
-        for (size_t i = 0; i < n0; i++) {
-            plan_region r = reg[i];
-            if (!(start[i] > 0.6 * makespan && r.wt > 0.25 * wcap && r.wt >= 2.0 * HL_MIN_REGION &&
-                  !r.it.clip && r.it.nseg == 1))
-                continue;
-            const int txn = r.it.tx >> 16, tyn = r.it.ty >> 16;
-            plan_region a = r, b = r;
-            if (txn * HL_TILE_W >= tyn * HL_TILE_H && txn > 1 && tyn <= HL_VOTE_RUNS) {
-                const int x0 = r.it.tx & 0xffff, m = txn / 2;
-                a.it.tx = x0 | (m << 16);
-                b.it.tx = (x0 + m) | ((txn - m) << 16);
-            } else if (tyn > 1) {
-                const int y0 = r.it.ty & 0xffff, m = tyn / 2;
-                a.it.ty = y0 | (m << 16);
-                b.it.ty = (y0 + m) | ((tyn - m) << 16);
-            } else {
-                continue;
-            }
-            a.wt = b.wt = 0.6 * r.wt;
-            reg[i] = a;
-            reg.push_back(b);
-        }
+        a.wt = b.wt = 0.6 * r.wt;
+        reg[i] = a;
+        reg.push_back(b);
     }
     std::stable_sort(reg.begin(), reg.end(), heavier);
+}
+
+/* The plan of windows of at most cap rows, blocks that fit one whole. */
+static void plan_in_windows(const hl_handle *h, const plan_img *im, int n, int cap, double target,
+                            const std::vector<slice_ext> &ext, std::vector<plan_region> &reg)
+{
+    const int slices = h->Tp / HL_SLICE;
+    for (int i = 0; i < n; i++)
+        for (int sl = 0; sl < slices; sl++) {
+            const double rows = region_rows(ext[sl], im[i].w, im[i].h);
+            if (rows > cap) {
+                block_windows(h, im[i], i, sl, cap, target, reg);
+                continue;
+            }
+            plan_region r;
+            memset(&r.it, 0, sizeof(r.it));
+            r.it.img = i;
+            r.it.slice = sl;
+            r.it.tx = ((im[i].w + HL_TILE_W - 1) / HL_TILE_W) << 16;
+            r.it.ty = ((im[i].h + HL_TILE_H - 1) / HL_TILE_H) << 16;
+            r.it.nseg = 1;
+            r.blk = i * slices + sl;
+            r.wt = (double)im[i].w * im[i].h + HL_ROW_PIXELS * rows;
+            reg.push_back(r);
+        }
+    std::stable_sort(reg.begin(), reg.end(), heavier);
+}
+
+/* Pixels that a launch of items of these weights takes: its heaviest item, a CTA's
+ * share (items do not share out evenly) or, in a list schedule of a little more items
+ * than CTAs, the first two on one CTA; and the slabs' rows. */
+static double plan_length(std::vector<double> &wt, double sum, double most, double slab_rows,
+                          int ctas)
+{
+    ctas = std::max(ctas, 1);
+    double len = std::max(1.1 * (sum + HL_ITEM_PIXELS * (double)wt.size()) / ctas,
+                          most + HL_ITEM_PIXELS);
+    if ((int)wt.size() > ctas) {
+        std::nth_element(wt.begin(), wt.begin() + ctas, wt.end(), std::greater<double>());
+        len = std::max(len, 2.0 * (wt[(size_t)ctas] + HL_ITEM_PIXELS));
+    }
+    return len + (slab_rows > 0.0 ? HL_MERGE_PIXELS : 0.0) + slab_rows * HL_SLAB_PIXELS / ctas;
+}
+
+/* Is a plan of windows the shorter one?  *cap: the windows' rows at most, in and out;
+ * *target: pixels of a part at most, 0 for whole windows. */
+static bool windows_win(const hl_handle *h, const plan_img *im, int n, int ctas,
+                        const std::vector<slice_ext> &ext, double total, int *cap, double *target)
+{
+    const int slices = h->Tp / HL_SLICE;
+    const double wcap = std::max(total / (HL_PLAN_SHARE * std::max(ctas, 1)), HL_MIN_REGION);
+    double sum = 0.0, most = 0.0, slab_rows = 0.0, best = 1e300;
+    bool grid = true, win = false;
+    std::vector<double> wt, part;
+    for (int i = 0; i < n && grid; i++)
+        for (int sl = 0; sl < slices && grid; sl++) {
+            const double area = (double)im[i].w * im[i].h;
+            int nx = 1, ny = 1;
+            hl_vote_item it;
+            if (!(area <= wcap && slide_item(h, ext[sl], im[i].w, im[i].h, sl, *cap, &it)))
+                grid = best_grid(ext[sl], im[i].w, im[i].h, *cap,
+                                 std::max(1.0, ceil(area / wcap)), &nx, &ny);
+            const double rows = region_rows(ext[sl], (double)im[i].w / nx, (double)im[i].h / ny);
+            const double w = area / (nx * ny) + HL_ROW_PIXELS * rows;
+            wt.insert(wt.end(), (size_t)nx * ny, w);
+            sum += nx * ny * w;
+            most = std::max(most, w);
+            slab_rows += nx * ny > 1 ? nx * ny * rows : 0.0;
+        }
+    if (grid)
+        best = plan_length(wt, sum, most, slab_rows, ctas);
+    std::vector<plan_band> band;
+    for (int i = 0; i < n; i++)
+        for (int sl = 0; sl < slices; sl++)
+            band.push_back(block_band(h, im[i].w, im[i].h, sl));
+    for (int c = *cap, top = *cap, worse = 0; c >= 128 && worse < 2; c = c * 2 / 3) {
+        wt.clear();
+        sum = most = 0.0;
+        for (int i = 0; i < n; i++)
+            for (int sl = 0; sl < slices; sl++) {
+                const plan_band &b = band[(size_t)(i * slices + sl)];
+                const double area = (double)im[i].w * im[i].h;
+                const double whole = region_rows(ext[sl], im[i].w, im[i].h);
+                int rows = 0;
+                const int nw = whole > c ? band_windows(b, c, &rows) : 1;
+                for (int j = 0; j < nw; j++) {
+                    wt.push_back(rows ? window_weight(h, b, area, j, rows)
+                                      : area + HL_ROW_PIXELS * whole);
+                    sum += wt.back();
+                    most = std::max(most, wt.back());
+                }
+            }
+        /* whole, then in parts: every item of a block that has any goes through slabs */
+        const double share = std::max(sum / std::max(ctas, 1), 0.5 * HL_MIN_REGION);
+        bool better = false;
+        for (double f : {0.0, 2.0, 1.5, 1.0}) {
+            if (f > 0.0 && most <= f * share)
+                continue;
+            part.clear();
+            slab_rows = 0.0;
+            double heaviest = 0.0;
+            size_t at = 0;
+            for (int i = 0; i < n; i++)
+                for (int sl = 0; sl < slices; sl++) {
+                    const double whole = region_rows(ext[sl], im[i].w, im[i].h);
+                    /* a slab's groups of eight columns are as tall as these lie apart */
+                    const double apart = 0.5 * sqrt((double)im[i].w * im[i].w +
+                                                    (double)im[i].h * im[i].h) *
+                                         std::min(7.0 * h->p.detheta, 1.0) / h->p.derho;
+                    int rows = 0;
+                    const int nw = whole > c ? band_windows(band[(size_t)(i * slices + sl)], c, &rows)
+                                             : 1;
+                    const size_t before = part.size();
+                    for (int j = 0; j < nw; j++, at++) {
+                        const int np = rows ? window_parts(wt[at], f * share) : 1;
+                        part.insert(part.end(), (size_t)np, wt[at] / np);
+                        heaviest = std::max(heaviest, wt[at] / np);
+                    }
+                    const size_t items = part.size() - before;
+                    slab_rows += items > (size_t)nw ? (double)items * (rows + apart) : 0.0;
+                }
+            const double len = plan_length(part, sum, heaviest, slab_rows, ctas);
+            if (len < best) {
+                best = len;
+                *cap = c;
+                *target = f * share;
+                win = better = true;
+            }
+        }
+        worse = better || c == top ? 0 : worse + 1;
+    }
+    return win;
+}
+
+/* Plans the vote of n images with windows of at most cap rows on ctas
+ * persistent CTAs; slabs: there is memory for them. */
+static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int ctas,
+                     bool slabs, vote_plan *pl)
+{
+    const int slices = h->Tp / HL_SLICE;
+    std::vector<slice_ext> ext;
+    slice_extents(h, ext);
+    double total = 0.0;
+    pl->exact = 0;
+    pl->add = !slabs;
+    pl->part16 = 1;
+    for (int i = 0; i < n; i++) {
+        if (im[i].R >= (1 << 22))
+            pl->exact = 1;
+        for (int sl = 0; sl < slices; sl++)
+            total += (double)im[i].w * im[i].h +
+                     HL_ROW_PIXELS * std::min(region_rows(ext[sl], im[i].w, im[i].h), 4.0 * cap);
+    }
+    std::vector<plan_region> reg;
+    int wcap = cap;
+    double target = 0.0;
+    const bool small = n * slices < 2 * ctas && total / std::max(ctas, 1) < HL_SMALL_PIXELS;
+    if ((h->p.derho < 1.0 || small) &&
+        windows_win(h, im, n, ctas, ext, total, &wcap, &target))
+        plan_in_windows(h, im, n, wcap, target, ext, reg);
+    else
+        plan_regions(h, im, n, cap, ctas, ext, total, reg);
+    bool slides = false;
+    int win_rows = 0;
+    for (const plan_region &r : reg) {
+        slides |= !r.it.win && r.it.nseg > 1;
+        win_rows = std::max(win_rows, r.it.win ? r.it.adv : 0);
+    }
+    pl->win = win_rows > 0;
     /* slabs and merge blocks of the blocks with several items */
     std::vector<int> count((size_t)n * slices, 0), first((size_t)n * slices, 0);
     std::vector<int> at((size_t)n * slices, -1);   /* in pl->blocks */
+    std::vector<char> parts((size_t)n * slices, 0);
     for (const plan_region &r : reg)
-        count[(size_t)r.blk]++;
+        parts[(size_t)r.blk] |= r.it.nparts > 1;
+    for (const plan_region &r : reg)   /* whole windows are final */
+        if (!r.it.win || parts[(size_t)r.blk])
+            count[(size_t)r.blk]++;
     pl->blocks.clear();
     int nslab = 0;
     for (int b = 0; b < n * slices; b++)
@@ -821,6 +1065,8 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
         }
     pl->slabs.assign((size_t)nslab, hl_slab{});
     for (const plan_region &r : reg) {
+        if (r.it.win && !parts[(size_t)r.blk])
+            continue;
         const int w = im[r.it.img].w, hh = im[r.it.img].h;
         pl->part16 &= hl_part16_ok(h->p.derho, std::min((r.it.tx >> 16) * HL_TILE_W, w),
                                    std::min((r.it.ty >> 16) * HL_TILE_H, hh));
@@ -832,7 +1078,7 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
         max_scratch += 8LL * im[i].R * h->Tp;
     /* slabs are numbered in 31 bits */
     max_scratch = std::min(std::max(max_scratch, HL_MAX_SCRATCH), 64LL * 0x7fffffff);
-    double most = 8.0;
+    double most = std::max(8, win_rows);
     const double irho = 1.0 / h->p.derho;
     for (size_t i = 0; i < reg.size(); i++) {
         hl_vote_item it = reg[i].it;
@@ -841,12 +1087,16 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
         const int y1 = std::min(((it.ty & 0xffff) + (it.ty >> 16)) * HL_TILE_H, hh);
         const double rows = region_rows(ext[it.slice], x1 - (it.tx & 0xffff) * HL_TILE_W,
                                         y1 - (it.ty & 0xffff) * HL_TILE_H);
-        most = std::max(most, std::min(rows, (double)cap));
+        if (!it.win)
+            most = std::max(most, std::min(rows, (double)cap));
         const size_t b = (size_t)reg[i].blk;
         it.slab = -1;
         if (count[b] > 1) {
             hl_slab sl = {};
-            slab_groups(h, im[it.img], it, x1, y1, &sl);
+            if (it.win)
+                window_groups(h, im[it.img], it, &sl);
+            else
+                slab_groups(h, im[it.img], it, x1, y1, &sl);
             long long units = 0;
             for (int g = 0; g < 4; g++) {
                 sl.o[g] = (int)units;
@@ -927,6 +1177,7 @@ static void plan_args(const vote_plan &p, const unsigned char *d_plan, unsigned 
     ma->slabs = reinterpret_cast<const hl_slab *>(d_plan);
     va->items = reinterpret_cast<const hl_vote_item *>(d_plan + o);
     va->nitems = (int)p.items.size();
+    va->win = p.win;
     va->win_rows = p.win_rows;
     va->exact = p.exact;
     va->part16 = p.part16;

@@ -95,17 +95,23 @@ typedef struct hl_vote_img {
 
 /* One work item of the vote: a rectangle of an image's compaction tiles (a
  * region) voted for one theta slice.  Every theta's window of rows starts at
- * the lowest rho the rectangle reaches, so `rows` of them hold every vote.
- * win > 0 or clip: a rectangle of one tile whose range needs several windows
- * (rho steps far below a pixel); votes outside the window are dropped. */
+ * the lowest rho the rectangle reaches, so `rows` of them hold every vote. */
 typedef struct hl_vote_item {
     int img, slice;
     int tx, ty;               /* first tile | tiles << 16 */
     int slab;                 /* its slab's first row group in scratch; -1: the
-                                 block's only item (or hl_vote_args.add) */
+                                 block's only item, or a whole window, or
+                                 hl_vote_args.add */
     int gb[4], gn[4], go[4];  /* the slab's column groups: see hl_slab */
-    int win, clip;
-    /* nseg > 1: a whole image whose range does not fit one window, voted in
+    /* win: a whole image's votes of one window of adv rows; column k's row 0 is
+     * floor(rho of the centre at theta_k) + off0.  Tiles that may reach the window
+     * are voted (hl_band_window: lo, hi, tang), every vote's row is tested.  The
+     * windows of a block hold all its rows, so each is final unless its points are
+     * shared out to nparts items (this one is part `part`).  nseg: groups of
+     * HL_VOTE_RUNS / 2 tile rows */
+    int win, part, nparts;
+    float lo, hi, tang;
+    /* else nseg > 1: a whole image whose range does not fit one window, voted in
      * nseg segments with the window sliding by adv rows after each: segment j
      * holds the tiles whose centre lies, at the slice's middle theta, [j adv,
      * (j + 1) adv) above -half from the image's centre; column k's row 0 is
@@ -154,6 +160,7 @@ typedef struct hl_vote_args {
      * monotonically increasing counter */
     const hl_vote_item *items;
     int nitems;
+    int win;                  /* some of them are of one window each */
     unsigned *work;           /* counter */
     unsigned work_base;       /* its value at launch */
     unsigned char *scratch;   /* slabs: row groups */

@@ -35,6 +35,10 @@
  * vote them straight from shared memory and arrive on the slot's empty barrier,
  * which the producer waits on before refilling it.  The producer moves on to
  * the next item as soon as the current one is issued.
+ * Where regions would get small (rho steps below 1) or a merge is not worth its
+ * launch, a block is voted in windows instead: an item takes the tiles that may
+ * reach its rows (hl_band.h), tests every vote's row against them, and its rows are
+ * final; a window heavier than a CTA's share is voted in parts of its points.
  * When an item is voted the consumers read it and clear what they read.  The
  * only item of its block is final: when peaks are wanted, its bins above the
  * threshold go to the accumulator, which is zero otherwise (the peak rule needs
@@ -63,8 +67,8 @@
  *
  * Bounds: every voted point lies in the item's rectangle (or band), whose rows
  * the window holds; the list's sentinel (+infinity pads an odd tile) and stale
- * ring data vote 0 at the place of a real point; items whose window may be too
- * small test every row.  A launch whose compaction reported an error votes
+ * ring data vote 0 at the place of a real point; a window's votes are tested one by
+ * one.  A launch whose compaction reported an error votes
  * nothing.
  * After the start there is no block-wide barrier, and every mbarrier wait is
  * bounded: a time-out sets a status bit that the host reads with the result
@@ -148,8 +152,9 @@ struct VoteSeg {
     int total;                         /* points of its stream */
     int rho_min, R, thr;               /* the image's */
     int slab;                          /* see hl_vote_item */
+    int win;                           /* an item of one window: see hl_vote_item */
     int last, adv;                     /* the item's last segment; rows to slide */
-    int rows;                          /* rows its votes can reach */
+    int rows;                          /* rows its votes can reach; of a window */
     float margin;                      /* one rho bin in pixels */
     float c[HL_SLICE], s[HL_SLICE];    /* cos / sin of the slice's thetas */
     int base[HL_SLICE];                /* rho of each column's row 0 */
@@ -164,9 +169,19 @@ struct VoteTab {
     unsigned key[8];
 };
 
-/* 32 points from pts on, 8 a round, 8 votes of each a lane. */
-template <bool UNIT, int CV>
-__device__ __forceinline__ void vote_rounds(const float2 *pts, const VoteTab &t, f2x ir)
+/* the vote at relative shared address rel, if it lies below lim */
+__device__ __forceinline__ void red_below(unsigned rel, unsigned lim, unsigned acc_base)
+{
+    asm volatile("{ .reg .pred p; setp.lt.u32 p, %0, %1; @p red.shared.add.u32 [%2], 1; }"
+                 ::"r"(rel), "r"(lim), "r"(rel + acc_base)
+                 : "memory");
+}
+
+/* 32 points from pts on, 8 a round, 8 votes of each a lane.  WIN: the table's keys
+ * are relative to the window, and only votes below lim, its bytes, count. */
+template <bool UNIT, int CV, bool WIN>
+__device__ __forceinline__ void vote_rounds(const float2 *pts, const VoteTab &t, f2x ir,
+                                            unsigned lim, unsigned acc_base)
 {
     pts += threadIdx.x & 7;
 #pragma unroll
@@ -177,14 +192,19 @@ __device__ __forceinline__ void vote_rounds(const float2 *pts, const VoteTab &t,
         for (int i = 0; i < 4; i++) {
             unsigned r0, r1;
             diag_bits<UNIT, CV>(X, Y, t.c[i], t.s[i], ir, r0, r1);
-            red_smem(128u * r0 + t.key[2 * i]);
-            red_smem(128u * r1 + t.key[2 * i + 1]);
+            if (WIN) {
+                red_below(128u * r0 + t.key[2 * i], lim, acc_base);
+                red_below(128u * r1 + t.key[2 * i + 1], lim, acc_base);
+            } else {
+                red_smem(128u * r0 + t.key[2 * i]);
+                red_smem(128u * r1 + t.key[2 * i + 1]);
+            }
         }
     }
 }
 
-/* Points that a clipped item's window may not hold, or whose |rho| may reach
- * 2^22: point by point, a lane a theta, by the conversion instruction, every
+/* Points whose |rho| may reach 2^22 (or that a window promised to hold and does
+ * not): point by point, a lane a theta, by the conversion instruction, every
  * row tested. */
 template <bool UNIT>
 __device__ __noinline__ void vote_clipped(const float2 *pts, unsigned real, const VoteSeg &g,
@@ -201,41 +221,14 @@ __device__ __noinline__ void vote_clipped(const float2 *pts, unsigned real, cons
     }
 }
 
-/* A warp's block of a slot: 32 places, n of them filled.  They are looked at
- * once, a lane a place: the ones with no point (past the end, or the list's
- * sentinel) are filled with one of the block's points, whose surplus votes the
- * warp takes off again, so that no vote needs a test; and which blocks lie on
- * one side of rho 0 over the whole slice (a sinusoid has at most one zero in
- * it, so its ends tell, with a bin to spare).  Blocks on one side vote by floor
- * or by ceil, the others by the sign of each vote.  Conflict-free red.shared
- * alone take 1.13 cycles a warp-vote an SM; the floor 1.5, truncation by sign
- * 2.15 (micro-benchmark, 31 warps). */
-template <bool UNIT>
-__device__ __forceinline__ void vote_block(float2 *pts, int n, int mode, const VoteTab &t,
-                                           f2x ir, const VoteSeg &g, int rows, int *acc,
-                                           float irho)
+/* Floor, ceil or truncation by sign for a warp's points: which blocks lie on one
+ * side of rho 0 over the whole slice (a sinusoid has at most one zero in it, so its
+ * ends tell, with a bin to spare) is looked at once. */
+template <bool UNIT, bool WIN>
+__device__ __forceinline__ void vote_cv(const float2 *pts, float2 q, bool there, int mode,
+                                        const VoteTab &t, f2x ir, const VoteSeg &g, unsigned lim,
+                                        unsigned acc_base)
 {
-    const int lane = threadIdx.x & 31;
-    const float2 q = pts[lane];
-    const bool there = lane < n && q.x < 1.0e29f;
-    const unsigned real = __ballot_sync(FULL, there);
-    if (mode == CV_EXACT) {   /* a clipped item, or the exact conversion */
-        vote_clipped<UNIT>(pts, real, g, rows, acc, irho);
-        return;
-    }
-    if (real != FULL) {
-        if (!real)
-            return;
-        const float2 f = pts[__ffs(real) - 1];
-        if (!there) {
-            pts[lane] = f;
-            /* the slot is refilled by the async proxy */
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        }
-        const int row = rho_of<UNIT>(f.x, f.y, g.c[lane], g.s[lane], irho) - g.base[lane];
-        atomicSub(acc + row * HL_SLICE + lane, 32 - __popc(real));
-        __syncwarp();
-    }
     int cv = mode;
     if (mode == CV_SIGN) {
         const float v0 = q.x * g.c[0] + q.y * g.s[0];
@@ -246,11 +239,54 @@ __device__ __forceinline__ void vote_block(float2 *pts, int n, int mode, const V
             cv = CV_CEIL;
     }
     if (cv == CV_FLOOR)
-        vote_rounds<UNIT, CV_FLOOR>(pts, t, ir);
+        vote_rounds<UNIT, CV_FLOOR, WIN>(pts, t, ir, lim, acc_base);
     else if (cv == CV_CEIL)
-        vote_rounds<UNIT, CV_CEIL>(pts, t, ir);
+        vote_rounds<UNIT, CV_CEIL, WIN>(pts, t, ir, lim, acc_base);
     else
-        vote_rounds<UNIT, CV_SIGN>(pts, t, ir);
+        vote_rounds<UNIT, CV_SIGN, WIN>(pts, t, ir, lim, acc_base);
+}
+
+/* A warp's block of a slot: 32 places, n of them filled.  They are looked at
+ * once, a lane a place: the ones with no point (past the end, or the list's
+ * sentinel) are filled with one of the block's points, whose surplus votes the
+ * warp takes off again, so that no vote needs a test -- in a window item, where
+ * every vote is tested, with the sentinel.  Conflict-free red.shared alone take
+ * 1.13 cycles a warp-vote an SM; the floor 1.5, truncation by sign 2.15
+ * (micro-benchmark, 31 warps). */
+template <bool UNIT, bool WIN>
+__device__ __forceinline__ void vote_block(float2 *pts, int n, int mode, const VoteTab &t,
+                                           f2x ir, const VoteSeg &g, int *acc, unsigned acc_base,
+                                           float irho)
+{
+    const int lane = threadIdx.x & 31;
+    const bool win = WIN && g.win;
+    const float2 q = pts[lane];
+    const bool there = lane < n && q.x < 1.0e29f;
+    const unsigned real = __ballot_sync(FULL, there);
+    if (!real)
+        return;
+    if (mode == CV_EXACT) {
+        vote_clipped<UNIT>(pts, real, g, g.rows, acc, irho);
+        return;
+    }
+    if (real != FULL) {
+        const float2 f = win ? make_float2(__int_as_float(0x7f800000), 0.0f)
+                               : pts[__ffs(real) - 1];
+        if (!there) {
+            pts[lane] = f;
+            /* the slot is refilled by the async proxy */
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        if (!win) {
+            const int row = rho_of<UNIT>(f.x, f.y, g.c[lane], g.s[lane], irho) - g.base[lane];
+            atomicSub(acc + row * HL_SLICE + lane, 32 - __popc(real));
+        }
+        __syncwarp();
+    }
+    if (win)
+        vote_cv<UNIT, true>(pts, q, there, mode, t, ir, g, 128u * (unsigned)g.rows, acc_base);
+    else
+        vote_cv<UNIT, false>(pts, q, there, mode, t, ir, g, 0u, acc_base);
 }
 
 /* Bounded wait that also gives up as soon as another warp of the CTA has
@@ -324,6 +360,7 @@ __device__ __forceinline__ bool cons_sync(VoteSmem &sm, unsigned &par,
  * points into the ring.  It runs ahead of the consumers by up to the ring's
  * depth, so the next item's setup and first copies overlap the current item's
  * last votes. */
+template <bool WIN>
 __device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &sm)
 {
     const int lane = threadIdx.x & 31;
@@ -347,6 +384,7 @@ __device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &s
             if (a.imgs)
                 im = a.imgs[it.img];
         }
+        const bool win = WIN && it.win;
         const int tx0 = it.tx & 0xffff, txn = it.tx >> 16;
         const int ty0 = it.ty & 0xffff, tyn = it.ty >> 16;
         /* the columns past T vote like the last theta: their counts are
@@ -365,18 +403,21 @@ __device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &s
             lo = fminf(lo, v);
             hi = fmaxf(hi, v);
         }
-        const bool slide = it.nseg > 1;
+        const bool slide = it.nseg > 1 && !win;
         const float ctx = 0.5f * (float)(im.w - 1), cty = 0.5f * (float)(im.h - 1);
-        int base = slide ? __float2int_rd(rho_f<false>(ctx, cty, cl, sl, a.irho)) + it.off0
-                         : __float2int_rz(lo) + it.win * a.win_rows;
+        int base = slide || win
+                       ? __float2int_rd(rho_f<false>(ctx, cty, cl, sl, a.irho)) + it.off0
+                       : __float2int_rz(lo);
         int top = __float2int_rz(hi);
-        if (have && !slide && !it.clip && __any_sync(FULL, top - base >= a.win_rows)) {
+        bool clip = false;
+        if (have && !slide && !win && __any_sync(FULL, top - base >= a.win_rows)) {
             if (lane == 0)   /* the plan promised more rows than there are */
                 atomicOr(a.status, HL_ST_RHO_OUT_OF_RANGE);
-            it.clip = 1;
+            clip = true;
         }
+        const int wrows = win ? min(it.adv, a.win_rows) : a.win_rows;
         if (!slide)
-            top = min(top, base + a.win_rows - 1);
+            top = min(top, base + wrows - 1);
         int mode = a.exact ? CV_EXACT
                            : (!__any_sync(FULL, lo < 0.0f)
                                   ? CV_FLOOR
@@ -384,66 +425,82 @@ __device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &s
         const bool mixed = mode == CV_SIGN;
         /* sliding: the middle theta's normal in rho units a tile */
         const int km = min(it.slice * HL_SLICE + HL_SLICE / 2, a.T - 1);
-        const float sm_ = slide ? a.sinv[km] * a.irho : 0.0f;
-        float cm = slide ? a.cosv[km] * a.irho : 0.0f;
-        cm = copysignf(fmaxf(fabsf(cm), 1.0e-9f), cm);
+        const float sm_ = slide ? a.sinv[km] * a.irho : win ? a.sinv[km] : 0.0f;
+        float cm = slide ? a.cosv[km] * a.irho : win ? a.cosv[km] : 0.0f;
+        if (!win)
+            cm = copysignf(fmaxf(fabsf(cm), 1.0e-9f), cm);
         const float icm = 1.0f / (cm * HL_TILE_W);
         const float x0 = __fmul_rn(ctx - HL_TILE_W / 2, 1.0f / HL_TILE_W);
-        const bool wide = txn == im.tiles_x && !slide;
+        const bool wide = txn == im.tiles_x && !slide && !win;
         const int nsegs = have ? max(it.nseg, 1) : 1;
 
-        for (int sj = 0; sj < nsegs && ok; sj++, base += it.adv) {
-        const int rows = __reduce_max_sync(FULL, max(min(top, base + a.win_rows - 1) - base + 1, 0));
-        if (it.clip)
+        for (int sj = 0; sj < nsegs && ok; sj++, base += slide ? it.adv : 0) {
+        const int rows = __reduce_max_sync(FULL, max(min(top, base + wrows - 1) - base + 1, 0));
+        if (clip)
             mode = CV_EXACT;   /* every row tested */
+        if (win && mixed)   /* rho 0 truncates from both sides */
+            mode = !__any_sync(FULL, base < 1)
+                       ? CV_FLOOR
+                       : (!__any_sync(FULL, base + rows > 0) ? CV_CEIL : CV_SIGN);
         if (slide && mixed)   /* by the segment's own rows */
             mode = !__any_sync(FULL, base < 0)
                        ? CV_FLOOR
                        : (!__any_sync(FULL, base + a.win_rows > 0) ? CV_CEIL : CV_SIGN);
-        /* the runs, four per lane: one a tile row, or one for a rectangle as
-         * wide as the image */
-        const int nruns = have && !skip ? (wide ? 1 : min(tyn, HL_VOTE_RUNS)) : 0;
-        int st[4], ln[4], sum = 0;
+        /* the runs, lane and every 32nd after it: one a tile row, or one for a
+         * rectangle as wide as the image; a window's item two a tile row.  Few
+         * runs are one round: a lane's are looked up one after the other */
+        const int nruns = !have || skip ? 0
+                          : wide        ? 1
+                          : win      ? 2 * min(tyn - sj * (HL_VOTE_RUNS / 2), HL_VOTE_RUNS / 2)
+                                        : min(tyn, HL_VOTE_RUNS);
+        int st[HL_VOTE_RUNS / 32], en[HL_VOTE_RUNS / 32];
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int r = 4 * lane + q;
-            st[q] = ln[q] = 0;
-            if (r < nruns) {
+        for (int q = 0; q < HL_VOTE_RUNS / 32; q++) {
+            st[q] = en[q] = 0;
+            if (32 * q < nruns) {
+                const int r = 32 * q + lane;
                 int ta = 0, tb = txn;   /* the run's tiles, from tx0 */
-                if (slide) {
-                    const float yk = __fmul_rn(
-                        (float)((ty0 + r) * HL_TILE_H + HL_TILE_H / 2) - cty, sm_);
-                    hl_band_tiles(sj, nsegs, it.adv, it.half, yk, cm, icm, x0, txn, &ta, &tb);
-                }
-                if (tb > ta) {
-                    const int t0 = (ty0 + r) * im.tiles_x + tx0;
+                const int ty = ty0 + (win ? sj * (HL_VOTE_RUNS / 2) + r / 2 : r);
+                const float y = (float)(ty * HL_TILE_H + HL_TILE_H / 2) - cty;
+                if (win)
+                    hl_band_window(r & 1, it.lo, it.hi, it.tang, cm, sm_, HL_TILE_W / 2 - ctx, y,
+                                   txn, &ta, &tb);
+                if (slide)
+                    hl_band_tiles(sj, nsegs, it.adv, it.half, __fmul_rn(y, sm_), cm, icm, x0, txn,
+                                  &ta, &tb);
+                if (r < nruns && tb > ta) {
+                    const int t0 = ty * im.tiles_x + tx0;
                     st[q] = im.tile_off[t0 + ta];
-                    ln[q] = im.tile_off[wide ? (ty0 + tyn) * im.tiles_x : t0 + tb] - st[q];
+                    en[q] = im.tile_off[wide ? (ty0 + tyn) * im.tiles_x : t0 + tb];
                 }
             }
-            sum += ln[q];
         }
-        int incl = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t1 = __shfl_up_sync(FULL, incl, o);
-            if (lane >= o)
-                incl += t1;
-        }
-        const int total = __shfl_sync(FULL, incl, 31);
-        int pos = incl - sum;
         __syncwarp();   /* the previous segment's runs are no longer read */
+        int all = 0;
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int r = 4 * lane + q;
-            if (r < nruns) {
-                sm.run_s[r] = st[q];
-                sm.rpre[r] = pos;
-                pos += ln[q];
-                if (r == nruns - 1)
-                    sm.rpre[nruns] = pos;
+        for (int q = 0; q < HL_VOTE_RUNS / 32; q++)
+            if (32 * q < nruns) {
+                const int r = 32 * q + lane;
+                int incl = en[q] - st[q];
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t1 = __shfl_up_sync(FULL, incl, o);
+                    if (lane >= o)
+                        incl += t1;
+                }
+                if (r < nruns) {
+                    sm.run_s[r] = st[q];
+                    sm.rpre[r] = all + incl - (en[q] - st[q]);
+                    if (r == nruns - 1)
+                        sm.rpre[nruns] = all + incl;
+                }
+                all += __shfl_sync(FULL, incl, 31);
             }
-        }
+        /* a part of them, from and to even places */
+        const int np = WIN ? max(it.nparts, 1) : 1, part = WIN ? it.part : 0;
+        const int from = (int)((long long)all * part / np) & ~1;
+        const int to = part + 1 < np ? (int)((long long)all * (part + 1) / np) & ~1 : all;
+        const int total = to - from;
 
         /* publish the segment once the consumers are done with the one that
          * last used its slot */
@@ -475,6 +532,8 @@ __device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &s
                 g.gn[q] = it.gn[q];
                 g.go[q] = it.go[q];
             }
+            if (WIN)
+                g.win = win;
             g.last = sj == nsegs - 1;
             g.adv = it.adv;
             g.rows = rows;
@@ -484,7 +543,7 @@ __device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &s
             mbar_arrive(&sm.seg_full[ds]);
         nseg++;
 
-        /* batch b is stream range [b * SLOT_CAP, ...): lane i copies the part
+        /* batch b is stream range [from + b * SLOT_CAP, ...): lane i copies the part
          * of run r0 + i overlapping it; a ballot finds the first run of the
          * next batch */
         const int nb = (total + SLOT_CAP - 1) / SLOT_CAP;
@@ -497,8 +556,8 @@ __device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &s
                 ok = false;
                 break;
             }
-            const int s0 = b * SLOT_CAP;
-            const int e0 = min(total, s0 + SLOT_CAP);
+            const int s0 = from + b * SLOT_CAP;
+            const int e0 = min(to, s0 + SLOT_CAP);
             if (lane == 0)
                 mbar_expect_tx(&sm.full[slot], (unsigned)(e0 - s0) * 8u);
             __syncwarp();
@@ -538,7 +597,9 @@ __device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &s
     }
 }
 
-template <bool UNIT>
+/* WIN: some of the items are of one window each.  Their selection and tests cost the
+ * others registers: 256 uneven images 1042 us in the one form for both, 1021 apart. */
+template <bool UNIT, bool WIN>
 __global__ void __launch_bounds__(1024, 1)
 hl_vote_kernel(hl_vote_args a)
 {
@@ -573,7 +634,7 @@ hl_vote_kernel(hl_vote_args a)
      * consumers meet on mbarriers, every wait bounded */
     __syncthreads();
     if (warp == 0) {
-        vote_producer(a, sm);
+        vote_producer<WIN>(a, sm);
         return;
     }
 
@@ -600,9 +661,10 @@ hl_vote_kernel(hl_vote_args a)
                     const int c0 = 8 * j + ((p + i) & 7), c1 = 8 * j + ((p + i + 1) & 7);
                     tab.c[i / 2] = f2_pack(g.c[c0], g.c[c1]);
                     tab.s[i / 2] = f2_pack(g.s[c0], g.s[c1]);
-                    tab.key[i] = acc_base + 4u * (unsigned)c0 -
+                    const unsigned at = WIN && g.win ? 0u : acc_base;
+                    tab.key[i] = at + 4u * (unsigned)c0 -
                                  128u * (unsigned)(RHO_MAGIC_BITS + g.base[c0]);
-                    tab.key[i + 1] = acc_base + 4u * (unsigned)c1 -
+                    tab.key[i + 1] = at + 4u * (unsigned)c1 -
                                      128u * (unsigned)(RHO_MAGIC_BITS + g.base[c1]);
                 }
             }
@@ -616,8 +678,8 @@ hl_vote_kernel(hl_vote_args a)
                 seq++;
                 const int n = min(SLOT_CAP, total - b * SLOT_CAP);
                 for (; i < n; i += 32 * ncons)
-                    vote_block<UNIT>(sm.raw[slot] + i, n - i, mode, tab, ir, g, a.win_rows,
-                                     s_acc, a.irho);
+                    vote_block<UNIT, WIN>(sm.raw[slot] + i, n - i, mode, tab, ir, g, s_acc, acc_base,
+                                     a.irho);
                 i -= n;
                 __syncwarp();
                 if (lane == 0)
@@ -625,6 +687,12 @@ hl_vote_kernel(hl_vote_args a)
             }
         }
 
+        if (WIN && g.win && !g.last) {   /* more rows of tiles for the same window */
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(&sm.seg_empty[ds]);
+            continue;
+        }
         /* the item is voted: store it and clear what is read, lane = column */
         if (!cons_sync(sm, cpar, a.status))
             return;
@@ -876,7 +944,9 @@ cudaError_t hl_launch_vote(const hl_vote_args *a, int threads, int grid,
                            cudaStream_t s)
 {
     const size_t smem = hl_vote_smem_bytes(a->win_rows);
-    const auto kernel = a->irho == 1.0f ? hl_vote_kernel<true> : hl_vote_kernel<false>;
+    const bool unit = a->irho == 1.0f;
+    const auto kernel = a->win ? (unit ? hl_vote_kernel<true, true> : hl_vote_kernel<false, true>)
+                               : (unit ? hl_vote_kernel<true, false> : hl_vote_kernel<false, false>);
     const cudaError_t e = cudaFuncSetAttribute(
         kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess)
