@@ -336,9 +336,12 @@ static inline cudaError_t hl_launch_pdl(void (*kernel)(Params...), dim3 grid, di
 #endif
 /* HoughCircle (hl_circle_bits.cu, hl_circle.cu) */
 /* Radii up to this are counted on bit planes (nine of them, three words left and
- * right), larger ones vote point by point.  1024 x 1024, the whole call: radii 5 to
- * 50, 1% edge pixels 94 against 135 us by points, 5% 94 against 317, 0.05% 94
- * against 94; 60 to 89, 1% 144 against 206, 0.05% 144 against 107. */
+ * right), larger ones vote point by point.  1024 x 1024, the whole call against the
+ * same by points, threshold 100 or twice the radius: radii 5 to 50, 5% edge pixels 97
+ * against 320 us, 1% 87 against 135, 0.05% 38 against 99; 60 to 89, 1% 147 against
+ * 209, 0.05% 37 against 111.  Slower where few edge pixels meet a low threshold or the
+ * whole accumulator is asked for: 60 to 89, 0.05%, threshold 30 135 against 111, the
+ * accumulator 184 against 150. */
 #define HL_CIRCLE_DENSE_R 89
 /* One image's edge map and its tiles.  A call's only image has bases 0. */
 typedef struct hl_circle_bits_img {
