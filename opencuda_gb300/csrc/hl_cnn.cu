@@ -1175,16 +1175,15 @@ struct HeadTrig {
 
 static const HeadTrig &head_trig()
 {
-    static HeadTrig t;
-    static bool init = false;
-    if (!init) {
+    static const HeadTrig t = [] {   /* once, whichever thread comes first */
+        HeadTrig v;
         for (int i = 0; i < HL_HEAD_T; i++) {
             const double th = ((double)i + 0.5) * 3.14159265358979323846 / HL_HEAD_T;
-            t.c[i] = (float)cos(th);
-            t.s[i] = (float)sin(th);
+            v.c[i] = (float)cos(th);
+            v.s[i] = (float)sin(th);
         }
-        init = true;
-    }
+        return v;
+    }();
     return t;
 }
 
