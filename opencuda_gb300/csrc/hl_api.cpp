@@ -450,10 +450,10 @@ extern "C" int hl_last_launch_count(const hl_handle *h)
  * form.  At rho steps from 1 on only launches of less than HL_SMALL_PIXELS and two
  * blocks a CTA are looked at: in others regions win.
  * T = 180, a call by fixed windows of rows, which this replaced / by regions alone /
- * now: 16 images of 1000 x 900, step 0.1 229 / 1368 / 193 us, 0.05 380 / 2088 / 287,
- * 0.25 149 / 217 / 139; one of 2048 x 2048, 0.1 95 / 362 / 113, 0.05 142 / 467 / 122;
- * 512 x 512, 0.1 45 / 171 / 48; 16 of 512 x 512, step 1 58 / 66 / 58. */
-#define HL_WINDOW_VOTE 2.0
+ * now: 16 images of 1000 x 900, step 0.1 229 / 1368 / 174 us, 0.05 380 / 2088 / 260,
+ * 0.25 149 / 217 / 126; one of 2048 x 2048, 0.1 94 / 362 / 102, 0.05 141 / 467 / 108;
+ * 512 x 512, 0.1 45 / 171 / 45; 16 of 512 x 512, step 1 58 / 66 / 58. */
+#define HL_WINDOW_VOTE 1.7
 #define HL_ITEM_PIXELS 120e3
 #define HL_SLAB_PIXELS 100.0
 #define HL_MERGE_PIXELS 60e3
