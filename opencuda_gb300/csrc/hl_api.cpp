@@ -656,13 +656,20 @@ static void slab_rows(hl_slab *sl, int g, double r0, double r1, int R4)
     }
 }
 
+/* 1 - cos(half the span) of the eight columns from k0 on */
+static double slab_bend(const hl_handle *h, int k0)
+{
+    const int k1 = std::min(k0 + 7, h->T - 1);
+    return 1.0 - cos(std::min(0.5 * (k1 - std::min(k0, k1)) * h->p.detheta, M_PI));
+}
+
 /* The rows that the votes of an item's four column groups can fall into, in
  * groups of four rows (sl's b, n, lo and hi).  A corner's rho is a sinusoid over
  * the group's thetas: no lower than at its ends less the distance times 1 -
- * cos(half the span), and as much higher; a row and 2^-20 of the value more for
+ * cos(half the span) (bend, of the slice's groups), and as much higher; a row and 2^-20 of the value more for
  * the vote rule's floats. */
 static void slab_groups(const hl_handle *h, const plan_img &im, const hl_vote_item &it, int x1,
-                        int y1, hl_slab *sl)
+                        int y1, const double *bend, hl_slab *sl)
 {
     const double irho = 1.0 / h->p.derho;
     const int R4 = (im.R + 3) / 4;
@@ -683,8 +690,7 @@ static void slab_groups(const hl_handle *h, const plan_img &im, const hl_vote_it
             lo = std::min(lo, v);
             hi = std::max(hi, v);
         }
-        const double half = std::min(0.5 * (k1 - k0) * h->p.detheta, M_PI);
-        const double slack = far * (1.0 - cos(half)) + far * (1.0 / (1 << 20)) + 1.0;
+        const double slack = far * bend[g] + far * (1.0 / (1 << 20)) + 1.0;
         slab_rows(sl, g, floor(lo - slack) - im.rho_min, ceil(hi + slack) - im.rho_min, R4);
     }
 }
@@ -1006,6 +1012,8 @@ static bool windows_win(const hl_handle *h, const plan_img *im, int n, int ctas,
             }
         }
         worse = better || c == top ? 0 : worse + 1;
+        if (n * slices >= 2 * ctas)
+            break;   /* items enough: smaller windows only repeat votes */
     }
     return win;
 }
@@ -1079,7 +1087,9 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
     /* slabs are numbered in 31 bits */
     max_scratch = std::min(std::max(max_scratch, HL_MAX_SCRATCH), 64LL * 0x7fffffff);
     double most = std::max(8, win_rows);
-    const double irho = 1.0 / h->p.derho;
+    std::vector<double> bend((size_t)slices * 4);
+    for (size_t g = 0; g < bend.size(); g++)
+        bend[g] = slab_bend(h, (int)g * 8);
     for (size_t i = 0; i < reg.size(); i++) {
         hl_vote_item it = reg[i].it;
         const int w = im[it.img].w, hh = im[it.img].h;
@@ -1096,7 +1106,7 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
             if (it.win)
                 window_groups(h, im[it.img], it, &sl);
             else
-                slab_groups(h, im[it.img], it, x1, y1, &sl);
+                slab_groups(h, im[it.img], it, x1, y1, &bend[(size_t)it.slice * 4], &sl);
             long long units = 0;
             for (int g = 0; g < 4; g++) {
                 sl.o[g] = (int)units;
@@ -2523,6 +2533,8 @@ static int batch_run_ws(hl_handle *h, hl_batch_ws **pb, const hl_image_desc *img
         gk.push_back(K);
         gk.push_back(h->p.thresdis);
         gk.push_back((long long)ang);
+        gk.push_back(b->plan.add);
+        gk.push_back((long long)b->plan.items.size());
         if (!b->gexec || gk != b->gkey) {
             if (b->gexec) {
                 cudaGraphExecDestroy(b->gexec);

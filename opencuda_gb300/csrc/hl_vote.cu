@@ -926,7 +926,9 @@ hl_merge_kernel(hl_merge_args a)
                     dst[(size_t)(4 * rg + u) * a.Tp + e] = v[e][u];
                     bits |= 1u << (2 * u + e);
                 }
-    bool full = false;
+    /* every warp comes here once: without a look first, the counter of a full list
+     * would grow with the accumulators */
+    bool full = __any_sync(FULL, bits != 0) && *(volatile int *)a.cand.count > a.cand.cap;
     note_warp(a.cand, blk.img, bits, full, [&](int b) {
         return (unsigned)(4 * rg + (b >> 1)) * (unsigned)a.T + (unsigned)(k + (b & 1));
     });
