@@ -771,8 +771,9 @@ static inline size_t small_smem(int R)
 int hl_small_fits(int T, int Tp, int R)
 {
     const int C = Tp / HL_SLICE;
+    /* a CTA's 227 KB hold the kernel's few static words too */
     return T > 0 && C >= 1 && C <= HL_SMALL_MAX_CTAS && R > 0 &&
-           small_smem(R) <= 227u * 1024u;
+           small_smem(R) + 64 <= 227u * 1024u;
 }
 
 /* Edge masks of this thread's four 16-pixel chunks c, c + SMALL_THREADS, ...
