@@ -467,10 +467,10 @@ struct vote_plan {
     unsigned chunks;           /* of a merge launch */
     int part16, win_rows, exact, win;
     /* the blocks' items add to the accumulator instead of going through slabs:
-     * where these would take more than HL_MAX_SCRATCH and twice the accumulators (images
-     * of 32 K and more a side, or a handful of angles: a slab's column groups are
-     * as tall as their thetas lie apart), or could not be allocated.  Dense: the accumulator is cleared
-     * before and scanned after */
+     * where these would take more than HL_MAX_SCRATCH and twice the accumulators
+     * (images of 32 K and more a side, or a handful of angles: a slab's column groups
+     * are as tall as their thetas lie apart), or could not be allocated.  Dense: the
+     * accumulator is cleared before and scanned after */
     int add;
 };
 #define HL_MAX_SCRATCH (1LL << 30)
@@ -666,8 +666,8 @@ static double slab_bend(const hl_handle *h, int k0)
 /* The rows that the votes of an item's four column groups can fall into, in
  * groups of four rows (sl's b, n, lo and hi).  A corner's rho is a sinusoid over
  * the group's thetas: no lower than at its ends less the distance times 1 -
- * cos(half the span) (bend, of the slice's groups), and as much higher; a row and 2^-20 of the value more for
- * the vote rule's floats. */
+ * cos(half the span) (bend, of the slice's groups), and as much higher; a row and
+ * 2^-20 of the value more for the vote rule's floats. */
 static void slab_groups(const hl_handle *h, const plan_img &im, const hl_vote_item &it, int x1,
                         int y1, const double *bend, hl_slab *sl)
 {
@@ -992,8 +992,8 @@ static bool windows_win(const hl_handle *h, const plan_img *im, int n, int ctas,
                                                     (double)im[i].h * im[i].h) *
                                          std::min(7.0 * h->p.detheta, 1.0) / h->p.derho;
                     int rows = 0;
-                    const int nw = whole > c ? band_windows(band[(size_t)(i * slices + sl)], c, &rows)
-                                             : 1;
+                    const int nw =
+                        whole > c ? band_windows(band[(size_t)(i * slices + sl)], c, &rows) : 1;
                     const size_t before = part.size();
                     for (int j = 0; j < nw; j++, at++) {
                         const int np = rows ? window_parts(wt[at], f * share) : 1;

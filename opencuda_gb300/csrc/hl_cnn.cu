@@ -643,7 +643,6 @@ hl_conv1_kernel(hl_conv_args a)
             make_uint4(v[0] | ((unsigned)v[1] << 16), v[2] | ((unsigned)v[3] << 16),
                        v[4] | ((unsigned)v[5] << 16), v[6] | ((unsigned)v[7] << 16));
         *reinterpret_cast<uint4 *>(row + 128) = make_uint4(v[8], 0u, 0u, 0u);
-        asm volatile("cp.async.wait_all;" ::: "memory");   /* the weights */
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         if (__syncthreads_or(failed))
             break;
@@ -676,7 +675,6 @@ hl_conv1_kernel(hl_conv_args a)
         cnn_mbar_wait(&sm.bar, phase ^ 1u);   /* as in hl_conv32_kernel */
     if (GRAD)
         conv_add_db(a, db, reinterpret_cast<float *>(sm.out));
-    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     if (tid < 32)
         tmem_dealloc(tmem, 32);

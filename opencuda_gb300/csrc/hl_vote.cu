@@ -61,15 +61,14 @@
  * SM's cycles against the 1.13 of the shared-memory atomics alone, and the
  * items' edges (first copies, store, barriers) about a quarter of the time.
  * 4096 x 4096, T = 720: 92 us (fixed rho windows 118 us), with the slab merge 109
- * (128).  256 images of 256..2048 a side, T = 360: 854 us (1267).  2048 points a slot: 1024 make every warp
- * wait on a barrier for every block it votes (4096 x 4096 158 against 153 us,
- * the batch 1364 against 1318).
+ * (128).  256 images of 256..2048 a side, T = 360: 854 us (1267).  2048 points a
+ * slot: 1024 make every warp wait on a barrier for every block it votes (4096 x 4096
+ * 158 against 153 us, the batch 1364 against 1318).
  *
  * Bounds: every voted point lies in the item's rectangle (or band), whose rows
  * the window holds; the list's sentinel (+infinity pads an odd tile) and stale
- * ring data vote 0 at the place of a real point; a window's votes are tested one by
- * one.  A launch whose compaction reported an error votes
- * nothing.
+ * ring data vote 0 at the place of a real point; a window's votes are clamped to it
+ * one by one.  A launch whose compaction reported an error votes nothing.
  * After the start there is no block-wide barrier, and every mbarrier wait is
  * bounded: a time-out sets a status bit that the host reads with the result
  * and an abort flag on which every other waiting warp gives up too; the
@@ -679,8 +678,8 @@ hl_vote_kernel(hl_vote_args a)
                 seq++;
                 const int n = min(SLOT_CAP, total - b * SLOT_CAP);
                 for (; i < n; i += 32 * ncons)
-                    vote_block<UNIT, WIN>(sm.raw[slot] + i, n - i, mode, tab, ir, g, s_acc, acc_base,
-                                     a.irho);
+                    vote_block<UNIT, WIN>(sm.raw[slot] + i, n - i, mode, tab, ir, g, s_acc,
+                                          acc_base, a.irho);
                 i -= n;
                 __syncwarp();
                 if (lane == 0)
@@ -737,7 +736,8 @@ hl_vote_kernel(hl_vote_args a)
                         const int x[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                         for (int e = 0; e < 4; e++)
-                            if (x[e] > thr && g.k0 + c + e < a.T && (unsigned)row(e) < (unsigned)g.R) {
+                            if (x[e] > thr && g.k0 + c + e < a.T &&
+                                (unsigned)row(e) < (unsigned)g.R) {
                                 g.acc[(size_t)row(e) * a.Tp + g.k0 + c + e] = x[e];
                                 bits |= 1u << e;
                             }
