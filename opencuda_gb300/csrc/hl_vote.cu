@@ -777,13 +777,15 @@ hl_vote_kernel(hl_vote_args a)
             const int gb = g.gb[grp], gn = g.gn[grp];
             const int most = max(max(g.gn[0], g.gn[1]), max(g.gn[2], g.gn[3]));
             const size_t at = ((size_t)g.slab + g.go[grp]) * 8 + cc;
+            const int rows = g.rows;   /* that votes can reach */
             for (int q = cw; q < most; q += ncons) {
                 int v[4];
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
+                    /* not the row of a window's other votes: it is cleared meanwhile */
                     const unsigned i = (unsigned)(4 * (gb + q) + u - rb);
                     v[u] = 0;
-                    if (q < gn && i < (unsigned)a.win_rows) {
+                    if (q < gn && i < (unsigned)rows) {
                         v[u] = col[i * HL_SLICE];
                         col[i * HL_SLICE] = 0;
                     }
