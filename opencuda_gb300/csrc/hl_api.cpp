@@ -1022,7 +1022,7 @@ static bool windows_win(const hl_handle *h, const plan_img *im, int n, int ctas,
  * persistent CTAs; slabs: there is memory for them. */
 static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int ctas,
                      bool slabs, vote_plan *pl)
-{
+try {
     const int slices = h->Tp / HL_SLICE;
     std::vector<slice_ext> ext;
     slice_extents(h, ext);
@@ -1139,6 +1139,8 @@ static int make_plan(const hl_handle *h, const plan_img *im, int n, int cap, int
         pl->chunks = std::max(pl->chunks, (unsigned)(mb.hi - mb.lo + 15) / 16);
     pl->win_rows = slides ? cap : std::min(cap, ((int)most + 7) / 8 * 8);
     return HL_NO_ERROR;
+} catch (const std::bad_alloc &) {   /* many windows of a very fine step */
+    return HL_OUT_OF_MEM;
 }
 
 /* rows a window may have: the override (at least what one tile needs at a
