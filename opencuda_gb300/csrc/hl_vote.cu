@@ -476,26 +476,30 @@ __device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &s
             }
         }
         __syncwarp();   /* the previous segment's runs are no longer read */
-        int all = 0;
+        /* laid end to end a lane's after the other's: the order is free */
+        const int rounds = (nruns + 31) / 32, nslots = 32 * rounds;
+        int sum = 0;
 #pragma unroll
         for (int q = 0; q < HL_VOTE_RUNS / 32; q++)
-            if (32 * q < nruns) {
-                const int r = 32 * q + lane;
-                int incl = en[q] - st[q];
+            sum += en[q] - st[q];
+        int incl = sum;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t1 = __shfl_up_sync(FULL, incl, o);
-                    if (lane >= o)
-                        incl += t1;
-                }
-                if (r < nruns) {
-                    sm.run_s[r] = st[q];
-                    sm.rpre[r] = all + incl - (en[q] - st[q]);
-                    if (r == nruns - 1)
-                        sm.rpre[nruns] = all + incl;
-                }
-                all += __shfl_sync(FULL, incl, 31);
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t1 = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o)
+                incl += t1;
+        }
+        const int all = __shfl_sync(FULL, incl, 31);
+        int pos = incl - sum;
+#pragma unroll
+        for (int q = 0; q < HL_VOTE_RUNS / 32; q++)
+            if (q < rounds) {
+                sm.run_s[rounds * lane + q] = st[q];
+                sm.rpre[rounds * lane + q] = pos;
+                pos += en[q] - st[q];
             }
+        if (lane == 31)
+            sm.rpre[nslots] = all;
         /* a part of them, from and to even places */
         const int np = WIN ? max(it.nparts, 1) : 1, part = WIN ? it.part : 0;
         const int from = (int)((long long)all * part / np) & ~1;
@@ -564,11 +568,11 @@ __device__ __forceinline__ void vote_producer(const hl_vote_args &a, VoteSmem &s
             /* runs from r0 on: every run ending at or before e0 lies wholly in
              * this batch; the first one reaching past e0 is shared with the
              * next batch and ends the scan */
-            int nextr = nruns;
-            for (int rb = r0; rb < nruns; rb += 32) {
+            int nextr = nslots;
+            for (int rb = r0; rb < nslots; rb += 32) {
                 const int r = rb + lane;
                 bool past = false;
-                if (r < nruns) {
+                if (r < nslots) {
                     const int rs = sm.rpre[r], re = sm.rpre[r + 1];
                     const int ps = max(s0, rs), pe = min(e0, re);
                     if (pe > ps)
